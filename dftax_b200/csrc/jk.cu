@@ -87,13 +87,37 @@ __global__ void __launch_bounds__(kGtThreads) gamma_partial_kernel(
   }
 }
 
-__global__ void reduce_rows_kernel(const double* __restrict__ part, int64_t nparts, int64_t ldb,
-                                   double* __restrict__ out) {
-  const int64_t c = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  if (c >= ldb) return;
+// out[c] = sum_p part[p][c], bound by the latency of its dependent adds: one
+// thread per column left them serial (592 partials: 61-81 us at every size, on
+// 1-15 blocks). A block takes 32 columns; thread (y, x) sums the partials y,
+// y + 32, ... of column x (a warp reads 256 contiguous bytes), and 32 sums are
+// added in a fixed order: 3-5 us, reproducible.
+constexpr int kRrCols = 32, kRrLanes = 32;
+__global__ void __launch_bounds__(kRrCols * kRrLanes) reduce_rows_kernel(
+    const double* __restrict__ part, int64_t nparts, int64_t ldb, double* __restrict__ out) {
+  __shared__ double red[kRrLanes][kRrCols + 1];
+  const int x = threadIdx.x % kRrCols, y = threadIdx.x / kRrCols;
+  const int64_t c = blockIdx.x * (int64_t)kRrCols + x;
   double s = 0.0;
-  for (int64_t p = 0; p < nparts; ++p) s += part[p * ldb + c];
-  out[c] = s;
+  if (c < ldb) {
+#pragma unroll 4
+    for (int64_t p = y; p < nparts; p += kRrLanes) s += part[p * ldb + c];
+  }
+  red[y][x] = s;
+  __syncthreads();
+  // warp y adds the lanes of column y by a shuffle tree (a fixed order)
+  double t = red[x][y];
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+  const int64_t cc = blockIdx.x * (int64_t)kRrCols + y;
+  if (x == 0 && cc < ldb) out[cc] = t;
+}
+
+static void launch_reduce_rows(const double* part, int64_t nparts, int64_t ldb, double* out,
+                               cudaStream_t s) {
+  reduce_rows_kernel<<<(unsigned)((ldb + kRrCols - 1) / kRrCols), kRrCols * kRrLanes, 0, s>>>(
+      part, nparts, ldb, out);
+  DFJK_LAUNCHED();
 }
 
 // J rows: one warp per row, J[m, n] and J[n, m]
@@ -163,9 +187,7 @@ static void gamma_rows(Plan& p, const double* Bc, int64_t nrows, const double* d
   gamma_partial_kernel<<<dim3((unsigned)xparts, (unsigned)ycols), kGtThreads, 0, s>>>(
       Bc, p.ldb, nrows, dvec, rows_per, part.as<double>());
   DFJK_LAUNCHED();
-  reduce_rows_kernel<<<(unsigned)((p.ldb + 255) / 256), 256, 0, s>>>(part.as<double>(), xparts,
-                                                                     p.ldb, add ? sum : out);
-  DFJK_LAUNCHED();
+  launch_reduce_rows(part.as<double>(), xparts, p.ldb, add ? sum : out, s);
   if (add) {
     add_to_kernel<<<(unsigned)((p.ldb + 255) / 256), 256, 0, s>>>(sum, p.ldb, out);
     DFJK_LAUNCHED();
@@ -193,9 +215,7 @@ static void gamma_from_dvec(Plan& p, const double* dvec, double* gamma, cudaStre
     gamma_partial_kernel<<<dim3((unsigned)xparts, (unsigned)ycols), kGtThreads, 0, s>>>(
         p.d_B.as<double>(), p.ldb, p.nrows, dvec, rows_per, part.as<double>());
     DFJK_LAUNCHED();
-    reduce_rows_kernel<<<(unsigned)((p.ldb + 255) / 256), 256, 0, s>>>(part.as<double>(), xparts,
-                                                                       p.ldb, gamma);
-    DFJK_LAUNCHED();
+    launch_reduce_rows(part.as<double>(), xparts, p.ldb, gamma, s);
   } else {
     DFJK_CUDA(cudaMemsetAsync(gamma, 0, p.ldb * sizeof(double), s));
   }
