@@ -247,12 +247,29 @@ static void j_from_gamma(Plan& p, const double* gamma, double* J, cudaStream_t s
 // K: half transform X[m][x][i] = sum_{(r, n) in list(m)} B[r][x0 + x] C'[n][i]
 // ---------------------------------------------------------------------------
 
-// Block tile 64 (x) x 80 (i), 16 list entries per k chunk, on the float64
-// tensor cores (mma.sync m8n8k4 f64: tcgen05 has no float64 kind). Eight
-// warps as 4 (x, 16 rows) x 2 (i, 40 columns); a warp holds 2 x 5 fragments
-// of 8 x 8. Shared rows are padded to 68 / 84 doubles so that the fragment
-// loads (k = lane % 4, row = lane / 4) fall in distinct banks.
-constexpr int kHtX = 64, kHtI = 80, kHtK = 16, kHtPX = 68, kHtPI = 84;
+// On the float64 tensor cores (mma.sync m8n8k4 f64: tcgen05 has no float64
+// kind). A block of eight warps computes 64 directions x HtTile::I columns of
+// one m, 16 list entries per k chunk, through a four-stage cp.async ring of
+// 16-byte copies with one barrier per chunk. Bound by the DMMA pipe once nocc
+// is above ~20 columns: the tile's width follows the columns (half_tile), since
+// columns of padding cost as much as real ones.
+//   * Warps: WI of them side by side over the columns, 8 / WI over the
+//     directions; a warp holds XF x IF fragments of 8 x 8.
+//   * The order of rows and columns inside a fragment is free, so neighbouring
+//     fragments interleave: a lane's elements of a pair of fragments are
+//     adjacent and come with one 16-byte load. Rows of 64 + 4 and I + 4 doubles
+//     put the 8 lanes of a load phase (4 k, 2 rows) in distinct banks.
+// (H2O)_12 (nocc 60): 1353 us with 80-column tiles, 8-byte copies and two
+// stages; see half_tile for the widths.
+constexpr int kHtX = 64, kHtK = 16, kHtPX = kHtX + 4, kHtStages = 4;
+
+template <int IF_, int WI_>
+struct HtTile {
+  static constexpr int IF = IF_, WI = WI_, WX = 8 / WI, XF = kHtX / (8 * WX);
+  static constexpr int I = 8 * IF * WI, PI = I + 4;
+  static constexpr int kStage = kHtK * (kHtPX + PI);   // doubles
+  static constexpr size_t smem = (size_t)kHtStages * kStage * sizeof(double);
+};
 
 __device__ __forceinline__ void dmma_8x8x4(double (&c)[2], double a, double b) {
   asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};"
@@ -260,90 +277,190 @@ __device__ __forceinline__ void dmma_8x8x4(double (&c)[2], double a, double b) {
                : "d"(a), "d"(b));
 }
 
-__device__ __forceinline__ void cp_async8(void* smem, const void* gmem, bool valid) {
-  // src-size 0 fills the 8 shared bytes with zeros (gmem must still be a valid address)
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"(
+__device__ __forceinline__ void cp_async16(void* smem, const void* gmem, bool valid) {
+  // src-size 0 fills the 16 shared bytes with zeros (gmem must still be a valid address)
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(
                    static_cast<unsigned>(__cvta_generic_to_shared(smem))),
-               "l"(gmem), "r"(valid ? 8 : 0)
+               "l"(gmem), "r"(valid ? 16 : 0)
                : "memory");
 }
 
 // The list of m is entries [kbeg[m], kend[m]) (kend == nullptr: up to
 // kbeg[m + 1]); entry e reads B row krow[e] - row0. accumulate: X += instead
-// of X = (a streamed plan sums the chunks of B rows).
-__global__ void __launch_bounds__(256) half_transform_kernel(
+// of X = (a streamed plan sums the chunks of B rows). ldb and ncol are even,
+// B and Cp 16-byte aligned and x0 a multiple of 64, so every copy and store is
+// aligned.
+template <class T>
+__global__ void __launch_bounds__(256, 2) half_transform_kernel(
     const double* __restrict__ B, int64_t ldb, int64_t x0, int64_t xc, const double* __restrict__ Cp,
     int64_t ncol, const int* __restrict__ kbeg, const int* __restrict__ kend,
     const int* __restrict__ krow, const int* __restrict__ kn, int64_t row0, int accumulate,
     double* __restrict__ X) {
-  // two buffers: chunk c + 1 is copied (cp.async) while chunk c is multiplied
-  __shared__ double Bs[2][kHtK][kHtPX];
-  __shared__ double Cs[2][kHtK][kHtPI];
+  constexpr int XF = T::XF, IF = T::IF, PI = T::PI;
+  constexpr int kCg = kHtK * T::I / 2, kCper = (kCg + 255) / 256;   // 16-byte copies of C' rows
+  extern __shared__ __align__(16) double ht_smem[];
   const int m = blockIdx.x;
   const int64_t xt = (int64_t)blockIdx.y * kHtX;   // within the chunk
-  const int64_t it = (int64_t)blockIdx.z * kHtI;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int wx = (warp & 3) * 16, wi = (warp >> 2) * 40;
+  const int64_t it = (int64_t)blockIdx.z * T::I;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int wx = (warp % T::WX) * 8 * XF, wi = (warp / T::WX) * 8 * IF;
   const int fr = lane >> 2, fk = lane & 3;   // fragment row / k of this lane
-  double acc[2][5][2];
+  double acc[XF][IF][2];
 #pragma unroll
-  for (int a = 0; a < 2; ++a)
+  for (int a = 0; a < XF; ++a)
 #pragma unroll
-    for (int b = 0; b < 5; ++b) acc[a][b][0] = acc[a][b][1] = 0.0;
+    for (int b = 0; b < IF; ++b) acc[a][b][0] = acc[a][b][1] = 0.0;
   const int e0 = kbeg[m], e1 = kend ? kend[m] : kbeg[m + 1];
-  // kHtK list entries: rows of B (x tile) and rows of C' (i tile)
-  auto stage = [&](int buf, int e) {
-    for (int q = threadIdx.x; q < kHtK * kHtX; q += 256) {
-      const int k = q / kHtX, x = q % kHtX;
-      const bool ok = e + k < e1 && xt + x < xc;
-      cp_async8(&Bs[buf][k][x], ok ? B + ((int64_t)krow[e + k] - row0) * ldb + x0 + xt + x : B, ok);
+  const int nch = (e1 - e0 + kHtK - 1) / kHtK;
+  // this thread's copies of a chunk: B rows tid / 32 and tid / 32 + 8 (one
+  // 16-byte piece of each), kCper pieces of C' rows. Their list entries are
+  // read one chunk ahead, so a copy never waits for its index.
+  const int bk = tid >> 5, bx = 2 * (tid & 31);
+  const bool bin = x0 + xt + bx < ldb;
+  int nr[2], nn[kCper];
+  auto fetch = [&](int c) {
+    const int e = e0 + c * kHtK;
+#pragma unroll
+    for (int j = 0; j < 2; ++j) nr[j] = e + bk + 8 * j < e1 ? krow[e + bk + 8 * j] : -1;
+#pragma unroll
+    for (int j = 0; j < kCper; ++j) {
+      const int k = (tid + 256 * j) / (T::I / 2);
+      nn[j] = k < kHtK && e + k < e1 ? kn[e + k] : -1;
     }
-    for (int q = threadIdx.x; q < kHtK * kHtI; q += 256) {
-      const int k = q / kHtI, i = q % kHtI;
-      const bool ok = e + k < e1 && it + i < ncol;
-      cp_async8(&Cs[buf][k][i], ok ? Cp + (int64_t)kn[e + k] * ncol + it + i : Cp, ok);
-    }
-    asm volatile("cp.async.commit_group;" ::: "memory");
   };
-  if (e0 < e1) stage(0, e0);
-  int buf = 0;
-  for (int e = e0; e < e1; e += kHtK, buf ^= 1) {
-    if (e + kHtK < e1) {
-      stage(buf ^ 1, e + kHtK);
-      asm volatile("cp.async.wait_group 1;" ::: "memory");
-    } else {
-      asm volatile("cp.async.wait_group 0;" ::: "memory");
+  auto stage = [&](int c) {
+    double* Bs = ht_smem + (c % kHtStages) * T::kStage;
+    double* Cs = Bs + kHtK * kHtPX;
+#pragma unroll
+    for (int j = 0; j < 2; ++j) {
+      const bool ok = nr[j] >= 0 && bin;
+      cp_async16(Bs + (bk + 8 * j) * kHtPX + bx,
+                 ok ? B + ((int64_t)nr[j] - row0) * ldb + x0 + xt + bx : B, ok);
     }
+#pragma unroll
+    for (int j = 0; j < kCper; ++j) {
+      const int q = tid + 256 * j, k = q / (T::I / 2), i = 2 * (q % (T::I / 2));
+      if (q >= kCg) break;
+      const bool ok = nn[j] >= 0 && it + i < ncol;
+      cp_async16(Cs + k * PI + i, ok ? Cp + (int64_t)nn[j] * ncol + it + i : Cp, ok);
+    }
+  };
+  auto commit = [] { asm volatile("cp.async.commit_group;" ::: "memory"); };
+  if (nch > 0) fetch(0);
+  for (int c = 0; c < kHtStages - 1; ++c) {
+    if (c < nch) {
+      stage(c);
+      if (c + 1 < nch) fetch(c + 1);
+    }
+    commit();
+  }
+  for (int c = 0; c < nch; ++c) {
+    // chunk c has landed, and every warp is done with the buffer of chunk c - 1
+    asm volatile("cp.async.wait_group %0;" ::"n"(kHtStages - 2) : "memory");
     __syncthreads();
+    if (c + kHtStages - 1 < nch) {
+      stage(c + kHtStages - 1);
+      if (c + kHtStages < nch) fetch(c + kHtStages);
+    }
+    commit();
+    const double* Bs = ht_smem + (c % kHtStages) * T::kStage;
+    const double* Cs = Bs + kHtK * kHtPX;
 #pragma unroll
     for (int kk = 0; kk < kHtK; kk += 4) {
-      double af[2], bf[5];
+      double af[XF], bf[IF];
+      if constexpr (XF == 2) {
+        const double2 v = *reinterpret_cast<const double2*>(Bs + (kk + fk) * kHtPX + wx + 2 * fr);
+        af[0] = v.x;
+        af[1] = v.y;
+      } else {
+        af[0] = Bs[(kk + fk) * kHtPX + wx + fr];
+      }
 #pragma unroll
-      for (int a = 0; a < 2; ++a) af[a] = Bs[buf][kk + fk][wx + 8 * a + fr];
+      for (int b = 0; b + 1 < IF; b += 2) {
+        const double2 v =
+            *reinterpret_cast<const double2*>(Cs + (kk + fk) * PI + wi + 8 * b + 2 * fr);
+        bf[b] = v.x;
+        bf[b + 1] = v.y;
+      }
+      if constexpr (IF % 2) bf[IF - 1] = Cs[(kk + fk) * PI + wi + 8 * (IF - 1) + fr];
 #pragma unroll
-      for (int b = 0; b < 5; ++b) bf[b] = Cs[buf][kk + fk][wi + 8 * b + fr];
+      for (int a = 0; a < XF; ++a)
 #pragma unroll
-      for (int a = 0; a < 2; ++a)
-#pragma unroll
-        for (int b = 0; b < 5; ++b) dmma_8x8x4(acc[a][b], af[a], bf[b]);
+        for (int b = 0; b < IF; ++b) dmma_8x8x4(acc[a][b], af[a], bf[b]);
     }
-    __syncthreads();
   }
-  // accumulator (a, b, r) holds x = wx + 8a + lane / 4, i = wi + 8b + 2 (lane % 4) + r
+  // fragment (a, b), register r of this lane: direction wx + XF (lane / 4) + a;
+  // column 8 b + 2 (2 (lane % 4) + r) + {0, 1} over a pair b, b + 1, and
+  // 8 b + 2 (lane % 4) + r in an unpaired last fragment
+  auto put = [&](double* o, double u, double v) {
+    if (accumulate) {
+      const double2 p = *reinterpret_cast<const double2*>(o);
+      u += p.x;
+      v += p.y;
+    }
+    *reinterpret_cast<double2*>(o) = make_double2(u, v);
+  };
 #pragma unroll
-  for (int a = 0; a < 2; ++a) {
-    const int64_t x = xt + wx + 8 * a + fr;
+  for (int a = 0; a < XF; ++a) {
+    const int64_t x = xt + wx + XF * fr + a;
     if (x >= xc) continue;
+    double* row = X + ((int64_t)m * xc + x) * ncol;
 #pragma unroll
-    for (int b = 0; b < 5; ++b)
+    for (int b = 0; b + 1 < IF; b += 2)
 #pragma unroll
       for (int r = 0; r < 2; ++r) {
-        const int64_t i = it + wi + 8 * b + 2 * fk + r;
-        if (i < ncol) {
-          double* o = X + ((int64_t)m * xc + x) * ncol + i;
-          *o = accumulate ? *o + acc[a][b][r] : acc[a][b][r];
-        }
+        const int64_t i = it + wi + 8 * b + 4 * fk + 2 * r;
+        if (i < ncol) put(row + i, acc[a][b][r], acc[a][b + 1][r]);
       }
+    if constexpr (IF % 2) {
+      const int64_t i = it + wi + 8 * (IF - 1) + 2 * fk;
+      if (i < ncol) put(row + i, acc[a][IF - 1][0], acc[a][IF - 1][1]);
+    }
+  }
+}
+
+template <class T>
+static void launch_half(const double* B, int64_t ldb, int64_t x0, int64_t xc, const double* Cp,
+                        int64_t ncol, const int* kbeg, const int* kend, const int* krow,
+                        const int* kn, int64_t row0, int accumulate, int64_t nao, double* X,
+                        cudaStream_t s) {
+  DFJK_CUDA(cudaFuncSetAttribute(half_transform_kernel<T>,
+                                 cudaFuncAttributeMaxDynamicSharedMemorySize, (int)T::smem));
+  const dim3 grid((unsigned)nao, (unsigned)((xc + kHtX - 1) / kHtX),
+                  (unsigned)((ncol + T::I - 1) / T::I));
+  half_transform_kernel<T><<<grid, 256, T::smem, s>>>(B, ldb, x0, xc, Cp, ncol, kbeg, kend, krow,
+                                                      kn, row0, accumulate, X);
+  DFJK_LAUNCHED();
+}
+
+// Column tile of the half transform: every tile streams the rows of B again
+// and pays a prologue and an epilogue, worth about 12 columns, so the width
+// with the smallest tiles x (width + 12) is taken (60 columns: one tile of 64,
+// 160: two of 80, 82: two of 48).
+static int half_tile(int64_t ncol) {
+  int best = 80;
+  int64_t cost = INT64_MAX;
+  for (int w : {80, 64, 48, 40, 32, 24, 16, 8}) {
+    const int64_t c = (ncol + w - 1) / w * (w + 12);
+    if (c < cost) {
+      cost = c;
+      best = w;
+    }
+  }
+  return best;
+}
+
+template <class... A>
+static void launch_half_any(int64_t ncol, A... a) {
+  switch (half_tile(ncol)) {
+    case 8: launch_half<HtTile<1, 1>>(a...); return;
+    case 16: launch_half<HtTile<2, 1>>(a...); return;
+    case 24: launch_half<HtTile<3, 1>>(a...); return;
+    case 32: launch_half<HtTile<4, 1>>(a...); return;
+    case 40: launch_half<HtTile<5, 1>>(a...); return;
+    case 48: launch_half<HtTile<3, 2>>(a...); return;
+    case 64: launch_half<HtTile<4, 2>>(a...); return;
+    default: launch_half<HtTile<5, 2>>(a...); return;
   }
 }
 
@@ -367,65 +484,93 @@ __global__ void list_bounds_kernel(const int* __restrict__ kptr, const int* __re
   ke[m] = lower(lo, hi, r1);
 }
 
-// K partials on the float64 tensor cores: for the lower-triangle tile pair
-// (tm >= tn, 64 x 64) of blockIdx.x and the k slice blockIdx.y,
+// K partials on the float64 tensor cores: for lower-triangle tile pair number
+// blockIdx.x (tm >= tn, 64 x 64) and the k slice blockIdx.y,
 // part[slice][tm*64 + r][tn*64 + c] = sum_k X[tm*64 + r][k] X[tn*64 + c][k]
-// over the slice (X row-major, nao x kt). Same fragment layout and cp.async
-// double buffering as the half transform; rows are staged k-major.
-constexpr int kSyT = 64, kSyK = 16, kSyP = 68;
+// over the slice (X row-major, nao x kt, kt even). Bound by the DMMA pipe.
+// Rows are staged as they lie, 16 k (eight 16-byte pieces, the piece index
+// xor 4 (row % 2)) per chunk through a four-stage cp.async ring with one barrier
+// per chunk; the k order inside a chunk is free, so a lane takes k pairs
+// 2 (lane % 4) and its two k steps come with one 16-byte load, whose phases of
+// two rows x four pieces fall in distinct banks. Tiles on the diagonal stage
+// their rows once, and warps whose part lies above the diagonal or past nao
+// skip their products.
+constexpr int kSyT = 64, kSyK = 16, kSyStages = 4;
+constexpr size_t kSySmem = (size_t)kSyStages * 2 * kSyT * kSyK * sizeof(double);
 
-__global__ void __launch_bounds__(256) syrk_part_kernel(const double* __restrict__ X, int64_t nao,
-                                                        int64_t kt, int64_t kslice,
-                                                        const int2* __restrict__ tiles,
-                                                        double* __restrict__ part) {
-  __shared__ double As[2][kSyK][kSyP];
-  __shared__ double Bs[2][kSyK][kSyP];
-  const int2 tp = tiles[blockIdx.x];
-  const int64_t r0 = (int64_t)tp.x * kSyT, c0 = (int64_t)tp.y * kSyT;
+__global__ void __launch_bounds__(256, 2) syrk_part_kernel(const double* __restrict__ X, int64_t nao,
+                                                           int64_t kt, int64_t kslice,
+                                                           double* __restrict__ part) {
+  extern __shared__ __align__(16) double sy_smem[];
+  int tm = (int)((sqrt(8.0 * blockIdx.x + 1.0) - 1.0) * 0.5);
+  while ((tm + 1) * (tm + 2) / 2 <= (int)blockIdx.x) ++tm;
+  while (tm * (tm + 1) / 2 > (int)blockIdx.x) --tm;
+  const int tn = (int)blockIdx.x - tm * (tm + 1) / 2;
+  const bool diag = tm == tn;
+  const int64_t r0 = (int64_t)tm * kSyT, c0 = (int64_t)tn * kSyT;
   const int64_t k0 = (int64_t)blockIdx.y * kslice;
   const int64_t k1 = k0 + kslice < kt ? k0 + kslice : kt;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int wr = (warp & 3) * 16, wc = (warp >> 2) * 32;
   const int fr = lane >> 2, fk = lane & 3;
+  const bool work = r0 + wr < nao && c0 + wc < nao && !(diag && wc > wr + 15);
   double acc[2][4][2];
 #pragma unroll
   for (int a = 0; a < 2; ++a)
 #pragma unroll
     for (int b = 0; b < 4; ++b) acc[a][b][0] = acc[a][b][1] = 0.0;
-  auto stage = [&](int buf, int64_t k) {
-    for (int q = threadIdx.x; q < kSyT * kSyK; q += 256) {
-      const int r = q / kSyK, kk = q % kSyK;
-      const bool ka = k + kk < k1;
-      const bool oa = ka && r0 + r < nao, ob = ka && c0 + r < nao;
-      cp_async8(&As[buf][kk][r], oa ? X + (r0 + r) * kt + k + kk : X, oa);
-      cp_async8(&Bs[buf][kk][r], ob ? X + (c0 + r) * kt + k + kk : X, ob);
+  const int nch = (int)((k1 - k0 + kSyK - 1) / kSyK);
+  // this thread's copies of a chunk: rows tid / 8 and tid / 8 + 32, piece tid % 8
+  const int sr = tid >> 3, sp = tid & 7;
+  auto stage = [&](int c) {
+    double* As = sy_smem + (size_t)(c % kSyStages) * (2 * kSyT * kSyK);
+    const int64_t k = k0 + (int64_t)c * kSyK + 2 * sp;
+#pragma unroll
+    for (int j = 0; j < 2; ++j) {
+      const int r = sr + 32 * j, o = r * kSyK + 2 * (sp ^ (4 * (r & 1)));
+      const bool oa = k < k1 && r0 + r < nao;
+      cp_async16(As + o, oa ? X + (r0 + r) * kt + k : X, oa);
+      if (!diag) {
+        const bool ob = k < k1 && c0 + r < nao;
+        cp_async16(As + kSyT * kSyK + o, ob ? X + (c0 + r) * kt + k : X, ob);
+      }
     }
-    asm volatile("cp.async.commit_group;" ::: "memory");
   };
-  if (k0 < k1) stage(0, k0);
-  int buf = 0;
-  for (int64_t k = k0; k < k1; k += kSyK, buf ^= 1) {
-    if (k + kSyK < k1) {
-      stage(buf ^ 1, k + kSyK);
-      asm volatile("cp.async.wait_group 1;" ::: "memory");
-    } else {
-      asm volatile("cp.async.wait_group 0;" ::: "memory");
-    }
+  auto commit = [] { asm volatile("cp.async.commit_group;" ::: "memory"); };
+  for (int c = 0; c < kSyStages - 1; ++c) {
+    if (c < nch) stage(c);
+    commit();
+  }
+  for (int c = 0; c < nch; ++c) {
+    asm volatile("cp.async.wait_group %0;" ::"n"(kSyStages - 2) : "memory");
     __syncthreads();
+    if (c + kSyStages - 1 < nch) stage(c + kSyStages - 1);
+    commit();
+    if (!work) continue;
+    const double* As = sy_smem + (size_t)(c % kSyStages) * (2 * kSyT * kSyK);
+    const double* Bs = diag ? As : As + kSyT * kSyK;
 #pragma unroll
-    for (int kk = 0; kk < kSyK; kk += 4) {
-      double af[2], bf[4];
+    for (int h = 0; h < 2; ++h) {
+      // k pairs 8 h + 2 fk, + 1 of this lane (rows differ by 8: the same parity)
+      const int piece = 2 * ((4 * h + fk) ^ (4 * (fr & 1)));
+      double2 af[2], bf[4];
 #pragma unroll
-      for (int a = 0; a < 2; ++a) af[a] = As[buf][kk + fk][wr + 8 * a + fr];
+      for (int a = 0; a < 2; ++a)
+        af[a] = *reinterpret_cast<const double2*>(As + (wr + 8 * a + fr) * kSyK + piece);
 #pragma unroll
-      for (int b = 0; b < 4; ++b) bf[b] = Bs[buf][kk + fk][wc + 8 * b + fr];
+      for (int b = 0; b < 4; ++b)
+        bf[b] = *reinterpret_cast<const double2*>(Bs + (wc + 8 * b + fr) * kSyK + piece);
 #pragma unroll
       for (int a = 0; a < 2; ++a)
 #pragma unroll
-        for (int b = 0; b < 4; ++b) dmma_8x8x4(acc[a][b], af[a], bf[b]);
+        for (int b = 0; b < 4; ++b) dmma_8x8x4(acc[a][b], af[a].x, bf[b].x);
+#pragma unroll
+      for (int a = 0; a < 2; ++a)
+#pragma unroll
+        for (int b = 0; b < 4; ++b) dmma_8x8x4(acc[a][b], af[a].y, bf[b].y);
     }
-    __syncthreads();
   }
+  if (!work) return;
   double* out = part + (int64_t)blockIdx.y * nao * nao;
 #pragma unroll
   for (int a = 0; a < 2; ++a) {
@@ -453,49 +598,50 @@ __global__ void syrk_reduce_kernel(const double* __restrict__ part, int64_t nspl
   K[t] = beta0 ? sign * acc : K[t] + sign * acc;
 }
 
+// C'[m][j] = sqrt|w| C[m][sel[j]] for j < nsel (sel == nullptr: column j), zero
+// in the padding columns up to ncp
 __global__ void scale_cols_kernel(const double* __restrict__ C, const double* __restrict__ w,
                                   int64_t nao, int64_t ncol, const int* __restrict__ sel,
-                                  int64_t nsel, double* __restrict__ out) {
+                                  int64_t nsel, int64_t ncp, double* __restrict__ out) {
   const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  if (i >= nao * nsel) return;
-  const int64_t m = i / nsel, j = i % nsel;
-  const int col = sel[j];
-  const double f = w ? sqrt(fabs(w[col])) : 1.0;
-  out[i] = C[m * ncol + col] * f;
-}
-
-__global__ void symmetrize_kernel(double* __restrict__ K, int64_t n) {
-  // cuBLAS filled the column-major lower triangle = row-major upper (j >= i)
-  const int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  if (t >= n * n) return;
-  const int64_t i = t / n, j = t % n;
-  if (j < i) K[t] = K[j * n + i];
+  if (i >= nao * ncp) return;
+  const int64_t m = i / ncp, j = i % ncp;
+  double v = 0.0;
+  if (j < nsel) {
+    const int64_t col = sel ? sel[j] : j;
+    v = C[m * ncol + col] * (w ? sqrt(fabs(w[col])) : 1.0);
+  }
+  out[i] = v;
 }
 
 // K (+)= sign * X X^T (float64, full square) for X nao x kt row-major: lower
-// 64 x 64 tile pairs times k slices, enough blocks for several waves, then a
-// fixed-order sum of the slices (bit-reproducible).
+// 64 x 64 tile pairs times k slices, then a fixed-order sum of the slices
+// (bit-reproducible). Two blocks run per SM; the slice count is the one whose
+// waves x (slice length + 128: a block's prologue and partial stores in units
+// of k) is smallest. One slice per 1024 k left a single block at small sizes
+// ((H2O)_1: 46 us) and 1.4 waves at (H2O)_12 (719 us).
 static void syrk_fp64(Plan& p, const double* X, int64_t kt, double sign, bool beta0, double* K,
                       cudaStream_t s) {
   const int64_t nao = p.nao;
-  const int64_t nt = (nao + kSyT - 1) / kSyT;
-  std::vector<int2> tl;
-  for (int64_t a = 0; a < nt; ++a)
-    for (int64_t b = 0; b <= a; ++b) tl.push_back(make_int2((int)a, (int)b));
-  int sm = 148;
-  cudaDeviceGetAttribute(&sm, cudaDevAttrMultiProcessorCount, p.ctx->device);
-  const int64_t want = 4 * (int64_t)sm;
-  int64_t nsplit = std::max<int64_t>(1, (want + (int64_t)tl.size() - 1) / (int64_t)tl.size());
-  nsplit = std::min<int64_t>(nsplit, std::max<int64_t>(1, kt / 1024));
-  nsplit = std::min<int64_t>(nsplit, 65535);
+  const int64_t nt = (nao + kSyT - 1) / kSyT, tiles = nt * (nt + 1) / 2;
+  const int64_t slots = 2 * (int64_t)num_sms(p.ctx->device);
+  const int64_t most = std::min<int64_t>(64, std::max<int64_t>(1, kt / 64));
+  int64_t nsplit = 1;
+  int64_t best = INT64_MAX;
+  for (int64_t q = 1; q <= most; ++q) {
+    const int64_t t = (tiles * q + slots - 1) / slots * ((kt + q - 1) / q + 128);
+    if (t < best) {
+      best = t;
+      nsplit = q;
+    }
+  }
   const int64_t kslice = ((kt + nsplit - 1) / nsplit + kSyK - 1) / kSyK * kSyK;
   nsplit = (kt + kslice - 1) / kslice;
-  p.ws_syrk_tiles.ensure(tl.size() * sizeof(int2));
-  DFJK_CUDA(cudaMemcpyAsync(p.ws_syrk_tiles.p, tl.data(), tl.size() * sizeof(int2),
-                            cudaMemcpyHostToDevice, s));
   p.ws_syrk.ensure((size_t)nsplit * nao * nao * sizeof(double));
-  syrk_part_kernel<<<dim3((unsigned)tl.size(), (unsigned)nsplit), 256, 0, s>>>(
-      X, nao, kt, kslice, p.ws_syrk_tiles.as<int2>(), p.ws_syrk.as<double>());
+  DFJK_CUDA(cudaFuncSetAttribute(syrk_part_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 (int)kSySmem));
+  syrk_part_kernel<<<dim3((unsigned)tiles, (unsigned)nsplit), 256, kSySmem, s>>>(
+      X, nao, kt, kslice, p.ws_syrk.as<double>());
   DFJK_LAUNCHED();
   syrk_reduce_kernel<<<(unsigned)((nao * nao + 255) / 256), 256, 0, s>>>(
       p.ws_syrk.as<double>(), nsplit, nao, sign, beta0 ? 1 : 0, K);
@@ -511,22 +657,26 @@ struct GammaFuse {
   double* gamma = nullptr;
 };
 
+// nsel columns of C: those of `sel` (host indices), or the first nsel when null
 static void k_accumulate(Plan& p, const double* C, const double* w, int64_t ncol,
-                         const std::vector<int>& sel, double sign, bool first, double* K,
-                         cudaStream_t s, GammaFuse* fuse = nullptr) {
-  Context& c = *p.ctx;
-  const int64_t nao = p.nao, nsel = (int64_t)sel.size();
+                         const std::vector<int>* sel, int64_t nsel, double sign, bool first,
+                         double* K, cudaStream_t s, GammaFuse* fuse = nullptr) {
+  const int64_t nao = p.nao;
   if (nsel == 0) return;
   DevBuf& dsel = p.ws_sel;
   DevBuf& Cp = p.ws_Cp;
-  dsel.ensure(sel.size() * sizeof(int));
-  DFJK_CUDA(cudaMemcpyAsync(dsel.p, sel.data(), sel.size() * sizeof(int), cudaMemcpyHostToDevice, s));
-  Cp.ensure((size_t)nao * nsel * sizeof(double));
-  scale_cols_kernel<<<(unsigned)((nao * nsel + 255) / 256), 256, 0, s>>>(C, w, nao, ncol,
-                                                                         dsel.as<int>(), nsel,
-                                                                         Cp.as<double>());
+  if (sel) {
+    dsel.ensure(nsel * sizeof(int));
+    DFJK_CUDA(cudaMemcpyAsync(dsel.p, sel->data(), nsel * sizeof(int), cudaMemcpyHostToDevice, s));
+  }
+  // an even number of columns (a zero one added) keeps the rows of C' and X
+  // 16-byte aligned for the wide copies and the TMA stores of both forms
+  const int64_t ncp = nsel + (nsel & 1);
+  Cp.ensure((size_t)nao * ncp * sizeof(double));
+  scale_cols_kernel<<<(unsigned)((nao * ncp + 255) / 256), 256, 0, s>>>(
+      C, w, nao, ncol, sel ? dsel.as<int>() : nullptr, nsel, ncp, Cp.as<double>());
   DFJK_LAUNCHED();
-  // x chunking so that X (nao * xc * nsel doubles) stays within budget; a
+  // x chunking so that X (nao * xc * ncp doubles) stays within budget; a
   // streamed plan rebuilds B once per x chunk, so it takes up to half the
   // free device memory
   int64_t budget = (int64_t)6 << 30;
@@ -535,21 +685,19 @@ static void k_accumulate(Plan& p, const double* C, const double* w, int64_t ncol
     DFJK_CUDA(cudaMemGetInfo(&fr, &tot));
     budget = std::max<int64_t>(budget, (int64_t)(fr / 2));
   }
-  int64_t xc = budget / (nao * nsel * (int64_t)sizeof(double));
+  int64_t xc = budget / (nao * ncp * (int64_t)sizeof(double));
   xc = std::max<int64_t>(kHtX, xc / kHtX * kHtX);
   xc = std::min<int64_t>(xc, (p.nfit + kHtX - 1) / kHtX * kHtX);
   DevBuf& X = p.ws_X;
-  X.ensure((size_t)nao * xc * nsel * sizeof(double));
-  DFJK_CUBLAS(cublasSetStream(c.cublas, s));
+  X.ensure((size_t)nao * xc * ncp * sizeof(double));
   bool beta0 = first;
   for (int64_t x0 = 0; x0 < p.nfit; x0 += xc) {
     const int64_t n = std::min(xc, p.nfit - x0);
-    dim3 grid((unsigned)nao, (unsigned)((n + kHtX - 1) / kHtX), (unsigned)((nsel + kHtI - 1) / kHtI));
     p.timer.mark(kPhKhalf, s);
     const bool oz = p.opts.precision == DFJK_MIXED && !p.opts.streamed;
     if (p.opts.streamed) {
       // X = sum over chunks of B rows of the half transform of each chunk
-      DFJK_CUDA(cudaMemsetAsync(X.p, 0, (size_t)nao * n * nsel * sizeof(double), s));
+      DFJK_CUDA(cudaMemsetAsync(X.p, 0, (size_t)nao * n * ncp * sizeof(double), s));
       p.ws_kb.ensure(nao * sizeof(int));
       p.ws_ke.ensure(nao * sizeof(int));
       const bool with_gamma = fuse && fuse->dvec;
@@ -560,29 +708,27 @@ static void k_accumulate(Plan& p, const double* C, const double* w, int64_t ncol
             p.d_kptr.as<int>(), p.d_krow.as<int>(), nao, r0, r0 + nr, p.ws_kb.as<int>(),
             p.ws_ke.as<int>());
         DFJK_LAUNCHED();
-        half_transform_kernel<<<grid, 256, 0, s>>>(Bc, p.ldb, x0, n, Cp.as<double>(), nsel,
-                                                   p.ws_kb.as<int>(), p.ws_ke.as<int>(),
-                                                   p.d_krow.as<int>(), p.d_kn.as<int>(), r0, 1,
-                                                   X.as<double>());
-        DFJK_LAUNCHED();
+        launch_half_any(ncp, Bc, p.ldb, x0, n, (const double*)Cp.as<double>(), ncp,
+                        (const int*)p.ws_kb.as<int>(), (const int*)p.ws_ke.as<int>(),
+                        (const int*)p.d_krow.as<int>(), (const int*)p.d_kn.as<int>(), r0, 1, nao,
+                        X.as<double>(), s);
       });
       if (with_gamma) fuse->dvec = nullptr;   // gamma is complete
     } else if (oz) {
-      if (x0 == 0) ozaki_prepare_c(p, Cp.as<double>(), nsel, s);
-      ozaki_k1(p, nsel, x0, n, X.as<double>(), s);   // int8 tensor cores, exact accumulation
+      if (x0 == 0) ozaki_prepare_c(p, Cp.as<double>(), ncp, s);
+      ozaki_k1(p, ncp, x0, n, X.as<double>(), s);   // int8 tensor cores, exact accumulation
     } else {
-      half_transform_kernel<<<grid, 256, 0, s>>>(p.d_B.as<double>(), p.ldb, x0, n, Cp.as<double>(),
-                                                 nsel, p.d_kptr.as<int>(), nullptr,
-                                                 p.d_krow.as<int>(), p.d_kn.as<int>(), 0, 0,
-                                                 X.as<double>());
-      DFJK_LAUNCHED();
+      launch_half_any(ncp, (const double*)p.d_B.as<double>(), p.ldb, x0, n,
+                      (const double*)Cp.as<double>(), ncp, (const int*)p.d_kptr.as<int>(),
+                      (const int*)nullptr, (const int*)p.d_krow.as<int>(),
+                      (const int*)p.d_kn.as<int>(), (int64_t)0, 0, nao, X.as<double>(), s);
     }
     p.timer.mark(kPhKhalf, s);
     p.timer.mark(kPhKsyrk, s);
     if (oz) {
-      ozaki_syrk(p, X.as<double>(), n * nsel, sign, beta0, K, s);   // full square, int8 tensor cores
+      ozaki_syrk(p, X.as<double>(), n * ncp, sign, beta0, K, s);   // int8 tensor cores
     } else {
-      syrk_fp64(p, X.as<double>(), n * nsel, sign, beta0, K, s);
+      syrk_fp64(p, X.as<double>(), n * ncp, sign, beta0, K, s);
     }
     p.timer.mark(kPhKsyrk, s);
     beta0 = false;
@@ -591,8 +737,13 @@ static void k_accumulate(Plan& p, const double* C, const double* w, int64_t ncol
 
 static void k_compute(Plan& p, const double* C, const double* w, int64_t ncol, double* K,
                       cudaStream_t s, GammaFuse* fuse = nullptr) {
+  // every K path below leaves the full square, exactly symmetric
+  if (!w) {
+    k_accumulate(p, C, nullptr, ncol, nullptr, ncol, 1.0, true, K, s, fuse);
+    return;
+  }
   std::vector<int> pos, neg;
-  if (w) {
+  {
     std::vector<double> hw(ncol);
     DFJK_CUDA(cudaMemcpyAsync(hw.data(), w, ncol * sizeof(double), cudaMemcpyDeviceToHost, s));
     DFJK_CUDA(cudaStreamSynchronize(s));
@@ -601,18 +752,13 @@ static void k_compute(Plan& p, const double* C, const double* w, int64_t ncol, d
       if (hw[i] > 0) pos.push_back((int)i);
       else if (hw[i] < 0) neg.push_back((int)i);
     }
-  } else {
-    for (int64_t i = 0; i < ncol; ++i) pos.push_back((int)i);
   }
   if (pos.empty() && neg.empty()) {
     DFJK_CUDA(cudaMemsetAsync(K, 0, (size_t)p.nao * p.nao * sizeof(double), s));
     return;
   }
-  k_accumulate(p, C, w, ncol, pos, 1.0, true, K, s, fuse);
-  k_accumulate(p, C, w, ncol, neg, -1.0, pos.empty(), K, s, fuse);
-  const int64_t n = p.nao;
-  symmetrize_kernel<<<(unsigned)((n * n + 255) / 256), 256, 0, s>>>(K, n);
-  DFJK_LAUNCHED();
+  k_accumulate(p, C, w, ncol, &pos, (int64_t)pos.size(), 1.0, true, K, s, fuse);
+  k_accumulate(p, C, w, ncol, &neg, (int64_t)neg.size(), -1.0, pos.empty(), K, s, fuse);
 }
 
 void jk_compute(Plan& p, const double* C, const double* w, int64_t ncol, double* J, double* K,
