@@ -117,6 +117,8 @@ struct Plan {
   DevBuf ws_oz_x, ws_oz_ex, ws_oz_kp;
   // float64 K = X X^T: per-slice partials
   DevBuf ws_syrk;
+  // density path: total density, low-rank columns, scalars read back, block partials of the dots, K
+  DevBuf ws_Ptot, ws_lowrank, ws_scal, ws_dots, ws_K;
 };
 
 // ---- mixed precision on the int8 tensor cores (ozaki.cu) ----
@@ -168,6 +170,20 @@ void jk_compute(Plan& p, const double* C, const double* w, int64_t ncol, double*
                 cudaStream_t s);
 // gamma = B^T vec(Ptot) over the plan's rows (ldb doubles; the J intermediate)
 void gamma_from_density(Plan& p, const double* Ptot, double* gamma, cudaStream_t s);
+
+// ---- rank-revealing factor of a density (lowrank.cu) ----
+// pivots down to this share of the largest are taken (the eigensolver route
+// keeps eigenvalues down to the same share of the largest)
+constexpr double kLowRankTol = 1e-14;
+// the factor stands for P when no element of P - C C^T exceeds this share of
+// max |P|: the pivots left out plus the rounding of r-term sums
+constexpr double kLowRankAccept = 3e-14;
+bool low_rank_supported(int64_t n);   // its workspace fits in shared memory
+// per spin channel of P (nspin x n x n, symmetric): columns Ct[k][i] (k < rank,
+// n x n per channel), the rank, max |P - C C^T| and max |P| (bits of a double;
+// the caller zeroes them). Enqueued only.
+void launch_low_rank(const double* P, int64_t n, int nspin, double* Ct, int* rank,
+                     unsigned long long* worst, unsigned long long* scale, cudaStream_t s);
 
 // ---- nuclear gradient of the DF energy (grad.cu) ----
 // E and dE/dR at a fixed density P (nspin x nao x nao, device): per orbital

@@ -17,6 +17,7 @@
 
 #include <algorithm>
 #include <cmath>
+#include <cstring>
 
 namespace dfjk {
 
@@ -599,9 +600,9 @@ __global__ void syrk_reduce_kernel(const double* __restrict__ part, int64_t nspl
 }
 
 // C'[m][j] = sqrt|w| C[m][sel[j]] for j < nsel (sel == nullptr: column j), zero
-// in the padding columns up to ncp
+// in the padding columns up to ncp; C[m][j] lies at C[m * sm + j * sc]
 __global__ void scale_cols_kernel(const double* __restrict__ C, const double* __restrict__ w,
-                                  int64_t nao, int64_t ncol, const int* __restrict__ sel,
+                                  int64_t nao, int64_t sm, int64_t sc, const int* __restrict__ sel,
                                   int64_t nsel, int64_t ncp, double* __restrict__ out) {
   const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   if (i >= nao * ncp) return;
@@ -609,7 +610,7 @@ __global__ void scale_cols_kernel(const double* __restrict__ C, const double* __
   double v = 0.0;
   if (j < nsel) {
     const int64_t col = sel ? sel[j] : j;
-    v = C[m * ncol + col] * (w ? sqrt(fabs(w[col])) : 1.0);
+    v = C[m * sm + col * sc] * (w ? sqrt(fabs(w[col])) : 1.0);
   }
   out[i] = v;
 }
@@ -657,8 +658,9 @@ struct GammaFuse {
   double* gamma = nullptr;
 };
 
-// nsel columns of C: those of `sel` (host indices), or the first nsel when null
-static void k_accumulate(Plan& p, const double* C, const double* w, int64_t ncol,
+// nsel columns of C: those of `sel` (host indices), or the first nsel when
+// null; C[m][j] lies at C[m * sm + j * sc]
+static void k_accumulate(Plan& p, const double* C, int64_t sm, int64_t sc, const double* w,
                          const std::vector<int>* sel, int64_t nsel, double sign, bool first,
                          double* K, cudaStream_t s, GammaFuse* fuse = nullptr) {
   const int64_t nao = p.nao;
@@ -674,7 +676,7 @@ static void k_accumulate(Plan& p, const double* C, const double* w, int64_t ncol
   const int64_t ncp = nsel + (nsel & 1);
   Cp.ensure((size_t)nao * ncp * sizeof(double));
   scale_cols_kernel<<<(unsigned)((nao * ncp + 255) / 256), 256, 0, s>>>(
-      C, w, nao, ncol, sel ? dsel.as<int>() : nullptr, nsel, ncp, Cp.as<double>());
+      C, w, nao, sm, sc, sel ? dsel.as<int>() : nullptr, nsel, ncp, Cp.as<double>());
   DFJK_LAUNCHED();
   // x chunking so that X (nao * xc * ncp doubles) stays within budget; a
   // streamed plan rebuilds B once per x chunk, so it takes up to half the
@@ -739,7 +741,7 @@ static void k_compute(Plan& p, const double* C, const double* w, int64_t ncol, d
                       cudaStream_t s, GammaFuse* fuse = nullptr) {
   // every K path below leaves the full square, exactly symmetric
   if (!w) {
-    k_accumulate(p, C, nullptr, ncol, nullptr, ncol, 1.0, true, K, s, fuse);
+    k_accumulate(p, C, ncol, 1, nullptr, nullptr, ncol, 1.0, true, K, s, fuse);
     return;
   }
   std::vector<int> pos, neg;
@@ -757,8 +759,8 @@ static void k_compute(Plan& p, const double* C, const double* w, int64_t ncol, d
     DFJK_CUDA(cudaMemsetAsync(K, 0, (size_t)p.nao * p.nao * sizeof(double), s));
     return;
   }
-  k_accumulate(p, C, w, ncol, &pos, (int64_t)pos.size(), 1.0, true, K, s, fuse);
-  k_accumulate(p, C, w, ncol, &neg, (int64_t)neg.size(), -1.0, pos.empty(), K, s, fuse);
+  k_accumulate(p, C, ncol, 1, w, &pos, (int64_t)pos.size(), 1.0, true, K, s, fuse);
+  k_accumulate(p, C, ncol, 1, w, &neg, (int64_t)neg.size(), -1.0, pos.empty(), K, s, fuse);
 }
 
 void jk_compute(Plan& p, const double* C, const double* w, int64_t ncol, double* J, double* K,
@@ -803,34 +805,67 @@ __global__ void add_kernel(const double* __restrict__ a, const double* __restric
   if (i < n) out[i] = a[i] + b[i];
 }
 
-__global__ void dot_kernel(const double* __restrict__ a, const double* __restrict__ b, int64_t n,
-                           double* __restrict__ out) {
+// The dots of an energy: block partials (sum of a[i] b[i], and F += c a when F
+// is given), added by the last block to finish in block order, so the result
+// does not depend on the schedule. One block of 256 threads left the trace of
+// P K a chain of n^2 / 256 loads (14 us at n = 180, 45 us at n = 318).
+constexpr int kDotBlocks = 128;
+
+__global__ void __launch_bounds__(256) dot_axpy_kernel(const double* __restrict__ a,
+                                                       const double* __restrict__ b, double c,
+                                                       int64_t n, double* F, double* part,
+                                                       unsigned* count, double* __restrict__ out) {
   __shared__ double sh[256];
-  double s = 0.0;
-  for (int64_t i = threadIdx.x; i < n; i += blockDim.x) s += a[i] * b[i];
-  sh[threadIdx.x] = s;
-  __syncthreads();
-  for (int o = blockDim.x / 2; o > 0; o >>= 1) {
-    if ((int)threadIdx.x < o) sh[threadIdx.x] += sh[threadIdx.x + o];
+  __shared__ bool last;
+  auto block_sum = [&](double s) {
+    sh[threadIdx.x] = s;
     __syncthreads();
+    for (int o = 128; o > 0; o >>= 1) {
+      if ((int)threadIdx.x < o) sh[threadIdx.x] += sh[threadIdx.x + o];
+      __syncthreads();
+    }
+    return sh[0];
+  };
+  double s = 0.0;
+  for (int64_t i = blockIdx.x * (int64_t)256 + threadIdx.x; i < n; i += (int64_t)gridDim.x * 256) {
+    const double v = a[i];
+    s += v * b[i];
+    if (F) F[i] += c * v;
   }
-  if (threadIdx.x == 0) *out = sh[0];
+  s = block_sum(s);
+  if (threadIdx.x == 0) {
+    part[blockIdx.x] = s;
+    __threadfence();
+    last = atomicInc(count, gridDim.x - 1) == gridDim.x - 1;   // wraps to 0 for the next call
+  }
+  __syncthreads();
+  if (!last) return;
+  __threadfence();
+  s = block_sum(threadIdx.x < gridDim.x ? __ldcg(part + threadIdx.x) : 0.0);
+  if (threadIdx.x == 0) *out = s;
 }
 
-__global__ void axpy_kernel(const double* __restrict__ x, double a, int64_t n, double* __restrict__ y) {
+// what an energy reads back from the device (ws_scal)
+struct EnergyScalars {
+  double dot[5];                      // gamma . gamma, then Tr(P_s K) per spin and operator
+  unsigned long long worst[2], scale[2];
+  int rank[2];
+  int nonfinite;
+  unsigned count;                     // of dot_axpy_kernel
+};
+
+__global__ void nonfinite_kernel(const double* __restrict__ x, int64_t n, int* __restrict__ bad) {
   const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  if (i < n) y[i] += a * x[i];
+  if (i < n && !isfinite(x[i])) atomicExch(bad, 1);
 }
 
-static double dot(const double* a, const double* b, int64_t n, cudaStream_t s) {
-  DevBuf r;
-  r.alloc(sizeof(double));
-  dot_kernel<<<1, 256, 0, s>>>(a, b, n, r.as<double>());
+static void dot_axpy(Plan& p, const double* a, const double* b, double c, int64_t n, double* F,
+                     double* out, cudaStream_t s) {
+  p.ws_dots.ensure(kDotBlocks * sizeof(double));
+  const unsigned blocks = (unsigned)std::max<int64_t>(1, std::min<int64_t>(kDotBlocks, (n + 1023) / 1024));
+  dot_axpy_kernel<<<blocks, 256, 0, s>>>(a, b, c, n, F, p.ws_dots.as<double>(),
+                                         &p.ws_scal.as<EnergyScalars>()->count, out);
   DFJK_LAUNCHED();
-  double h = 0;
-  DFJK_CUDA(cudaMemcpyAsync(&h, r.p, sizeof(double), cudaMemcpyDeviceToHost, s));
-  DFJK_CUDA(cudaStreamSynchronize(s));
-  return h;
 }
 
 // K of a symmetric density Q (device, nao x nao): Q = V diag(l) V^T on the
@@ -878,8 +913,8 @@ static void density_factor(Plan& p, const double* Q, DevBuf& Ct, DevBuf& dw, cud
 // hf_lr: the long-range exchange of range-separated hybrids through the plan's
 // long-range fit (terms.py:604-612)
 void gamma_from_density(Plan& p, const double* Ptot, double* gamma, cudaStream_t s) {
-  DevBuf dvec;
-  dvec.alloc(std::max<int64_t>(p.nrows, 1) * sizeof(double));
+  DevBuf& dvec = p.ws_dvec;
+  dvec.ensure(std::max<int64_t>(p.nrows, 1) * sizeof(double));
   if (p.nrows > 0) {
     dvec_from_density_kernel<<<(unsigned)((p.nrows + 255) / 256), 256, 0, s>>>(
         Ptot, p.nao, p.d_row_m.as<int>(), p.d_row_n.as<int>(), p.d_row_w.as<int8_t>(), p.nrows,
@@ -889,58 +924,79 @@ void gamma_from_density(Plan& p, const double* Ptot, double* gamma, cudaStream_t
   gamma_from_dvec(p, dvec.as<double>(), gamma, s);
 }
 
+// Two host synchronizations: the ranks (with the density check), and the
+// scalars at the end.
 double energy(Plan& p, const double* P, int nspin, double hf, double hf_lr, double* F,
               cudaStream_t s) {
   const int64_t n = p.nao, nn = n * n;
-  DevBuf Ptot, dvec, gamma, J;
+  const bool exch = hf != 0.0 || hf_lr != 0.0;
+  p.ws_scal.ensure(sizeof(EnergyScalars));
+  EnergyScalars* sc = p.ws_scal.as<EnergyScalars>();
+  DFJK_CUDA(cudaMemsetAsync(sc, 0, sizeof(EnergyScalars), s));
+  nonfinite_kernel<<<(unsigned)((nn * nspin + 255) / 256), 256, 0, s>>>(P, nn * nspin, &sc->nonfinite);
+  DFJK_LAUNCHED();
+  const bool low = exch && low_rank_supported(n);
+  if (low) {
+    p.ws_lowrank.ensure((size_t)nn * nspin * sizeof(double));
+    launch_low_rank(P, n, nspin, p.ws_lowrank.as<double>(), sc->rank, sc->worst, sc->scale, s);
+  }
   const double* Pt = P;
   if (nspin == 2) {
-    Ptot.alloc(nn * sizeof(double));
-    add_kernel<<<(unsigned)((nn + 255) / 256), 256, 0, s>>>(P, P + nn, nn, Ptot.as<double>());
+    p.ws_Ptot.ensure(nn * sizeof(double));
+    add_kernel<<<(unsigned)((nn + 255) / 256), 256, 0, s>>>(P, P + nn, nn, p.ws_Ptot.as<double>());
     DFJK_LAUNCHED();
-    Pt = Ptot.as<double>();
+    Pt = p.ws_Ptot.as<double>();
   }
-  check_finite(p, P, nn * nspin, s, "the density");
-  dvec.alloc(std::max<int64_t>(p.nrows, 1) * sizeof(double));
-  gamma.alloc(p.ldb * sizeof(double));
-  if (p.nrows > 0) {
-    dvec_from_density_kernel<<<(unsigned)((p.nrows + 255) / 256), 256, 0, s>>>(
-        Pt, n, p.d_row_m.as<int>(), p.d_row_n.as<int>(), p.d_row_w.as<int8_t>(), p.nrows,
-        dvec.as<double>());
-    DFJK_LAUNCHED();
-  }
-  gamma_from_dvec(p, dvec.as<double>(), gamma.as<double>(), s);
-  double e = 0.5 * dot(gamma.as<double>(), gamma.as<double>(), p.ldb, s);
+  p.ws_gamma.ensure(p.ldb * sizeof(double));
+  double* gamma = p.ws_gamma.as<double>();
+  gamma_from_density(p, Pt, gamma, s);
+  dot_axpy(p, gamma, gamma, 0.0, p.ldb, nullptr, &sc->dot[0], s);
   if (F) {
-    J.alloc(nn * sizeof(double));
-    j_from_gamma(p, gamma.as<double>(), J.as<double>(), s);
-    for (int sp = 0; sp < nspin; ++sp)
-      DFJK_CUDA(cudaMemcpyAsync(F + sp * nn, J.p, nn * sizeof(double), cudaMemcpyDeviceToDevice, s));
+    j_from_gamma(p, gamma, F, s);
+    if (nspin == 2)
+      DFJK_CUDA(cudaMemcpyAsync(F + nn, F, nn * sizeof(double), cudaMemcpyDeviceToDevice, s));
   }
-  if (hf != 0.0 || hf_lr != 0.0) {
-    DevBuf K, Ct, dw;
-    K.alloc(nn * sizeof(double));
-    for (int sp = 0; sp < nspin; ++sp) {
-      const double* Ps = P + sp * nn;
-      density_factor(p, Ps, Ct, dw, s);
-      const struct { Plan* plan; double coeff; } terms[2] = {{&p, hf},
-                                                             {p.lr ? &p.lr->p : nullptr, hf_lr}};
-      for (const auto& t : terms) {
-        if (t.coeff == 0.0) continue;
-        k_compute(*t.plan, Ct.as<double>(), dw.as<double>(), n, K.as<double>(), s);
-        const double tr = dot(Ps, K.as<double>(), nn, s);
-        // exchange quadratic (terms.py:500-509)
-        e += (nspin == 1 ? -0.25 : -0.5) * t.coeff * tr;
-        if (F) {
-          const double a = (nspin == 1 ? -0.5 : -1.0) * t.coeff;
-          axpy_kernel<<<(unsigned)((nn + 255) / 256), 256, 0, s>>>(K.as<double>(), a, nn,
-                                                                    F + sp * nn);
-          DFJK_LAUNCHED();
-        }
+  EnergyScalars h;
+  DFJK_CUDA(cudaMemcpyAsync(&h, sc, sizeof h, cudaMemcpyDeviceToHost, s));
+  DFJK_CUDA(cudaStreamSynchronize(s));
+  if (h.nonfinite) fail(DFJK_ERR_NUMERIC, "non-finite values in the density");
+  if (!exch) return 0.5 * h.dot[0];
+  auto value = [](unsigned long long bits) {
+    double v;
+    static_assert(sizeof v == sizeof bits, "bits of a double");
+    std::memcpy(&v, &bits, sizeof v);
+    return v;
+  };
+  p.ws_K.ensure(nn * sizeof(double));
+  double* K = p.ws_K.as<double>();
+  for (int sp = 0; sp < nspin; ++sp) {
+    const double* Ps = P + sp * nn;
+    const bool factored = low && value(h.worst[sp]) <= kLowRankAccept * value(h.scale[sp]);
+    DevBuf Ct, dw;
+    if (!factored) density_factor(p, Ps, Ct, dw, s);   // indefinite, or too rough a factor
+    const struct { Plan* plan; double coeff; } terms[2] = {{&p, hf},
+                                                           {p.lr ? &p.lr->p : nullptr, hf_lr}};
+    for (int t = 0; t < 2; ++t) {
+      if (terms[t].coeff == 0.0) continue;
+      Plan& q = *terms[t].plan;
+      if (!factored) {
+        k_compute(q, Ct.as<double>(), dw.as<double>(), n, K, s);
+      } else if (h.rank[sp] > 0) {
+        k_accumulate(q, p.ws_lowrank.as<double>() + sp * nn, 1, n, nullptr, nullptr, h.rank[sp],
+                     1.0, true, K, s);
+      } else {
+        DFJK_CUDA(cudaMemsetAsync(K, 0, nn * sizeof(double), s));
       }
+      // the trace of the exchange quadratic (terms.py:500-509), and F += a K
+      const double a = (nspin == 1 ? -0.5 : -1.0) * terms[t].coeff;
+      dot_axpy(p, K, Ps, a, nn, F ? F + sp * nn : nullptr, &sc->dot[1 + 2 * t + sp], s);
     }
   }
+  DFJK_CUDA(cudaMemcpyAsync(h.dot, sc->dot, sizeof h.dot, cudaMemcpyDeviceToHost, s));
   DFJK_CUDA(cudaStreamSynchronize(s));
+  double e = 0.5 * h.dot[0];
+  for (int sp = 0; sp < nspin; ++sp)
+    e += (nspin == 1 ? -0.25 : -0.5) * (hf * h.dot[1 + sp] + hf_lr * h.dot[3 + sp]);
   return e;
 }
 

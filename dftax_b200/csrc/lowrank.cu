@@ -1,0 +1,199 @@
+// Rank-revealing factor of a density matrix: P = C C^T by Cholesky with
+// diagonal pivoting.
+//
+// K(P) is cheapest from r columns with P = C C^T, r the rank (the occupied
+// orbitals of a closed-shell density). An eigendecomposition gives them, but
+// its tridiagonalization is a chain of n grid-wide steps (1.1 ms for n = 180,
+// 2.3 ms for n = 318, 11 ms for n = 960). A density is positive semidefinite,
+// so Cholesky with the largest remaining diagonal as pivot gives them in r
+// steps and stops by itself: Higham, "Analysis of the Cholesky decomposition
+// of a semi-definite matrix" (1990), bounds its error by a small multiple of
+// r eps |P|. Whether P was positive semidefinite is read off the residual
+// P - C C^T, every element of which is checked; the caller takes the
+// eigensolver when it is not small.
+#include "internal.h"
+
+namespace dfjk {
+namespace {
+
+constexpr int kCta = 8;         // CTAs per cluster, one cluster per spin channel
+constexpr int kLanes = 8;       // k lanes (warps) per block
+constexpr int kRows = 32;       // rows per pass
+
+__device__ __forceinline__ void cluster_barrier() {
+  asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+  asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+
+struct Pivot {
+  double v;
+  long long i;
+};
+
+// the larger value, the lower index among equal ones
+__device__ __forceinline__ Pivot better(Pivot a, Pivot b) {
+  return b.v > a.v || (b.v == a.v && b.i < a.i) ? b : a;
+}
+
+// Columns Ct[k][i] (k < rank) of P[spin] for the cluster of blockIdx.x / 8;
+// rank[spin] out. Left-looking: step k forms column p of the residual from P
+// and the k columns so far, C[i][k] = (P[p][i] - sum_q C[i][q] C[p][q]) /
+// sqrt(d_p), and updates the residual diagonal d. Each CTA owns a run of rows
+// (its part of d in shared memory); a warp per k lane sums every eighth q
+// over 32 rows at a time. One cluster barrier per step carries the CTAs' pivot
+// candidates (distributed shared memory, two sets of slots) and makes the new
+// column visible. Bound by that barrier and the L2 latency of the pivot row,
+// about 2 us a step; the arithmetic is n r^2 in all.
+__global__ void __cluster_dims__(kCta, 1, 1) __launch_bounds__(kLanes * 32)
+    pivoted_cholesky_kernel(const double* __restrict__ Pall, int64_t n, double rel_tol,
+                            double* Ctall, int* __restrict__ rank) {
+  extern __shared__ double sm[];
+  __shared__ double red[kLanes][kRows];
+  __shared__ Pivot slot[2][kCta];
+  const int spin = blockIdx.x / kCta, cta = blockIdx.x % kCta;
+  const double* P = Pall + (int64_t)spin * n * n;
+  double* Ct = Ctall + (int64_t)spin * n * n;
+  const int64_t per = (n + kCta - 1) / kCta;
+  const int64_t lo = cta * per, hi = lo + per < n ? lo + per : n;
+  double* d = sm;            // residual diagonal of rows lo .. hi - 1 (-1: pivoted)
+  double* crow = sm + per;   // C[p][0 .. k - 1]
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  Pivot best{-1.0, 0};
+  if (warp == 0)
+    for (int64_t i = lo + lane; i < hi; i += 32) {
+      d[i - lo] = P[i * n + i];
+      best = better(best, Pivot{d[i - lo], i});
+    }
+  double first = 0.0;
+  int64_t k = 0;
+  for (;; ++k) {
+    if (warp == 0) {
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) {
+        Pivot q{__shfl_xor_sync(0xffffffffu, best.v, o), __shfl_xor_sync(0xffffffffu, best.i, o)};
+        best = better(best, q);
+      }
+      if (lane < kCta) {
+        // this CTA's candidate into slot [k & 1][cta] of CTA `lane`
+        uint32_t a = static_cast<uint32_t>(__cvta_generic_to_shared(&slot[k & 1][cta])), r;
+        asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(lane));
+        asm volatile("st.shared::cluster.f64 [%0], %1;" ::"r"(r), "d"(best.v) : "memory");
+        asm volatile("st.shared::cluster.b64 [%0], %1;" ::"r"(r + 8), "l"(best.i) : "memory");
+      }
+      __syncwarp();
+    }
+    cluster_barrier();
+    Pivot p = slot[k & 1][0];
+#pragma unroll
+    for (int c = 1; c < kCta; ++c) p = better(p, slot[k & 1][c]);
+    if (k == 0) first = p.v;
+    // the same decision in every CTA: all read the same eight candidates
+    if (k == n || !(p.v > rel_tol * first) || !(p.v > 0.0)) break;
+    for (int64_t q = threadIdx.x; q < k; q += kLanes * 32) crow[q] = __ldcg(Ct + q * n + p.i);
+    __syncthreads();
+    const double inv = 1.0 / sqrt(p.v);
+    best = Pivot{-1.0, 0};
+    for (int64_t r0 = lo; r0 < hi; r0 += kRows) {
+      const int64_t i = r0 + lane;
+      double s = 0.0;
+      if (i < hi)
+        for (int64_t q = warp; q < k; q += kLanes) s += Ct[q * n + i] * crow[q];
+      red[warp][lane] = s;
+      __syncthreads();
+      if (warp == 0 && i < hi) {
+        double t = 0.0;
+#pragma unroll
+        for (int w = 0; w < kLanes; ++w) t += red[w][lane];
+        double di = d[i - lo], c = 0.0;
+        if (i == p.i) {
+          c = sqrt(p.v);
+          di = -1.0;
+        } else if (di >= 0.0) {
+          // (rounding can leave a residual diagonal just below zero: its row
+          // is finished then, as a pivoted one is)
+          c = (P[p.i * n + i] - t) * inv;
+          di -= c * c;
+        }
+        d[i - lo] = di;
+        Ct[k * n + i] = c;
+        if (di >= 0.0) best = better(best, Pivot{di, i});
+      }
+      __syncthreads();
+    }
+  }
+  // (the last barrier of the loop: no CTA still writes into another's slots)
+  if (cta == 0 && threadIdx.x == 0) rank[spin] = (int)k;
+}
+
+// worst[spin] = max |P - C C^T| over every element, and scale[spin] = max |P|
+// (bits of non-negative doubles order as integers); 32 x 32 tiles, the rank
+// read on the device
+__global__ void __launch_bounds__(256) residual_kernel(const double* __restrict__ Pall, int64_t n,
+                                                       const double* __restrict__ Ctall,
+                                                       const int* __restrict__ rank,
+                                                       unsigned long long* __restrict__ worst,
+                                                       unsigned long long* __restrict__ scale) {
+  __shared__ double A[32][33], B[32][33];
+  const int spin = blockIdx.z;
+  const double* P = Pall + (int64_t)spin * n * n;
+  const double* Ct = Ctall + (int64_t)spin * n * n;
+  const int r = rank[spin];
+  const int64_t i0 = blockIdx.y * 32, j0 = blockIdx.x * 32;
+  const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
+  double s[4] = {0.0, 0.0, 0.0, 0.0};
+  for (int q0 = 0; q0 < r; q0 += 32) {
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      const int q = q0 + ty + 8 * u;
+      A[ty + 8 * u][tx] = q < r && i0 + tx < n ? Ct[(int64_t)q * n + i0 + tx] : 0.0;
+      B[ty + 8 * u][tx] = q < r && j0 + tx < n ? Ct[(int64_t)q * n + j0 + tx] : 0.0;
+    }
+    __syncthreads();
+#pragma unroll 8
+    for (int q = 0; q < 32; ++q) {
+      const double b = B[q][tx];
+#pragma unroll
+      for (int u = 0; u < 4; ++u) s[u] += A[q][ty + 8 * u] * b;
+    }
+    __syncthreads();
+  }
+  double w = 0.0, m = 0.0;
+#pragma unroll
+  for (int u = 0; u < 4; ++u) {
+    const int64_t i = i0 + ty + 8 * u, j = j0 + tx;
+    if (i < n && j < n) {
+      const double v = P[i * n + j];
+      w = fmax(w, fabs(v - s[u]));
+      m = fmax(m, fabs(v));
+    }
+  }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    w = fmax(w, __shfl_xor_sync(0xffffffffu, w, o));
+    m = fmax(m, __shfl_xor_sync(0xffffffffu, m, o));
+  }
+  if (tx == 0) {
+    atomicMax(worst + spin, (unsigned long long)__double_as_longlong(w));
+    atomicMax(scale + spin, (unsigned long long)__double_as_longlong(m));
+  }
+}
+
+size_t chol_smem(int64_t n) { return (size_t)((n + kCta - 1) / kCta + n) * sizeof(double); }
+
+}  // namespace
+
+bool low_rank_supported(int64_t n) { return chol_smem(n) <= (size_t)200 << 10; }
+
+void launch_low_rank(const double* P, int64_t n, int nspin, double* Ct, int* rank,
+                     unsigned long long* worst, unsigned long long* scale, cudaStream_t s) {
+  const size_t smem = chol_smem(n);
+  DFJK_CUDA(cudaFuncSetAttribute(pivoted_cholesky_kernel,
+                                 cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  pivoted_cholesky_kernel<<<kCta * nspin, kLanes * 32, smem, s>>>(P, n, kLowRankTol, Ct, rank);
+  DFJK_LAUNCHED();
+  const unsigned t = (unsigned)((n + 31) / 32);
+  residual_kernel<<<dim3(t, t, (unsigned)nspin), 256, 0, s>>>(P, n, Ct, rank, worst, scale);
+  DFJK_LAUNCHED();
+}
+
+}  // namespace dfjk

@@ -1,0 +1,69 @@
+"""Energy and Fock of densities through the pivoted Cholesky factor and through
+the eigensolver it falls back to: every rank from zero to full, one and two
+channels, graded eigenvalues down to the cutoff, an indefinite and a negative
+density. The reference contracts the plan's own dense (mn|P) and V+ in float64.
+
+Tolerance: rounding of (mn|P) V+ amplified by the metric's condition number,
+5e-10 (see test_gpu_jk_shapes.py), relative to |J| + |K| of the density without
+cancellation; a factor accepted with a residual of 3e-14 max |P| per element
+moves K by less than nao * 3e-14 of that, below it.
+"""
+
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+REL = 5e-10
+
+
+def _densities(n, rng):
+    q, _ = np.linalg.qr(rng.standard_normal((n, n)))
+    occ = lambda r: 2.0 * q[:, :r] @ q[:, :r].T  # noqa: E731
+    graded = (q * 10.0 ** -np.linspace(0.0, 16.0, n)) @ q.T
+    yield "rank 1", occ(1)[None]
+    yield "rank n/3", occ(n // 3)[None]
+    yield "full rank", occ(n)[None]
+    yield "zero", np.zeros((1, n, n))
+    yield "graded", 0.5 * (graded + graded.T)[None]
+    yield "open shell, one empty channel", np.stack([0.5 * occ(n // 3), np.zeros((n, n))])
+    yield "open shell", np.stack([0.5 * occ(7), 0.5 * occ(5)])
+    yield "indefinite", (occ(5) - 0.3 * occ(9))[None]
+    yield "zero diagonal", np.kron(np.eye(n // 2), [[0.0, 1.0], [1.0, 0.0]])[None]
+    yield "negative", -occ(4)[None]
+
+
+@pytest.mark.parametrize("name,precision,hf_lr", [("water", "fp64", 0.0), ("alkane2", "fp64", 0.0),
+                                                  ("water3", "mixed", 0.0), ("water", "fp64", 0.4)])
+def test_energy_of_any_density(name, precision, hf_lr):
+    import torch
+
+    from dftax_b200 import Plan, systems
+
+    sym, xyz, orb, aux, _ = systems.workload(name, seed=3)
+    plan = Plan(orb, aux, precision=precision, omega=0.3 if hf_lr else 0.0).build()
+    terms = [(plan, 0.25)] + ([(plan.long_range, hf_lr)] if hf_lr else [])
+    T, V = plan.eri3c_dense(), plan.metric_pinv()
+    rel = REL if precision == "fp64" else 1e-7
+    for what, P in _densities(orb.nao, np.random.default_rng(1)):
+        Pt = torch.as_tensor(P, device="cuda")
+        e, F = plan.energy(Pt, 0.25, hf_coeff_lr=hf_lr)
+        g = torch.einsum("mnP,mn->P", T, Pt.sum(0))
+        J = T @ (V @ g)
+        ref, size = 0.5 * float(g @ (V @ g)), float(J.norm())
+        Fr = J[None].repeat(len(P), 1, 1)
+        half = 0.5 if len(P) == 1 else 1.0
+        for p, a in terms:
+            t, v = (T, V) if p is plan else (p.eri3c_dense(), p.metric_pinv())
+            for s in range(len(P)):
+                Y = torch.einsum("mlP,ls->msP", t, Pt[s])
+                K = torch.einsum("msP,PQ,nsQ->mn", Y, v, t)
+                ref -= 0.5 * half * a * float((Pt[s] * K).sum())
+                Fr[s] -= half * a * K
+                A = torch.linalg.eigh(Pt[s])
+                A = (A[1] * A[0].abs()) @ A[1].T
+                size += float(torch.einsum("mlP,ls,PQ,nsQ->mn", t, A, v, t).norm())
+        assert float((F - Fr).norm()) <= rel * size, (what, float((F - Fr).norm()), size)
+        assert abs(e - ref) <= rel * size * max(float(Pt.norm()), 1e-300), (what, e, ref)
+        e2, F2 = plan.energy(Pt, 0.25, hf_coeff_lr=hf_lr)
+        assert e2 == e and torch.equal(F, F2), what
