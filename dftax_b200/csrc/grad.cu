@@ -29,34 +29,34 @@ ShellView view(const Shells& s) {
                    s.d_cen.as<double>(), s.d_pexp.as<double>(), s.d_pcoef.as<double>()};
 }
 
-bool launch_grad3c(int l1, int l2, int lc, dim3 grid, cudaStream_t s, const Grad3cArgs& a) {
+bool launch_grad3c(int l1, int l2, int lc, unsigned npair, cudaStream_t s, const Grad3cArgs& a) {
   switch (l1 * 4 + l2) {
-    case 0: return launch_grad3c_00(lc, grid, s, a);
-    case 4: return launch_grad3c_10(lc, grid, s, a);
-    case 5: return launch_grad3c_11(lc, grid, s, a);
-    case 8: return launch_grad3c_20(lc, grid, s, a);
-    case 9: return launch_grad3c_21(lc, grid, s, a);
-    case 10: return launch_grad3c_22(lc, grid, s, a);
-    case 12: return launch_grad3c_30(lc, grid, s, a);
-    case 13: return launch_grad3c_31(lc, grid, s, a);
-    case 14: return launch_grad3c_32(lc, grid, s, a);
-    case 15: return launch_grad3c_33(lc, grid, s, a);
+    case 0: return launch_grad3c_00(lc, npair, s, a);
+    case 4: return launch_grad3c_10(lc, npair, s, a);
+    case 5: return launch_grad3c_11(lc, npair, s, a);
+    case 8: return launch_grad3c_20(lc, npair, s, a);
+    case 9: return launch_grad3c_21(lc, npair, s, a);
+    case 10: return launch_grad3c_22(lc, npair, s, a);
+    case 12: return launch_grad3c_30(lc, npair, s, a);
+    case 13: return launch_grad3c_31(lc, npair, s, a);
+    case 14: return launch_grad3c_32(lc, npair, s, a);
+    case 15: return launch_grad3c_33(lc, npair, s, a);
     default: return false;
   }
 }
 
-bool launch_pair_deriv(int l1, int l2, unsigned blocks, cudaStream_t s, const PairDerivArgs& a) {
+bool launch_pair_deriv(int l1, int l2, int64_t npp, cudaStream_t s, const PairDerivArgs& a) {
   switch (l1 * 4 + l2) {
-    case 0: launch_pair_deriv_00(blocks, s, a); return true;
-    case 4: launch_pair_deriv_10(blocks, s, a); return true;
-    case 5: launch_pair_deriv_11(blocks, s, a); return true;
-    case 8: launch_pair_deriv_20(blocks, s, a); return true;
-    case 9: launch_pair_deriv_21(blocks, s, a); return true;
-    case 10: launch_pair_deriv_22(blocks, s, a); return true;
-    case 12: launch_pair_deriv_30(blocks, s, a); return true;
-    case 13: launch_pair_deriv_31(blocks, s, a); return true;
-    case 14: launch_pair_deriv_32(blocks, s, a); return true;
-    case 15: launch_pair_deriv_33(blocks, s, a); return true;
+    case 0: launch_pair_deriv_00(npp, s, a); return true;
+    case 4: launch_pair_deriv_10(npp, s, a); return true;
+    case 5: launch_pair_deriv_11(npp, s, a); return true;
+    case 8: launch_pair_deriv_20(npp, s, a); return true;
+    case 9: launch_pair_deriv_21(npp, s, a); return true;
+    case 10: launch_pair_deriv_22(npp, s, a); return true;
+    case 12: launch_pair_deriv_30(npp, s, a); return true;
+    case 13: launch_pair_deriv_31(npp, s, a); return true;
+    case 14: launch_pair_deriv_32(npp, s, a); return true;
+    case 15: launch_pair_deriv_33(npp, s, a); return true;
     default: return false;
   }
 }
@@ -125,8 +125,12 @@ __global__ void trace_kernel(const double* __restrict__ M, int64_t n, int64_t ld
 // ---------------------------------------------------------------------------
 // 2-center derivative: (P|Q) depends on A - B only, so
 //   d(P|Q)/dA_x = hob sum_{c1,c2} T_P[c1][p] T_Q[c2][q] R_{c1 + c2 + e_x}(A - B) = -d/dB_x.
-// One thread per unordered pair of shells of the (LP, LQ) groups; the
-// contribution -1/2 sum_{p,q} W[p][q] d(p|q) counts both orders of a pair.
+// One warp per unordered pair of shells of the (LP, LQ) groups; the
+// contribution -1/2 sum_{p,q} W[p][q] d(p|q) counts both orders of a pair. The
+// warp projects W onto cartesian components through shared memory, builds R
+// with the 3-center kernel's ladder and spreads the (c1, c2) products over its
+// lanes. (A thread per pair kept all of it in local memory: 66 threads for
+// (f|f) on four waters took 177 us.)
 // ---------------------------------------------------------------------------
 
 struct Grad2cArgs {
@@ -148,7 +152,10 @@ template <int LP, int LQ>
 __global__ void __launch_bounds__(128) grad2c_kernel(Grad2cArgs a) {
   constexpr int NP = 2 * LP + 1, NQ = 2 * LQ + 1, CP = nc_(LP), CQ = nc_(LQ);
   constexpr int M1 = LP + LQ + 1, NR = hcount(M1);
-  const int64_t gid = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+  __shared__ double sW[4][NP * NQ], sH[4][CP * NQ], sC[4][CP * CQ];
+  __shared__ double sR[4][2][NR], sB[4][M1 + 1];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int64_t gid = blockIdx.x * (int64_t)4 + warp;
   if (gid >= (int64_t)a.countP * a.countQ) return;
   const int ip = (int)(gid / a.countQ), iq = (int)(gid % a.countQ);
   if (LP == LQ && ip >= iq) return;   // same group: each unordered pair once; a shell with itself has no derivative
@@ -158,23 +165,24 @@ __global__ void __launch_bounds__(128) grad2c_kernel(Grad2cArgs a) {
   const double Z = a.aux.cen[3 * sp + 2] - a.aux.cen[3 * sq + 2];
   const double* TP = a.c2s + a.offP;
   const double* TQ = a.c2s + a.offQ;
-  // W projected on the cartesian components: Wc[c1][c2] = sum_{p,q} T_P W T_Q
-  double Wc[CP * CQ];
+  // W projected on the cartesian components: sum_{p,q} T_P[c1][p] W[p][q] T_Q[c2][q]
   const int r0 = a.colP + ip * NP, c0 = a.colQ + iq * NQ;
-#pragma unroll 1
-  for (int c1 = 0; c1 < CP; ++c1)
-#pragma unroll 1
-    for (int c2 = 0; c2 < CQ; ++c2) {
-      double s = 0.0;
-#pragma unroll 1
-      for (int p = 0; p < NP; ++p) {
-        const double tp = __ldg(TP + c1 * NP + p);
-        if (tp == 0.0) continue;
-#pragma unroll 1
-        for (int q = 0; q < NQ; ++q) s += tp * __ldg(TQ + c2 * NQ + q) * a.W[(int64_t)(r0 + p) * a.ld + c0 + q];
-      }
-      Wc[c1 * CQ + c2] = s;
-    }
+  for (int q = lane; q < NP * NQ; q += 32)
+    sW[warp][q] = a.W[(int64_t)(r0 + q / NQ) * a.ld + c0 + q % NQ];
+  __syncwarp();
+  for (int q = lane; q < CP * NQ; q += 32) {
+    double s = 0.0;
+    for (int k = 0; k < NP; ++k) s += __ldg(TP + q / NQ * NP + k) * sW[warp][k * NQ + q % NQ];
+    sH[warp][q] = s;
+  }
+  __syncwarp();
+  for (int q = lane; q < CP * CQ; q += 32) {
+    double s = 0.0;
+    for (int k = 0; k < NQ; ++k) s += sH[warp][q / CQ * NQ + k] * __ldg(TQ + q % CQ * NQ + k);
+    sC[warp][q] = s;
+  }
+  HermiteGroup<M1, 32> ladder;
+  ladder.init(lane);
   double f[3] = {0.0, 0.0, 0.0};
 #pragma unroll 1
   for (int i = 0; i < a.aux.nprim[sp]; ++i) {
@@ -183,35 +191,34 @@ __global__ void __launch_bounds__(128) grad2c_kernel(Grad2cArgs a) {
     for (int j = 0; j < a.aux.nprim[sq]; ++j) {
       const double be = a.aux.pexp[a.aux.prim0[sq] + j], cb = a.aux.pcoef[a.aux.prim0[sq] + j];
       const double rho = al * be / (al + be);
-      double F[M1 + 1];
-      boys_operator<M1>(rho * (X * X + Y * Y + Z * Z), rho, a.omega, a.boys, a.boys_asym, F);
-      double R[NR];
-      hermite_r<M1>(rho, X, Y, Z, F, R);
+      const double* R = ladder.run(rho * (X * X + Y * Y + Z * Z), rho, a.omega, X, Y, Z, a.boys,
+                                   a.boys_asym, sB[warp], sR[warp][0], sR[warp][1], lane);
       double hob = kTwoPi25 * ca * cb / (al * be * sqrt(al + be));
 #pragma unroll
       for (int k = 0; k < LP; ++k) hob *= 0.5 / al;
 #pragma unroll
       for (int k = 0; k < LQ; ++k) hob *= -0.5 / be;
-#pragma unroll 1
-      for (int c1 = 0; c1 < CP; ++c1) {
-        const int x1 = comp_x(LP, c1), y1 = comp_y(LP, c1), z1 = comp_z(LP, c1);
-#pragma unroll 1
-        for (int c2 = 0; c2 < CQ; ++c2) {
-          const double wc = hob * Wc[c1 * CQ + c2];
-          if (wc == 0.0) continue;
-          const int x = x1 + comp_x(LQ, c2), y = y1 + comp_y(LQ, c2), z = z1 + comp_z(LQ, c2);
-          f[0] += wc * R[hidx(x + 1, y, z)];
-          f[1] += wc * R[hidx(x, y + 1, z)];
-          f[2] += wc * R[hidx(x, y, z + 1)];
-        }
+      for (int q = lane; q < CP * CQ; q += 32) {
+        const int c1 = q / CQ, c2 = q % CQ;
+        const double wc = hob * sC[warp][q];
+        const int x1 = comp_x(LP, c1), y1 = comp_y(LP, c1), x2 = comp_x(LQ, c2), y2 = comp_y(LQ, c2);
+        const int x = x1 + x2, y = y1 + y2, z = LP + LQ - x - y;
+        f[0] += wc * R[hidx(x + 1, y, z)];
+        f[1] += wc * R[hidx(x, y + 1, z)];
+        f[2] += wc * R[hidx(x, y, z + 1)];
       }
+      __syncwarp();   // sB and R are rewritten by the next primitives
     }
   }
   // -1/2 (W_pq + W_qp) d(p|q)/dA = -f on P's center, +f on Q's (dB = -dA)
 #pragma unroll
   for (int d = 0; d < 3; ++d) {
-    atomicAdd(a.grad_aux + 3 * sp + d, -f[d]);
-    atomicAdd(a.grad_aux + 3 * sq + d, f[d]);
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) f[d] += __shfl_xor_sync(0xffffffffu, f[d], o);
+    if (lane == d) {
+      atomicAdd(a.grad_aux + 3 * sp + d, -f[d]);
+      atomicAdd(a.grad_aux + 3 * sq + d, f[d]);
+    }
   }
 }
 
@@ -244,7 +251,7 @@ void launch_grad2c(Plan& p, const double* W, double* grad_aux, cudaStream_t s) {
       a.omega = p.atten;
       a.grad_aux = grad_aux;
       const int64_t n = (int64_t)a.countP * a.countQ;
-      const unsigned blocks = (unsigned)((n + 127) / 128);
+      const unsigned blocks = (unsigned)((n + 3) / 4);
       bool done = false;
 #define X(A, B)                                              \
   if (lp == A && lq == B) {                                  \
@@ -267,7 +274,6 @@ void launch_grad3c_pairs(Plan& p, const ClassRange& cr, int64_t b, int64_t e, do
   const Context& c = *p.ctx;
   const int64_t pp_b = p.pair_pp0[b];
   const int64_t pp_e = p.pair_pp0[e - 1] + p.pair_npp[e - 1];
-  const int nab = (2 * cr.l1 + 1) * (2 * cr.l2 + 1);
   {
     PairDerivArgs a;
     a.pp_pair = p.d_pp_pair.as<int>();
@@ -282,8 +288,7 @@ void launch_grad3c_pairs(Plan& p, const ClassRange& cr, int64_t b, int64_t e, do
     a.pp_begin = pp_b;
     a.pp_count = pp_e - pp_b;
     a.dsph = dsph;
-    const int64_t threads = a.pp_count * 3 * nab;
-    if (!launch_pair_deriv(cr.l1, cr.l2, (unsigned)((threads + 127) / 128), s, a))
+    if (!launch_pair_deriv(cr.l1, cr.l2, a.pp_count, s, a))
       fail(DFJK_ERR_UNSUPPORTED, "pair derivative class (%d,%d) not compiled", cr.l1, cr.l2);
     DFJK_LAUNCHED();
   }
@@ -317,8 +322,7 @@ void launch_grad3c_pairs(Plan& p, const ClassRange& cr, int64_t b, int64_t e, do
     a.omega = p.atten;
     a.grad_orb = grad_orb;
     a.grad_aux = grad_aux;
-    dim3 grid((unsigned)(e - b), (unsigned)((a.aux_count + 127) / 128));
-    if (!launch_grad3c(cr.l1, cr.l2, lc, grid, s, a))
+    if (!launch_grad3c(cr.l1, cr.l2, lc, (unsigned)(e - b), s, a))
       fail(DFJK_ERR_UNSUPPORTED, "3-center derivative class (%d,%d|%d) not compiled", cr.l1, cr.l2, lc);
     DFJK_LAUNCHED();
   }

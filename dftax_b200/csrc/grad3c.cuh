@@ -3,7 +3,7 @@
 // the kept shell pairs, columns = auxiliary functions in sorted order).
 //
 // For one kept shell pair (a, b) (a has the larger l, center A; b center B)
-// and one auxiliary shell c (center C) a thread forms
+// and one auxiliary shell c (center C) a group of lanes forms
 //   fA = sum_{i,m} G[i][m] d(ab|c)[i][m]/dA,  fC = sum_{i,m} G[i][m] d(ab|c)[i][m]/dC,
 // and fB = -fA - fC (the integral is unchanged when all three centers move
 // together). In the McMurchie-Davidson form of eri3c.cuh,
@@ -16,7 +16,7 @@
 // (dftax/ks/forces.py:245-270 through dftax/integrals/eri3c_bucketed.py:376-426).
 #pragma once
 
-#include "md_device.cuh"
+#include "eri3c.cuh"
 
 namespace dfjk {
 
@@ -33,67 +33,69 @@ struct PairDerivArgs {
   double* dsph;         // [pp - pp_begin][3][na*nb][hcount(l1 + l2 + 1)]
 };
 
-// One thread per (primitive pair, spherical function pair, direction).
+// A primitive pair's tables by one warp (LAB <= 2) or one block: the three
+// axes' E tables (shared, by three lanes), the derivative axis' coefficients,
+// then one output (direction, function pair, Hermite entry) per lane. A thread
+// per function pair and direction left (dd) at 750 threads on four waters and
+// its Hermite sums in local memory: 149 us.
 template <int L1, int L2>
 __global__ void __launch_bounds__(128) pair_deriv_kernel(PairDerivArgs a) {
   constexpr int NA = 2 * L1 + 1, NB = 2 * L2 + 1, NAB = NA * NB, NH1 = hcount(L1 + L2 + 1);
   constexpr int CA = nc_(L1), CB = nc_(L2), T1 = L1 + L2 + 2;
-  const int64_t gid = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  const int64_t local = gid / (3 * NAB);
-  if (local >= a.pp_count) return;
-  const int rem = (int)(gid % (3 * NAB));
-  const int dir = rem / NAB, ab = rem % NAB;
-  const int ia = ab / NB, ib = ab % NB;
-  const int64_t pp = a.pp_begin + local;
-  const int pr = a.pp_pair[pp];
-  const int s1 = a.pair_s1[pr], s2 = a.pair_s2[pr];
-  const int p1 = a.orb.prim0[s1] + a.pp_pa[pp], p2 = a.orb.prim0[s2] + a.pp_pb[pp];
-  const double al = a.orb.pexp[p1], be = a.orb.pexp[p2];
-  double E[3][L1 + 2][L2 + 1][T1];
-#pragma unroll 1
-  for (int x = 0; x < 3; ++x) e_axis<L1 + 1, L2>(al, be, a.orb.cen[3 * s1 + x] - a.orb.cen[3 * s2 + x], E[x]);
-  // coefficient of Hermite order t on axis x for exponents (li, mi): the plain
-  // table, or on the derivative axis 2 al E[li+1] - li E[li-1]
-  auto coef = [&](int x, int li, int mi, int t) -> double {
-    if (x != dir) return t <= li + mi ? E[x][li][mi][t] : 0.0;
-    double v = 2.0 * al * E[x][li + 1][mi][t];
-    if (li > 0 && t <= li - 1 + mi) v -= li * E[x][li - 1][mi][t];
-    return v;
-  };
-  double out[NH1];
+  constexpr int TPP = L1 + L2 <= 2 ? 32 : 128, PPB = 128 / TPP;
+  // [0]: E of the axis, [1]: 2 al E[li + 1] - li E[li - 1] (zero past their orders)
+  __shared__ double sE[PPB][2][3][L1 + 1][L2 + 1][T1];
+  const int g = threadIdx.x / TPP, gl = threadIdx.x % TPP;
+  const int64_t local = blockIdx.x * (int64_t)PPB + g;
+  const bool on = local < a.pp_count;
+  const int64_t pp = a.pp_begin + (on ? local : 0);
+  if (gl < 3) {
+    const int pr = a.pp_pair[pp], s1 = a.pair_s1[pr], s2 = a.pair_s2[pr];
+    const double al = a.orb.pexp[a.orb.prim0[s1] + a.pp_pa[pp]];
+    const double be = a.orb.pexp[a.orb.prim0[s2] + a.pp_pb[pp]];
+    double E[L1 + 2][L2 + 1][T1];
+    e_axis<L1 + 1, L2>(al, be, a.orb.cen[3 * s1 + gl] - a.orb.cen[3 * s2 + gl], E);
 #pragma unroll
-  for (int h = 0; h < NH1; ++h) out[h] = 0.0;
+    for (int i = 0; i <= L1; ++i)
+#pragma unroll
+      for (int j = 0; j <= L2; ++j)
+#pragma unroll
+        for (int t = 0; t < T1; ++t) {
+          sE[g][0][gl][i][j][t] = E[i][j][t];
+          double v = 2.0 * al * E[i + 1][j][t];
+          if (i > 0) v -= i * E[i - 1][j][t];
+          sE[g][1][gl][i][j][t] = v;
+        }
+  }
+  __syncthreads();
+  if (!on) return;
   const double* TA = a.c2s + a.off1;
   const double* TB = a.c2s + a.off2;
+  double* dst = a.dsph + local * (3 * NAB * NH1);
 #pragma unroll 1
-  for (int ca = 0; ca < CA; ++ca) {
-    const double ta = TA[ca * NA + ia];
-    if (ta == 0.0) continue;
-    const int la[3] = {comp_x(L1, ca), comp_y(L1, ca), comp_z(L1, ca)};
+  for (int q = gl; q < 3 * NAB * NH1; q += TPP) {
+    const int h = q % NH1, ab = q / NH1 % NAB, dir = q / (NH1 * NAB);
+    const int ia = ab / NB, ib = ab % NB;
+    int t, u, v;
+    hdecode(h, t, u, v);
+    double sum = 0.0;
 #pragma unroll 1
-    for (int cb = 0; cb < CB; ++cb) {
-      const double tab = ta * TB[cb * NB + ib];
-      if (tab == 0.0) continue;
-      const int lb[3] = {comp_x(L2, cb), comp_y(L2, cb), comp_z(L2, cb)};
-      const int tx = la[0] + lb[0] + (dir == 0), ty = la[1] + lb[1] + (dir == 1),
-                tz = la[2] + lb[2] + (dir == 2);
+    for (int ca = 0; ca < CA; ++ca) {
+      const double ta = TA[ca * NA + ia];
+      if (ta == 0.0) continue;
+      const int ax = comp_x(L1, ca), ay = comp_y(L1, ca), az = L1 - ax - ay;
 #pragma unroll 1
-      for (int t = 0; t <= tx; ++t) {
-        const double ct = tab * coef(0, la[0], lb[0], t);
-        if (ct == 0.0) continue;
-#pragma unroll 1
-        for (int u = 0; u <= ty; ++u) {
-          const double cu = ct * coef(1, la[1], lb[1], u);
-          if (cu == 0.0) continue;
-#pragma unroll 1
-          for (int v = 0; v <= tz; ++v) out[hidx(t, u, v)] += cu * coef(2, la[2], lb[2], v);
-        }
+      for (int cb = 0; cb < CB; ++cb) {
+        const double tab = ta * TB[cb * NB + ib];
+        if (tab == 0.0) continue;
+        const int bx = comp_x(L2, cb), by = comp_y(L2, cb), bz = L2 - bx - by;
+        // orders past an axis' own are zero in the tables
+        sum += tab * sE[g][dir == 0][0][ax][bx][t] * sE[g][dir == 1][1][ay][by][u] *
+               sE[g][dir == 2][2][az][bz][v];
       }
     }
+    dst[q] = sum;
   }
-  double* dst = a.dsph + ((local * 3 + dir) * NAB + ab) * NH1;
-#pragma unroll 1
-  for (int h = 0; h < NH1; ++h) dst[h] = out[h];
 }
 
 struct Grad3cArgs {
@@ -124,195 +126,306 @@ struct Grad3cArgs {
   double* grad_aux;          // [aux shell][3]
 };
 
-// Hermite R^0_{tuv} for t+u+v <= M (packed by hidx) with runtime loops: the
-// same in-place ladder as hermite_r, kept rolled so the high orders of the
-// derivative classes compile to a small kernel (R lives in local memory).
-// F holds F_n(t) on entry and (-2 rho)^n F_n(t) on return.
-__device__ __forceinline__ void hermite_r_rolled(int M, double rho, double X, double Y, double Z,
-                                                 double* F, double* R) {
-  const double m2r = -2.0 * rho;
-  double pw = 1.0;
-  for (int n = 0; n <= M; ++n) {
-    F[n] *= pw;
-    pw *= m2r;
-  }
-  R[0] = F[M];
-#pragma unroll 1
-  for (int n = M - 1; n >= 0; --n) {
-#pragma unroll 1
-    for (int k = M - n; k >= 1; --k) {
-#pragma unroll 1
-      for (int t = k; t >= 0; --t) {
-#pragma unroll 1
-        for (int v = 0; v <= k - t; ++v) {
-          const int u = k - t - v;
-          double val;
-          if (v > 0) {
-            val = Z * R[hidx(t, u, v - 1)];
-            if (v > 1) val += (v - 1) * R[hidx(t, u, v - 2)];
-          } else if (u > 0) {
-            val = Y * R[hidx(t, u - 1, 0)];
-            if (u > 1) val += (u - 1) * R[hidx(t, u - 2, 0)];
-          } else {
-            val = X * R[hidx(t - 1, 0, 0)];
-            if (t > 1) val += (t - 1) * R[hidx(t - 2, 0, 0)];
-          }
-          R[hidx(t, u, v)] = val;
-        }
+// The Hermite R ladder of order M by a group of TL lanes: lane gl holds the
+// entries h = gl + TL j, each with what its recursion reads packed into a word
+// (order, axis, the second term's factor, the two entries).
+template <int M, int TL>
+struct HermiteGroup {
+  static constexpr int NR = hcount(M), RJ = (NR + TL - 1) / TL;
+  static_assert(M < 15 && NR <= 512, "packed table fields");
+  uint32_t tab[RJ];
+
+  __device__ __forceinline__ void init(int gl) {
+#pragma unroll
+    for (int j = 0; j < RJ; ++j) {
+      const int h = gl + TL * j;
+      tab[j] = 15u;   // past every order
+      if (h < NR) {
+        int t, u, v;
+        hdecode(h, t, u, v);
+        const int ax = v > 0 ? 2 : (u > 0 ? 1 : 0), k = v > 0 ? v : (u > 0 ? u : t);
+        const int dt = ax == 0, du = ax == 1, dv = ax == 2;
+        const int e1 = k > 0 ? hidx(t - dt, u - du, v - dv) : 0;
+        const int e2 = k > 1 ? hidx(t - 2 * dt, u - 2 * du, v - 2 * dv) : 0;
+        const int mul = k > 1 ? k - 1 : 0;
+        tab[j] = (uint32_t)(t + u + v) | (uint32_t)ax << 4 | (uint32_t)mul << 6 |
+                 (uint32_t)e1 << 10 | (uint32_t)e2 << 19;
       }
     }
-    R[0] = F[n];
   }
-}
+
+  // R_{tuv} (t + u + v <= M, packed by hidx) at (X, Y, Z), T = rho r^2, of the
+  // Coulomb (omega = 0) or erf(omega r)/r operator, in sRa or sRb (the one
+  // returned; NR doubles each, sB: M + 1). Whole warps call it together; it
+  // ends with the lanes in step.
+  __device__ __forceinline__ const double* run(double T, double rho, double omega, double X,
+                                               double Y, double Z, const double* __restrict__ boys,
+                                               const double* __restrict__ asym, double* sB,
+                                               double* sRa, double* sRb, int gl) const {
+    double sat = 1.0, rs = 1.0;
+    if (omega > 0.0) {
+      sat = omega * omega / (omega * omega + rho);
+      rs = sqrt(sat);
+    }
+    const double x = -2.0 * rho * sat;
+    for (int o = gl; o <= M; o += TL) {
+      double f = rs * boys_order(o, sat * T, boys, asym);
+      for (int k = 0; k < o; ++k) f *= x;
+      sB[o] = f;
+    }
+    __syncwarp();
+    double* src = sRa;
+    double* dst = sRb;
+    if (gl == 0) src[0] = sB[M];
+    __syncwarp();
+#pragma unroll 1
+    for (int n = M - 1; n >= 0; --n) {
+#pragma unroll
+      for (int j = 0; j < RJ; ++j) {
+        const uint32_t e = tab[j];
+        const int ord = e & 15, ax = e >> 4 & 3, mul = e >> 6 & 15;
+        if (ord > M - n) continue;
+        double val;
+        if (ord == 0) {
+          val = sB[n];
+        } else {
+          val = (ax == 0 ? X : (ax == 1 ? Y : Z)) * src[e >> 10 & 511];
+          if (mul) val += mul * src[e >> 19];
+        }
+        dst[gl + TL * j] = val;
+      }
+      __syncwarp();
+      double* tmp = src;
+      src = dst;
+      dst = tmp;
+    }
+    return src;
+  }
+};
+
+// A group of lanes (a warp, or 8 lanes when LAB <= 1) per (pair, auxiliary
+// shell):
+//   * the Boys values, one order per lane;
+//   * the Hermite R ladder of order LAB + LC + 1, level by level in two shared
+//     buffers, each lane updating a fixed set of (t, u, v) entries;
+//   * W_m[h] = pref sum_c T[c][m] R[h + c], h of order <= LAB + 1, the lane's h
+//     in registers and in shared memory;
+//   * for each bra row i: gh_m[h] += G[i][m] Esph[i][h] and, unless the pair is
+//     one shell with itself, fA_d += D_d[i][h] sum_m G[i][m] W_m[h];
+//   * fC_d = -sum_{m,h} gh_m[h] W_m[h + e_d].
+// Bound by latency at few triples and by the G contraction, NAB (2 NC + 3) NH1
+// products, at many. One thread per triple (R, W, gh and the derivative sums,
+// up to 1000 doubles, in local memory) took 7.9 ms for (H2O)_4, where (dd|d)
+// has 280 triples.
+template <int LA, int LB, int LC>
+struct GradShape {
+  static constexpr int NC = 2 * LC + 1, NCC = nc_(LC), LAB = LA + LB;
+  static constexpr int NAB = (2 * LA + 1) * (2 * LB + 1);
+  static constexpr int NH = hcount(LAB), NH1 = hcount(LAB + 1), M1 = LAB + LC + 1, NR = hcount(M1);
+  static constexpr int TL = LAB <= 1 ? 8 : 32, GPB = 128 / TL;   // lanes per group, groups per block
+  // Hermite entries per lane, and components m held at a time: at most 15 sums
+  // of each kind per lane (27 or 36 at once spilled kilobytes)
+  static constexpr int HJ = (NH1 + TL - 1) / TL;
+  static constexpr int MP = (NC * HJ + 14) / 15, MC = (NC + MP - 1) / MP;
+  static constexpr int GROUP = 2 * NR + MC * NH1 + NAB * NC + (M1 + 1);   // doubles
+  static constexpr size_t smem = (size_t)(NCC * NC + GPB * GROUP) * sizeof(double) +
+                                 (size_t)NH1 * NCC * sizeof(short);
+};
 
 template <int LA, int LB, int LC>
 __global__ void __launch_bounds__(128) grad3c_kernel(Grad3cArgs a) {
-  constexpr int NA = 2 * LA + 1, NB = 2 * LB + 1, NC = 2 * LC + 1, NCC = nc_(LC);
-  constexpr int LAB = LA + LB, NH = hcount(LAB), NH1 = hcount(LAB + 1), NAB = NA * NB;
-  constexpr int M1 = LAB + LC + 1, NR = hcount(M1);
-  __shared__ double sT[NCC * NC];
-  __shared__ int sC[NCC][3];
+  using S = GradShape<LA, LB, LC>;
+  constexpr int NC = S::NC, NCC = S::NCC, NAB = S::NAB, NH = S::NH, NH1 = S::NH1, M1 = S::M1;
+  constexpr int NR = S::NR, TL = S::TL, GPB = S::GPB;
+  constexpr int HJ = S::HJ, MC = S::MC;
+  extern __shared__ double gsm[];
   __shared__ double red[4][6];
-  for (int q = threadIdx.x; q < NCC * NC; q += blockDim.x) sT[q] = a.c2s_aux[q];
-  for (int q = threadIdx.x; q < NCC; q += blockDim.x) {
-    sC[q][0] = comp_x(LC, q);
-    sC[q][1] = comp_y(LC, q);
-    sC[q][2] = comp_z(LC, q);
+  const int grp = threadIdx.x / TL, gl = threadIdx.x % TL;
+  double* sT = gsm;
+  double* sRa = sT + NCC * NC + grp * S::GROUP;
+  double* sRb = sRa + NR;
+  double* sW = sRb + NR;
+  double* sG = sW + MC * NH1;
+  double* sB = sG + NAB * NC;
+  short* sI = reinterpret_cast<short*>(gsm + NCC * NC + GPB * S::GROUP);   // hidx(h + c)
+  for (int q = threadIdx.x; q < NCC * NC; q += 128) sT[q] = a.c2s_aux[q];
+  for (int q = threadIdx.x; q < NH1 * NCC; q += 128) {
+    int t, u, v;
+    hdecode(q / NCC, t, u, v);
+    const int c = q % NCC;
+    sI[q] = (short)hidx(t + comp_x(LC, c), u + comp_y(LC, c), v + comp_z(LC, c));
+  }
+  HermiteGroup<M1, TL> ladder;
+  ladder.init(gl);
+  // h + e_d of the lane's Hermite entries
+  int up[HJ][3];
+#pragma unroll
+  for (int j = 0; j < HJ; ++j) {
+    int t = 0, u = 0, v = 0;
+    if (gl + TL * j < NH) hdecode(gl + TL * j, t, u, v);
+    up[j][0] = hidx(t + 1, u, v);
+    up[j][1] = hidx(t, u + 1, v);
+    up[j][2] = hidx(t, u, v + 1);
   }
   __syncthreads();
-  const int slot = blockIdx.y * blockDim.x + threadIdx.x;
   const int64_t pr = a.pair_begin + blockIdx.x;
   const int s1 = a.pair_s1[pr], s2 = a.pair_s2[pr];
   const bool same = s1 == s2;   // fA + fB = -fC lands on one shell: no d/dA needed
-  double fA[3] = {0.0, 0.0, 0.0}, fC[3] = {0.0, 0.0, 0.0};
-  if (slot < a.aux_count) {
+  const int64_t pp0 = a.pair_pp0[pr];
+  const int npp = a.pair_npp[pr];
+  const double* Gp = a.G + (a.pair_row0[pr] - a.row_base) * a.ld + a.col_base;
+  double fab[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};   // this lane's part of fA and fB
+  for (int base = blockIdx.y * GPB; base < a.aux_count; base += gridDim.y * GPB) {
+    // groups past the last shell run along with zero weights
+    const bool on = base + grp < a.aux_count;
+    const int slot = on ? base + grp : a.aux_count - 1;
     const int kc = a.aux_sorted[a.aux_begin + slot];
     const double C0 = a.aux.cen[3 * kc], C1 = a.aux.cen[3 * kc + 1], C2 = a.aux.cen[3 * kc + 2];
     const int cp0 = a.aux.prim0[kc], cnp = a.aux.nprim[kc];
-    const int64_t pp0 = a.pair_pp0[pr];
-    const int npp = a.pair_npp[pr];
-    const double* Grow = a.G + (a.pair_row0[pr] - a.row_base) * a.ld + a.col_base + slot * NC;
-    double R[NR], w[NH1], gh[NH], dh[3 * NH1];
+    const int cmax = TL == 32 ? cnp : __reduce_max_sync(0xffffffffu, cnp);
+    for (int q = gl; q < NAB * NC; q += TL)
+      sG[q] = on ? Gp[(int64_t)(q / NC) * a.ld + slot * NC + q % NC] : 0.0;
+    double fA[3] = {0.0, 0.0, 0.0}, fC[3] = {0.0, 0.0, 0.0};
 #pragma unroll 1
     for (int q = 0; q < npp; ++q) {
       const int64_t pp = pp0 + q;
-      const double P0 = a.pp_P[3 * pp], P1 = a.pp_P[3 * pp + 1], P2 = a.pp_P[3 * pp + 2];
-      const double g = a.pp_g[pp];
-      const double pab = a.pp_pref[pp];
+      const double X = a.pp_P[3 * pp] - C0, Y = a.pp_P[3 * pp + 1] - C1, Z = a.pp_P[3 * pp + 2] - C2;
+      const double g = a.pp_g[pp], pab = a.pp_pref[pp];
       const double* E = a.esph + (pp - a.esph_pp0) * (NAB * NH);
       const double* D = a.dsph + (pp - a.dsph_pp0) * (3 * NAB * NH1);
 #pragma unroll 1
-      for (int ic = 0; ic < cnp; ++ic) {
-        const double gc = a.aux.pexp[cp0 + ic], cc = a.aux.pcoef[cp0 + ic];
+      for (int ic = 0; ic < cmax; ++ic) {
+        // (a group with fewer primitives repeats its last with a zero factor)
+        const int pc = cp0 + (ic < cnp ? ic : cnp - 1);
+        const double gc = a.aux.pexp[pc], cc = ic < cnp ? a.aux.pcoef[pc] : 0.0;
         const double rho = g * gc / (g + gc);
-        const double X = P0 - C0, Y = P1 - C1, Z = P2 - C2;
-        double F[M1 + 1];
-        boys_operator<M1>(rho * (X * X + Y * Y + Z * Z), rho, a.omega, a.boys, a.boys_asym, F);
-        hermite_r_rolled(M1, rho, X, Y, Z, F, R);
+        const double T = rho * (X * X + Y * Y + Z * Z);
+        const double* src = ladder.run(T, rho, a.omega, X, Y, Z, a.boys, a.boys_asym, sB, sRa, sRb, gl);
         double hob = 1.0;
+#pragma unroll
         for (int k = 0; k < LC; ++k) hob *= -0.5 / gc;
         const double pref = pab * cc * kTwoPi25 / (g * gc * sqrt(g + gc)) * hob;
+        // MC components m at a time, so that w and gh stay in registers
 #pragma unroll 1
-        for (int m = 0; m < NC; ++m) {
-          // W_m[h] = pref sum_c T[c][m] R_{h + c}, h of order <= LAB + 1
+        for (int m0 = 0; m0 < NC; m0 += MC) {
+          double w[HJ][MC], gh[HJ][MC];
+#pragma unroll
+          for (int j = 0; j < HJ; ++j) {
+            const int h = gl + TL * j;
+#pragma unroll
+            for (int m = 0; m < MC; ++m) w[j][m] = gh[j][m] = 0.0;
+            if (h >= NH1) continue;
 #pragma unroll 1
-          for (int t = 0; t <= LAB + 1; ++t)
-#pragma unroll 1
-            for (int u = 0; u <= LAB + 1 - t; ++u)
-#pragma unroll 1
-              for (int v = 0; v <= LAB + 1 - t - u; ++v) {
-                double sum = 0.0;
-#pragma unroll 1
-                for (int c = 0; c < NCC; ++c)
-                  sum += sT[c * NC + m] * R[hidx(t + sC[c][0], u + sC[c][1], v + sC[c][2])];
-                w[hidx(t, u, v)] = sum * pref;
-              }
-          // G-weighted Hermite coefficients of the bra: plain and d/dA
-#pragma unroll 1
-          for (int h = 0; h < NH; ++h) gh[h] = 0.0;
-#pragma unroll 1
-          for (int h = 0; h < 3 * NH1; ++h) dh[h] = 0.0;
+            for (int c = 0; c < NCC; ++c) {
+              const double r = src[sI[h * NCC + c]];
+#pragma unroll
+              for (int m = 0; m < MC; ++m)
+                if (m0 + m < NC) w[j][m] += sT[c * NC + m0 + m] * r;
+            }
+#pragma unroll
+            for (int m = 0; m < MC; ++m) {
+              w[j][m] *= pref;
+              sW[m * NH1 + h] = w[j][m];
+            }
+          }
+          __syncwarp();
 #pragma unroll 1
           for (int i = 0; i < NAB; ++i) {
-            const double gi = Grow[(int64_t)i * a.ld + m];
-            if (gi == 0.0) continue;
-            const double* Ei = E + i * NH;
-#pragma unroll 4
-            for (int h = 0; h < NH; ++h) gh[h] += gi * __ldg(Ei + h);
-            if (!same) {
-#pragma unroll 1
-              for (int d = 0; d < 3; ++d) {
-                const double* Di = D + (d * NAB + i) * NH1;
-#pragma unroll 4
-                for (int h = 0; h < NH1; ++h) dh[d * NH1 + h] += gi * __ldg(Di + h);
+            double gi[MC];
+#pragma unroll
+            for (int m = 0; m < MC; ++m) gi[m] = m0 + m < NC ? sG[i * NC + m0 + m] : 0.0;
+#pragma unroll
+            for (int j = 0; j < HJ; ++j) {
+              const int h = gl + TL * j;
+              if (h < NH) {
+                const double e = __ldg(E + i * NH + h);
+#pragma unroll
+                for (int m = 0; m < MC; ++m) gh[j][m] += gi[m] * e;
+              }
+              if (!same && h < NH1) {
+                double v = 0.0;
+#pragma unroll
+                for (int m = 0; m < MC; ++m) v += gi[m] * w[j][m];
+#pragma unroll
+                for (int d = 0; d < 3; ++d) fA[d] += v * __ldg(D + (d * NAB + i) * NH1 + h);
               }
             }
           }
-#pragma unroll 1
-          for (int t = 0; t <= LAB; ++t)
-#pragma unroll 1
-            for (int u = 0; u <= LAB - t; ++u)
-#pragma unroll 1
-              for (int v = 0; v <= LAB - t - u; ++v) {
-                const double e = gh[hidx(t, u, v)];
-                fC[0] -= e * w[hidx(t + 1, u, v)];
-                fC[1] -= e * w[hidx(t, u + 1, v)];
-                fC[2] -= e * w[hidx(t, u, v + 1)];
-              }
-          if (!same) {
-#pragma unroll 1
-            for (int d = 0; d < 3; ++d) {
-              double sum = 0.0;
-#pragma unroll 4
-              for (int h = 0; h < NH1; ++h) sum += dh[d * NH1 + h] * w[h];
-              fA[d] += sum;
-            }
+#pragma unroll
+          for (int j = 0; j < HJ; ++j) {
+            if (gl + TL * j >= NH) continue;
+#pragma unroll
+            for (int m = 0; m < MC; ++m)
+#pragma unroll
+              for (int d = 0; d < 3; ++d) fC[d] -= gh[j][m] * sW[m * NH1 + up[j][d]];
           }
+          __syncwarp();   // sW is rewritten by the next components
         }
       }
     }
-    // the auxiliary shells of the block differ: one atomic add each
-    for (int d = 0; d < 3; ++d) atomicAdd(a.grad_aux + 3 * kc + d, fC[d]);
+#pragma unroll
+    for (int d = 0; d < 3; ++d) {
+      fab[d] += fA[d];
+      fab[3 + d] -= fA[d] + fC[d];
+#pragma unroll
+      for (int o = TL / 2; o > 0; o >>= 1) fC[d] += __shfl_xor_sync(0xffffffffu, fC[d], o);
+    }
+    if (on && gl < 3) atomicAdd(a.grad_aux + 3 * kc + gl, gl == 0 ? fC[0] : (gl == 1 ? fC[1] : fC[2]));
+    __syncwarp();   // sG is rewritten by the next shell
   }
   // fA and fB = -fA - fC summed over the block (one shell pair)
-  double v[6] = {fA[0], fA[1], fA[2], -fA[0] - fC[0], -fA[1] - fC[1], -fA[2] - fC[2]};
 #pragma unroll
   for (int k = 0; k < 6; ++k)
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v[k] += __shfl_xor_sync(0xffffffffu, v[k], o);
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  if (lane == 0)
+    for (int o = 16; o > 0; o >>= 1) fab[k] += __shfl_xor_sync(0xffffffffu, fab[k], o);
+  if ((threadIdx.x & 31) == 0)
 #pragma unroll
-    for (int k = 0; k < 6; ++k) red[warp][k] = v[k];
+    for (int k = 0; k < 6; ++k) red[threadIdx.x >> 5][k] = fab[k];
   __syncthreads();
   if (threadIdx.x < 6) {
     double sum = 0.0;
-    for (int q = 0; q < (int)(blockDim.x >> 5); ++q) sum += red[q][threadIdx.x];
+#pragma unroll
+    for (int q = 0; q < 4; ++q) sum += red[q][threadIdx.x];
     const int sh = threadIdx.x < 3 ? s1 : s2;
     atomicAdd(a.grad_orb + 3 * sh + threadIdx.x % 3, sum);
   }
 }
 
+// npair shell pairs; each block walks about four auxiliary shells per group
+// once the pairs alone fill the device
+template <int LA, int LB, int LC>
+inline void launch_grad3c_one(unsigned npair, cudaStream_t s, const Grad3cArgs& a) {
+  using S = GradShape<LA, LB, LC>;
+  if (S::smem > (size_t)48 << 10)
+    cudaFuncSetAttribute(grad3c_kernel<LA, LB, LC>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                         (int)S::smem);
+  const unsigned full = (unsigned)((a.aux_count + S::GPB - 1) / S::GPB);
+  const unsigned gy = (uint64_t)npair * full > 8 * 148 ? (full + 3) / 4 : full;
+  grad3c_kernel<LA, LB, LC><<<dim3(npair, gy), 128, S::smem, s>>>(a);
+}
+
 template <int LA, int LB>
-inline bool launch_grad3c_lc(int lc, dim3 grid, cudaStream_t s, const Grad3cArgs& a) {
+inline bool launch_grad3c_lc(int lc, unsigned npair, cudaStream_t s, const Grad3cArgs& a) {
   switch (lc) {
-    case 0: grad3c_kernel<LA, LB, 0><<<grid, 128, 0, s>>>(a); return true;
-    case 1: grad3c_kernel<LA, LB, 1><<<grid, 128, 0, s>>>(a); return true;
-    case 2: grad3c_kernel<LA, LB, 2><<<grid, 128, 0, s>>>(a); return true;
-    case 3: grad3c_kernel<LA, LB, 3><<<grid, 128, 0, s>>>(a); return true;
-    case 4: grad3c_kernel<LA, LB, 4><<<grid, 128, 0, s>>>(a); return true;
+    case 0: launch_grad3c_one<LA, LB, 0>(npair, s, a); return true;
+    case 1: launch_grad3c_one<LA, LB, 1>(npair, s, a); return true;
+    case 2: launch_grad3c_one<LA, LB, 2>(npair, s, a); return true;
+    case 3: launch_grad3c_one<LA, LB, 3>(npair, s, a); return true;
+    case 4: launch_grad3c_one<LA, LB, 4>(npair, s, a); return true;
     default: return false;
   }
 }
 
+// npp primitive pairs
 template <int LA, int LB>
-inline void launch_pair_deriv_t(unsigned blocks, cudaStream_t s, const PairDerivArgs& a) {
-  pair_deriv_kernel<LA, LB><<<blocks, 128, 0, s>>>(a);
+inline void launch_pair_deriv_t(int64_t npp, cudaStream_t s, const PairDerivArgs& a) {
+  constexpr int per = LA + LB <= 2 ? 4 : 1;
+  pair_deriv_kernel<LA, LB><<<(unsigned)((npp + per - 1) / per), 128, 0, s>>>(a);
 }
 
 #define DFJK_GRAD3C_DECL(A, B)                                                              \
-  bool launch_grad3c_##A##B(int lc, dim3 grid, cudaStream_t s, const Grad3cArgs& a);       \
-  void launch_pair_deriv_##A##B(unsigned blocks, cudaStream_t s, const PairDerivArgs& a);
+  bool launch_grad3c_##A##B(int lc, unsigned npair, cudaStream_t s, const Grad3cArgs& a);  \
+  void launch_pair_deriv_##A##B(int64_t npp, cudaStream_t s, const PairDerivArgs& a);
 DFJK_GRAD3C_DECL(0, 0)
 DFJK_GRAD3C_DECL(1, 0)
 DFJK_GRAD3C_DECL(1, 1)

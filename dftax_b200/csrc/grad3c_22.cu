@@ -3,12 +3,12 @@
 
 namespace dfjk {
 
-bool launch_grad3c_22(int lc, dim3 grid, cudaStream_t s, const Grad3cArgs& a) {
-  return launch_grad3c_lc<2, 2>(lc, grid, s, a);
+bool launch_grad3c_22(int lc, unsigned npair, cudaStream_t s, const Grad3cArgs& a) {
+  return launch_grad3c_lc<2, 2>(lc, npair, s, a);
 }
 
-void launch_pair_deriv_22(unsigned blocks, cudaStream_t s, const PairDerivArgs& a) {
-  launch_pair_deriv_t<2, 2>(blocks, s, a);
+void launch_pair_deriv_22(int64_t npp, cudaStream_t s, const PairDerivArgs& a) {
+  launch_pair_deriv_t<2, 2>(npp, s, a);
 }
 
 }  // namespace dfjk

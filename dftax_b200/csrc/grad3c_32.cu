@@ -3,12 +3,12 @@
 
 namespace dfjk {
 
-bool launch_grad3c_32(int lc, dim3 grid, cudaStream_t s, const Grad3cArgs& a) {
-  return launch_grad3c_lc<3, 2>(lc, grid, s, a);
+bool launch_grad3c_32(int lc, unsigned npair, cudaStream_t s, const Grad3cArgs& a) {
+  return launch_grad3c_lc<3, 2>(lc, npair, s, a);
 }
 
-void launch_pair_deriv_32(unsigned blocks, cudaStream_t s, const PairDerivArgs& a) {
-  launch_pair_deriv_t<3, 2>(blocks, s, a);
+void launch_pair_deriv_32(int64_t npp, cudaStream_t s, const PairDerivArgs& a) {
+  launch_pair_deriv_t<3, 2>(npp, s, a);
 }
 
 }  // namespace dfjk
