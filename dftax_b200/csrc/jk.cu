@@ -13,6 +13,7 @@
 // run them on the int8 tensor cores (ozaki.cu). J is float64 in both.
 // which are the P-gradients of dftax's DFCoulomb.energy (terms.py:592-613):
 // J = int3c (V+ gamma), K = einsum("mlP,PQ,nsQ,ls->mn") (hybrid.py:23-41).
+#include "dmma.cuh"
 #include "internal.h"
 
 #include <algorithm>
@@ -272,20 +273,6 @@ struct HtTile {
   static constexpr size_t smem = (size_t)kHtStages * kStage * sizeof(double);
 };
 
-__device__ __forceinline__ void dmma_8x8x4(double (&c)[2], double a, double b) {
-  asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};"
-               : "+d"(c[0]), "+d"(c[1])
-               : "d"(a), "d"(b));
-}
-
-__device__ __forceinline__ void cp_async16(void* smem, const void* gmem, bool valid) {
-  // src-size 0 fills the 16 shared bytes with zeros (gmem must still be a valid address)
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(
-                   static_cast<unsigned>(__cvta_generic_to_shared(smem))),
-               "l"(gmem), "r"(valid ? 16 : 0)
-               : "memory");
-}
-
 // The list of m is entries [kbeg[m], kend[m]) (kend == nullptr: up to
 // kbeg[m + 1]); entry e reads B row krow[e] - row0. accumulate: X += instead
 // of X = (a streamed plan sums the chunks of B rows). ldb and ncol are even,
@@ -346,24 +333,23 @@ __global__ void __launch_bounds__(256, 2) half_transform_kernel(
       cp_async16(Cs + k * PI + i, ok ? Cp + (int64_t)nn[j] * ncol + it + i : Cp, ok);
     }
   };
-  auto commit = [] { asm volatile("cp.async.commit_group;" ::: "memory"); };
   if (nch > 0) fetch(0);
   for (int c = 0; c < kHtStages - 1; ++c) {
     if (c < nch) {
       stage(c);
       if (c + 1 < nch) fetch(c + 1);
     }
-    commit();
+    cp_async_commit();
   }
   for (int c = 0; c < nch; ++c) {
     // chunk c has landed, and every warp is done with the buffer of chunk c - 1
-    asm volatile("cp.async.wait_group %0;" ::"n"(kHtStages - 2) : "memory");
+    cp_async_wait<kHtStages - 2>();
     __syncthreads();
     if (c + kHtStages - 1 < nch) {
       stage(c + kHtStages - 1);
       if (c + kHtStages < nch) fetch(c + kHtStages);
     }
-    commit();
+    cp_async_commit();
     const double* Bs = ht_smem + (c % kHtStages) * T::kStage;
     const double* Cs = Bs + kHtK * kHtPX;
 #pragma unroll
@@ -537,16 +523,15 @@ __global__ void __launch_bounds__(256, 2) syrk_part_kernel(const double* __restr
       }
     }
   };
-  auto commit = [] { asm volatile("cp.async.commit_group;" ::: "memory"); };
   for (int c = 0; c < kSyStages - 1; ++c) {
     if (c < nch) stage(c);
-    commit();
+    cp_async_commit();
   }
   for (int c = 0; c < nch; ++c) {
-    asm volatile("cp.async.wait_group %0;" ::"n"(kSyStages - 2) : "memory");
+    cp_async_wait<kSyStages - 2>();
     __syncthreads();
     if (c + kSyStages - 1 < nch) stage(c + kSyStages - 1);
-    commit();
+    cp_async_commit();
     if (!work) continue;
     const double* As = sy_smem + (size_t)(c % kSyStages) * (2 * kSyT * kSyK);
     const double* Bs = diag ? As : As + kSyT * kSyK;

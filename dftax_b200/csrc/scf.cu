@@ -52,6 +52,9 @@ struct dfscf {
   dfjk::DevBuf P, C, eps, F, J, K, Vxc, Cocc, wocc;
   dfjk::DevBuf dF, dE, A1, A2, Fo, work, info, vec;
   dfjk::DevBuf Fx;                                   // the DIIS Fock matrix of the iteration
+  // the caller's density and XC matrix of the evaluation entry points: the
+  // captured XC graph reads and writes these, whatever buffers a call brings
+  dfjk::DevBuf Pin, Vout;
   dfjk::DevBuf sp_X, sp_X2, sp_Z, sp_Y, sp_Q, sp_st, sp_info, sp_work;   // purification
   bool sp_have_Q = false;      // sp_Q holds the last occupied orbitals (X^T-basis)
   int sp_steps = 16;           // projection steps the last converged density took
@@ -313,6 +316,14 @@ double energy_fock(dfscf& f, const double* P, bool from_orbitals, double* Fout, 
   f.res.e_xc = e_xc;
   f.res.e_nn = f.e_nn;
   return e_one + e_coul + e_xc + f.e_nn;
+}
+
+// the caller's density in this handle's own buffer
+const double* stage_density(dfscf& f, const double* P, cudaStream_t s) {
+  const size_t b = (size_t)f.nao * f.nao * sizeof(double);
+  f.Pin.ensure(b);
+  DFJK_CUDA(cudaMemcpyAsync(f.Pin.p, P, b, cudaMemcpyDeviceToDevice, s));
+  return f.Pin.as<double>();
 }
 
 // orbitals of F into f.C / f.eps and (write_P) the aufbau density into f.P
@@ -619,8 +630,9 @@ void run(dfscf& f, const double* P0, cudaStream_t s) {
 }
 
 // Points per XC chunk, chosen by timing: the chunk size sets the shapes of the
-// two DGEMMs per chunk (G x nsig x nsig) and the launches per evaluation.
-// Candidates 2048, 4096, 8192 and 16384 points are timed on the core-guess
+// two products per chunk (G x nsig x nsig) and the launches per evaluation.
+// Candidates 2048 (from 2^16 points on: below, its chunks are too few functions
+// each to pay for their launches), 4096, 8192 and 16384 points are timed on the core-guess
 // density (three evaluations each: a direct one, the graph capture, and a
 // timed graph replay) for the first molecule of each (nao / 128, log2 points,
 // XC streams) bucket; the choice is kept for the process, so later molecules
@@ -647,6 +659,7 @@ void autotune_chunk(dfscf& f, const int (&nout)[8], const std::vector<double>& p
     double best_ms = INFINITY;
     for (int64_t G : {2048, 4096, 8192, 16384}) {
       if ((int64_t)6 * f.nao * G * 8 > ((int64_t)3 << 30)) continue;
+      if (G < 4096 && f.npts < ((int64_t)1 << 16)) continue;
       // as the SCF runs it: the first call launches directly, the second
       // captures the CUDA graph, the timed ones replay it
       xc_chunk(f.p->orb, nout, pv, G, f.o.ao_thresh, f.xcw);
@@ -915,8 +928,12 @@ dfjk_status dfscf_xc(dfscf* f, const double* P, double* exc, double* Vxc, void* 
                                   static_cast<cudaStream_t>(stream)));
       return;
     }
-    *exc = xc_energy_fock(*f->c, f->ov, f->pts.as<double>(), f->wts.as<double>(), P, Vxc,
-                          xc_params(*f), f->xcw, static_cast<cudaStream_t>(stream));
+    cudaStream_t s = static_cast<cudaStream_t>(stream);
+    const size_t b = (size_t)f->nao * f->nao * sizeof(double);
+    const double* Pd = stage_density(*f, P, s);
+    if (Vxc) f->Vout.ensure(b);
+    *exc = xc_energy_fock(*f->c, f->ov, f->pts.as<double>(), f->wts.as<double>(), Pd,
+                          Vxc ? f->Vout.as<double>() : nullptr, xc_params(*f), f->xcw, s, Vxc);
   });
 }
 
@@ -925,7 +942,7 @@ dfjk_status dfscf_energy_fock(dfscf* f, const double* P, double* e, double* F, v
   return guard(f->c, [&] {
     DFJK_CUDA(cudaSetDevice(f->c->device));
     cudaStream_t s = static_cast<cudaStream_t>(stream);
-    *e = energy_fock(*f, P, false, F ? F : f->A2.as<double>(), s);
+    *e = energy_fock(*f, stage_density(*f, P, s), false, F ? F : f->A2.as<double>(), s);
     DFJK_CUDA(cudaStreamSynchronize(s));
   });
 }

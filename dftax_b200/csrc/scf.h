@@ -37,22 +37,20 @@ struct XcChunks {
   std::vector<int> ao_cnt;
   int max_ao = 0;
   int64_t total_ao = 0;                // sum of ao_cnt (the dense form would be nchunk * nao)
-  double gemm_flop = 0.0;              // FLOP of one evaluation's two DGEMMs: sum 4 G ao_cnt^2
+  double gemm_flop = 0.0;              // FLOP of one evaluation's two products: sum 4 G ao_cnt^2
   DevBuf d_sh, d_sh_out0, d_ao_map;    // shells, their first compact AO, compact -> AO
 };
 
 // XC on a point grid (xc.cu)
 // The chunks of one XC evaluation run on kXcBranches concurrent branches
-// (chunk k on branch k % kXcBranches), each with its own buffers, and the
-// context's stream and cuBLAS handle of that branch (no shared GEMM
-// workspace), and its own V accumulator; one chunk's kernels fill only part
+// (chunk k on branch k % kXcBranches), each with its own buffers, the
+// context's stream of that branch and its own V accumulator; one chunk's kernels fill only part
 // of the GPU. The accumulators are summed in branch order at the end and the
 // energy partials are per chunk, so the result does not depend on how the
 // branches interleave.
 struct XcBranch {
-  DevBuf phi, dphi, X, W;       // [nsig][G] AO values, 3 gradients, Phi P, weighted AO
-  DevBuf Pc, Vc;                // P on a chunk's AOs, its V block
-  DevBuf vr, vg;                // per point: v_rho, v_grad (3)
+  DevBuf phi, dphi, W;          // [nsig][G] AO values, 3 gradients, weighted AO
+  DevBuf Pc, Vc;                // P on a chunk's AOs, the slices of its V block
 };
 
 struct XcWork {
@@ -94,11 +92,12 @@ struct XcParams {
 // E_xc of the closed-shell density P (nao x nao, symmetric, device) and, when
 // Vxc != nullptr, its P-gradient symmetrized (device, nao x nao), over the grid
 // points pts [n][3] with weights w [n] (device, in xc_prepare's order), chunk
-// by chunk as ws.ch lays them out. Uses the context's cuBLAS handle on
-// stream s. Returns E_xc (host synchronizing).
+// by chunk as ws.ch lays them out, on the context's branch streams forked from
+// and joined to s. Returns E_xc (host synchronizing); Vcopy, when given,
+// receives a copy of Vxc before that.
 double xc_energy_fock(const Context& c, const OrbView& ov, const double* pts, const double* w,
                       const double* P, double* Vxc, const XcParams& xp, XcWork& ws,
-                      cudaStream_t s);
+                      cudaStream_t s, double* Vcopy = nullptr);
 
 // Becke cell weights: w[i] = raw[i] * P_owner(i) / sum_A P_A at point i
 void launch_becke_partition(const double* pts, const int* owner, const double* raw, int64_t n,

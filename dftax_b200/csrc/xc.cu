@@ -6,21 +6,23 @@
 //                                per point and shell, points fastest, so the
 //                                stores of a warp are contiguous), as
 //                                dftax/energy/gto.py:371-412 evaluates them;
-//   X = Phi P                    cuBLAS DGEMM;
-//   rho_g = sum_mu X Phi, grad rho_g = 2 sum_mu X dPhi        (rho_kernel);
+//   X = Phi P on the float64 tensor cores, kept in registers;
+//   rho_g = sum_mu X Phi, grad rho_g = 2 sum_mu X dPhi;
 //   e_g = w rho eps_xc(rho, grad rho) and its derivatives v_rho, v_grad by
 //   forward-mode dual numbers over the same expression as dftax's PBE
 //   (xc.py:87-252, PBE0 :584-601; points with rho <= 1e-10 contribute nothing,
 //   as the double-where of grid.py:31-44 makes them);
-//   W = v_rho/2 Phi + v_grad . dPhi, V += Phi^T W               (cuBLAS DGEMM);
+//   W = v_rho/2 Phi + v_grad . dPhi                    (all of it: rho_w_kernel)
+//   V += Phi^T W on the float64 tensor cores                       (v_kernel);
 // and at the end Vxc = V + V^T, the symmetrized P-gradient of E_xc
 // (scf.py:42-46). The chunks run on kXcBranches concurrent streams (chunk k
 // on branch k % kXcBranches, one V accumulator each, summed in branch order
 // at the end); the energy is summed per block in a fixed order and then over
 // blocks on the host, so the result is reproducible. The SCF calls this with
 // the same buffers every iteration: the second call captures its launches
-// (about eight per chunk, the branches forked and joined by events) in a
+// (about seven per chunk, the branches forked and joined by events) in a
 // CUDA graph and later calls replay it.
+#include "dmma.cuh"
 #include "md_device.cuh"
 #include "scf.h"
 
@@ -33,8 +35,6 @@ namespace dfjk {
 namespace {
 
 constexpr int kAoThreads = 128;
-constexpr size_t kXcBlasWorkspace = (size_t)8 << 20;   // per XC branch cuBLAS handle
-constexpr int kPtThreads = 256;
 
 // ---------------------------------------------------------------------------
 // Becke partition
@@ -182,81 +182,26 @@ __global__ void __launch_bounds__(kAoThreads) ao_kernel(OrbView ov, const int* _
   ao_shell<L>(ov, s, dx, dy, dz, live, o, G, plane, phi, dphi);
 }
 
-// Pc[k1][k2] = P[map[k1]][map[k2]]
+// Pc[k1][k2] = P[map[k1]][map[k2]], rows of ldp (nsig rounded up to even: the
+// copies of rho_w_kernel are 16 bytes wide), zero in the padding
 __global__ void gather_p_kernel(const double* __restrict__ P, int nao, const int* __restrict__ map,
-                                int nsig, double* __restrict__ Pc) {
+                                int nsig, int ldp, double* __restrict__ Pc) {
   const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  if (i >= (int64_t)nsig * nsig) return;
-  const int64_t a = i / nsig, b = i % nsig;
-  Pc[i] = P[(int64_t)map[a] * nao + map[b]];
+  if (i >= (int64_t)nsig * ldp) return;
+  const int64_t a = i / ldp, b = i % ldp;
+  Pc[i] = b < nsig ? P[(int64_t)map[a] * nao + map[b]] : 0.0;
 }
 
-// V[map[k1]][map[k2]] += Vc[k1][k2] (column-major Vc; the map is one-to-one)
-__global__ void scatter_v_kernel(const double* __restrict__ Vc, int nsig, const int* __restrict__ map,
-                                 int nao, double* __restrict__ V) {
+// V[map[k1]][map[k2]] += sum_z part[z][k1][k2], slices in order (the map is
+// one-to-one; V + V^T is taken at the end, so the product's order does not matter)
+__global__ void scatter_v_kernel(const double* __restrict__ part, int nslice, int nsig,
+                                 const int* __restrict__ map, int nao, double* __restrict__ V) {
   const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  if (i >= (int64_t)nsig * nsig) return;
-  const int64_t a = i % nsig, b = i / nsig;
-  V[(int64_t)map[b] * nao + map[a]] += Vc[i];
-}
-
-// rho[g] = sum_mu X Phi, grad[x][g] = 2 sum_mu X dPhi_x. A block takes 16
-// points with 16 lanes of mu each (mu = lane, lane + 16, ...: a warp reads 16
-// consecutive points of two mu rows), so an 8192-point chunk fills 512
-// blocks; the 16 partial sums are added in a fixed order, so the result does
-// not depend on the launch.
-// rho and grad rho of 2 kRhoPairs points per block: each thread takes two
-// neighbouring points (16-byte loads; G is a multiple of 256, so the pair
-// stays inside the chunk, and the padding points hold zeros) and every
-// kRhoLanes-th function from ml, two functions per step; the kRhoLanes
-// partial sums are added in a fixed order
-constexpr int kRhoPairs = 16, kRhoLanes = 16;
-__global__ void __launch_bounds__(kRhoPairs * kRhoLanes) rho_kernel(
-    const double* __restrict__ X, const double* __restrict__ phi, const double* __restrict__ dphi,
-    int nao, int64_t G, int64_t ng, double* __restrict__ rho, double* __restrict__ grad) {
-  __shared__ double2 red[4][kRhoLanes][kRhoPairs];
-  const int gi = threadIdx.x % kRhoPairs, ml = threadIdx.x / kRhoPairs;
-  const int64_t g = 2 * (blockIdx.x * (int64_t)kRhoPairs + gi);
-  const int64_t plane = (int64_t)nao * G;
-  double2 r = {0.0, 0.0}, a = {0.0, 0.0}, b = {0.0, 0.0}, c = {0.0, 0.0};
-  auto ld2 = [](const double* p) { return *reinterpret_cast<const double2*>(p); };
-  auto acc = [&](int64_t o) {
-    const double2 x = ld2(X + o), f = ld2(phi + o), dx = ld2(dphi + o),
-                  dy = ld2(dphi + plane + o), dz = ld2(dphi + 2 * plane + o);
-    r.x += x.x * f.x;
-    r.y += x.y * f.y;
-    a.x += x.x * dx.x;
-    a.y += x.y * dx.y;
-    b.x += x.x * dy.x;
-    b.y += x.y * dy.y;
-    c.x += x.x * dz.x;
-    c.y += x.y * dz.y;
-  };
-  if (g < ng) {
-    int mu = ml;
-    for (; mu + kRhoLanes < nao; mu += 2 * kRhoLanes) {
-      acc((int64_t)mu * G + g);
-      acc((int64_t)(mu + kRhoLanes) * G + g);
-    }
-    if (mu < nao) acc((int64_t)mu * G + g);
-  }
-  red[0][ml][gi] = r;
-  red[1][ml][gi] = a;
-  red[2][ml][gi] = b;
-  red[3][ml][gi] = c;
-  __syncthreads();
-  if (ml < 4 && g < ng) {
-    double2 t = {0.0, 0.0};
-#pragma unroll
-    for (int q = 0; q < kRhoLanes; ++q) {
-      t.x += red[ml][q][gi].x;
-      t.y += red[ml][q][gi].y;
-    }
-    const double f = ml == 0 ? 1.0 : 2.0;
-    double* out = ml == 0 ? rho : grad + (ml - 1) * G;
-    out[g] = f * t.x;
-    if (g + 1 < ng) out[g + 1] = f * t.y;
-  }
+  const int64_t nn = (int64_t)nsig * nsig;
+  if (i >= nn) return;
+  double s = 0.0;
+  for (int z = 0; z < nslice; ++z) s += part[z * nn + i];
+  V[(int64_t)map[i / nsig] * nao + map[i % nsig]] += s;
 }
 
 // ---------------------------------------------------------------------------
@@ -365,24 +310,136 @@ __device__ D4 pbe_eps(D4 rho, D4 gx, D4 gy, D4 gz, double xs, double cs) {
   return xs * ex + cs * (eps_pw + H);
 }
 
-// per point: rho, grad in, v_rho, v_grad out (in place); e per block
-__global__ void __launch_bounds__(kPtThreads) pbe_kernel(double* __restrict__ rho,
-                                                         double* __restrict__ grad,
-                                                         const double* __restrict__ w, int64_t G,
-                                                         int64_t ng, double xs, double cs,
-                                                         double thresh, double* __restrict__ ered) {
-  __shared__ double red[kPtThreads];
-  const int64_t g = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  double e = 0.0;
-  if (g < ng) {
-    const double r = rho[g];
-    double vr = 0.0, v0 = 0.0, v1 = 0.0, v2 = 0.0;
-    if (r > thresh) {
+// One block: 64 points of a chunk, everything between the AO values and V.
+//   * X = Phi Pc for all nsig functions, 64 columns at a time, on the float64
+//     tensor cores: 16 functions per step through a four-stage cp.async ring
+//     that runs on across the column blocks (the order of points and columns
+//     inside a fragment is free: a lane's pair of fragments is one 16-byte load);
+//   * after each column block the lane's X meets Phi and dPhi of the same
+//     (point, function) pairs and adds to rho and grad rho; X is never stored;
+//   * the partial sums of a point's lanes are added in a fixed order, 64 threads
+//     evaluate the functional, and the block writes W for its points while
+//     their Phi and dPhi are still in the caches.
+// As five launches per chunk (DGEMM, density, functional, weights, with X and
+// the density arrays in memory between them) (H2O)_6 took 1523 us per
+// evaluation, its DGEMMs at 7-11 TFLOP/s on 165 functions.
+constexpr int kRpPts = 64, kRpCols = 64, kRpK = 16, kRpPitch = 68, kRpStages = 4;
+constexpr int kRpStage = 2 * kRpK * kRpPitch;   // doubles
+constexpr size_t kRpSmem = (size_t)kRpStages * kRpStage * sizeof(double);
+
+__global__ void __launch_bounds__(256, 2) rho_w_kernel(
+    const double* __restrict__ Pc, int ldp, const double* __restrict__ phi,
+    const double* __restrict__ dphi, int nsig, int64_t G, const double* __restrict__ w, int64_t ng,
+    double xs, double cs, double thresh, double* __restrict__ W, double* __restrict__ ered) {
+  extern __shared__ __align__(16) double rsm[];
+  __shared__ double red[2][4][kRpPts];   // per column half: rho, grad
+  __shared__ double sv[4][kRpPts];       // v_rho / 2, v_grad (weighted)
+  __shared__ double se[kRpPts];
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int wx = (warp & 3) * 16, wi = (warp >> 2) * 32;
+  const int fr = lane >> 2, fk = lane & 3;
+  const int64_t g0 = blockIdx.x * (int64_t)kRpPts;
+  const int64_t plane = (int64_t)nsig * G;
+  const int nk = (nsig + kRpK - 1) / kRpK, ncb = (nsig + kRpCols - 1) / kRpCols;
+  const int steps = nk * ncb;
+  const int bk = tid >> 5, bx = 2 * (tid & 31);
+  auto stage = [&](int q) {
+    double* As = rsm + (q % kRpStages) * kRpStage;
+    double* Bs = As + kRpK * kRpPitch;
+    const int k0 = q % nk * kRpK, c = q / nk * kRpCols + bx;
+#pragma unroll
+    for (int j = 0; j < 2; ++j) {
+      const int k = k0 + bk + 8 * j;
+      const bool in = k < nsig, inc = in && c < ldp;
+      cp_async16(As + (bk + 8 * j) * kRpPitch + bx, in ? phi + k * G + g0 + bx : phi, in);
+      cp_async16(Bs + (bk + 8 * j) * kRpPitch + bx, inc ? Pc + (int64_t)k * ldp + c : Pc, inc);
+    }
+  };
+  for (int q = 0; q < kRpStages - 1; ++q) {
+    if (q < steps) stage(q);
+    cp_async_commit();
+  }
+  double acc[2][4][2], sum[4][2];   // sum: rho, grad of the lane's two points
+#pragma unroll
+  for (int a = 0; a < 2; ++a)
+#pragma unroll
+    for (int b = 0; b < 4; ++b) acc[a][b][0] = acc[a][b][1] = 0.0;
+#pragma unroll
+  for (int d = 0; d < 4; ++d) sum[d][0] = sum[d][1] = 0.0;
+  for (int q = 0; q < steps; ++q) {
+    cp_async_wait<kRpStages - 2>();
+    __syncthreads();
+    if (q + kRpStages - 1 < steps) stage(q + kRpStages - 1);
+    cp_async_commit();
+    const double* As = rsm + (q % kRpStages) * kRpStage;
+    const double* Bs = As + kRpK * kRpPitch;
+    if (q / nk * kRpCols + wi < nsig) {   // else the warp's columns lie past the functions
+#pragma unroll
+      for (int kk = 0; kk < kRpK; kk += 4) {
+        const double2 av = *reinterpret_cast<const double2*>(As + (kk + fk) * kRpPitch + wx + 2 * fr);
+        const double af[2] = {av.x, av.y};
+        double bf[4];
+#pragma unroll
+        for (int b = 0; b < 4; b += 2) {
+          const double2 v =
+              *reinterpret_cast<const double2*>(Bs + (kk + fk) * kRpPitch + wi + 8 * b + 2 * fr);
+          bf[b] = v.x;
+          bf[b + 1] = v.y;
+        }
+#pragma unroll
+        for (int a = 0; a < 2; ++a)
+#pragma unroll
+          for (int b = 0; b < 4; ++b) dmma_8x8x4(acc[a][b], af[a], bf[b]);
+      }
+    }
+    if (q % nk == nk - 1) {
+      // fragment (a, b), register r: point wx + 2 (lane / 4) + a, column
+      // wi + 8 (b & ~1) + 4 (lane % 4) + 2 r + (b & 1)
+      const int c0 = q / nk * kRpCols + wi;
+      const double* at = phi + g0 + wx + 2 * fr;
+      const double* dat = dphi + g0 + wx + 2 * fr;
+#pragma unroll
+      for (int b = 0; b < 4; ++b)
+#pragma unroll
+        for (int r = 0; r < 2; ++r) {
+          const int c = c0 + 8 * (b & ~1) + 4 * fk + 2 * r + (b & 1);
+          if (c < nsig) {
+            const double x0 = acc[0][b][r], x1 = acc[1][b][r];
+            const double2 f = __ldg(reinterpret_cast<const double2*>(at + c * G));
+            sum[0][0] += x0 * f.x;
+            sum[0][1] += x1 * f.y;
+#pragma unroll
+            for (int d = 0; d < 3; ++d) {
+              const double2 v = __ldg(reinterpret_cast<const double2*>(dat + d * plane + c * G));
+              sum[1 + d][0] += x0 * v.x;
+              sum[1 + d][1] += x1 * v.y;
+            }
+          }
+          acc[0][b][r] = acc[1][b][r] = 0.0;
+        }
+    }
+  }
+  // the four lanes of a point, then the two column halves
+#pragma unroll
+  for (int d = 0; d < 4; ++d)
+#pragma unroll
+    for (int a = 0; a < 2; ++a) {
+      double s = sum[d][a];
+      s += __shfl_xor_sync(0xffffffffu, s, 1);
+      s += __shfl_xor_sync(0xffffffffu, s, 2);
+      if (fk == 0) red[warp >> 2][d][wx + 2 * fr + a] = s;
+    }
+  __syncthreads();
+  if (tid < kRpPts) {
+    const int64_t g = g0 + tid;
+    double e = 0.0, vr = 0.0, v0 = 0.0, v1 = 0.0, v2 = 0.0;
+    const double r = red[0][0][tid] + red[1][0][tid];
+    if (g < ng && r > thresh) {
       const double wg = w[g];
       const D4 R = {r, {1.0, 0.0, 0.0, 0.0}};
-      const D4 X = {grad[g], {0.0, 1.0, 0.0, 0.0}};
-      const D4 Y = {grad[G + g], {0.0, 0.0, 1.0, 0.0}};
-      const D4 Z = {grad[2 * G + g], {0.0, 0.0, 0.0, 1.0}};
+      const D4 X = {2.0 * (red[0][1][tid] + red[1][1][tid]), {0.0, 1.0, 0.0, 0.0}};
+      const D4 Y = {2.0 * (red[0][2][tid] + red[1][2][tid]), {0.0, 0.0, 1.0, 0.0}};
+      const D4 Z = {2.0 * (red[0][3][tid] + red[1][3][tid]), {0.0, 0.0, 0.0, 1.0}};
       const D4 f = R * pbe_eps(R, X, Y, Z, xs, cs);
       e = wg * f.v;
       vr = wg * f.d[0];
@@ -390,33 +447,124 @@ __global__ void __launch_bounds__(kPtThreads) pbe_kernel(double* __restrict__ rh
       v1 = wg * f.d[2];
       v2 = wg * f.d[3];
     }
-    rho[g] = vr;
-    grad[g] = v0;
-    grad[G + g] = v1;
-    grad[2 * G + g] = v2;
+    se[tid] = e;
+    sv[0][tid] = 0.5 * vr;
+    sv[1][tid] = v0;
+    sv[2][tid] = v1;
+    sv[3][tid] = v2;
   }
-  red[threadIdx.x] = e;
   __syncthreads();
-  for (int o = kPtThreads / 2; o > 0; o >>= 1) {
-    if ((int)threadIdx.x < o) red[threadIdx.x] += red[threadIdx.x + o];
-    __syncthreads();
+  if (warp == 0) {
+    double e = se[lane] + se[lane + 32];
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) e += __shfl_xor_sync(0xffffffffu, e, o);
+    if (lane == 0) ered[blockIdx.x] = e;
   }
-  if (threadIdx.x == 0) ered[blockIdx.x] = red[0];
+  if (!W) return;
+  // W[mu][g] = v_rho/2 Phi + v_grad . dPhi: two points per lane, a function per warp
+  double2 v[4];
+#pragma unroll
+  for (int d = 0; d < 4; ++d) v[d] = make_double2(sv[d][2 * lane], sv[d][2 * lane + 1]);
+#pragma unroll 2
+  for (int c = warp; c < nsig; c += 8) {
+    const int64_t o = c * G + g0 + 2 * lane;
+    const double2 f = __ldg(reinterpret_cast<const double2*>(phi + o));
+    double2 s = make_double2(v[0].x * f.x, v[0].y * f.y);
+#pragma unroll
+    for (int d = 0; d < 3; ++d) {
+      const double2 t = __ldg(reinterpret_cast<const double2*>(dphi + d * plane + o));
+      s.x += v[1 + d].x * t.x;
+      s.y += v[1 + d].y * t.y;
+    }
+    *reinterpret_cast<double2*>(W + o) = s;
+  }
 }
 
-// W[mu][g] = v_rho/2 Phi + v_grad . dPhi (zero past ng)
-__global__ void w_kernel(const double* __restrict__ phi, const double* __restrict__ dphi,
-                         const double* __restrict__ vr, const double* __restrict__ vg, int nao,
-                         int64_t G, int64_t ng, double* __restrict__ W) {
-  const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  const int64_t plane = (int64_t)nao * G;
-  if (i >= plane) return;
-  const int64_t g = i % G;
-  double v = 0.0;
-  if (g < ng)
-    v = 0.5 * vr[g] * phi[i] + vg[g] * dphi[i] + vg[G + g] * dphi[plane + i] +
-        vg[2 * G + g] * dphi[2 * plane + i];
-  W[i] = v;
+// part[z][mu][nu] = sum_g Phi[mu][g] W[nu][g] over slice z of kVSlice points:
+// 64 x 64 tiles on the float64 tensor cores, both operands staged as they lie
+// (16 points a step, the 16-byte piece index xor 4 (row % 2): load phases of
+// two rows x four pieces fall in distinct banks; the point order inside a step
+// is free) through a four-stage cp.async ring with one barrier per step. The
+// output is small and the sum long, so slices fill the device; 512 points keep
+// a block's prologue and partial store near a tenth of its products.
+constexpr int kVT = 64, kVK = 16, kVStages = 4, kVSlice = 512;
+constexpr size_t kVSmem = (size_t)kVStages * 2 * kVT * kVK * sizeof(double);
+
+__global__ void __launch_bounds__(256, 2) v_kernel(const double* __restrict__ phi,
+                                                   const double* __restrict__ W, int nsig, int64_t G,
+                                                   double* __restrict__ part) {
+  extern __shared__ __align__(16) double vsm[];
+  const int r0 = blockIdx.x * kVT, c0 = blockIdx.y * kVT;
+  const int64_t k0 = blockIdx.z * (int64_t)kVSlice;
+  const int64_t k1 = k0 + kVSlice < G ? k0 + kVSlice : G;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int wr = (warp & 3) * 16, wc = (warp >> 2) * 32;
+  const int fr = lane >> 2, fk = lane & 3;
+  const bool work = r0 + wr < nsig && c0 + wc < nsig;
+  double acc[2][4][2];
+#pragma unroll
+  for (int a = 0; a < 2; ++a)
+#pragma unroll
+    for (int b = 0; b < 4; ++b) acc[a][b][0] = acc[a][b][1] = 0.0;
+  const int nst = (int)((k1 - k0) / kVK);   // G and the slices are multiples of 16
+  const int sr = tid >> 3, sp = tid & 7;
+  auto stage = [&](int q) {
+    double* As = vsm + (size_t)(q % kVStages) * (2 * kVT * kVK);
+    const int64_t k = k0 + (int64_t)q * kVK + 2 * sp;
+#pragma unroll
+    for (int j = 0; j < 2; ++j) {
+      const int r = sr + 32 * j, o = r * kVK + 2 * (sp ^ (4 * (r & 1)));
+      const bool oa = r0 + r < nsig, ob = c0 + r < nsig;
+      cp_async16(As + o, oa ? phi + (int64_t)(r0 + r) * G + k : phi, oa);
+      cp_async16(As + kVT * kVK + o, ob ? W + (int64_t)(c0 + r) * G + k : W, ob);
+    }
+  };
+  for (int q = 0; q < kVStages - 1; ++q) {
+    if (q < nst) stage(q);
+    cp_async_commit();
+  }
+  for (int q = 0; q < nst; ++q) {
+    cp_async_wait<kVStages - 2>();
+    __syncthreads();
+    if (q + kVStages - 1 < nst) stage(q + kVStages - 1);
+    cp_async_commit();
+    if (!work) continue;
+    const double* As = vsm + (size_t)(q % kVStages) * (2 * kVT * kVK);
+    const double* Bs = As + kVT * kVK;
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      const int piece = 2 * ((4 * h + fk) ^ (4 * (fr & 1)));
+      double2 af[2], bf[4];
+#pragma unroll
+      for (int a = 0; a < 2; ++a)
+        af[a] = *reinterpret_cast<const double2*>(As + (wr + 8 * a + fr) * kVK + piece);
+#pragma unroll
+      for (int b = 0; b < 4; ++b)
+        bf[b] = *reinterpret_cast<const double2*>(Bs + (wc + 8 * b + fr) * kVK + piece);
+#pragma unroll
+      for (int a = 0; a < 2; ++a)
+#pragma unroll
+        for (int b = 0; b < 4; ++b) dmma_8x8x4(acc[a][b], af[a].x, bf[b].x);
+#pragma unroll
+      for (int a = 0; a < 2; ++a)
+#pragma unroll
+        for (int b = 0; b < 4; ++b) dmma_8x8x4(acc[a][b], af[a].y, bf[b].y);
+    }
+  }
+  if (!work) return;
+  double* out = part + blockIdx.z * (int64_t)nsig * nsig;
+#pragma unroll
+  for (int a = 0; a < 2; ++a) {
+    const int r = r0 + wr + 8 * a + fr;
+    if (r >= nsig) continue;
+#pragma unroll
+    for (int b = 0; b < 4; ++b)
+#pragma unroll
+      for (int q = 0; q < 2; ++q) {
+        const int c = c0 + wc + 8 * b + 2 * fk + q;
+        if (c < nsig) out[(int64_t)r * nsig + c] = acc[a][b][q];
+      }
+  }
 }
 
 // out = sum over the nb branch accumulators V_b (n x n, stride n*n) of
@@ -660,17 +808,12 @@ static void xc_enqueue(const Context& c, const OrbView& ov, const double* pts, c
   const XcChunks& ch = ws.ch;
   const int64_t G = ch.G;
   const int64_t nchunk = (int64_t)ch.g0.size();
-  const int64_t nblk = (G + kPtThreads - 1) / kPtThreads;
-  const double one = 1.0, zero = 0.0;
+  const int64_t nblk = G / kRpPts;
+  const int nslice = (int)((G + kVSlice - 1) / kVSlice);
   const int nb = std::min(std::max(ws.nbr, 1), kXcBranches);
   // fork: every branch starts after the caller's prior work on s
   DFJK_CUDA(cudaEventRecord(c.xc_fork, s));
-  for (int q = 0; q < nb; ++q) {
-    DFJK_CUDA(cudaStreamWaitEvent(c.xc_stream[q], c.xc_fork, 0));
-    DFJK_CUBLAS(cublasSetStream(c.xc_blas[q], c.xc_stream[q]));
-    // (setting the stream resets the workspace: give it back each time)
-    DFJK_CUBLAS(cublasSetWorkspace(c.xc_blas[q], c.xc_ws[q].p, kXcBlasWorkspace));
-  }
+  for (int q = 0; q < nb; ++q) DFJK_CUDA(cudaStreamWaitEvent(c.xc_stream[q], c.xc_fork, 0));
   if (Vxc)
     for (int q = 0; q < nb; ++q)
       DFJK_CUDA(cudaMemsetAsync(ws.Vacc.as<double>() + q * nn, 0, nn * sizeof(double),
@@ -678,16 +821,14 @@ static void xc_enqueue(const Context& c, const OrbView& ov, const double* pts, c
   for (int64_t k = 0; k < nchunk; ++k) {
     XcBranch& b = ws.br[k % nb];
     cudaStream_t bs = c.xc_stream[k % nb];
-    cublasHandle_t blas = c.xc_blas[k % nb];
     double* Vacc = ws.Vacc.as<double>() + (k % nb) * nn;
     const int64_t g0 = ch.g0[k], ng = ch.ng[k];
-    const int nsig = ch.ao_cnt[k], nsh = ch.sh_cnt[k];
+    const int nsig = ch.ao_cnt[k], ldp = nsig + (nsig & 1);
     const int* map = ch.d_ao_map.as<int>() + ch.ao_off[k];
     if (nsig == 0) {
       DFJK_CUDA(cudaMemsetAsync(ws.ered.as<double>() + k * nblk, 0, nblk * sizeof(double), bs));
       continue;
     }
-    const int64_t plane = (int64_t)nsig * G;
     // the chunk's shells are grouped by l: one launch per l present
     int j0 = ch.sh_off[k];
     for (int l = 0; l < kXcMaxL + 1; ++l) {
@@ -707,33 +848,22 @@ static void xc_enqueue(const Context& c, const OrbView& ov, const double* pts, c
       DFJK_LAUNCHED();
       j0 += cnt;
     }
-    (void)nsh;
-    gather_p_kernel<<<(unsigned)(((int64_t)nsig * nsig + 255) / 256), 256, 0, bs>>>(
-        P, nao, map, nsig, b.Pc.as<double>());
+    gather_p_kernel<<<(unsigned)(((int64_t)nsig * ldp + 255) / 256), 256, 0, bs>>>(
+        P, nao, map, nsig, ldp, b.Pc.as<double>());
     DFJK_LAUNCHED();
-    // X (G x nsig, column-major: [k][g]) = Phi Pc
-    DFJK_CUBLAS(cublasDgemm(blas, CUBLAS_OP_N, CUBLAS_OP_N, (int)G, nsig, nsig, &one,
-                            b.phi.as<double>(), (int)G, b.Pc.as<double>(), nsig, &zero,
-                            b.X.as<double>(), (int)G));
-    rho_kernel<<<(unsigned)((ng + 2 * kRhoPairs - 1) / (2 * kRhoPairs)), kRhoPairs * kRhoLanes, 0, bs>>>(
-        b.X.as<double>(), b.phi.as<double>(), b.dphi.as<double>(), nsig, G, ng,
-        b.vr.as<double>(), b.vg.as<double>());
-    DFJK_LAUNCHED();
-    pbe_kernel<<<(unsigned)nblk, kPtThreads, 0, bs>>>(b.vr.as<double>(), b.vg.as<double>(),
-                                                      w + g0, G, ng, xp.x_scale, xp.c_scale,
-                                                      xp.rho_thresh, ws.ered.as<double>() + k * nblk);
+    rho_w_kernel<<<(unsigned)nblk, 256, kRpSmem, bs>>>(
+        b.Pc.as<double>(), ldp, b.phi.as<double>(), b.dphi.as<double>(), nsig, G, w + g0, ng,
+        xp.x_scale, xp.c_scale, xp.rho_thresh, Vxc ? b.W.as<double>() : nullptr,
+        ws.ered.as<double>() + k * nblk);
     DFJK_LAUNCHED();
     if (Vxc) {
-      w_kernel<<<(unsigned)((plane + 255) / 256), 256, 0, bs>>>(
-          b.phi.as<double>(), b.dphi.as<double>(), b.vr.as<double>(), b.vg.as<double>(), nsig,
-          G, ng, b.W.as<double>());
+      // Vc = Phi^T W by slices, scattered into this branch's V
+      const unsigned nt = (unsigned)((nsig + kVT - 1) / kVT);
+      v_kernel<<<dim3(nt, nt, (unsigned)nslice), 256, kVSmem, bs>>>(
+          b.phi.as<double>(), b.W.as<double>(), nsig, G, b.Vc.as<double>());
       DFJK_LAUNCHED();
-      // Vc = Phi^T W, scattered into this branch's V
-      DFJK_CUBLAS(cublasDgemm(blas, CUBLAS_OP_T, CUBLAS_OP_N, nsig, nsig, (int)G, &one,
-                              b.phi.as<double>(), (int)G, b.W.as<double>(), (int)G, &zero,
-                              b.Vc.as<double>(), nsig));
       scatter_v_kernel<<<(unsigned)(((int64_t)nsig * nsig + 255) / 256), 256, 0, bs>>>(
-          b.Vc.as<double>(), nsig, map, nao, Vacc);
+          b.Vc.as<double>(), nslice, nsig, map, nao, Vacc);
       DFJK_LAUNCHED();
     }
   }
@@ -751,33 +881,31 @@ static void xc_enqueue(const Context& c, const OrbView& ov, const double* pts, c
 
 double xc_energy_fock(const Context& c, const OrbView& ov, const double* pts, const double* w,
                       const double* P, double* Vxc, const XcParams& xp, XcWork& ws,
-                      cudaStream_t s) {
+                      cudaStream_t s, double* Vcopy) {
   const int nao = ov.nao;
   const XcChunks& ch = ws.ch;
   const int64_t G = ch.G;
   const int64_t nchunk = (int64_t)ch.g0.size();
-  const int64_t nblk = (G + kPtThreads - 1) / kPtThreads;
+  const int64_t nblk = G / kRpPts;   // G is a multiple of 256
   const int64_t plane_max = (int64_t)std::max(ch.max_ao, 1) * G;
-  const size_t sq = (size_t)std::max(ch.max_ao, 1) * std::max(ch.max_ao, 1) * sizeof(double);
+  const size_t mx = (size_t)std::max(ch.max_ao, 1);
+  const size_t nslice = (size_t)((G + kVSlice - 1) / kVSlice);
   for (int q = 0; q < std::min(std::max(ws.nbr, 1), kXcBranches); ++q) {
     XcBranch& b = ws.br[q];
     b.phi.ensure(plane_max * sizeof(double));
     b.dphi.ensure(3 * plane_max * sizeof(double));
-    b.X.ensure(plane_max * sizeof(double));
     b.W.ensure(plane_max * sizeof(double));
-    b.Pc.ensure(sq);
-    b.Vc.ensure(sq);
-    b.vr.ensure(G * sizeof(double));
-    b.vg.ensure(3 * G * sizeof(double));
+    b.Pc.ensure(mx * (mx + 1) * sizeof(double));
+    if (Vxc) b.Vc.ensure(nslice * mx * mx * sizeof(double));
   }
-  // the context's branch streams, events and handles are made here on first
-  // use, never during a capture
+  DFJK_CUDA(cudaFuncSetAttribute(rho_w_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kRpSmem));
+  DFJK_CUDA(cudaFuncSetAttribute(v_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kVSmem));
+  // the context's branch streams and events are made here on first use, never
+  // during a capture
   Context& cx = const_cast<Context&>(c);
   for (int q = 0; q < kXcBranches; ++q) {
     if (!cx.xc_stream[q]) DFJK_CUDA(cudaStreamCreateWithFlags(&cx.xc_stream[q], cudaStreamNonBlocking));
     if (!cx.xc_done[q]) DFJK_CUDA(cudaEventCreateWithFlags(&cx.xc_done[q], cudaEventDisableTiming));
-    if (!cx.xc_blas[q]) DFJK_CUBLAS(cublasCreate(&cx.xc_blas[q]));
-    cx.xc_ws[q].ensure(kXcBlasWorkspace);
   }
   if (!cx.xc_fork) DFJK_CUDA(cudaEventCreateWithFlags(&cx.xc_fork, cudaEventDisableTiming));
   ws.ered.ensure((size_t)std::max<int64_t>(nchunk, 1) * nblk * sizeof(double));
@@ -788,8 +916,7 @@ double xc_energy_fock(const Context& c, const OrbView& ov, const double* pts, co
     DFJK_CUDA(cudaGraphLaunch(ws.exec, s));
     count_launch(ws.graph_kernels);
   } else if (!ws.graph_off && ws.calls > 0 && Vxc) {
-    // capture this call's work (the buffers above are already sized, and the
-    // first, direct call let cuBLAS set up its workspace outside capture)
+    // capture this call's work (the buffers above are already sized)
     if (ws.exec) {
       DFJK_CUDA(cudaGraphExecDestroy(ws.exec));
       ws.exec = nullptr;
@@ -829,6 +956,9 @@ double xc_energy_fock(const Context& c, const OrbView& ov, const double* pts, co
     xc_enqueue(c, ov, pts, w, P, Vxc, xp, ws, s);
   }
   ++ws.calls;
+  if (Vcopy && Vxc)
+    DFJK_CUDA(cudaMemcpyAsync(Vcopy, Vxc, (size_t)nao * nao * sizeof(double),
+                              cudaMemcpyDeviceToDevice, s));
   std::vector<double> e((size_t)nchunk * nblk);
   if (!e.empty())
     DFJK_CUDA(cudaMemcpyAsync(e.data(), ws.ered.p, e.size() * sizeof(double),

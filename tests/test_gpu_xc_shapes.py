@@ -1,0 +1,41 @@
+"""XC energy and matrix at the sizes where the quadrature kernels' tiles end:
+point counts around the 64-point blocks and 512-point slices, chunks of 256 to
+8192 points, 30 to 114 functions (one and two 64-column blocks, even and odd
+counts), with and without the matrix, against the oracle's dense quadrature.
+
+Tolerance: sums of up to 5000 x 114^2 float64 products, 2^-53 * sqrt of that
+< 1e-12 relative.
+"""
+
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+REL = 1e-12
+
+
+@pytest.mark.parametrize("name,npts,chunk", [("water", 1, 256), ("water", 63, 256), ("water", 65, 512),
+                                             ("water3", 1000, 256), ("water3", 4097, 768),
+                                             ("alkane1", 5000, 8192), ("alkane2", 2500, 2048)])
+def test_xc_shapes(name, npts, chunk):
+    import torch
+
+    from dftax_b200 import df, systems
+    from dftax_b200.ks import KS
+    from oracle import ks as oks
+
+    sym, xyz, orb, aux, nocc = systems.workload(name, seed=1)
+    rng = np.random.default_rng(npts)
+    pts = xyz[rng.integers(0, len(xyz), npts)] + rng.standard_normal((npts, 3))
+    w = rng.uniform(0.01, 0.1, npts)
+    ks = KS(sym, xyz, orb, coulomb=df(aux), grid=(pts, w), grid_chunk=chunk)
+    C = systems.random_occupied(orb.nao, nocc, seed=3)
+    P = 2.0 * C @ C.T
+    e0, V0 = oks.exc_and_vxc(orb, pts, w, P)
+    for _ in range(3):   # direct, captured, replayed; the caller's buffers change
+        e, V = ks.xc_energy(torch.as_tensor(P, device="cuda"))
+        assert abs(e - e0) <= REL * abs(e0)
+        assert np.linalg.norm(V.cpu().numpy() - V0) <= REL * np.linalg.norm(V0)
+    e1, none = ks.xc_energy(P, want_fock=False)
+    assert none is None and abs(e1 - e0) <= REL * abs(e0)
