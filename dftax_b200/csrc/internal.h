@@ -131,6 +131,9 @@ void ozaki_prepare_c(Plan& p, const double* Cp, int64_t nsel, cudaStream_t s);
 void ozaki_k1(Plan& p, int64_t nsel, int64_t x0, int64_t n, double* X, cudaStream_t s);
 void ozaki_syrk(Plan& p, const double* X, int64_t kt, double sign, bool beta0, double* K,
                 cudaStream_t s);
+// error flag of the tensor-core pipeline since ozaki_prepare_c (one host
+// synchronization per K)
+void ozaki_check_k(Plan& p, cudaStream_t s);
 
 // ---- 3-center row chunks (api.cu) ----
 int64_t chunk_budget(const Plan& p);   // bytes of one chunk of 3-center rows

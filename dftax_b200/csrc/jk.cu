@@ -720,6 +720,7 @@ static void k_accumulate(Plan& p, const double* C, int64_t sm, int64_t sc, const
     p.timer.mark(kPhKsyrk, s);
     beta0 = false;
   }
+  if (p.opts.precision == DFJK_MIXED && !p.opts.streamed) ozaki_check_k(p, s);
 }
 
 static void k_compute(Plan& p, const double* C, const double* w, int64_t ncol, double* K,

@@ -429,14 +429,27 @@ void ozaki_prepare_c(Plan& p, const double* Cp, int64_t nsel, cudaStream_t s) {
   DFJK_CUDA(cudaMemsetAsync(p.ws_oz_err.p, 0, sizeof(int), s));
 }
 
-// X[m][x - x0][i] (float64, ld n * nsel) for fitted directions [x0, x0 + n)
+// Tile of occupied columns of the half transform: an MMA is bound by the 128 +
+// BN operand rows it reads from shared memory, and every tile streams all B_x
+// planes, so the width with the smallest tiles x (128 + BN) is taken (42
+// columns: 48; 82: one tile of 96; 100: two of 64; 160: two of 80).
+static OzakiShape half_shape(int64_t nsel) {
+  OzakiShape best = kOzHalf;
+  int64_t cost = INT64_MAX;
+  for (OzakiShape q : {kOzHalf48, kOzHalf64, kOzHalf, kOzHalfWide}) {
+    const int64_t bn = ozaki_shape(q).bn, c = (nsel + bn - 1) / bn * (128 + bn);
+    if (c < cost) {
+      cost = c;
+      best = q;
+    }
+  }
+  return best;
+}
+
+// X[m][x - x0][i] (float64, ld n * nsel, nsel even) for fitted directions [x0, x0 + n)
 void ozaki_k1(Plan& p, int64_t nsel, int64_t x0, int64_t n, double* X, cudaStream_t s) {
   constexpr int ND = kOzKDigits;
-  // every tile of occupied columns streams all B_x planes: take 96-column
-  // tiles when they need fewer tiles than 80-column ones (81 columns: 1, not 2)
-  const int64_t t80 = (nsel + ozaki_shape(kOzHalf).bn - 1) / ozaki_shape(kOzHalf).bn;
-  const int64_t t96 = (nsel + ozaki_shape(kOzHalfWide).bn - 1) / ozaki_shape(kOzHalfWide).bn;
-  const OzakiShape shape = t96 < t80 ? kOzHalfWide : kOzHalf;
+  const OzakiShape shape = half_shape(nsel);
   const OzakiShapeInfo sh = ozaki_shape(shape);
   const int bk = sh.box_k;
   const int64_t nao = p.nao, nao_p = p.nao_p16;
@@ -460,33 +473,70 @@ void ozaki_k1(Plan& p, int64_t nsel, int64_t x0, int64_t n, double* X, cudaStrea
   a.batch_stride_out = nsel;
   a.err = p.ws_oz_err.as<int>();
   // several fitted directions per CTA (one TMEM allocation and one copy ring
-  // for all of them) while the grid still fills the device four times over
+  // for all of them), at most 32: the count whose waves x (directions + 1, a
+  // CTA's setup and last epilogue) is smallest, so that the last wave is full
+  // (14 directions left C10H22 at 4.3 waves of 148 CTAs, 15 make 4)
   int sm = 148;
   cudaDeviceGetAttribute(&sm, cudaDevAttrMultiProcessorCount, p.ctx->device);
   const int64_t tiles = ((nsel + sh.bn - 1) / sh.bn) * ((nao + 127) / 128);
-  a.zper = (int)std::max<int64_t>(1, std::min<int64_t>(16, tiles * n / (4 * (int64_t)sm)));
+  int64_t best = INT64_MAX;
+  a.zper = 1;
+  for (int64_t z = 32; z >= 1; --z) {
+    const int64_t t = (tiles * ((n + z - 1) / z) + sm - 1) / sm * (z + 1);
+    if (t < best) {
+      best = t;
+      a.zper = (int)z;
+    }
+  }
   const int64_t zstep = (int64_t)65535 * a.zper;
   for (int64_t z0 = 0; z0 < n; z0 += zstep) {
     const int64_t nz = std::min<int64_t>(zstep, n - z0);
     a.plane0 = (int)(x0 + z0);
     a.out = X + z0 * nsel;
-    // X[m][z][i] leaves through TMA tensor stores when its strides allow
-    a.tma_out = ozaki_out_mappable(a.out, a.batch_stride_out, a.ld_out) ? 1 : 0;
-    if (a.tma_out) ozaki_map_out(&maps.out, a.out, nsel, nz, nao, a.batch_stride_out, a.ld_out);
+    // X[m][z][i] leaves through TMA tensor stores
+    ozaki_map_out(&maps.out, a.out, nsel, nz, nao, a.batch_stride_out, a.ld_out);
     ozaki_launch(shape, maps, a, (int)nz, s);
   }
-  check_oz_err(p, s);
+}
+
+void ozaki_check_k(Plan& p, cudaStream_t s) { check_oz_err(p, s); }
+
+// Slice (k bytes) of K = X X^T over kt values: one block per SM works on a
+// (tile, slice), so the slices are as many as make waves x (k tiles of a slice
+// + 14, a block's setup and epilogue in k tiles) smallest, none above kOzSlice.
+// Slices of 8192 gave 1.4 waves for C10H22 (301 us) and one block for (H2O)_3
+// (141 us).
+static int64_t syrk_slice(int64_t kt, int64_t nao, int dev) {
+  const OzakiShapeInfo sh = ozaki_shape(kOzSyrk);
+  int sm = 148;
+  cudaDeviceGetAttribute(&sm, cudaDevAttrMultiProcessorCount, dev);
+  int64_t tiles = 0;
+  for (int64_t m0 = 0; m0 < nao; m0 += 128)
+    tiles += (std::min(nao, m0 + 128) + sh.bn - 1) / sh.bn;
+  const int64_t ktiles = (kt + sh.box_k - 1) / sh.box_k;
+  const int64_t least = (kt + kOzSlice - 1) / kOzSlice;
+  const int64_t most = std::max(least, std::min<int64_t>(std::max<int64_t>(1, ktiles / 2), 2 * least + 32));
+  int64_t best = INT64_MAX, slice = kOzSlice;
+  for (int64_t q = least; q <= most; ++q) {
+    const int64_t per = (ktiles + q - 1) / q;
+    const int64_t t = (tiles * q + sm - 1) / sm * (per + 14);
+    if (t < best) {
+      best = t;
+      slice = per * sh.box_k;
+    }
+  }
+  return slice;
 }
 
 // K (+)= sign * X X^T for one chunk of X (nao x kt, row-major): k in slices of
-// kOzSlice bytes, each with its own row exponents and its own float64 partial
+// syrk_slice bytes, each with its own row exponents and its own float64 partial
 // (full square, exactly symmetric: both triangles come from the same integer
 // sums), then summed in a fixed order, so K is bit-reproducible.
 void ozaki_syrk(Plan& p, const double* X, int64_t kt, double sign, bool beta0, double* K,
                 cudaStream_t s) {
   constexpr int ND = kOzSDigits;
-  constexpr int64_t KS = kOzSlice;
-  static_assert(KS <= kOzMaxK, "a k slice must stay within the exact int32 range");
+  static_assert(kOzSlice <= kOzMaxK, "a k slice must stay within the exact int32 range");
+  const int64_t KS = syrk_slice(kt, p.nao, p.ctx->device);
   const OzakiShapeInfo sh = ozaki_shape(kOzSyrk);
   const int bk = sh.box_k;
   const int64_t nao = p.nao;
@@ -527,7 +577,6 @@ void ozaki_syrk(Plan& p, const double* X, int64_t kt, double sign, bool beta0, d
   reduce_slices_kernel<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(p.ws_oz_kp.as<double>(), nsl,
                                                                    nao, sign, beta0 ? 1 : 0, K);
   DFJK_LAUNCHED();
-  check_oz_err(p, s);
 }
 
 }  // namespace dfjk

@@ -17,13 +17,16 @@ constexpr int kOzMaxDigits = 7;
 constexpr int64_t kOzMaxK = 32640;
 // 7 digits: order 6 sums 2*65*128 + 5*128*128 = 98560 per k, below 2^31 for k <= 21788
 constexpr int64_t kOzMaxK7 = 21788;
-constexpr int64_t kOzSlice = 8192;  // k bytes per slice of the K = X X^T product
+constexpr int64_t kOzSlice = 8192;  // most k bytes per slice of the K = X X^T product
 
 // The products and the tile shape each one runs with (ozaki_gemm.cu).
-// kOzHalfWide: the half transform with 96 occupied columns per tile, used when
-// it needs fewer tiles than 80 columns would (each tile streams every B_x plane)
+// kOzHalf48 / kOzHalf64 / kOzHalf / kOzHalfWide: the half transform with 48, 64,
+// 80 or 96 occupied columns per tile (half_shape in ozaki.cu)
 // kOzBuild64: the build product of float64 plans, 7 digits on SM pairs
-enum OzakiShape { kOzBuild = 0, kOzHalf = 1, kOzSyrk = 2, kOzHalfWide = 3, kOzBuild64 = 4 };
+enum OzakiShape {
+  kOzBuild = 0, kOzHalf = 1, kOzSyrk = 2, kOzHalfWide = 3, kOzBuild64 = 4, kOzHalf48 = 5,
+  kOzHalf64 = 6
+};
 
 // digits per value of the build product B = (ij|P) L of a plan
 inline int build_digits(const Plan& p) {
@@ -38,7 +41,7 @@ OzakiShapeInfo ozaki_shape(OzakiShape shape);
 struct OzakiMaps {
   CUtensorMap a[kOzMaxDigits];   // A digit planes, box (box_k, 128 rows, 1)
   CUtensorMap b[kOzMaxDigits];   // B digit planes, box (box_k, box_b rows, 1)
-  CUtensorMap out;               // float64 output when tma_out: box (16, 1, 32), 128-byte swizzle
+  CUtensorMap out;               // float64 output (all but K = X X^T): box (16, 1, 32), 128-byte swizzle
 };
 
 struct OzakiArgs {
@@ -55,7 +58,6 @@ struct OzakiArgs {
   int* err;                // set non-zero when a bounded wait gives up
   int zper;                // batches per CTA (one TMEM allocation, one ring); 0 or 1: one
   int zcount;              // batches of the launch (set by ozaki_launch)
-  int tma_out;             // half transform: 1 writes through maps.out (the build product always does)
   int lower;               // 1: tiles wholly above the diagonal (n0 > m0 + 127) are skipped
 };
 
@@ -64,9 +66,8 @@ struct OzakiArgs {
 void ozaki_map(CUtensorMap* m, const void* base, int64_t d0, int64_t d1, int64_t d2,
                int64_t stride1, int64_t stride2, int box_k, int box1);
 
-// float64 output map over [rows][batches][cols] (strides in elements), and
-// whether a base and strides allow one (16-byte alignment)
-bool ozaki_out_mappable(const double* base, int64_t batch_stride, int64_t ld);
+// float64 output map over [rows][batches][cols] (strides in elements; base and
+// strides multiples of 16 bytes)
 void ozaki_map_out(CUtensorMap* m, double* base, int64_t cols, int64_t batches, int64_t rows,
                    int64_t batch_stride, int64_t ld);
 

@@ -17,11 +17,10 @@
 //
 // Tiles: 128 (m) x BN (n) x BK (k, bytes), K-major operands, TMA with the
 // BK-byte swizzle into an ST-stage mbarrier ring (ND digit planes per operand
-// per stage). Two shapes are compiled: ND 4, BK 64, BN 80, three 52 KB stages
-// and 64 KB of output staging for TMA stores (K half transform: n = occupied
-// orbitals, 160 = 2 x 80 for (H2O)_32), and
-// ND 5, BK 64, BN 96, three 70 KB stages (K = X X^T; 5 x 96 of the 512 TMEM
-// columns). The build product runs on SM pairs (ozaki_gemm_i8_pair below,
+// per stage). The K half transform (n = occupied orbitals) runs ND 4, BK 64 with
+// BN 48, 64, 80 (three stages of 45-52 KB) or 96 (two) and 64 KB of output
+// staging for TMA stores; K = X X^T runs ND 5, BK 64, BN 96, three 70 KB stages
+// (5 x 96 of the 512 TMEM columns). The build product runs on SM pairs (ozaki_gemm_i8_pair below,
 // M = 256, four 55 KB stages). Warp 0 lane 0 issues
 // copies, warp 1 lane 0 issues MMAs (BK/32 per digit pair per k tile), and
 // eight warps drain tensor memory (warps w and w + 4 own rows 32 (w % 4) ..
@@ -167,12 +166,18 @@ __device__ __forceinline__ double scale_pow2(double x, int e) {
 // 2^53 and so exact as a float64 (order 0 < 2^28, the others < 2^31), and one
 // FMA joins them with a single rounding.
 template <int ND>
+__device__ __forceinline__ long long combine_int(const uint32_t (&v)[ND][16], int j) {
+  static_assert(ND <= 5, "the int64 sum of more orders would overflow");
+  long long s = (int)v[0][j];
+#pragma unroll
+  for (int o = 1; o < ND; ++o) s = s * 256 + (int)v[o][j];
+  return s;
+}
+
+template <int ND>
 __device__ __forceinline__ double combine_orders(const uint32_t (&v)[ND][16], int j, int e) {
   if constexpr (ND <= 5) {
-    long long s = (int)v[0][j];
-#pragma unroll
-    for (int o = 1; o < ND; ++o) s = s * 256 + (int)v[o][j];
-    return scale_pow2((double)s, e - 14 - 8 * (ND - 1));
+    return scale_pow2((double)combine_int<ND>(v, j), e - 14 - 8 * (ND - 1));
   } else {
     static_assert(ND <= 8, "the low part holds at most four orders");
     long long hi = (int)v[0][j];
@@ -196,16 +201,12 @@ __device__ __forceinline__ void tma_store_3d(const CUtensorMap* map, uint32_t sr
 
 // one lane's 128-byte row of a 32 x 16 float64 block in shared memory, in the
 // 128-byte swizzle of the output tensor maps (16-byte chunk j at j ^ (row % 8))
-template <int ND>
-__device__ __forceinline__ void stage_row(uint8_t* buf, int lane, const uint32_t (&v)[ND][16],
-                                          int era, const int* ecol) {
+template <class F>
+__device__ __forceinline__ void stage_row(uint8_t* buf, int lane, F value) {
 #pragma unroll
-  for (int j = 0; j < 16; j += 2) {
-    const double r0 = combine_orders<ND>(v, j, era + ecol[j]);
-    const double r1 = combine_orders<ND>(v, j + 1, era + ecol[j + 1]);
+  for (int j = 0; j < 16; j += 2)
     *reinterpret_cast<double2*>(buf + lane * 128 + (((j >> 1) ^ (lane & 7)) << 4)) =
-        make_double2(r0, r1);
-  }
+        make_double2(value(j), value(j + 1));
 }
 
 template <int ND, int BK, int BN, int ST, bool TOUT>
@@ -356,25 +357,47 @@ __global__ void __launch_bounds__(320, 1) ozaki_gemm_i8(const __grid_constant__ 
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
       const int bz = a.b_batched ? a.plane0 + z : 0;
       const int era = row < a.M ? a.ea[(int64_t)(a.plane0 + z) * a.ea_stride + row] : 0;
-      double* orow = a.out + (int64_t)z * a.batch_stride_out + (int64_t)row * a.ld_out;
       const int* ebz = a.eb + (int64_t)bz * a.eb_stride;
-      for (int c = 16 * h; c < BN; c += 32) {
-        uint32_t v[ND][16];
+      auto release = [&] {
+        asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+        __syncwarp();
+        if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(drained)) : "memory");
+      };
+      if constexpr (TOUT) {
+        // the accumulators first, combined to one int64 per value in registers:
+        // the next batch's MMAs start while these are scaled and stored (with
+        // the release after the stores, MMAs and epilogue took turns: 12 us
+        // per 128 x 80 tile of (H2O)_32 instead of the MMAs' 8)
+        constexpr int NCH = (BN / 16 + 1) / 2;   // this warp's 16-column chunks
+        long long acc[NCH][16];
 #pragma unroll
-        for (int o = 0; o < ND; ++o) tmem_ld16_issue(trow + (uint32_t)o * ACC + c, v[o]);
-        tmem_ld_wait();
+        for (int i = 0; i < NCH; ++i) {
+          const int c = 16 * h + 32 * i;
+          if (c >= BN) break;
+          uint32_t v[ND][16];
 #pragma unroll
-        for (int o = 0; o < ND; ++o) reg_fence16(v[o]);
-        if constexpr (TOUT) {
+          for (int o = 0; o < ND; ++o) tmem_ld16_issue(trow + (uint32_t)o * ACC + c, v[o]);
+          tmem_ld_wait();
+#pragma unroll
+          for (int o = 0; o < ND; ++o) reg_fence16(v[o]);
+#pragma unroll
+          for (int j = 0; j < 16; ++j) acc[i][j] = combine_int<ND>(v, j);
+        }
+        release();
+#pragma unroll
+        for (int i = 0; i < NCH; ++i) {
+          const int c = 16 * h + 32 * i;
+          if (c >= BN) break;
           // columns past N read exponent 0; the tensor map clips them and rows past M
-          int ecol[16];
-#pragma unroll
-          for (int j = 0; j < 16; ++j) ecol[j] = n0 + c + j < a.N ? ebz[n0 + c + j] : 0;
           uint8_t* buf = stg + (uint32_t)((warp - 2) * 2 + (nst & 1)) * 4096;
           // the block handed over two chunks ago has been read out of this buffer
           if (lane == 0) asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory");
           __syncwarp();
-          stage_row<ND>(buf, lane, v, era, ecol);
+          stage_row(buf, lane, [&](int j) {
+            const int col = n0 + c + j;
+            const int e = era + (col < a.N ? ebz[col] : 0);
+            return scale_pow2((double)acc[i][j], e - 14 - 8 * (ND - 1));
+          });
           asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
           __syncwarp();
           if (lane == 0) {
@@ -382,7 +405,16 @@ __global__ void __launch_bounds__(320, 1) ozaki_gemm_i8(const __grid_constant__ 
             asm volatile("cp.async.bulk.commit_group;" ::: "memory");
           }
           ++nst;
-        } else {
+        }
+      } else {
+        double* orow = a.out + (int64_t)z * a.batch_stride_out + (int64_t)row * a.ld_out;
+        for (int c = 16 * h; c < BN; c += 32) {
+          uint32_t v[ND][16];
+#pragma unroll
+          for (int o = 0; o < ND; ++o) tmem_ld16_issue(trow + (uint32_t)o * ACC + c, v[o]);
+          tmem_ld_wait();
+#pragma unroll
+          for (int o = 0; o < ND; ++o) reg_fence16(v[o]);
           if (row >= a.M) continue;
 #pragma unroll
           for (int j = 0; j < 16; ++j) {
@@ -391,10 +423,8 @@ __global__ void __launch_bounds__(320, 1) ozaki_gemm_i8(const __grid_constant__ 
             orow[col] = combine_orders<ND>(v, j, era + ebz[col]);
           }
         }
+        release();
       }
-      asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-      __syncwarp();
-      if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(drained)) : "memory");
     }
     // the staging blocks must be read out before the CTA's shared memory goes
     if (TOUT && lane == 0) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
@@ -617,7 +647,7 @@ __global__ void __launch_bounds__(320, 1) ozaki_gemm_i8_pair(const __grid_consta
 #pragma unroll
         for (int o = 0; o < ND; ++o) reg_fence16(v[o]);
         uint8_t* buf = stg + (uint32_t)(c / 16) * STG;
-        stage_row<ND>(buf, lane, v, era, ebs + c);
+        stage_row(buf, lane, [&](int j) { return combine_orders<ND>(v, j, era + ebs[c + j]); });
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
         __syncwarp();
         if (lane == 0) {
@@ -717,6 +747,8 @@ void launch_pair(const OzakiMaps& maps, const OzakiArgs& a, cudaStream_t s) {
 // the n tile
 OzakiShapeInfo ozaki_shape(OzakiShape shape) {
   switch (shape) {
+    case kOzHalf48: return {kOzKDigits, 64, 48, 3, 48};
+    case kOzHalf64: return {kOzKDigits, 64, 64, 3, 64};
     case kOzHalf: return {kOzKDigits, 64, 80, 3, 80};
     case kOzHalfWide: return {kOzKDigits, 64, 96, 2, 96};
     case kOzBuild: return {kOzBDigits, 64, 96, 4, 48};
@@ -743,14 +775,9 @@ void ozaki_map(CUtensorMap* m, const void* base, int64_t d0, int64_t d1, int64_t
   if (r != CUDA_SUCCESS) fail(DFJK_ERR_CUDA, "cuTensorMapEncodeTiled failed (%d)", (int)r);
 }
 
-bool ozaki_out_mappable(const double* base, int64_t batch_stride, int64_t ld) {
-  return !(reinterpret_cast<uintptr_t>(base) & 15) && (batch_stride * 8) % 16 == 0 &&
-         (ld * 8) % 16 == 0;
-}
-
 void ozaki_map_out(CUtensorMap* m, double* base, int64_t cols, int64_t batches, int64_t rows,
                    int64_t batch_stride, int64_t ld) {
-  if (!ozaki_out_mappable(base, batch_stride, ld))
+  if ((reinterpret_cast<uintptr_t>(base) & 15) || (batch_stride * 8) % 16 || (ld * 8) % 16)
     fail(DFJK_ERR_INVALID, "output tensor map: base or strides not 16-byte aligned");
   cuuint64_t dims[3] = {(cuuint64_t)cols, (cuuint64_t)batches, (cuuint64_t)rows};
   cuuint64_t strides[2] = {(cuuint64_t)(batch_stride * 8), (cuuint64_t)(ld * 8)};
@@ -768,15 +795,11 @@ void ozaki_launch(OzakiShape shape, const OzakiMaps& maps, const OzakiArgs& a, i
   static_assert(kOzKDigits == 4 && kOzBDigits == 5 && kOzSDigits == 5 && kOzB64Digits == 7,
                 "the compiled shapes follow the digit counts");
   switch (shape) {
-    case kOzHalf:
-      if (a.tma_out) launch<4, 64, 80, 3, true>(maps, a, grid_z, s);
-      else launch<4, 64, 80, 3, false>(maps, a, grid_z, s);
-      return;
-    case kOzHalfWide:
-      // two stages: three would not leave room for the output staging
-      if (a.tma_out) launch<4, 64, 96, 2, true>(maps, a, grid_z, s);
-      else launch<4, 64, 96, 2, false>(maps, a, grid_z, s);
-      return;
+    case kOzHalf48: launch<4, 64, 48, 3, true>(maps, a, grid_z, s); return;
+    case kOzHalf64: launch<4, 64, 64, 3, true>(maps, a, grid_z, s); return;
+    case kOzHalf: launch<4, 64, 80, 3, true>(maps, a, grid_z, s); return;
+    // two stages: three would not leave room for the output staging
+    case kOzHalfWide: launch<4, 64, 96, 2, true>(maps, a, grid_z, s); return;
     case kOzBuild:
       if (grid_z != 1) fail(DFJK_ERR_INVALID, "the two-SM build product takes one batch");
       launch_pair<5, 64, 96, 4>(maps, a, s);
