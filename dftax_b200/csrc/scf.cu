@@ -55,6 +55,7 @@ struct dfscf {
   // the caller's density and XC matrix of the evaluation entry points: the
   // captured XC graph reads and writes these, whatever buffers a call brings
   dfjk::DevBuf Pin, Vout;
+  dfjk::DevBuf dots;                                 // results of a batch of dot products
   dfjk::DevBuf sp_X, sp_X2, sp_Z, sp_Y, sp_Q, sp_st, sp_info, sp_work;   // purification
   bool sp_have_Q = false;      // sp_Q holds the last occupied orbitals (X^T-basis)
   int sp_steps = 16;           // projection steps the last converged density took
@@ -231,11 +232,50 @@ struct PartTimer {
   }
 };
 
-double ddot(Context& c, const double* a, const double* b, int64_t n, cudaStream_t s) {
-  double r = 0.0;
-  DFJK_CUBLAS(cublasSetStream(c.cublas, s));
-  DFJK_CUBLAS(cublasDdot(c.cublas, (int)n, a, 1, b, 1, &r));
-  return r;
+// Dot products out[k] = sum_i a[k][i] b[k][i] of n values, one block each (a
+// fixed order); the host reads the results of a batch at once. (One cuBLAS dot
+// per product, each waited for, took 2 ms of a (H2O)_3 solve.)
+constexpr int kDotsMax = 8;
+struct DotList {
+  const double* a[kDotsMax];
+  const double* b[kDotsMax];
+};
+
+__global__ void __launch_bounds__(1024) dots_kernel(DotList l, int64_t n, double* __restrict__ out) {
+  __shared__ double red[32];
+  const double* a = l.a[blockIdx.x];
+  const double* b = l.b[blockIdx.x];
+  double s = 0.0;
+#pragma unroll 4
+  for (int64_t i = threadIdx.x; i < n; i += 1024) s += a[i] * b[i];
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = s;
+  __syncthreads();
+  if (threadIdx.x < 32) {
+    s = red[threadIdx.x];
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+    if (threadIdx.x == 0) out[blockIdx.x] = s;
+  }
+}
+
+// enqueues `count` dots into f.dots and their copy to host[0 .. count - 1],
+// valid after the next synchronization of s
+void dots(dfscf& f, const std::vector<std::pair<const double*, const double*>>& ab, int64_t n,
+          double* host, cudaStream_t s) {
+  f.dots.ensure(ab.size() * sizeof(double));
+  for (size_t k0 = 0; k0 < ab.size(); k0 += kDotsMax) {
+    DotList l{};
+    const size_t c = std::min<size_t>(kDotsMax, ab.size() - k0);
+    for (size_t k = 0; k < c; ++k) {
+      l.a[k] = ab[k0 + k].first;
+      l.b[k] = ab[k0 + k].second;
+    }
+    dots_kernel<<<(unsigned)c, 1024, 0, s>>>(l, n, f.dots.as<double>() + k0);
+    DFJK_LAUNCHED();
+  }
+  DFJK_CUDA(cudaMemcpyAsync(host, f.dots.p, ab.size() * sizeof(double), cudaMemcpyDeviceToHost, s));
 }
 
 void gemm(Context& c, cublasOperation_t ta, cublasOperation_t tb, int m, int n, int k,
@@ -278,8 +318,9 @@ double energy_fock(dfscf& f, const double* P, bool from_orbitals, double* Fout, 
   Context& c = *f.c;
   const int64_t n = f.nao, nn = n * n;
   const double hf = f.o.hf_coeff;
-  double e_coul;
   PartTimer tm(s);
+  double d[3] = {0.0, 0.0, 0.0};   // Tr(P H), Tr(P J), Tr(P K)
+  double e_coul = 0.0;
   if (from_orbitals) {
     // C_occ row-major [nao][nocc] for the plan's J/K; weight 2 per orbital
     const double one = 1.0, zero = 0.0;
@@ -288,20 +329,24 @@ double energy_fock(dfscf& f, const double* P, bool from_orbitals, double* Fout, 
                             f.nao, &zero, f.C.as<double>(), f.nocc, f.Cocc.as<double>(), f.nocc));
     jk_compute(*f.p, f.Cocc.as<double>(), f.wocc.as<double>(), f.nocc, f.J.as<double>(),
                hf != 0.0 ? f.K.as<double>() : nullptr, s);
-    e_coul = 0.5 * ddot(c, P, f.J.as<double>(), nn, s);
-    if (hf != 0.0) e_coul -= 0.25 * hf * ddot(c, P, f.K.as<double>(), nn, s);
     fock_kernel<<<blocks(nn), 256, 0, s>>>(f.H.as<double>(), f.J.as<double>(),
                                            hf != 0.0 ? f.K.as<double>() : nullptr, nullptr,
                                            -0.5 * hf, nn, Fout);
     DFJK_LAUNCHED();
+    std::vector<std::pair<const double*, const double*>> ab{{P, f.H.as<double>()},
+                                                            {P, f.J.as<double>()}};
+    if (hf != 0.0) ab.push_back({P, f.K.as<double>()});
+    dots(f, ab, nn, d, s);
   } else {
     // the plan's DFCoulomb energy and gradient (J - a_x/2 K) of any symmetric P
     e_coul = energy(*f.p, P, 1, hf, 0.0, f.J.as<double>(), s);
     fock_kernel<<<blocks(nn), 256, 0, s>>>(f.H.as<double>(), f.J.as<double>(), nullptr, nullptr,
                                            0.0, nn, Fout);
     DFJK_LAUNCHED();
+    dots(f, {{P, f.H.as<double>()}}, nn, d, s);
   }
-  tm.add(f.res.ms_jk);
+  tm.add(f.res.ms_jk);   // (synchronizes: the dots have arrived)
+  if (from_orbitals) e_coul = 0.5 * d[1] - 0.25 * hf * d[2];
   double e_xc = 0.0;
   if (has_xc(f)) {
     e_xc = xc_energy_fock(c, f.ov, f.pts.as<double>(), f.wts.as<double>(), P, f.Vxc.as<double>(),
@@ -310,12 +355,11 @@ double energy_fock(dfscf& f, const double* P, bool from_orbitals, double* Fout, 
     DFJK_LAUNCHED();
     tm.add(f.res.ms_xc);
   }
-  const double e_one = ddot(c, P, f.H.as<double>(), nn, s);
-  f.res.e_one = e_one;
+  f.res.e_one = d[0];
   f.res.e_coul = e_coul;
   f.res.e_xc = e_xc;
   f.res.e_nn = f.e_nn;
-  return e_one + e_coul + e_xc + f.e_nn;
+  return d[0] + e_coul + e_xc + f.e_nn;
 }
 
 // the caller's density in this handle's own buffer
@@ -357,21 +401,13 @@ void make_density_eig(dfscf& f, const double* Fm, cudaStream_t s, bool write_P =
 
 constexpr int kSp2Max = 96;     // projection steps before giving up (no gap)
 
-// The aufbau density of F by SP2 purification into f.P, with C_occ (only
-// the occupied columns of f.C). Returns false, with f.P untouched, when the
-// projection does not converge to a rank-nocc projector.
-bool sp2_density(dfscf& f, const double* Fm, cudaStream_t s) {
+// The projection launched step by step (a DGEMM and an update kernel each):
+// matrices too large for the one-launch form. X ends in Xb[the result].
+int sp2_steps(dfscf& f, double* const (&Xb)[2], double* Z, double* st, bool* done, double* t1_last,
+              cudaStream_t s) {
   Context& c = *f.c;
-  PartTimer tm(s);
-  const int n = f.nao, m = f.nmo, k = f.nocc;
+  const int m = f.nmo, k = f.nocc;
   const int64_t mm = (int64_t)m * m;
-  gemm(c, CUBLAS_OP_N, CUBLAS_OP_N, n, m, n, 1.0, Fm, n, f.X.as<double>(), n, 0.0, f.A1.as<double>(),
-       n, s);
-  gemm(c, CUBLAS_OP_T, CUBLAS_OP_N, m, m, n, 1.0, f.X.as<double>(), n, f.A1.as<double>(), n, 0.0,
-       f.Fo.as<double>(), m, s);
-  double* Xb[2] = {f.sp_X.as<double>(), f.sp_X2.as<double>()};
-  double* Z = f.sp_Z.as<double>();
-  double* st = f.sp_st.as<double>();   // [0..1] bounds, then 3 per step
   gershgorin_kernel<<<1, 1024, 0, s>>>(f.Fo.as<double>(), m, st);
   DFJK_LAUNCHED();
   sp2_init_kernel<<<blocks(mm), 256, 0, s>>>(f.Fo.as<double>(), m, st, Xb[0]);
@@ -384,10 +420,9 @@ bool sp2_density(dfscf& f, const double* Fm, cudaStream_t s) {
   // host check comes after as many steps as the last converged projection
   // took (the spectra of consecutive iterations are alike), then every 4.
   std::vector<double> hs(3 * kSp2Max);
-  double e1 = INFINITY, e2 = INFINITY, t1_last = 0.0;
-  bool done = false;
+  double e1 = INFINITY, e2 = INFINITY;
   int it = 0, cur = 0;
-  while (it < kSp2Max && !done) {
+  while (it < kSp2Max && !*done) {
     const int g = std::min(it == 0 ? std::max(f.sp_steps, 4) : 4, kSp2Max - it);
     for (int j = 0; j < g; ++j) {
       gemm(c, CUBLAS_OP_N, CUBLAS_OP_N, m, m, m, 1.0, Xb[cur], m, Xb[cur], m, 0.0, Z, m, s);
@@ -400,15 +435,15 @@ bool sp2_density(dfscf& f, const double* Fm, cudaStream_t s) {
                               cudaMemcpyDeviceToHost, s));
     DFJK_CUDA(cudaStreamSynchronize(s));
     bool bad = false;
-    for (int j = 0; j < g && !done; ++j) {
+    for (int j = 0; j < g && !*done; ++j) {
       const double e = std::fabs(hs[3 * j] - hs[3 * j + 1]);
-      t1_last = hs[3 * j];
+      *t1_last = hs[3 * j];
       if (!std::isfinite(e)) {
         bad = true;
         break;
       }
       if (e < 1e-15 * m || (e < 1e-9 && e >= e2)) {
-        done = true;
+        *done = true;
         f.sp_steps = it + j + 1;
       }
       e2 = e1;
@@ -416,6 +451,36 @@ bool sp2_density(dfscf& f, const double* Fm, cudaStream_t s) {
     }
     if (bad) break;
     it += g;
+  }
+  return cur;
+}
+
+// The aufbau density of F by SP2 purification into f.P, with C_occ (only
+// the occupied columns of f.C). Returns false, with f.P untouched, when the
+// projection does not converge to a rank-nocc projector.
+bool sp2_density(dfscf& f, const double* Fm, cudaStream_t s) {
+  Context& c = *f.c;
+  PartTimer tm(s);
+  const int n = f.nao, m = f.nmo, k = f.nocc;
+  gemm(c, CUBLAS_OP_N, CUBLAS_OP_N, n, m, n, 1.0, Fm, n, f.X.as<double>(), n, 0.0, f.A1.as<double>(),
+       n, s);
+  gemm(c, CUBLAS_OP_T, CUBLAS_OP_N, m, m, n, 1.0, f.X.as<double>(), n, f.A1.as<double>(), n, 0.0,
+       f.Fo.as<double>(), m, s);
+  double* Xb[2] = {f.sp_X.as<double>(), f.sp_X2.as<double>()};
+  double* Z = f.sp_Z.as<double>();
+  double* st = f.sp_st.as<double>();   // [0..1] bounds, then 3 per step
+  double t1_last = 0.0;
+  bool done = false;
+  int cur = 0;
+  if (m <= kSp2ClusterMax) {
+    launch_sp2_cluster(f.Fo.as<double>(), m, k, kSp2Max, Xb[0], st, s);
+    double rec[3];
+    DFJK_CUDA(cudaMemcpyAsync(rec, st, sizeof rec, cudaMemcpyDeviceToHost, s));
+    DFJK_CUDA(cudaStreamSynchronize(s));
+    t1_last = rec[1];
+    done = rec[2] == 1.0;
+  } else {
+    cur = sp2_steps(f, Xb, Z, st, &done, &t1_last, s);
   }
   const double* Xs = Xb[cur];
   if (!done || !(std::fabs(t1_last - k) < 1e-6)) {
@@ -484,8 +549,8 @@ void make_density(dfscf& f, const double* Fm, cudaStream_t s) {
   make_density_eig(f, Fm, s);
 }
 
-// err = X^T (F P S - S P F) X into f.Fo's slot of dE; returns |err|
-double commutator(dfscf& f, const double* Fm, const double* Pm, double* err, cudaStream_t s) {
+// err = X^T (F P S - S P F) X into its slot of dE
+void commutator(dfscf& f, const double* Fm, const double* Pm, double* err, cudaStream_t s) {
   Context& c = *f.c;
   const int n = f.nao, m = f.nmo;
   gemm(c, CUBLAS_OP_N, CUBLAS_OP_N, n, n, n, 1.0, Fm, n, Pm, n, 0.0, f.A1.as<double>(), n, s);
@@ -497,10 +562,6 @@ double commutator(dfscf& f, const double* Fm, const double* Pm, double* err, cud
        f.A2.as<double>(), n, s);
   gemm(c, CUBLAS_OP_T, CUBLAS_OP_N, m, m, n, 1.0, f.X.as<double>(), n, f.A2.as<double>(), n, 0.0, err,
        m, s);
-  double r = 0.0;
-  DFJK_CUBLAS(cublasSetStream(c.cublas, s));
-  DFJK_CUBLAS(cublasDnrm2(c.cublas, m * m, err, 1, &r));
-  return r;
 }
 
 // DIIS coefficients of the filled slots (scf.py:245-273), host
@@ -573,13 +634,16 @@ void run(dfscf& f, const double* P0, cudaStream_t s) {
     const int slot = it % md;
     double* dFs = f.dF.as<double>() + slot * nn;
     double* dEs = f.dE.as<double>() + slot * mm;
-    derr = commutator(f, f.F.as<double>(), f.P.as<double>(), dEs, s);
+    commutator(f, f.F.as<double>(), f.P.as<double>(), dEs, s);
     DFJK_CUDA(cudaMemcpyAsync(dFs, f.F.p, nn * sizeof(double), cudaMemcpyDeviceToDevice, s));
     // the new row of error overlaps: B[slot][j] = <err_slot, err_j>
     const int count = std::min(it + 1, md);
     std::vector<double> row(md, 0.0);
-    for (int j = 0; j < count; ++j)
-      row[j] = ddot(c, dEs, f.dE.as<double>() + j * mm, mm, s);
+    std::vector<std::pair<const double*, const double*>> ab;
+    for (int j = 0; j < count; ++j) ab.push_back({dEs, f.dE.as<double>() + j * mm});
+    dots(f, ab, mm, row.data(), s);
+    DFJK_CUDA(cudaStreamSynchronize(s));
+    derr = std::sqrt(row[slot]);
     for (int j = 0; j < count; ++j) {
       f.B[(size_t)slot * md + j] = row[j];
       f.B[(size_t)j * md + slot] = row[j];
