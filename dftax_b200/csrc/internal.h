@@ -100,7 +100,7 @@ struct Plan {
   int64_t k0 = 0;    // first kept eigen-direction
   PhaseTimer timer;
   // persistent workspaces (grow-only), reused by every build and J/K call
-  DevBuf ws_raw, ws_syevd, ws_info, ws_flag, ws_dvec, ws_gamma, ws_part, ws_X, ws_Cp, ws_sel;
+  DevBuf ws_raw, ws_syevd, ws_info, ws_flag, ws_gamma, ws_part, ws_X, ws_Cp, ws_sel;
   // streamed plans: one chunk of B rows, the chunk's K-list bounds
   DevBuf ws_bchunk, ws_kb, ws_ke;
   // mixed precision: int8 digit planes of the square B_x for the tensor-core half transform

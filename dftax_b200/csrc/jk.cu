@@ -3,8 +3,8 @@
 // B is row-major [nrows][ldb]: one row per AO pair (m, n) of a kept shell
 // pair, one column per kept metric direction (B = (mn|P) L, L L^T = V+).
 //
-//   J: dvec[r] = w_r D[m, n]             (w_r = 2 off-diagonal pair, else 1)
-//      gamma   = B^T dvec                 (stream B once; CTA partials + reduce)
+//   J: d[r] = w_r D[m, n]                (w_r = 2 off-diagonal pair, else 1)
+//      gamma = B^T d                      (stream B once; CTA partials + reduce)
 //      J[m, n] = J[n, m] = B[r] . gamma   (stream B again; warp per row)
 //   K: X[m][x][i] = sum_{(r, n) in list(m)} B[r][x] C'[n][i]   (half transform)
 //      K = X X^T over the (x, i) index, C' = C sqrt|w|
@@ -26,61 +26,73 @@ namespace dfjk {
 // J
 // ---------------------------------------------------------------------------
 
-__global__ void dvec_from_c_kernel(const double* __restrict__ C, const double* __restrict__ w,
-                                   int64_t ncol, const int* __restrict__ rm,
-                                   const int* __restrict__ rn, const int8_t* __restrict__ kind,
-                                   int64_t nrows, double* __restrict__ dvec) {
-  const int64_t warp = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
-  const int lane = threadIdx.x & 31;
-  if (warp >= nrows) return;
-  const int m = rm[warp], n = rn[warp];
-  const double* cm = C + (int64_t)m * ncol;
-  const double* cn = C + (int64_t)n * ncol;
-  double s = 0.0;
-  for (int64_t i = lane; i < ncol; i += 32) s += (w ? w[i] : 1.0) * cm[i] * cn[i];
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-  if (lane == 0) dvec[warp] = (kind[warp] == 2 ? 2.0 : 1.0) * s;
-}
+// The density whose J is taken: sum_i w_i C[m][i] C[n][i] of ncol orbitals (w
+// null: ones), or the matrix D when C is null.
+struct DensitySource {
+  const double* C;
+  const double* w;
+  int64_t ncol;
+  const double* D;
+};
 
-__global__ void dvec_from_density_kernel(const double* __restrict__ D, int64_t nao,
-                                         const int* __restrict__ rm, const int* __restrict__ rn,
-                                         const int8_t* __restrict__ kind, int64_t nrows,
-                                         double* __restrict__ dvec) {
-  const int64_t r = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  if (r >= nrows) return;
-  const int m = rm[r], n = rn[r];
-  // off-diagonal pairs stand for both (m, n) and (n, m)
-  const double v = kind[r] == 2 ? D[(int64_t)m * nao + n] + D[(int64_t)n * nao + m]
-                                : D[(int64_t)m * nao + n];
-  dvec[r] = v;
-}
-
-// gamma partials: CTA (bx, by) sums rows [r0, r1) for columns [by*2048, +2048)
+// gamma partials: CTA (bx, by) sums rows [r0, r1) for columns [by*2048, +2048).
+// The rows' weights d[r] = w_r D[m, n] are formed 32 at a time by the block
+// itself (a warp takes four), so no launch and no array come before it.
 constexpr int kGtThreads = 256;
 constexpr int kGtCols = kGtThreads * 8;
+constexpr int kGtRows = 32;
 
 __global__ void __launch_bounds__(kGtThreads) gamma_partial_kernel(
-    const double* __restrict__ B, int64_t ldb, int64_t nrows, const double* __restrict__ dvec,
+    const double* __restrict__ B, int64_t ldb, int64_t nrows, DensitySource src, int64_t nao,
+    const int* __restrict__ rm, const int* __restrict__ rn, const int8_t* __restrict__ kind,
     int64_t rows_per_cta, double* __restrict__ part) {
+  __shared__ double sd[kGtRows];
   const int64_t r0 = blockIdx.x * rows_per_cta;
   const int64_t r1 = min(nrows, r0 + rows_per_cta);
   const int64_t c0 = (int64_t)blockIdx.y * kGtCols + 2 * threadIdx.x;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   double2 acc[4];
 #pragma unroll
   for (int j = 0; j < 4; ++j) acc[j] = make_double2(0.0, 0.0);
-  for (int64_t r = r0; r < r1; ++r) {
-    const double d = __ldg(dvec + r);
-    const double* row = B + r * ldb;
+  for (int64_t t0 = r0; t0 < r1; t0 += kGtRows) {
+    if (src.C) {
 #pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      const int64_t c = c0 + j * 2 * kGtThreads;
-      if (c < ldb) {
-        const double2 b = __ldcs(reinterpret_cast<const double2*>(row + c));
-        acc[j].x += d * b.x;
-        acc[j].y += d * b.y;
+      for (int q = 0; q < kGtRows / 8; ++q) {
+        const int64_t r = t0 + warp + 8 * q;
+        double s = 0.0;
+        if (r < r1) {
+          const double* cm = src.C + (int64_t)rm[r] * src.ncol;
+          const double* cn = src.C + (int64_t)rn[r] * src.ncol;
+          for (int64_t i = lane; i < src.ncol; i += 32)
+            s += (src.w ? src.w[i] : 1.0) * cm[i] * cn[i];
+        }
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+        // off-diagonal pairs stand for both (m, n) and (n, m)
+        if (lane == 0 && r < r1) sd[warp + 8 * q] = kind[r] == 2 ? 2.0 * s : s;
+      }
+    } else if (threadIdx.x < kGtRows && t0 + threadIdx.x < r1) {
+      const int64_t r = t0 + threadIdx.x;
+      const int64_t m = rm[r], n = rn[r];
+      sd[threadIdx.x] = kind[r] == 2 ? src.D[m * nao + n] + src.D[n * nao + m] : src.D[m * nao + n];
+    }
+    __syncthreads();
+    const int nr = (int)min(r1 - t0, (int64_t)kGtRows);
+#pragma unroll 2
+    for (int q = 0; q < nr; ++q) {
+      const double d = sd[q];
+      const double* row = B + (t0 + q) * ldb;
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const int64_t c = c0 + j * 2 * kGtThreads;
+        if (c < ldb) {
+          const double2 b = __ldcs(reinterpret_cast<const double2*>(row + c));
+          acc[j].x += d * b.x;
+          acc[j].y += d * b.y;
+        }
       }
     }
+    __syncthreads();
   }
 #pragma unroll
   for (int j = 0; j < 4; ++j) {
@@ -174,20 +186,23 @@ __global__ void add_to_kernel(const double* __restrict__ x, int64_t n, double* _
   if (i < n) y[i] += x[i];
 }
 
-// gamma (+)= Bc^T dvec over nrows rows of Bc: fixed-order partial sums
-static void gamma_rows(Plan& p, const double* Bc, int64_t nrows, const double* dvec, double* out,
-                       bool add, cudaStream_t s) {
+// gamma (+)= Bc^T d over nrows rows of Bc (rows from row0 of the plan): fixed-
+// order partial sums. At least eight rows per block, so that a small B leaves
+// few partials to add.
+static void gamma_rows(Plan& p, const double* Bc, int64_t row0, int64_t nrows,
+                       const DensitySource& src, double* out, bool add, cudaStream_t s) {
   const int sms = num_sms(p.ctx->device);
   const int64_t ycols = (p.ldb + kGtCols - 1) / kGtCols;
   int64_t xparts = std::max<int64_t>(1, (int64_t)sms * 4 / ycols);
-  xparts = std::min<int64_t>(xparts, std::max<int64_t>(1, nrows));
+  xparts = std::min<int64_t>(xparts, (nrows + 7) / 8);
   const int64_t rows_per = (nrows + xparts - 1) / xparts;
   xparts = (nrows + rows_per - 1) / rows_per;
   DevBuf& part = p.ws_part;
-  part.ensure((size_t)(std::max<int64_t>(xparts, 1) + (add ? 1 : 0)) * p.ldb * sizeof(double));
+  part.ensure((size_t)(xparts + (add ? 1 : 0)) * p.ldb * sizeof(double));
   double* sum = part.as<double>() + xparts * p.ldb;   // the chunk's gamma when adding
   gamma_partial_kernel<<<dim3((unsigned)xparts, (unsigned)ycols), kGtThreads, 0, s>>>(
-      Bc, p.ldb, nrows, dvec, rows_per, part.as<double>());
+      Bc, p.ldb, nrows, src, p.nao, p.d_row_m.as<int>() + row0, p.d_row_n.as<int>() + row0,
+      p.d_row_w.as<int8_t>() + row0, rows_per, part.as<double>());
   DFJK_LAUNCHED();
   launch_reduce_rows(part.as<double>(), xparts, p.ldb, add ? sum : out, s);
   if (add) {
@@ -196,35 +211,23 @@ static void gamma_rows(Plan& p, const double* Bc, int64_t nrows, const double* d
   }
 }
 
-// gamma = B^T dvec into `gamma` (ldb doubles)
-static void gamma_from_dvec(Plan& p, const double* dvec, double* gamma, cudaStream_t s) {
-  if (p.opts.streamed) {
+// gamma = B^T d into `gamma` (ldb doubles)
+static void gamma_of(Plan& p, const DensitySource& src, double* gamma, cudaStream_t s) {
+  if (p.opts.streamed || p.nrows == 0) {
     DFJK_CUDA(cudaMemsetAsync(gamma, 0, p.ldb * sizeof(double), s));
+    if (p.nrows == 0) return;
     for_each_b_chunk(p, s, [&](int64_t r0, int64_t nr, const double* Bc) {
-      if (nr > 0) gamma_rows(p, Bc, nr, dvec + r0, gamma, true, s);
+      if (nr > 0) gamma_rows(p, Bc, r0, nr, src, gamma, true, s);
     });
     return;
   }
-  const int sms = num_sms(p.ctx->device);
-  const int64_t ycols = (p.ldb + kGtCols - 1) / kGtCols;
-  int64_t xparts = std::max<int64_t>(1, (int64_t)sms * 4 / ycols);
-  xparts = std::min<int64_t>(xparts, std::max<int64_t>(1, p.nrows));
-  const int64_t rows_per = (p.nrows + xparts - 1) / xparts;
-  xparts = (p.nrows + rows_per - 1) / rows_per;
-  DevBuf& part = p.ws_part;
-  part.ensure((size_t)std::max<int64_t>(xparts, 1) * p.ldb * sizeof(double));
-  if (p.nrows > 0) {
-    gamma_partial_kernel<<<dim3((unsigned)xparts, (unsigned)ycols), kGtThreads, 0, s>>>(
-        p.d_B.as<double>(), p.ldb, p.nrows, dvec, rows_per, part.as<double>());
-    DFJK_LAUNCHED();
-    launch_reduce_rows(part.as<double>(), xparts, p.ldb, gamma, s);
-  } else {
-    DFJK_CUDA(cudaMemsetAsync(gamma, 0, p.ldb * sizeof(double), s));
-  }
+  gamma_rows(p, p.d_B.as<double>(), 0, p.nrows, src, gamma, false, s);
 }
 
 static void j_from_gamma(Plan& p, const double* gamma, double* J, cudaStream_t s) {
-  DFJK_CUDA(cudaMemsetAsync(J, 0, (size_t)p.nao * p.nao * sizeof(double), s));
+  // without screening every element belongs to a row
+  if (p.opts.screen > 0.0 || p.nrows == 0)
+    DFJK_CUDA(cudaMemsetAsync(J, 0, (size_t)p.nao * p.nao * sizeof(double), s));
   if (p.nrows == 0) return;
   const int sms = num_sms(p.ctx->device);
   if (p.opts.streamed) {
@@ -251,8 +254,8 @@ static void j_from_gamma(Plan& p, const double* gamma, double* J, cudaStream_t s
 
 // On the float64 tensor cores (mma.sync m8n8k4 f64: tcgen05 has no float64
 // kind). A block of eight warps computes 64 directions x HtTile::I columns of
-// one m, 16 list entries per k chunk, through a four-stage cp.async ring of
-// 16-byte copies with one barrier per chunk. Bound by the DMMA pipe once nocc
+// one m, 16 list entries per k chunk, through a ring of three or four stages of
+// 16-byte copies (three blocks per SM) with one barrier per chunk. Bound by the DMMA pipe once nocc
 // is above ~20 columns: the tile's width follows the columns (half_tile), since
 // columns of padding cost as much as real ones.
 //   * Warps: WI of them side by side over the columns, 8 / WI over the
@@ -263,14 +266,15 @@ static void j_from_gamma(Plan& p, const double* gamma, double* J, cudaStream_t s
 //     put the 8 lanes of a load phase (4 k, 2 rows) in distinct banks.
 // (H2O)_12 (nocc 60): 1353 us with 80-column tiles, 8-byte copies and two
 // stages; see half_tile for the widths.
-constexpr int kHtX = 64, kHtK = 16, kHtPX = kHtX + 4, kHtStages = 4;
+constexpr int kHtX = 64, kHtK = 16, kHtPX = kHtX + 4;
 
 template <int IF_, int WI_>
 struct HtTile {
   static constexpr int IF = IF_, WI = WI_, WX = 8 / WI, XF = kHtX / (8 * WX);
   static constexpr int I = 8 * IF * WI, PI = I + 4;
   static constexpr int kStage = kHtK * (kHtPX + PI);   // doubles
-  static constexpr size_t smem = (size_t)kHtStages * kStage * sizeof(double);
+  static constexpr int kStages = 3 * 4 * kStage * 8 <= 224 * 1024 ? 4 : 3;
+  static constexpr size_t smem = (size_t)kStages * kStage * sizeof(double);
 };
 
 // The list of m is entries [kbeg[m], kend[m]) (kend == nullptr: up to
@@ -279,12 +283,12 @@ struct HtTile {
 // B and Cp 16-byte aligned and x0 a multiple of 64, so every copy and store is
 // aligned.
 template <class T>
-__global__ void __launch_bounds__(256, 2) half_transform_kernel(
+__global__ void __launch_bounds__(256, 3) half_transform_kernel(
     const double* __restrict__ B, int64_t ldb, int64_t x0, int64_t xc, const double* __restrict__ Cp,
     int64_t ncol, const int* __restrict__ kbeg, const int* __restrict__ kend,
     const int* __restrict__ krow, const int* __restrict__ kn, int64_t row0, int accumulate,
     double* __restrict__ X) {
-  constexpr int XF = T::XF, IF = T::IF, PI = T::PI;
+  constexpr int XF = T::XF, IF = T::IF, PI = T::PI, kHtStages = T::kStages;
   constexpr int kCg = kHtK * T::I / 2, kCper = (kCg + 255) / 256;   // 16-byte copies of C' rows
   extern __shared__ __align__(16) double ht_smem[];
   const int m = blockIdx.x;
@@ -485,7 +489,7 @@ __global__ void list_bounds_kernel(const int* __restrict__ kptr, const int* __re
 constexpr int kSyT = 64, kSyK = 16, kSyStages = 4;
 constexpr size_t kSySmem = (size_t)kSyStages * 2 * kSyT * kSyK * sizeof(double);
 
-__global__ void __launch_bounds__(256, 2) syrk_part_kernel(const double* __restrict__ X, int64_t nao,
+__global__ void __launch_bounds__(256, 3) syrk_part_kernel(const double* __restrict__ X, int64_t nao,
                                                            int64_t kt, int64_t kslice,
                                                            double* __restrict__ part) {
   extern __shared__ __align__(16) double sy_smem[];
@@ -602,7 +606,7 @@ __global__ void scale_cols_kernel(const double* __restrict__ C, const double* __
 
 // K (+)= sign * X X^T (float64, full square) for X nao x kt row-major: lower
 // 64 x 64 tile pairs times k slices, then a fixed-order sum of the slices
-// (bit-reproducible). Two blocks run per SM; the slice count is the one whose
+// (bit-reproducible). Three blocks run per SM; the slice count is the one whose
 // waves x (slice length + 128: a block's prologue and partial stores in units
 // of k) is smallest. One slice per 1024 k left a single block at small sizes
 // ((H2O)_1: 46 us) and 1.4 waves at (H2O)_12 (719 us).
@@ -610,7 +614,7 @@ static void syrk_fp64(Plan& p, const double* X, int64_t kt, double sign, bool be
                       cudaStream_t s) {
   const int64_t nao = p.nao;
   const int64_t nt = (nao + kSyT - 1) / kSyT, tiles = nt * (nt + 1) / 2;
-  const int64_t slots = 2 * (int64_t)num_sms(p.ctx->device);
+  const int64_t slots = 3 * (int64_t)num_sms(p.ctx->device);
   const int64_t most = std::min<int64_t>(64, std::max<int64_t>(1, kt / 64));
   int64_t nsplit = 1;
   int64_t best = INT64_MAX;
@@ -635,12 +639,12 @@ static void syrk_fp64(Plan& p, const double* X, int64_t kt, double sign, bool be
 }
 
 // K (+)= sign * X X^T for the selected columns of C (scaled by sqrt|w|)
-// fuse (streamed plans only, may be null): gamma = B^T dvec is also summed
-// in the first pass over B's chunks (one rebuild of B fewer per J/K call);
-// its dvec is cleared once gamma is done.
+// fuse (streamed plans only, may be null): gamma = B^T d is also summed in the
+// first pass over B's chunks (one rebuild of B fewer per J/K call).
 struct GammaFuse {
-  const double* dvec = nullptr;
+  DensitySource src;
   double* gamma = nullptr;
+  bool done = false;
 };
 
 // nsel columns of C: those of `sel` (host indices), or the first nsel when
@@ -657,12 +661,17 @@ static void k_accumulate(Plan& p, const double* C, int64_t sm, int64_t sc, const
     DFJK_CUDA(cudaMemcpyAsync(dsel.p, sel->data(), nsel * sizeof(int), cudaMemcpyHostToDevice, s));
   }
   // an even number of columns (a zero one added) keeps the rows of C' and X
-  // 16-byte aligned for the wide copies and the TMA stores of both forms
+  // 16-byte aligned for the wide copies and the TMA stores of both forms;
+  // unweighted columns that already lie so are used where they are
   const int64_t ncp = nsel + (nsel & 1);
-  Cp.ensure((size_t)nao * ncp * sizeof(double));
-  scale_cols_kernel<<<(unsigned)((nao * ncp + 255) / 256), 256, 0, s>>>(
-      C, w, nao, sm, sc, sel ? dsel.as<int>() : nullptr, nsel, ncp, Cp.as<double>());
-  DFJK_LAUNCHED();
+  const double* Cc = C;
+  if (w || sel || sc != 1 || sm != ncp || (reinterpret_cast<uintptr_t>(C) & 15)) {
+    Cp.ensure((size_t)nao * ncp * sizeof(double));
+    Cc = Cp.as<double>();
+    scale_cols_kernel<<<(unsigned)((nao * ncp + 255) / 256), 256, 0, s>>>(
+        C, w, nao, sm, sc, sel ? dsel.as<int>() : nullptr, nsel, ncp, Cp.as<double>());
+    DFJK_LAUNCHED();
+  }
   // x chunking so that X (nao * xc * ncp doubles) stays within budget; a
   // streamed plan rebuilds B once per x chunk, so it takes up to half the
   // free device memory
@@ -687,26 +696,26 @@ static void k_accumulate(Plan& p, const double* C, int64_t sm, int64_t sc, const
       DFJK_CUDA(cudaMemsetAsync(X.p, 0, (size_t)nao * n * ncp * sizeof(double), s));
       p.ws_kb.ensure(nao * sizeof(int));
       p.ws_ke.ensure(nao * sizeof(int));
-      const bool with_gamma = fuse && fuse->dvec;
+      const bool with_gamma = fuse && !fuse->done;
       if (with_gamma) DFJK_CUDA(cudaMemsetAsync(fuse->gamma, 0, p.ldb * sizeof(double), s));
       for_each_b_chunk(p, s, [&](int64_t r0, int64_t nr, const double* Bc) {
-        if (with_gamma && nr > 0) gamma_rows(p, Bc, nr, fuse->dvec + r0, fuse->gamma, true, s);
+        if (with_gamma && nr > 0) gamma_rows(p, Bc, r0, nr, fuse->src, fuse->gamma, true, s);
         list_bounds_kernel<<<(unsigned)((nao + 255) / 256), 256, 0, s>>>(
             p.d_kptr.as<int>(), p.d_krow.as<int>(), nao, r0, r0 + nr, p.ws_kb.as<int>(),
             p.ws_ke.as<int>());
         DFJK_LAUNCHED();
-        launch_half_any(ncp, Bc, p.ldb, x0, n, (const double*)Cp.as<double>(), ncp,
+        launch_half_any(ncp, Bc, p.ldb, x0, n, Cc, ncp,
                         (const int*)p.ws_kb.as<int>(), (const int*)p.ws_ke.as<int>(),
                         (const int*)p.d_krow.as<int>(), (const int*)p.d_kn.as<int>(), r0, 1, nao,
                         X.as<double>(), s);
       });
-      if (with_gamma) fuse->dvec = nullptr;   // gamma is complete
+      if (with_gamma) fuse->done = true;
     } else if (oz) {
-      if (x0 == 0) ozaki_prepare_c(p, Cp.as<double>(), ncp, s);
+      if (x0 == 0) ozaki_prepare_c(p, Cc, ncp, s);
       ozaki_k1(p, ncp, x0, n, X.as<double>(), s);   // int8 tensor cores, exact accumulation
     } else {
       launch_half_any(ncp, (const double*)p.d_B.as<double>(), p.ldb, x0, n,
-                      (const double*)Cp.as<double>(), ncp, (const int*)p.d_kptr.as<int>(),
+                      Cc, ncp, (const int*)p.d_kptr.as<int>(),
                       (const int*)nullptr, (const int*)p.d_krow.as<int>(),
                       (const int*)p.d_kn.as<int>(), (int64_t)0, 0, nao, X.as<double>(), s);
     }
@@ -754,27 +763,20 @@ void jk_compute(Plan& p, const double* C, const double* w, int64_t ncol, double*
   for (int ph = kPhJ; ph <= kPhKsyrk; ++ph) p.timer.reset(ph);
   if (J) {
     p.timer.mark(kPhJ, s);
-    DevBuf& dvec = p.ws_dvec;
     DevBuf& gamma = p.ws_gamma;
-    dvec.ensure(std::max<int64_t>(p.nrows, 1) * sizeof(double));
     gamma.ensure(p.ldb * sizeof(double));
-    if (p.nrows > 0) {
-      dvec_from_c_kernel<<<(unsigned)((p.nrows * 32 + 255) / 256), 256, 0, s>>>(
-          C, w, ncol, p.d_row_m.as<int>(), p.d_row_n.as<int>(), p.d_row_w.as<int8_t>(), p.nrows,
-          dvec.as<double>());
-      DFJK_LAUNCHED();
-    }
+    const DensitySource src{C, w, ncol, nullptr};
     if (p.opts.streamed && K) {
       // one pass over B's chunks gives gamma and the K half transform; J
       // takes a second
-      GammaFuse fuse{dvec.as<double>(), gamma.as<double>()};
+      GammaFuse fuse{src, gamma.as<double>(), false};
       k_compute(p, C, w, ncol, K, s, &fuse);
-      if (fuse.dvec) gamma_from_dvec(p, dvec.as<double>(), gamma.as<double>(), s);
+      if (!fuse.done) gamma_of(p, src, gamma.as<double>(), s);
       j_from_gamma(p, gamma.as<double>(), J, s);
       p.timer.mark(kPhJ, s);
       return;
     }
-    gamma_from_dvec(p, dvec.as<double>(), gamma.as<double>(), s);
+    gamma_of(p, src, gamma.as<double>(), s);
     j_from_gamma(p, gamma.as<double>(), J, s);
     p.timer.mark(kPhJ, s);
   }
@@ -899,15 +901,7 @@ static void density_factor(Plan& p, const double* Q, DevBuf& Ct, DevBuf& dw, cud
 // hf_lr: the long-range exchange of range-separated hybrids through the plan's
 // long-range fit (terms.py:604-612)
 void gamma_from_density(Plan& p, const double* Ptot, double* gamma, cudaStream_t s) {
-  DevBuf& dvec = p.ws_dvec;
-  dvec.ensure(std::max<int64_t>(p.nrows, 1) * sizeof(double));
-  if (p.nrows > 0) {
-    dvec_from_density_kernel<<<(unsigned)((p.nrows + 255) / 256), 256, 0, s>>>(
-        Ptot, p.nao, p.d_row_m.as<int>(), p.d_row_n.as<int>(), p.d_row_w.as<int8_t>(), p.nrows,
-        dvec.as<double>());
-    DFJK_LAUNCHED();
-  }
-  gamma_from_dvec(p, dvec.as<double>(), gamma, s);
+  gamma_of(p, DensitySource{nullptr, nullptr, 0, Ptot}, gamma, s);
 }
 
 // Two host synchronizations: the ranks (with the density check), and the
