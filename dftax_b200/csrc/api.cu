@@ -764,10 +764,23 @@ int64_t rows_of(const Plan& p, int64_t b, int64_t e) {
   return end_row - p.pair_row0[b];
 }
 
+void side_streams(Context& c) {
+  if (c.side_fork) return;
+  for (int q = 0; q < kXcBranches; ++q) {
+    if (!c.side_stream[q]) DFJK_CUDA(cudaStreamCreateWithFlags(&c.side_stream[q], cudaStreamNonBlocking));
+    if (!c.side_done[q]) DFJK_CUDA(cudaEventCreateWithFlags(&c.side_done[q], cudaEventDisableTiming));
+  }
+  DFJK_CUDA(cudaEventCreateWithFlags(&c.side_fork, cudaEventDisableTiming));
+}
+
 // Everything a build does before its 3-center rows: the metric factor, the
 // primitive pairs, the workspaces and L's digit planes. Returns the pair
 // chunks of the rows, or no chunks when the plan is streamed (built then).
-static std::vector<std::pair<int64_t, int64_t>> build_begin(Plan& p, cudaStream_t s) {
+// rows_ahead (may be null): where the rows fit in one chunk and the metric has
+// to be computed, they are computed beside it on a side stream, and *rows_ahead
+// is set; s then waits for them.
+static std::vector<std::pair<int64_t, int64_t>> build_begin(Plan& p, cudaStream_t s,
+                                                            bool* rows_ahead = nullptr) {
   p.built = 0;
   // the first build of a plan uses the metric factor computed while the plan
   // was created (same code and inputs); every later build recomputes it
@@ -776,18 +789,6 @@ static std::vector<std::pair<int64_t, int64_t>> build_begin(Plan& p, cudaStream_
   for (int ph = kPhMetric; ph <= kPhBgemm; ++ph)
     if (ph != kPhMetric || !have_metric) p.timer.reset(ph);
   p.timer.reset(kPhKplanes);
-  // The eigensolver keeps the whole device busy: running the 3-center rows
-  // beside it on a second stream (at either priority) was measured to save
-  // under 3% of a (H2O)_32 build while holding the whole tensor, so the
-  // phases run in order on s.
-  if (!have_metric) {
-    p.timer.mark(kPhMetric, s);
-    compute_metric_factor(p, s);
-    p.timer.mark(kPhMetric, s);
-  }
-  p.timer.mark(kPhPairs, s);
-  launch_pair_setup(p, s);
-  p.timer.mark(kPhPairs, s);
   const int64_t ld = p.naux;
   const int64_t kp = (p.naux + 15) / 16 * 16;
   auto chunks = pair_chunks(p, ld, chunk_budget(p));
@@ -795,6 +796,36 @@ static std::vector<std::pair<int64_t, int64_t>> build_begin(Plan& p, cudaStream_
   for (auto& ch : chunks) maxrows = std::max(maxrows, rows_of(p, ch.first, ch.second));
   DevBuf& raw = p.ws_raw;
   raw.ensure((size_t)maxrows * ld * sizeof(double));
+  auto pairs = [&](cudaStream_t q) {
+    p.timer.mark(kPhPairs, q);
+    launch_pair_setup(p, q);
+    p.timer.mark(kPhPairs, q);
+  };
+  // The eigensolver is a chain of latency-bound steps that leaves much of the
+  // device idle up to a few thousand functions; the rows need nothing from it.
+  // (Several chunks would need the whole tensor staged: from (H2O)_17 on, where
+  // the overlap was measured to save under 3% of a build.)
+  const bool ahead = rows_ahead && !have_metric && !p.opts.streamed && chunks.size() == 1;
+  Context& c = *p.ctx;
+  if (ahead) {
+    SideFork side(c, 1, s);   // after the earlier work on the plan's buffers
+    pairs(side.stream(0));
+    p.timer.mark(kPhEri3c, side.stream(0));
+    launch_eri3c_rows(p, chunks[0].first, chunks[0].second, 0, raw.p, ld, false, side.stream(0));
+    p.timer.mark(kPhEri3c, side.stream(0));
+    p.timer.mark(kPhMetric, s);
+    compute_metric_factor(p, s);
+    p.timer.mark(kPhMetric, s);
+    side.join();
+    *rows_ahead = true;
+  } else {
+    if (!have_metric) {
+      p.timer.mark(kPhMetric, s);
+      compute_metric_factor(p, s);
+      p.timer.mark(kPhMetric, s);
+    }
+    pairs(s);
+  }
   // B = (ij|P) L on the int8 tensor cores with exact accumulation: 5 digits
   // per value in mixed precision, 7 (2^-56 of each row's scale, below
   // float64's own rounding of the row maximum) for float64 plans
@@ -840,13 +871,16 @@ static void build_end(Plan& p, cudaStream_t s) {
 }
 
 void build(Plan& p, cudaStream_t s) {
-  auto chunks = build_begin(p, s);
+  bool ahead = false;
+  auto chunks = build_begin(p, s, &ahead);
   if (p.built) return;   // streamed
   for (auto& ch : chunks) {
     const int64_t r0 = p.pair_row0[ch.first], nr = rows_of(p, ch.first, ch.second);
-    p.timer.mark(kPhEri3c, s);
-    launch_eri3c_rows(p, ch.first, ch.second, r0, p.ws_raw.p, p.naux, false, s);
-    p.timer.mark(kPhEri3c, s);
+    if (!ahead) {
+      p.timer.mark(kPhEri3c, s);
+      launch_eri3c_rows(p, ch.first, ch.second, r0, p.ws_raw.p, p.naux, false, s);
+      p.timer.mark(kPhEri3c, s);
+    }
     build_product(p, r0, nr, s);
   }
   build_end(p, s);
@@ -1025,10 +1059,10 @@ dfjk_status dfjk_destroy(dfjk_ctx* h) {
   if (h->c.cublas) cublasDestroy(h->c.cublas);
   if (h->c.cusolver) cusolverDnDestroy(h->c.cusolver);
   for (int q = 0; q < dfjk::kXcBranches; ++q) {
-    if (h->c.xc_done[q]) cudaEventDestroy(h->c.xc_done[q]);
-    if (h->c.xc_stream[q]) cudaStreamDestroy(h->c.xc_stream[q]);
+    if (h->c.side_done[q]) cudaEventDestroy(h->c.side_done[q]);
+    if (h->c.side_stream[q]) cudaStreamDestroy(h->c.side_stream[q]);
   }
-  if (h->c.xc_fork) cudaEventDestroy(h->c.xc_fork);
+  if (h->c.side_fork) cudaEventDestroy(h->c.side_fork);
   const int dev = h->c.device;
   {
     std::lock_guard<std::recursive_mutex> cap(dfjk::capture_mutex());

@@ -421,22 +421,48 @@ double energy_gradient(Plan& p, const double* P, int nspin, double hf, double* g
     G.alloc((size_t)maxrows * naux * sizeof(double));
     const int64_t dsph_budget = (int64_t)512 << 20;   // bytes of derivative tables per launch
     dsph.alloc((size_t)dsph_budget);
+    auto per_pp = [](const ClassRange& cr) {
+      const int nab = (2 * cr.l1 + 1) * (2 * cr.l2 + 1);
+      return 3 * (int64_t)nab * hcount(cr.l1 + cr.l2 + 1) * (int64_t)sizeof(double);
+    };
     for (auto& ch : chunks) {
       const int64_t r0 = p.pair_row0[ch.first], nr = rows_of(p, ch.first, ch.second);
       DFJK_CUBLAS(cublasDgemm(c.cublas, CUBLAS_OP_N, CUBLAS_OP_N, (int)naux, (int)nr, (int)ldb, &one,
                               p.d_L.as<double>(), (int)naux, H.as<double>() + r0 * ldb, (int)ldb,
                               &zero, G.as<double>(), (int)naux));
+      struct Run { const ClassRange* cr; int64_t b, e, bytes; };
+      std::vector<Run> runs;
+      int64_t total = 0;
       for (const ClassRange& cr : p.classes) {
         const int64_t b = std::max(ch.first, cr.begin), e = std::min(ch.second, cr.begin + cr.count);
         if (b >= e) continue;
-        const int nab = (2 * cr.l1 + 1) * (2 * cr.l2 + 1);
-        const int64_t per_pp = 3 * (int64_t)nab * hcount(cr.l1 + cr.l2 + 1) * (int64_t)sizeof(double);
+        int64_t npp = 0;
+        for (int64_t q = b; q < e; ++q) npp += p.pair_npp[q];
+        runs.push_back({&cr, b, e, npp * per_pp(cr)});
+        total += runs.back().bytes;
+      }
+      if (total <= dsph_budget) {
+        // all classes' tables fit side by side: the classes, independent and
+        // mostly too small to fill the device, run on streams of their own
+        SideFork side(c, kXcBranches, s);
+        double* d = dsph.as<double>();
+        for (size_t k = 0; k < runs.size(); ++k) {
+          launch_grad3c_pairs(p, *runs[k].cr, runs[k].b, runs[k].e, d, G.as<double>(), r0, grad_orb,
+                              grad_aux, side.stream((int)(k % kXcBranches)));
+          d += runs[k].bytes / (int64_t)sizeof(double);
+        }
+        side.join();
+        continue;
+      }
+      for (const Run& run : runs) {
+        const ClassRange& cr = *run.cr;
+        const int64_t per = per_pp(cr);
         // sub-runs whose primitive pairs' derivative tables fit in dsph
-        int64_t q = b;
-        while (q < e) {
+        int64_t q = run.b;
+        while (q < run.e) {
           int64_t qe = q, npp = 0;
-          while (qe < e && (qe == q || (npp + p.pair_npp[qe]) * per_pp <= dsph_budget)) npp += p.pair_npp[qe++];
-          if (npp * per_pp > dsph_budget)
+          while (qe < run.e && (qe == q || (npp + p.pair_npp[qe]) * per <= dsph_budget)) npp += p.pair_npp[qe++];
+          if (npp * per > dsph_budget)
             fail(DFJK_ERR_MEMORY, "derivative tables of one shell pair exceed %lld bytes",
                  (long long)dsph_budget);
           launch_grad3c_pairs(p, cr, q, qe, dsph.as<double>(), G.as<double>(), r0, grad_orb,

@@ -33,11 +33,13 @@ struct Context {
   std::string last_error;
   cublasHandle_t cublas = nullptr;
   cusolverDnHandle_t cusolver = nullptr;
-  // streams and join events of the XC branches, made on first use and kept for
-  // the context's life (every SCF of the context reuses them)
-  cudaStream_t xc_stream[kXcBranches] = {};
-  cudaEvent_t xc_done[kXcBranches] = {};
-  cudaEvent_t xc_fork = nullptr;
+  // streams beside the caller's for work that does not depend on one another
+  // (XC groups, a build's rows beside its metric, a density's factor beside J,
+  // the derivative classes), with their join events; made on first use
+  // (side_streams) and kept for the context's life
+  cudaStream_t side_stream[kXcBranches] = {};
+  cudaEvent_t side_done[kXcBranches] = {};
+  cudaEvent_t side_fork = nullptr;
   DevBuf boys;   // kBoysNgrid x (kBoysNmax+1) doubles
   DevBuf boys_asym;  // 0.5*Gamma(n+1/2), n = 0..kBoysNmax
   // device address of the no-alloc J path's fixed scratch array on this
@@ -48,6 +50,35 @@ struct Context {
 // Device address of the no-alloc scratch array on the current device
 // (cudaGetSymbolAddress; loads the module that holds it).
 double* noalloc_scratch_address();
+
+void side_streams(Context& c);   // makes them (api.cu)
+
+// Streams 0 .. n-1 of the context ordered after s's work so far, and s after
+// theirs on destruction (an exception in between included), so no work outlives
+// the buffers of the call that enqueued it.
+class SideFork {
+ public:
+  SideFork(Context& c, int n, cudaStream_t s) : c_(c), n_(n), s_(s) {
+    side_streams(c);
+    DFJK_CUDA(cudaEventRecord(c.side_fork, s));
+    for (int q = 0; q < n; ++q) DFJK_CUDA(cudaStreamWaitEvent(c.side_stream[q], c.side_fork, 0));
+  }
+  cudaStream_t stream(int q) const { return c_.side_stream[q]; }
+  void join() {
+    for (; n_ > 0; --n_) {
+      cudaEventRecord(c_.side_done[n_ - 1], c_.side_stream[n_ - 1]);
+      cudaStreamWaitEvent(s_, c_.side_done[n_ - 1], 0);
+    }
+  }
+  ~SideFork() { join(); }
+  SideFork(const SideFork&) = delete;
+  SideFork& operator=(const SideFork&) = delete;
+
+ private:
+  Context& c_;
+  int n_;
+  cudaStream_t s_;
+};
 
 struct ClassRange {   // a contiguous run of shell pairs of one (l1, l2) class
   int l1, l2;

@@ -916,10 +916,12 @@ double energy(Plan& p, const double* P, int nspin, double hf, double hf_lr, doub
   nonfinite_kernel<<<(unsigned)((nn * nspin + 255) / 256), 256, 0, s>>>(P, nn * nspin, &sc->nonfinite);
   DFJK_LAUNCHED();
   const bool low = exch && low_rank_supported(n);
-  if (low) {
-    p.ws_lowrank.ensure((size_t)nn * nspin * sizeof(double));
-    launch_low_rank(P, n, nspin, p.ws_lowrank.as<double>(), sc->rank, sc->worst, sc->scale, s);
-  }
+  if (low) p.ws_lowrank.ensure((size_t)nn * nspin * sizeof(double));
+  // the density's factor, a chain of small steps on a few SMs, runs beside J
+  SideFork side(*p.ctx, low ? 1 : 0, s);
+  if (low)
+    launch_low_rank(P, n, nspin, p.ws_lowrank.as<double>(), sc->rank, sc->worst, sc->scale,
+                    side.stream(0));
   const double* Pt = P;
   if (nspin == 2) {
     p.ws_Ptot.ensure(nn * sizeof(double));
@@ -936,6 +938,7 @@ double energy(Plan& p, const double* P, int nspin, double hf, double hf_lr, doub
     if (nspin == 2)
       DFJK_CUDA(cudaMemcpyAsync(F + nn, F, nn * sizeof(double), cudaMemcpyDeviceToDevice, s));
   }
+  side.join();
   EnergyScalars h;
   DFJK_CUDA(cudaMemcpyAsync(&h, sc, sizeof h, cudaMemcpyDeviceToHost, s));
   DFJK_CUDA(cudaStreamSynchronize(s));

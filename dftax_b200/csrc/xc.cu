@@ -812,15 +812,15 @@ static void xc_enqueue(const Context& c, const OrbView& ov, const double* pts, c
   const int nslice = (int)((G + kVSlice - 1) / kVSlice);
   const int nb = std::min(std::max(ws.nbr, 1), kXcBranches);
   // fork: every branch starts after the caller's prior work on s
-  DFJK_CUDA(cudaEventRecord(c.xc_fork, s));
-  for (int q = 0; q < nb; ++q) DFJK_CUDA(cudaStreamWaitEvent(c.xc_stream[q], c.xc_fork, 0));
+  DFJK_CUDA(cudaEventRecord(c.side_fork, s));
+  for (int q = 0; q < nb; ++q) DFJK_CUDA(cudaStreamWaitEvent(c.side_stream[q], c.side_fork, 0));
   if (Vxc)
     for (int q = 0; q < nb; ++q)
       DFJK_CUDA(cudaMemsetAsync(ws.Vacc.as<double>() + q * nn, 0, nn * sizeof(double),
-                                c.xc_stream[q]));
+                                c.side_stream[q]));
   for (int64_t k = 0; k < nchunk; ++k) {
     XcBranch& b = ws.br[k % nb];
-    cudaStream_t bs = c.xc_stream[k % nb];
+    cudaStream_t bs = c.side_stream[k % nb];
     double* Vacc = ws.Vacc.as<double>() + (k % nb) * nn;
     const int64_t g0 = ch.g0[k], ng = ch.ng[k];
     const int nsig = ch.ao_cnt[k], ldp = nsig + (nsig & 1);
@@ -869,8 +869,8 @@ static void xc_enqueue(const Context& c, const OrbView& ov, const double* pts, c
   }
   // join: s waits for every branch
   for (int q = 0; q < nb; ++q) {
-    DFJK_CUDA(cudaEventRecord(c.xc_done[q], c.xc_stream[q]));
-    DFJK_CUDA(cudaStreamWaitEvent(s, c.xc_done[q], 0));
+    DFJK_CUDA(cudaEventRecord(c.side_done[q], c.side_stream[q]));
+    DFJK_CUDA(cudaStreamWaitEvent(s, c.side_done[q], 0));
   }
   if (Vxc) {
     symmetrize_sum_kernel<<<(unsigned)((nn + 255) / 256), 256, 0, s>>>(ws.Vacc.as<double>(),
@@ -900,14 +900,8 @@ double xc_energy_fock(const Context& c, const OrbView& ov, const double* pts, co
   }
   DFJK_CUDA(cudaFuncSetAttribute(rho_w_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kRpSmem));
   DFJK_CUDA(cudaFuncSetAttribute(v_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kVSmem));
-  // the context's branch streams and events are made here on first use, never
-  // during a capture
-  Context& cx = const_cast<Context&>(c);
-  for (int q = 0; q < kXcBranches; ++q) {
-    if (!cx.xc_stream[q]) DFJK_CUDA(cudaStreamCreateWithFlags(&cx.xc_stream[q], cudaStreamNonBlocking));
-    if (!cx.xc_done[q]) DFJK_CUDA(cudaEventCreateWithFlags(&cx.xc_done[q], cudaEventDisableTiming));
-  }
-  if (!cx.xc_fork) DFJK_CUDA(cudaEventCreateWithFlags(&cx.xc_fork, cudaEventDisableTiming));
+  // the side streams and events are made here on first use, never during a capture
+  side_streams(const_cast<Context&>(c));
   ws.ered.ensure((size_t)std::max<int64_t>(nchunk, 1) * nblk * sizeof(double));
   if (Vxc) ws.Vacc.ensure((size_t)std::max(ws.nbr, 1) * nao * nao * sizeof(double));
   const void* args[4] = {P, Vxc, pts, w};
