@@ -109,14 +109,17 @@ int64_t estimate(const dfbatch_request* r) {
   if (mixed) b += 4 * ldb * nao * nao16;                        // K digit planes
   const int64_t nocc = std::max(1, r->nocc);
   const int64_t x = std::min<int64_t>((int64_t)6 << 30, nao * ldb * nocc * 8);
-  b += x + x * 5 / 8 + (ldb * nocc / 8192 + 2) * nao * nao * 8;  // K half transform, slices, partials
+  // K half transform, its digit slices, the partials of K (at most 64 slices of
+  // a float64 plan, 2 ceil(k / 8192) + 32 of a mixed one)
+  b += x + x * 5 / 8 + (2 * (ldb * nocc / 8192) + 66) * nao * nao * 8;
   const int64_t diis = r->scf_opts.diis_space > 0 ? r->scf_opts.diis_space : 8;
-  b += (18 + 2 * diis) * nao * nao * 8;                          // SCF matrices (purification too), DIIS
+  b += (22 + 2 * diis) * nao * nao * 8;                          // SCF matrices (purification, density factor too), DIIS
   const int64_t G = r->scf_opts.grid_chunk > 0 ? r->scf_opts.grid_chunk : 16384;
   // XC chunk buffers and a V accumulator on each of the solve's XC streams
   // (one unless the request asks for more: xc.cu), the grid
   const int64_t nbr = r->scf_opts.xc_streams > 0 ? r->scf_opts.xc_streams : 1;
-  b += nbr * (6 * nao * G * 8 + 2 * nao * nao * 8) + r->npoint * 4 * 8;
+  const int64_t grp = std::max<int64_t>(dfjk::kXcGroupBytes, 5 * nao * G * 8);
+  b += nbr * (grp + (G / 512 + 3) * nao * nao * 8) + r->npoint * 4 * 8;
   return b + b / 10 + ((int64_t)256 << 20);
 }
 

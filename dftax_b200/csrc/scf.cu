@@ -312,6 +312,9 @@ XcParams xc_params(const dfscf& f) {
 
 bool has_xc(const dfscf& f) { return f.npts > 0 && (f.o.x_scale != 0.0 || f.o.c_scale != 0.0); }
 
+// the chunk size is chosen by timing (autotune_chunk), which lays the chunks out
+bool tunes(const dfscf& f) { return f.o.grid_chunk <= 0 && has_xc(f); }
+
 // E(P) and F(P) into f.F; J, K through the C_occ of f.C (from_orbitals) or
 // through the plan's density path for a general symmetric P
 double energy_fock(dfscf& f, const double* P, bool from_orbitals, double* Fout, cudaStream_t s) {
@@ -695,8 +698,8 @@ void run(dfscf& f, const double* P0, cudaStream_t s) {
 
 // Points per XC chunk, chosen by timing: the chunk size sets the shapes of the
 // two products per chunk (G x nsig x nsig) and the launches per evaluation.
-// Candidates 2048 (from 2^16 points on: below, its chunks are too few functions
-// each to pay for their launches), 4096, 8192 and 16384 points are timed on the core-guess
+// Candidates 512, 1024, 2048 (from 2^16 points on: below, there are too few
+// chunks of them to fill the groups), 4096, 8192 and 16384 points are timed on the core-guess
 // density (three evaluations each: a direct one, the graph capture, and a
 // timed graph replay) for the first molecule of each (nao / 128, log2 points,
 // XC streams) bucket; the choice is kept for the process, so later molecules
@@ -721,7 +724,7 @@ void autotune_chunk(dfscf& f, const int (&nout)[8], const std::vector<double>& p
   if (best == 0) {
     make_density_eig(f, f.H.as<double>(), s);   // core-guess density to time on
     double best_ms = INFINITY;
-    for (int64_t G : {2048, 4096, 8192, 16384}) {
+    for (int64_t G : {512, 1024, 2048, 4096, 8192, 16384}) {
       if ((int64_t)6 * f.nao * G * 8 > ((int64_t)3 << 30)) continue;
       if (G < 4096 && f.npts < ((int64_t)1 << 16)) continue;
       // as the SCF runs it: the first call launches directly, the second
@@ -800,7 +803,7 @@ dfjk_status dfscf_create(dfjk_plan* pl, int32_t natom, const double* atom_xyz,
     if (f->o.diis_space < 1 || f->o.max_iter < 0) fail(DFJK_ERR_INVALID, "invalid SCF options");
     if (f->o.xc_streams < 0 || f->o.xc_streams > kXcBranches)
       fail(DFJK_ERR_INVALID, "xc_streams must be 0..%d", kXcBranches);
-    f->xcw.nbr = f->o.xc_streams > 0 ? f->o.xc_streams : kXcBranches;
+    f->xcw.nbr = f->o.xc_streams > 0 ? f->o.xc_streams : kXcDefaultBranches;
     if (f->o.density != 0 && f->o.density != 1) fail(DFJK_ERR_INVALID, "density must be 0 or 1");
     for (int64_t i = 0; i < 3 * (int64_t)natom; ++i)
       if (!std::isfinite(atom_xyz[i])) fail(DFJK_ERR_NUMERIC, "non-finite atom coordinate");
@@ -824,7 +827,7 @@ dfjk_status dfscf_create(dfjk_plan* pl, int32_t natom, const double* atom_xyz,
       wv.assign(grid_w, grid_w + npoint);
       xc_sort(pv, wv);
       const int64_t G = f->o.grid_chunk > 0 ? (f->o.grid_chunk + 255) / 256 * 256 : 8192;
-      xc_chunk(p.orb, nout, pv, G, f->o.ao_thresh, f->xcw);
+      if (!tunes(*f)) xc_chunk(p.orb, nout, pv, G, f->o.ao_thresh, f->xcw);
       upload(f->pts, pv);
       upload(f->wts, wv);
     }
@@ -897,7 +900,7 @@ dfjk_status dfscf_create(dfjk_plan* pl, int32_t natom, const double* atom_xyz,
     f->dE.alloc((size_t)f->o.diis_space * m * m * sizeof(double));
     DFJK_CUDA(cudaMemsetAsync(f->dE.p, 0, (size_t)f->o.diis_space * m * m * sizeof(double), s));
     DFJK_CUDA(cudaMemsetAsync(f->dF.p, 0, (size_t)f->o.diis_space * nn * sizeof(double), s));
-    if (npoint > 0 && f->o.grid_chunk <= 0 && has_xc(*f)) autotune_chunk(*f, nout, pv, s);
+    if (tunes(*f)) autotune_chunk(*f, nout, pv, s);
     DFJK_CUDA(cudaStreamSynchronize(s));
   });
   if (st != DFJK_OK) {

@@ -28,36 +28,59 @@ void launch_one_electron(const Context& c, const OrbView& ov, int nshell, const 
 // are not negligible anywhere in its bounding box (xc_prepare)
 constexpr int kXcMaxL = 3;   // orbital l the AO kernel evaluates (f)
 
+// What the kernels read about a chunk; the offsets (in doubles) lie within the
+// buffers of its group
+struct XcChunkInfo {
+  int nsig, ldp;             // functions of the chunk, and rounded up to even
+  int64_t g0, ng;            // first point and count
+  int64_t phi, pc, part;     // AO values (dphi at 3 phi), P block, V slices
+  int64_t ao;                // first entry of the compact AO map
+};
+
+// A run of chunks whose kernels share their launches: the chunks' AO values,
+// gradients and weighted AOs take at most kXcGroupBytes (or one chunk).
+constexpr int64_t kXcGroupBytes = (int64_t)256 << 20;
+struct XcGroup {
+  int first = 0, count = 0;            // chunks
+  int max_nsig = 0;
+  int e_off = 0, e_cnt[kXcMaxL + 1] = {};   // shell entries, by l
+};
+
 struct XcChunks {
   int64_t G = 0;                       // points per chunk (the last may hold fewer)
-  std::vector<int64_t> g0, ng;         // first point and count of each chunk
-  std::vector<int> sh_off, sh_cnt;     // each chunk's range in the shell list
-  std::vector<int> sh_lcnt;            // [chunk][l]: its shells of each l, in this order
-  std::vector<int64_t> ao_off;         // each chunk's range in the compact AO map
-  std::vector<int> ao_cnt;
-  int max_ao = 0;
-  int64_t total_ao = 0;                // sum of ao_cnt (the dense form would be nchunk * nao)
-  double gemm_flop = 0.0;              // FLOP of one evaluation's two products: sum 4 G ao_cnt^2
-  DevBuf d_sh, d_sh_out0, d_ao_map;    // shells, their first compact AO, compact -> AO
+  std::vector<XcChunkInfo> info;
+  std::vector<XcGroup> groups;
+  int64_t max_phi = 0, max_pc = 0, max_part = 0, max_points = 0;   // largest group, doubles
+  double gemm_flop = 0.0;              // FLOP of one evaluation's two products: sum 4 G nsig^2
+  // shell entries (shell, its first compact AO, chunk), by group and l; compact
+  // AO -> AO of each chunk; AO -> compact AO or -1 ([chunk][nao]); info
+  DevBuf d_e_sh, d_e_out0, d_e_chunk, d_ao_map, d_pos, d_info;
 };
 
 // XC on a point grid (xc.cu)
-// The chunks of one XC evaluation run on kXcBranches concurrent branches
-// (chunk k on branch k % kXcBranches), each with its own buffers, the
-// context's stream of that branch and its own V accumulator; one chunk's kernels fill only part
-// of the GPU. The accumulators are summed in branch order at the end and the
-// energy partials are per chunk, so the result does not depend on how the
-// branches interleave.
+// The groups of one XC evaluation run on up to kXcBranches concurrent branches
+// (group k on branch k % branches), each with its own buffers, the context's
+// stream of that branch and its own V accumulator, so that one group's kernels
+// fill the tails of another's. The accumulators are summed in branch order at
+// the end and the energy partials are per chunk, so the result does not depend
+// on how the branches interleave.
 struct XcBranch {
-  DevBuf phi, dphi, W;          // [nsig][G] AO values, 3 gradients, weighted AO
-  DevBuf Pc, Vc;                // P on a chunk's AOs, the slices of its V block
+  DevBuf phi, dphi, W;          // per chunk [nsig][G]: AO values, 3 gradients, weighted AO
+  DevBuf Pc, Vc;                // P on each chunk's AOs, the slices of its V block
+  DevBuf vals;                  // per chunk [4][G]: rho, grad rho, then v_rho / 2, v_grad
 };
+
+// branches of an evaluation unless the caller asks for another number. (H2O)_6 by
+// group size and branches, 1024-point chunks: 48 MB x 2 (both groups in L2)
+// 1900 us, 96 x 4 1250, 256 x 2 1205, 256 x 4 1108, 1024 x 1 1374: launches that
+// fill the device count for more than L2 residency.
+constexpr int kXcDefaultBranches = 4;
 
 struct XcWork {
   XcChunks ch;
-  int nbr = kXcBranches;        // branches in use, 1..kXcBranches
+  int nbr = kXcDefaultBranches; // branches in use, 1..kXcBranches
   XcBranch br[kXcBranches];
-  DevBuf Vacc;                  // kXcBranches x nao x nao: V accumulated per branch
+  DevBuf Vacc;                  // V accumulators (nao x nao), one or more per branch
   DevBuf ered;                  // energy partials per chunk and block
   // the evaluation's device work as a CUDA graph, captured on the second call
   // with the same arguments and replayed while they stay the same

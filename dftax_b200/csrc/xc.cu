@@ -12,16 +12,18 @@
 //   forward-mode dual numbers over the same expression as dftax's PBE
 //   (xc.py:87-252, PBE0 :584-601; points with rho <= 1e-10 contribute nothing,
 //   as the double-where of grid.py:31-44 makes them);
-//   W = v_rho/2 Phi + v_grad . dPhi                    (all of it: rho_w_kernel)
-//   V += Phi^T W on the float64 tensor cores                       (v_kernel);
+//   W = v_rho/2 Phi + v_grad . dPhi;
+//   V += Phi^T W on the float64 tensor cores;
 // and at the end Vxc = V + V^T, the symmetrized P-gradient of E_xc
-// (scf.py:42-46). The chunks run on kXcBranches concurrent streams (chunk k
-// on branch k % kXcBranches, one V accumulator each, summed in branch order
-// at the end); the energy is summed per block in a fixed order and then over
-// blocks on the host, so the result is reproducible. The SCF calls this with
-// the same buffers every iteration: the second call captures its launches
-// (about seven per chunk, the branches forked and joined by events) in a
-// CUDA graph and later calls replay it.
+// (scf.py:42-46). Small chunks keep few functions each and so cost the fewest
+// products, but one chunk's kernels fill a fraction of the device: runs of
+// chunks (groups) share their launches, and the groups run on two or more
+// concurrent streams (group k on branch k % branches, one V accumulator each,
+// summed in branch order at the end). The energy is summed per block in a fixed
+// order and then over blocks on the host, so the result is reproducible. The
+// SCF calls this with the same buffers every iteration: the second call
+// captures its launches (nine or ten per group, the branches forked and
+// joined by events) in a CUDA graph and later calls replay it.
 #include "dmma.cuh"
 #include "md_device.cuh"
 #include "scf.h"
@@ -153,188 +155,297 @@ __device__ __forceinline__ void ao_shell(const OrbView& ov, int s, double dx, do
   }
 }
 
-// Phi[k][g] (ld G), dPhi[x][k][g] for the chunk's shells of angular momentum
-// L: shell j of the list is orbital shell shl[j] with compact AOs k =
-// out0c[j] .. ; grid (ceil(G / 128), shells of the list). One instance per L,
-// so the s and p shells, most of the work, do not carry the registers of the
-// d and f cases.
+// Phi[k][g] (ld G), dPhi[x][k][g] of a group's shell entries of angular
+// momentum L: entry j is shell e_sh[j] of chunk e_chunk[j] with compact AOs k =
+// e_out0[j] .. ; grid (G / 128, entries / kAoPer), kAoPer entries per block (one
+// each made the launch of 90 000 blocks of 128 threads the bound). One instance
+// per L, so the s and p shells, most of the work, do not carry the registers of
+// the d and f cases.
+constexpr int kAoPer = 4;
 template <int L>
-__global__ void __launch_bounds__(kAoThreads) ao_kernel(OrbView ov, const int* __restrict__ shl,
-                                                        const int* __restrict__ out0c,
-                                                        const double* __restrict__ pts,
-                                                        int64_t g0, int64_t ng, int64_t G, int nsig,
+__global__ void __launch_bounds__(kAoThreads) ao_kernel(OrbView ov, const int* __restrict__ e_sh,
+                                                        const int* __restrict__ e_out0,
+                                                        const int* __restrict__ e_chunk, int nent,
+                                                        const XcChunkInfo* __restrict__ info,
+                                                        const double* __restrict__ pts, int64_t G,
                                                         double* __restrict__ phi,
                                                         double* __restrict__ dphi) {
   const int64_t g = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  const int s = shl[blockIdx.y];
-  if (g >= G) return;
   const ShellView& sh = ov.sh;
-  const int64_t o = (int64_t)out0c[blockIdx.y] * G + g;
-  const int64_t plane = (int64_t)nsig * G;
-  const bool live = g < ng;
-  double dx = 0.0, dy = 0.0, dz = 0.0;
-  if (live) {
-    const double* p = pts + 3 * (g0 + g);
-    dx = p[0] - sh.cen[3 * s];
-    dy = p[1] - sh.cen[3 * s + 1];
-    dz = p[2] - sh.cen[3 * s + 2];
+#pragma unroll 1
+  for (int q = 0; q < kAoPer; ++q) {
+    const int j = blockIdx.y * kAoPer + q;
+    if (j >= nent) return;
+    const int s = e_sh[j];
+    const XcChunkInfo& ci = info[e_chunk[j]];
+    const bool live = g < ci.ng;
+    double dx = 0.0, dy = 0.0, dz = 0.0;
+    if (live) {
+      const double* p = pts + 3 * (ci.g0 + g);
+      dx = p[0] - sh.cen[3 * s];
+      dy = p[1] - sh.cen[3 * s + 1];
+      dz = p[2] - sh.cen[3 * s + 2];
+    }
+    ao_shell<L>(ov, s, dx, dy, dz, live, (int64_t)e_out0[j] * G + g, G, (int64_t)ci.nsig * G,
+                phi + ci.phi, dphi + 3 * ci.phi);
   }
-  ao_shell<L>(ov, s, dx, dy, dz, live, o, G, plane, phi, dphi);
 }
 
-// Pc[k1][k2] = P[map[k1]][map[k2]], rows of ldp (nsig rounded up to even: the
-// copies of rho_w_kernel are 16 bytes wide), zero in the padding
+// Pc[k1][k2] = P[map[k1]][map[k2]] of chunk blockIdx.y of a group, rows of ldp
+// (nsig rounded up to even: the copies of rho_kernel are 16 bytes wide), zero
+// in the padding
 __global__ void gather_p_kernel(const double* __restrict__ P, int nao, const int* __restrict__ map,
-                                int nsig, int ldp, double* __restrict__ Pc) {
-  const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  if (i >= (int64_t)nsig * ldp) return;
-  const int64_t a = i / ldp, b = i % ldp;
-  Pc[i] = b < nsig ? P[(int64_t)map[a] * nao + map[b]] : 0.0;
+                                const XcChunkInfo* __restrict__ info, double* __restrict__ Pc) {
+  const XcChunkInfo& ci = info[blockIdx.y];
+  const int64_t n = (int64_t)ci.nsig * ci.ldp;
+  const int* mp = map + ci.ao;
+  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n;
+       i += (int64_t)gridDim.x * blockDim.x) {
+    const int64_t a = i / ci.ldp, b = i % ci.ldp;
+    Pc[ci.pc + i] = b < ci.nsig ? P[(int64_t)mp[a] * nao + mp[b]] : 0.0;
+  }
 }
 
-// V[map[k1]][map[k2]] += sum_z part[z][k1][k2], slices in order (the map is
-// one-to-one; V + V^T is taken at the end, so the product's order does not matter)
-__global__ void scatter_v_kernel(const double* __restrict__ part, int nslice, int nsig,
-                                 const int* __restrict__ map, int nao, double* __restrict__ V) {
+// V_y[m][n] += the group's chunks y, y + parts, ... (y = blockIdx.y) that hold
+// both functions, chunk by chunk and slice by slice (V + V^T is taken at the end,
+// so the products' order does not matter). nao^2 threads alone walk a small
+// molecule's 50 chunks in a chain (72 us a group for (H2O)_6): several
+// accumulators share it there.
+__global__ void reduce_v_kernel(const double* __restrict__ part, int nslice, int count,
+                                const XcChunkInfo* __restrict__ info, const int* __restrict__ pos,
+                                int nao, double* __restrict__ V) {
   const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  const int64_t nn = (int64_t)nsig * nsig;
-  if (i >= nn) return;
+  if (i >= (int64_t)nao * nao) return;
+  const int m = (int)(i / nao), n = (int)(i % nao);
   double s = 0.0;
-  for (int z = 0; z < nslice; ++z) s += part[z * nn + i];
-  V[(int64_t)map[i / nsig] * nao + map[i % nsig]] += s;
+  for (int k = blockIdx.y; k < count; k += gridDim.y) {
+    const int a = pos[(int64_t)k * nao + m], b = pos[(int64_t)k * nao + n];
+    if (a < 0 || b < 0) continue;
+    const XcChunkInfo& ci = info[k];
+    const int64_t nn = (int64_t)ci.nsig * ci.nsig;
+    const double* p = part + ci.part + (int64_t)a * ci.nsig + b;
+    for (int z = 0; z < nslice; ++z) s += p[z * nn];
+  }
+  V[blockIdx.y * (int64_t)nao * nao + i] += s;
 }
 
 // ---------------------------------------------------------------------------
-// PBE by forward-mode dual numbers: value and d/d(rho, gx, gy, gz)
+// PBE by forward-mode dual numbers. Exchange depends on the density and the norm
+// of its gradient, correlation on the density and its own (differently guarded)
+// norm: two derivatives carried through each, and the norms' derivatives by hand,
+// instead of four (rho, gx, gy, gz) through both.
 // ---------------------------------------------------------------------------
 
-struct D4 {
-  double v, d[4];
+struct D2 {
+  double v, d[2];
 };
-__device__ __forceinline__ D4 dc(double c) { return {c, {0.0, 0.0, 0.0, 0.0}}; }
-__device__ __forceinline__ D4 operator+(D4 a, D4 b) {
-  return {a.v + b.v, {a.d[0] + b.d[0], a.d[1] + b.d[1], a.d[2] + b.d[2], a.d[3] + b.d[3]}};
+__device__ __forceinline__ D2 dc(double c) { return {c, {0.0, 0.0}}; }
+__device__ __forceinline__ D2 operator+(D2 a, D2 b) {
+  return {a.v + b.v, {a.d[0] + b.d[0], a.d[1] + b.d[1]}};
 }
-__device__ __forceinline__ D4 operator*(D4 a, D4 b) {
-  D4 r;
+__device__ __forceinline__ D2 operator*(D2 a, D2 b) {
+  D2 r;
   r.v = a.v * b.v;
 #pragma unroll
-  for (int k = 0; k < 4; ++k) r.d[k] = a.d[k] * b.v + a.v * b.d[k];
+  for (int k = 0; k < 2; ++k) r.d[k] = a.d[k] * b.v + a.v * b.d[k];
   return r;
 }
 // quotient rule as (a' - (a/b) b') / b: one division
-__device__ __forceinline__ D4 operator/(D4 a, D4 b) {
-  D4 r;
+__device__ __forceinline__ D2 operator/(D2 a, D2 b) {
+  D2 r;
   const double ib = 1.0 / b.v;
   r.v = a.v * ib;
 #pragma unroll
-  for (int k = 0; k < 4; ++k) r.d[k] = (a.d[k] - r.v * b.d[k]) * ib;
+  for (int k = 0; k < 2; ++k) r.d[k] = (a.d[k] - r.v * b.d[k]) * ib;
   return r;
 }
-__device__ __forceinline__ D4 operator+(D4 a, double c) { a.v += c; return a; }
-__device__ __forceinline__ D4 operator+(double c, D4 a) { a.v += c; return a; }
-__device__ __forceinline__ D4 operator-(double c, D4 a) {
-  return {c - a.v, {-a.d[0], -a.d[1], -a.d[2], -a.d[3]}};
+__device__ __forceinline__ D2 operator+(D2 a, double c) { a.v += c; return a; }
+__device__ __forceinline__ D2 operator+(double c, D2 a) { a.v += c; return a; }
+__device__ __forceinline__ D2 operator-(double c, D2 a) {
+  return {c - a.v, {-a.d[0], -a.d[1]}};
 }
-__device__ __forceinline__ D4 operator*(D4 a, double c) {
-  return {a.v * c, {a.d[0] * c, a.d[1] * c, a.d[2] * c, a.d[3] * c}};
+__device__ __forceinline__ D2 operator*(D2 a, double c) {
+  return {a.v * c, {a.d[0] * c, a.d[1] * c}};
 }
-__device__ __forceinline__ D4 operator*(double c, D4 a) { return a * c; }
-__device__ __forceinline__ D4 operator/(D4 a, double c) { return a * (1.0 / c); }
-__device__ __forceinline__ D4 operator/(double c, D4 a) { return dc(c) / a; }
-__device__ __forceinline__ D4 dscale(D4 a, double f) {   // chain rule with df/dx = f
-  D4 r;
+__device__ __forceinline__ D2 operator*(double c, D2 a) { return a * c; }
+__device__ __forceinline__ D2 operator/(D2 a, double c) { return a * (1.0 / c); }
+__device__ __forceinline__ D2 operator/(double c, D2 a) { return dc(c) / a; }
+__device__ __forceinline__ D2 dscale(D2 a, double f) {   // chain rule with df/dx = f
+  D2 r;
 #pragma unroll
-  for (int k = 0; k < 4; ++k) r.d[k] = a.d[k] * f;
+  for (int k = 0; k < 2; ++k) r.d[k] = a.d[k] * f;
   return r;
 }
-__device__ __forceinline__ D4 dsqrt(D4 a) {
+__device__ __forceinline__ D2 dsqrt(D2 a) {
   const double q = sqrt(a.v);
-  D4 r = dscale(a, 0.5 / q);
+  D2 r = dscale(a, 0.5 / q);
   r.v = q;
   return r;
 }
 // a^(1/3) for a > 0, with d/da = a^(1/3) / (3 a)
-__device__ __forceinline__ D4 dcbrt(D4 a) {
+__device__ __forceinline__ D2 dcbrt(D2 a) {
   const double q = cbrt(a.v);
-  D4 r = dscale(a, q / (3.0 * a.v));
+  D2 r = dscale(a, q / (3.0 * a.v));
   r.v = q;
   return r;
 }
-__device__ __forceinline__ D4 dlog1p(D4 a) {
-  D4 r = dscale(a, 1.0 / (1.0 + a.v));
+__device__ __forceinline__ D2 dlog1p(D2 a) {
+  D2 r = dscale(a, 1.0 / (1.0 + a.v));
   r.v = log1p(a.v);
   return r;
 }
-__device__ __forceinline__ D4 dexpm1(D4 a) {
+__device__ __forceinline__ D2 dexpm1(D2 a) {
   const double q = expm1(a.v);
-  D4 r = dscale(a, a.v > -0.5 ? q + 1.0 : exp(a.v));   // e^a = expm1(a) + 1 without cancellation
+  D2 r = dscale(a, a.v > -0.5 ? q + 1.0 : exp(a.v));   // e^a = expm1(a) + 1 without cancellation
   r.v = q;
   return r;
 }
 // jnp.clip(x, lo): the bound itself (derivative 0) below lo
-__device__ __forceinline__ D4 dclip(D4 a, double lo) { return a.v < lo ? dc(lo) : a; }
+__device__ __forceinline__ D2 dclip(D2 a, double lo) { return a.v < lo ? dc(lo) : a; }
 
-// eps_xc per particle of x_scale PBE exchange + c_scale PBE correlation,
-// unpolarized (xc.py: PBEExchange._unpolarized, PBECorrelation with zeta = 0)
-__device__ D4 pbe_eps(D4 rho, D4 gx, D4 gy, D4 gz, double xs, double cs) {
+// eps per particle of PBE exchange, unpolarized (xc.py: PBEExchange._unpolarized);
+// gnorm = |grad rho + 1e-30|
+__device__ __forceinline__ D2 pbe_x(D2 rho, D2 gnorm) {
   constexpr double pi = 3.141592653589793;
-  // exchange
-  const D4 ax = gx + 1e-30, ay = gy + 1e-30, az = gz + 1e-30;
-  const D4 gnorm = dsqrt(ax * ax + ay * ay + az * az);
-  const D4 kF = dcbrt(3 * pi * pi * rho + 1e-30);
-  const D4 s = gnorm / dclip(2 * kF * rho, 1e-30);
+  const D2 kF = dcbrt(3 * pi * pi * rho + 1e-30);
+  const D2 s = gnorm / dclip(2 * kF * rho, 1e-30);
   const double kappa = 0.804, mu = 0.2195149727645171;
-  const D4 ex_unif = -3 * kF / (4 * pi);
-  const D4 fx = 1 + kappa - kappa / (1 + mu * s * s / kappa);
-  const D4 ex = ex_unif * fx;
-  // correlation: PW92 paramagnetic channel + PBE H with phi = 1
+  const D2 ex_unif = -3 * kF / (4 * pi);
+  const D2 fx = 1 + kappa - kappa / (1 + mu * s * s / kappa);
+  return ex_unif * fx;
+}
+
+// eps per particle of PBE correlation with zeta = 0 (xc.py: PBECorrelation): PW92
+// paramagnetic channel + PBE H with phi = 1; gn = sqrt(|grad rho|^2 + 1e-30)
+__device__ __forceinline__ D2 pbe_c(D2 rho, D2 gn) {
+  constexpr double pi = 3.141592653589793;
   const double gamma = (1.0 - 0.6931471805599453) / (pi * pi);
   const double beta = 0.06672455060314922;
   const double A = 0.0310907, a1 = 0.21370, b1 = 7.5957, b2 = 3.5876, b3 = 1.6382, b4 = 0.49294;
-  const D4 rt = dclip(rho, 1e-20);
-  const D4 rs = dcbrt(3 / (4 * pi * rt) + 1e-20);
-  const D4 rss = dsqrt(rs);
-  const D4 den = 2.0 * A * (b1 * rss + b2 * rs + b3 * rs * rss + b4 * rs * rs);
-  const D4 eps_pw = -2.0 * A * (1.0 + a1 * rs) * dlog1p(1.0 / dclip(den, 1e-20));
-  const D4 kf = dcbrt(3 * pi * pi * rt + 1e-20);
-  const D4 ks = dsqrt(4 * kf / pi);
-  const D4 gn = dsqrt(gx * gx + gy * gy + gz * gz + 1e-30);
-  const D4 t = gn / dclip(2 * ks * rt, 1e-20);
-  const D4 dA = gamma * dexpm1(-1.0 * eps_pw / gamma);
-  const D4 Ac = beta / dclip(dA, 1e-20);
-  const D4 t2 = t * t;
-  const D4 f1 = t2 + Ac * (t2 * t2);
-  const D4 frac = beta * f1 / dclip(gamma * (1.0 + Ac * f1), 1e-20);
-  const D4 H = gamma * dlog1p(frac);
-  return xs * ex + cs * (eps_pw + H);
+  const D2 rt = dclip(rho, 1e-20);
+  const D2 rs = dcbrt(3 / (4 * pi * rt) + 1e-20);
+  const D2 rss = dsqrt(rs);
+  const D2 den = 2.0 * A * (b1 * rss + b2 * rs + b3 * rs * rss + b4 * rs * rs);
+  const D2 eps_pw = -2.0 * A * (1.0 + a1 * rs) * dlog1p(1.0 / dclip(den, 1e-20));
+  const D2 kf = dcbrt(3 * pi * pi * rt + 1e-20);
+  const D2 ks = dsqrt(4 * kf / pi);
+  const D2 t = gn / dclip(2 * ks * rt, 1e-20);
+  const D2 dA = gamma * dexpm1(-1.0 * eps_pw / gamma);
+  const D2 Ac = beta / dclip(dA, 1e-20);
+  const D2 t2 = t * t;
+  const D2 f1 = t2 + Ac * (t2 * t2);
+  const D2 frac = beta * f1 / dclip(gamma * (1.0 + Ac * f1), 1e-20);
+  return eps_pw + gamma * dlog1p(frac);
 }
 
-// One block: 64 points of a chunk, everything between the AO values and V.
+// per point of chunk blockIdx.y: rho, grad in, v_rho / 2, v_grad (weighted) out in
+// place (vals [4][G] per chunk); e per block
+constexpr int kPtThreads = 128;
+__global__ void __launch_bounds__(kPtThreads) pbe_kernel(double* __restrict__ vals,
+                                                         const XcChunkInfo* __restrict__ info,
+                                                         int64_t G, const double* __restrict__ wts,
+                                                         double xs, double cs, double thresh,
+                                                         double* __restrict__ eg) {
+  __shared__ double red[kPtThreads / 32];
+  const XcChunkInfo ci = info[blockIdx.y];
+  const int64_t g = blockIdx.x * (int64_t)kPtThreads + threadIdx.x;
+  double* v = vals + blockIdx.y * 4 * G + g;
+  double e = 0.0, vr = 0.0, v0 = 0.0, v1 = 0.0, v2 = 0.0;
+  const double r = g < ci.ng ? v[0] : 0.0;
+  if (r > thresh) {
+    const double w = wts[ci.g0 + g], gx = v[G], gy = v[2 * G], gz = v[3 * G];
+    const double ax = gx + 1e-30, ay = gy + 1e-30, az = gz + 1e-30;
+    const double na = sqrt(ax * ax + ay * ay + az * az);
+    const double nb = sqrt(gx * gx + gy * gy + gz * gz + 1e-30);
+    const D2 R = {r, {1.0, 0.0}};
+    const D2 fx = R * (xs * pbe_x(R, D2{na, {0.0, 1.0}}));
+    const D2 fc = R * (cs * pbe_c(R, D2{nb, {0.0, 1.0}}));
+    e = w * (fx.v + fc.v);
+    vr = 0.5 * w * (fx.d[0] + fc.d[0]);
+    const double qa = w * fx.d[1] / na, qb = w * fc.d[1] / nb;
+    v0 = qa * ax + qb * gx;
+    v1 = qa * ay + qb * gy;
+    v2 = qa * az + qb * gz;
+  }
+  v[0] = vr;
+  v[G] = v0;
+  v[2 * G] = v1;
+  v[3 * G] = v2;
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) e += __shfl_xor_sync(0xffffffffu, e, o);
+  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = e;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+#pragma unroll
+    for (int q = 1; q < kPtThreads / 32; ++q) e += red[q];
+    eg[blockIdx.y * (int64_t)gridDim.x + blockIdx.x] = e;
+  }
+}
+
+// W[mu][g] = v_rho/2 Phi + v_grad . dPhi of chunk blockIdx.z: two points per
+// thread (16-byte accesses), kWPer functions per block. Bound by memory: 40 bytes
+// per function and point.
+constexpr int kWThreads = 128, kWPer = 8;
+__global__ void __launch_bounds__(kWThreads) w_kernel(const double* __restrict__ phig,
+                                                      const double* __restrict__ dphig,
+                                                      const double* __restrict__ vals,
+                                                      const XcChunkInfo* __restrict__ info, int64_t G,
+                                                      double* __restrict__ Wg) {
+  const XcChunkInfo ci = info[blockIdx.z];
+  const int c0 = blockIdx.y * kWPer;
+  if (c0 >= ci.nsig) return;
+  const int64_t g = 2 * (blockIdx.x * (int64_t)kWThreads + threadIdx.x);   // G is a multiple of 256
+  const int64_t plane = (int64_t)ci.nsig * G;
+  const double* phi = phig + ci.phi + g;
+  const double* dphi = dphig + 3 * ci.phi + g;
+  double* W = Wg + ci.phi + g;
+  double2 v[4];
+#pragma unroll
+  for (int d = 0; d < 4; ++d)
+    v[d] = *reinterpret_cast<const double2*>(vals + (blockIdx.z * 4 + d) * G + g);
+#pragma unroll
+  for (int q = 0; q < kWPer; ++q) {
+    const int c = c0 + q;
+    if (c >= ci.nsig) break;
+    const int64_t o = c * G;
+    const double2 f = __ldg(reinterpret_cast<const double2*>(phi + o));
+    double2 s = make_double2(v[0].x * f.x, v[0].y * f.y);
+#pragma unroll
+    for (int d = 0; d < 3; ++d) {
+      const double2 t = __ldg(reinterpret_cast<const double2*>(dphi + d * plane + o));
+      s.x += v[1 + d].x * t.x;
+      s.y += v[1 + d].y * t.y;
+    }
+    *reinterpret_cast<double2*>(W + o) = s;
+  }
+}
+
+// rho and grad rho of 64 points of a chunk per block (grid (G / 64, chunks of the
+// group)), without X in memory:
 //   * X = Phi Pc for all nsig functions, 64 columns at a time, on the float64
 //     tensor cores: 16 functions per step through a four-stage cp.async ring
 //     that runs on across the column blocks (the order of points and columns
 //     inside a fragment is free: a lane's pair of fragments is one 16-byte load);
 //   * after each column block the lane's X meets Phi and dPhi of the same
-//     (point, function) pairs and adds to rho and grad rho; X is never stored;
-//   * the partial sums of a point's lanes are added in a fixed order, 64 threads
-//     evaluate the functional, and the block writes W for its points while
-//     their Phi and dPhi are still in the caches.
-// As five launches per chunk (DGEMM, density, functional, weights, with X and
-// the density arrays in memory between them) (H2O)_6 took 1523 us per
-// evaluation, its DGEMMs at 7-11 TFLOP/s on 165 functions.
+//     (point, function) pairs and adds to rho and grad rho;
+//   * the partial sums of a point's lanes are added in a fixed order.
+// As a cuBLAS DGEMM and a density kernel per chunk (H2O)_6 took 800 us. (With the
+// functional and W in the same block, 64 of 256 threads on the former, a block
+// took twice as long: 689 us per evaluation against the split kernels' sum.)
 constexpr int kRpPts = 64, kRpCols = 64, kRpK = 16, kRpPitch = 68, kRpStages = 4;
 constexpr int kRpStage = 2 * kRpK * kRpPitch;   // doubles
 constexpr size_t kRpSmem = (size_t)kRpStages * kRpStage * sizeof(double);
 
-__global__ void __launch_bounds__(256, 2) rho_w_kernel(
-    const double* __restrict__ Pc, int ldp, const double* __restrict__ phi,
-    const double* __restrict__ dphi, int nsig, int64_t G, const double* __restrict__ w, int64_t ng,
-    double xs, double cs, double thresh, double* __restrict__ W, double* __restrict__ ered) {
+__global__ void __launch_bounds__(256, 3) rho_kernel(
+    const double* __restrict__ Pg, const double* __restrict__ phig, const double* __restrict__ dphig,
+    const XcChunkInfo* __restrict__ info, int64_t G, double* __restrict__ vals) {
+  const XcChunkInfo ci = info[blockIdx.y];
+  const int nsig = ci.nsig, ldp = ci.ldp;
+  const double* Pc = Pg + ci.pc;
+  const double* phi = phig + ci.phi;
+  const double* dphi = dphig + 3 * ci.phi;
   extern __shared__ __align__(16) double rsm[];
   __shared__ double red[2][4][kRpPts];   // per column half: rho, grad
-  __shared__ double sv[4][kRpPts];       // v_rho / 2, v_grad (weighted)
-  __shared__ double se[kRpPts];
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int wx = (warp & 3) * 16, wi = (warp >> 2) * 32;
   const int fr = lane >> 2, fk = lane & 3;
@@ -430,57 +541,14 @@ __global__ void __launch_bounds__(256, 2) rho_w_kernel(
       if (fk == 0) red[warp >> 2][d][wx + 2 * fr + a] = s;
     }
   __syncthreads();
-  if (tid < kRpPts) {
-    const int64_t g = g0 + tid;
-    double e = 0.0, vr = 0.0, v0 = 0.0, v1 = 0.0, v2 = 0.0;
-    const double r = red[0][0][tid] + red[1][0][tid];
-    if (g < ng && r > thresh) {
-      const double wg = w[g];
-      const D4 R = {r, {1.0, 0.0, 0.0, 0.0}};
-      const D4 X = {2.0 * (red[0][1][tid] + red[1][1][tid]), {0.0, 1.0, 0.0, 0.0}};
-      const D4 Y = {2.0 * (red[0][2][tid] + red[1][2][tid]), {0.0, 0.0, 1.0, 0.0}};
-      const D4 Z = {2.0 * (red[0][3][tid] + red[1][3][tid]), {0.0, 0.0, 0.0, 1.0}};
-      const D4 f = R * pbe_eps(R, X, Y, Z, xs, cs);
-      e = wg * f.v;
-      vr = wg * f.d[0];
-      v0 = wg * f.d[1];
-      v1 = wg * f.d[2];
-      v2 = wg * f.d[3];
-    }
-    se[tid] = e;
-    sv[0][tid] = 0.5 * vr;
-    sv[1][tid] = v0;
-    sv[2][tid] = v1;
-    sv[3][tid] = v2;
-  }
-  __syncthreads();
-  if (warp == 0) {
-    double e = se[lane] + se[lane + 32];
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) e += __shfl_xor_sync(0xffffffffu, e, o);
-    if (lane == 0) ered[blockIdx.x] = e;
-  }
-  if (!W) return;
-  // W[mu][g] = v_rho/2 Phi + v_grad . dPhi: two points per lane, a function per warp
-  double2 v[4];
-#pragma unroll
-  for (int d = 0; d < 4; ++d) v[d] = make_double2(sv[d][2 * lane], sv[d][2 * lane + 1]);
-#pragma unroll 2
-  for (int c = warp; c < nsig; c += 8) {
-    const int64_t o = c * G + g0 + 2 * lane;
-    const double2 f = __ldg(reinterpret_cast<const double2*>(phi + o));
-    double2 s = make_double2(v[0].x * f.x, v[0].y * f.y);
-#pragma unroll
-    for (int d = 0; d < 3; ++d) {
-      const double2 t = __ldg(reinterpret_cast<const double2*>(dphi + d * plane + o));
-      s.x += v[1 + d].x * t.x;
-      s.y += v[1 + d].y * t.y;
-    }
-    *reinterpret_cast<double2*>(W + o) = s;
+  {
+    const int d = tid / kRpPts, g = tid % kRpPts;   // 256 threads: four sums of 64 points
+    vals[(blockIdx.y * 4 + d) * G + g0 + g] = (d == 0 ? 1.0 : 2.0) * (red[0][d][g] + red[1][d][g]);
   }
 }
 
-// part[z][mu][nu] = sum_g Phi[mu][g] W[nu][g] over slice z of kVSlice points:
+// part[z][mu][nu] = sum_g Phi[mu][g] W[nu][g] over slice z = blockIdx.y of
+// kVSlice points of chunk blockIdx.z (tile blockIdx.x, of the chunk's own count):
 // 64 x 64 tiles on the float64 tensor cores, both operands staged as they lie
 // (16 points a step, the 16-byte piece index xor 4 (row % 2): load phases of
 // two rows x four pieces fall in distinct banks; the point order inside a step
@@ -490,12 +558,18 @@ __global__ void __launch_bounds__(256, 2) rho_w_kernel(
 constexpr int kVT = 64, kVK = 16, kVStages = 4, kVSlice = 512;
 constexpr size_t kVSmem = (size_t)kVStages * 2 * kVT * kVK * sizeof(double);
 
-__global__ void __launch_bounds__(256, 2) v_kernel(const double* __restrict__ phi,
-                                                   const double* __restrict__ W, int nsig, int64_t G,
+__global__ void __launch_bounds__(256, 3) v_kernel(const double* __restrict__ phig,
+                                                   const double* __restrict__ Wg,
+                                                   const XcChunkInfo* __restrict__ info, int64_t G,
                                                    double* __restrict__ part) {
   extern __shared__ __align__(16) double vsm[];
-  const int r0 = blockIdx.x * kVT, c0 = blockIdx.y * kVT;
-  const int64_t k0 = blockIdx.z * (int64_t)kVSlice;
+  const XcChunkInfo ci = info[blockIdx.z];
+  const int nsig = ci.nsig, nt = (nsig + kVT - 1) / kVT;
+  if ((int)blockIdx.x >= nt * nt) return;
+  const double* phi = phig + ci.phi;
+  const double* W = Wg + ci.phi;
+  const int r0 = (int)blockIdx.x / nt * kVT, c0 = (int)blockIdx.x % nt * kVT;
+  const int64_t k0 = blockIdx.y * (int64_t)kVSlice;
   const int64_t k1 = k0 + kVSlice < G ? k0 + kVSlice : G;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int wr = (warp & 3) * 16, wc = (warp >> 2) * 32;
@@ -552,7 +626,7 @@ __global__ void __launch_bounds__(256, 2) v_kernel(const double* __restrict__ ph
     }
   }
   if (!work) return;
-  double* out = part + blockIdx.z * (int64_t)nsig * nsig;
+  double* out = part + ci.part + blockIdx.y * (int64_t)nsig * nsig;
 #pragma unroll
   for (int a = 0; a < 2; ++a) {
     const int r = r0 + wr + 8 * a + fr;
@@ -631,10 +705,10 @@ static uint64_t morton3(uint64_t x, uint64_t y, uint64_t z) {
 void xc_sort(std::vector<double>& pts, std::vector<double>& w) {
   const int64_t n = (int64_t)w.size();
   if (n == 0) return;
-  // contiguous index ranges, one per host thread (one thread below 64 k points)
-  const int T = n < ((int64_t)1 << 16)
-                    ? 1
-                    : (int)std::min<unsigned>(16, std::max(1u, std::thread::hardware_concurrency()));
+  // contiguous index ranges of at least 32 k points, one per host thread (starting
+  // 15 threads for each of the seven passes cost more than sorting 100 k points)
+  const int T = (int)std::max<int64_t>(
+      1, std::min<int64_t>(n >> 15, std::min<unsigned>(16, std::max(1u, std::thread::hardware_concurrency()))));
   auto lo_of = [&](int t) { return n * t / T; };
   // Morton order of 1-Bohr cells
   std::vector<double> los((size_t)3 * T, INFINITY);
@@ -703,18 +777,22 @@ void xc_sort(std::vector<double>& pts, std::vector<double>& w) {
   w.swap(w2);
 }
 
+// slices of a chunk's V product
+static int64_t xc_slices(int64_t G) { return (G + kVSlice - 1) / kVSlice; }
+
+// V accumulators per branch: enough that their nao^2 threads each come to about
+// 2^18
+static int64_t v_parts(int64_t nao) {
+  return std::min<int64_t>(8, std::max<int64_t>(1, ((int64_t)1 << 18) / (nao * nao)));
+}
+
 void xc_chunk(const Shells& sh, const int (&nout)[8], const std::vector<double>& pts, int64_t G,
               double thresh, XcWork& ws) {
   XcChunks& out = ws.ch;
   const int64_t n = (int64_t)pts.size() / 3;
-  out.g0.clear();
-  out.ng.clear();
-  out.sh_off.clear();
-  out.sh_cnt.clear();
-  out.ao_off.clear();
-  out.ao_cnt.clear();
-  out.max_ao = 0;
-  out.total_ao = 0;
+  out.info.clear();
+  out.groups.clear();
+  out.max_phi = out.max_pc = out.max_part = out.max_points = 0;
   out.gemm_flop = 0.0;
   out.G = G;
   if (ws.exec) cudaGraphExecDestroy(ws.exec);
@@ -737,8 +815,36 @@ void xc_chunk(const Shells& sh, const int (&nout)[8], const std::vector<double>&
     }
     return b;
   };
-  std::vector<int> shl, out0c, aomap;
-  out.sh_lcnt.clear();
+  const int nao = sh.nout;
+  std::vector<int> aomap, pos;
+  struct Entry {
+    int sh, out0, chunk;
+  };
+  std::vector<Entry> ents[kXcMaxL + 1];   // of the open group, by l
+  std::vector<int> e_sh, e_out0, e_chunk;
+  XcGroup grp;
+  int64_t phi = 0, pc = 0, part = 0;
+  const int64_t nslice = xc_slices(G);
+  auto close = [&] {
+    if (grp.count == 0) return;
+    grp.e_off = (int)e_sh.size();
+    for (int l = 0; l <= kXcMaxL; ++l) {
+      grp.e_cnt[l] = (int)ents[l].size();
+      for (const Entry& e : ents[l]) {
+        e_sh.push_back(e.sh);
+        e_out0.push_back(e.out0);
+        e_chunk.push_back(e.chunk);
+      }
+      ents[l].clear();
+    }
+    out.max_phi = std::max(out.max_phi, phi);
+    out.max_pc = std::max(out.max_pc, pc);
+    out.max_part = std::max(out.max_part, part);
+    out.max_points = std::max(out.max_points, grp.count * G);
+    out.groups.push_back(grp);
+    grp = XcGroup{};
+    phi = pc = part = 0;
+  };
   for (int64_t g0 = 0; g0 < n; g0 += G) {
     const int64_t ng = std::min(G, n - g0);
     double bl[3] = {INFINITY, INFINITY, INFINITY}, bh[3] = {-INFINITY, -INFINITY, -INFINITY};
@@ -747,11 +853,11 @@ void xc_chunk(const Shells& sh, const int (&nout)[8], const std::vector<double>&
         bl[d] = std::min(bl[d], pts[3 * i + d]);
         bh[d] = std::max(bh[d], pts[3 * i + d]);
       }
-    out.g0.push_back(g0);
-    out.ng.push_back(ng);
-    out.sh_off.push_back((int)shl.size());
-    out.ao_off.push_back((int64_t)aomap.size());
-    int nao_c = 0;
+    std::vector<Entry> mine;
+    int nsig = 0;
+    const int64_t ao = (int64_t)aomap.size();
+    pos.resize(pos.size() + nao, -1);
+    int* ps = pos.data() + pos.size() - nao;
     for (int s = 0; s < sh.n; ++s) {
       double d2 = 0.0;
       for (int d = 0; d < 3; ++d) {
@@ -760,43 +866,37 @@ void xc_chunk(const Shells& sh, const int (&nout)[8], const std::vector<double>&
         d2 += e * e;
       }
       if (bound(s, std::sqrt(d2)) <= thresh) continue;
-      shl.push_back(s);
-      out0c.push_back(nao_c);
+      mine.push_back({s, nsig, 0});
       const int no = nout[sh.l[s]];
-      for (int m = 0; m < no; ++m) aomap.push_back(sh.out0[s] + m);
-      nao_c += no;
-    }
-    out.sh_cnt.push_back((int)shl.size() - out.sh_off.back());
-    // this chunk's shells grouped by l (stable), each keeping its compact
-    // AOs: only the launch order changes, not the layout of Phi
-    {
-      const int j0 = out.sh_off.back(), j1 = (int)shl.size();
-      std::vector<std::pair<int, int>> seg;
-      int cnt[kXcMaxL + 1] = {};
-      for (int j = j0; j < j1; ++j) {
-        const int l = std::min<int>(sh.l[shl[j]], kXcMaxL);
-        seg.push_back({shl[j], out0c[j]});
-        ++cnt[l];
+      for (int m = 0; m < no; ++m) {
+        aomap.push_back(sh.out0[s] + m);
+        ps[sh.out0[s] + m] = nsig + m;
       }
-      int pos = j0;
-      for (int l = 0; l <= kXcMaxL; ++l) {
-        for (const auto& e : seg)
-          if (std::min<int>(sh.l[e.first], kXcMaxL) == l) {
-            shl[pos] = e.first;
-            out0c[pos] = e.second;
-            ++pos;
-          }
-        out.sh_lcnt.push_back(cnt[l]);
-      }
+      nsig += no;
     }
-    out.ao_cnt.push_back(nao_c);
-    out.max_ao = std::max(out.max_ao, nao_c);
-    out.total_ao += nao_c;
-    out.gemm_flop += 4.0 * (double)G * nao_c * nao_c;   // X = Phi P and Phi^T W
+    // AO values, three gradients and the weighted AOs: 40 bytes per function and point
+    if (grp.count > 0 && (phi + (int64_t)nsig * G) * 40 > kXcGroupBytes) close();
+    XcChunkInfo ci{nsig, nsig + (nsig & 1), g0, ng, phi, pc, part, ao};
+    if (grp.count == 0) grp.first = (int)out.info.size();
+    for (Entry e : mine) {
+      e.chunk = grp.count;
+      ents[std::min<int>(sh.l[e.sh], kXcMaxL)].push_back(e);
+    }
+    ++grp.count;
+    grp.max_nsig = std::max(grp.max_nsig, nsig);
+    phi += (int64_t)nsig * G;
+    pc += (int64_t)nsig * ci.ldp;
+    part += nslice * nsig * nsig;
+    out.info.push_back(ci);
+    out.gemm_flop += 4.0 * (double)G * nsig * nsig;   // X = Phi P and Phi^T W
   }
-  upload(out.d_sh, shl);
-  upload(out.d_sh_out0, out0c);
+  close();
+  upload(out.d_e_sh, e_sh);
+  upload(out.d_e_out0, e_out0);
+  upload(out.d_e_chunk, e_chunk);
   upload(out.d_ao_map, aomap);
+  upload(out.d_pos, pos);
+  upload(out.d_info, out.info);
 }
 
 // enqueues one evaluation's device work on s (buffers already sized)
@@ -807,63 +907,68 @@ static void xc_enqueue(const Context& c, const OrbView& ov, const double* pts, c
   const int64_t nn = (int64_t)nao * nao;
   const XcChunks& ch = ws.ch;
   const int64_t G = ch.G;
-  const int64_t nchunk = (int64_t)ch.g0.size();
-  const int64_t nblk = G / kRpPts;
-  const int nslice = (int)((G + kVSlice - 1) / kVSlice);
+  const int64_t nblk = G / kPtThreads;
+  const int nslice = (int)xc_slices(G);
+  const int64_t parts = v_parts(nao);
   const int nb = std::min(std::max(ws.nbr, 1), kXcBranches);
   // fork: every branch starts after the caller's prior work on s
   DFJK_CUDA(cudaEventRecord(c.side_fork, s));
   for (int q = 0; q < nb; ++q) DFJK_CUDA(cudaStreamWaitEvent(c.side_stream[q], c.side_fork, 0));
   if (Vxc)
     for (int q = 0; q < nb; ++q)
-      DFJK_CUDA(cudaMemsetAsync(ws.Vacc.as<double>() + q * nn, 0, nn * sizeof(double),
+      DFJK_CUDA(cudaMemsetAsync(ws.Vacc.as<double>() + q * parts * nn, 0, parts * nn * sizeof(double),
                                 c.side_stream[q]));
-  for (int64_t k = 0; k < nchunk; ++k) {
+  for (size_t k = 0; k < ch.groups.size(); ++k) {
+    const XcGroup& gr = ch.groups[k];
     XcBranch& b = ws.br[k % nb];
     cudaStream_t bs = c.side_stream[k % nb];
-    double* Vacc = ws.Vacc.as<double>() + (k % nb) * nn;
-    const int64_t g0 = ch.g0[k], ng = ch.ng[k];
-    const int nsig = ch.ao_cnt[k], ldp = nsig + (nsig & 1);
-    const int* map = ch.d_ao_map.as<int>() + ch.ao_off[k];
-    if (nsig == 0) {
-      DFJK_CUDA(cudaMemsetAsync(ws.ered.as<double>() + k * nblk, 0, nblk * sizeof(double), bs));
-      continue;
-    }
-    // the chunk's shells are grouped by l: one launch per l present
-    int j0 = ch.sh_off[k];
+    double* Vacc = ws.Vacc.as<double>() + (k % nb) * parts * nn;
+    const XcChunkInfo* info = ch.d_info.as<XcChunkInfo>() + gr.first;
+    double* phi = b.phi.as<double>();
+    double* dphi = b.dphi.as<double>();
+    // the group's shell entries lie by l: one launch per l present
+    int j0 = gr.e_off;
     for (int l = 0; l < kXcMaxL + 1; ++l) {
-      const int cnt = ch.sh_lcnt[(size_t)k * (kXcMaxL + 1) + l];
+      const int cnt = gr.e_cnt[l];
       if (cnt == 0) continue;
-      const dim3 grid((unsigned)((G + kAoThreads - 1) / kAoThreads), (unsigned)cnt);
-      const int* shl = ch.d_sh.as<int>() + j0;
-      const int* o0 = ch.d_sh_out0.as<int>() + j0;
-      double* ph = b.phi.as<double>();
-      double* dph = b.dphi.as<double>();
+      const dim3 grid((unsigned)((G + kAoThreads - 1) / kAoThreads), (unsigned)((cnt + kAoPer - 1) / kAoPer));
+      const int* es = ch.d_e_sh.as<int>() + j0;
+      const int* eo = ch.d_e_out0.as<int>() + j0;
+      const int* ec = ch.d_e_chunk.as<int>() + j0;
       switch (l) {
-        case 0: ao_kernel<0><<<grid, kAoThreads, 0, bs>>>(ov, shl, o0, pts, g0, ng, G, nsig, ph, dph); break;
-        case 1: ao_kernel<1><<<grid, kAoThreads, 0, bs>>>(ov, shl, o0, pts, g0, ng, G, nsig, ph, dph); break;
-        case 2: ao_kernel<2><<<grid, kAoThreads, 0, bs>>>(ov, shl, o0, pts, g0, ng, G, nsig, ph, dph); break;
-        default: ao_kernel<3><<<grid, kAoThreads, 0, bs>>>(ov, shl, o0, pts, g0, ng, G, nsig, ph, dph); break;
+        case 0: ao_kernel<0><<<grid, kAoThreads, 0, bs>>>(ov, es, eo, ec, cnt, info, pts, G, phi, dphi); break;
+        case 1: ao_kernel<1><<<grid, kAoThreads, 0, bs>>>(ov, es, eo, ec, cnt, info, pts, G, phi, dphi); break;
+        case 2: ao_kernel<2><<<grid, kAoThreads, 0, bs>>>(ov, es, eo, ec, cnt, info, pts, G, phi, dphi); break;
+        default: ao_kernel<3><<<grid, kAoThreads, 0, bs>>>(ov, es, eo, ec, cnt, info, pts, G, phi, dphi); break;
       }
       DFJK_LAUNCHED();
       j0 += cnt;
     }
-    gather_p_kernel<<<(unsigned)(((int64_t)nsig * ldp + 255) / 256), 256, 0, bs>>>(
-        P, nao, map, nsig, ldp, b.Pc.as<double>());
-    DFJK_LAUNCHED();
-    rho_w_kernel<<<(unsigned)nblk, 256, kRpSmem, bs>>>(
-        b.Pc.as<double>(), ldp, b.phi.as<double>(), b.dphi.as<double>(), nsig, G, w + g0, ng,
-        xp.x_scale, xp.c_scale, xp.rho_thresh, Vxc ? b.W.as<double>() : nullptr,
-        ws.ered.as<double>() + k * nblk);
-    DFJK_LAUNCHED();
-    if (Vxc) {
-      // Vc = Phi^T W by slices, scattered into this branch's V
-      const unsigned nt = (unsigned)((nsig + kVT - 1) / kVT);
-      v_kernel<<<dim3(nt, nt, (unsigned)nslice), 256, kVSmem, bs>>>(
-          b.phi.as<double>(), b.W.as<double>(), nsig, G, b.Vc.as<double>());
+    if (gr.max_nsig > 0) {
+      const int64_t pn = (int64_t)gr.max_nsig * (gr.max_nsig + 1);
+      gather_p_kernel<<<dim3((unsigned)std::min<int64_t>(64, (pn + 255) / 256), (unsigned)gr.count), 256, 0, bs>>>(
+          P, nao, ch.d_ao_map.as<int>(), info, b.Pc.as<double>());
       DFJK_LAUNCHED();
-      scatter_v_kernel<<<(unsigned)(((int64_t)nsig * nsig + 255) / 256), 256, 0, bs>>>(
-          b.Vc.as<double>(), nslice, nsig, map, nao, Vacc);
+    }
+    rho_kernel<<<dim3((unsigned)(G / kRpPts), (unsigned)gr.count), 256, kRpSmem, bs>>>(
+        b.Pc.as<double>(), phi, dphi, info, G, b.vals.as<double>());
+    DFJK_LAUNCHED();
+    pbe_kernel<<<dim3((unsigned)nblk, (unsigned)gr.count), kPtThreads, 0, bs>>>(
+        b.vals.as<double>(), info, G, w, xp.x_scale, xp.c_scale, xp.rho_thresh,
+        ws.ered.as<double>() + gr.first * nblk);
+    DFJK_LAUNCHED();
+    if (Vxc && gr.max_nsig > 0) {
+      w_kernel<<<dim3((unsigned)(G / (2 * kWThreads)), (unsigned)((gr.max_nsig + kWPer - 1) / kWPer),
+                      (unsigned)gr.count), kWThreads, 0, bs>>>(phi, dphi, b.vals.as<double>(), info, G,
+                                                               b.W.as<double>());
+      DFJK_LAUNCHED();
+      const unsigned nt = (unsigned)((gr.max_nsig + kVT - 1) / kVT);
+      v_kernel<<<dim3(nt * nt, (unsigned)nslice, (unsigned)gr.count), 256, kVSmem, bs>>>(
+          phi, b.W.as<double>(), info, G, b.Vc.as<double>());
+      DFJK_LAUNCHED();
+      reduce_v_kernel<<<dim3((unsigned)((nn + 255) / 256), (unsigned)parts), 256, 0, bs>>>(
+          b.Vc.as<double>(), nslice, gr.count, info, ch.d_pos.as<int>() + (int64_t)gr.first * nao,
+          nao, Vacc);
       DFJK_LAUNCHED();
     }
   }
@@ -874,7 +979,7 @@ static void xc_enqueue(const Context& c, const OrbView& ov, const double* pts, c
   }
   if (Vxc) {
     symmetrize_sum_kernel<<<(unsigned)((nn + 255) / 256), 256, 0, s>>>(ws.Vacc.as<double>(),
-                                                                        nb, nao, Vxc);
+                                                                        (int)(nb * parts), nao, Vxc);
     DFJK_LAUNCHED();
   }
 }
@@ -885,25 +990,23 @@ double xc_energy_fock(const Context& c, const OrbView& ov, const double* pts, co
   const int nao = ov.nao;
   const XcChunks& ch = ws.ch;
   const int64_t G = ch.G;
-  const int64_t nchunk = (int64_t)ch.g0.size();
-  const int64_t nblk = G / kRpPts;   // G is a multiple of 256
-  const int64_t plane_max = (int64_t)std::max(ch.max_ao, 1) * G;
-  const size_t mx = (size_t)std::max(ch.max_ao, 1);
-  const size_t nslice = (size_t)((G + kVSlice - 1) / kVSlice);
+  const int64_t nchunk = (int64_t)ch.info.size();
+  const int64_t nblk = G / kPtThreads;   // G is a multiple of 256
   for (int q = 0; q < std::min(std::max(ws.nbr, 1), kXcBranches); ++q) {
     XcBranch& b = ws.br[q];
-    b.phi.ensure(plane_max * sizeof(double));
-    b.dphi.ensure(3 * plane_max * sizeof(double));
-    b.W.ensure(plane_max * sizeof(double));
-    b.Pc.ensure(mx * (mx + 1) * sizeof(double));
-    if (Vxc) b.Vc.ensure(nslice * mx * mx * sizeof(double));
+    b.phi.ensure(ch.max_phi * sizeof(double));
+    b.dphi.ensure(3 * ch.max_phi * sizeof(double));
+    b.W.ensure(ch.max_phi * sizeof(double));
+    b.vals.ensure(4 * ch.max_points * sizeof(double));
+    b.Pc.ensure(ch.max_pc * sizeof(double));
+    if (Vxc) b.Vc.ensure(ch.max_part * sizeof(double));
   }
-  DFJK_CUDA(cudaFuncSetAttribute(rho_w_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kRpSmem));
+  DFJK_CUDA(cudaFuncSetAttribute(rho_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kRpSmem));
   DFJK_CUDA(cudaFuncSetAttribute(v_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kVSmem));
   // the side streams and events are made here on first use, never during a capture
   side_streams(const_cast<Context&>(c));
   ws.ered.ensure((size_t)std::max<int64_t>(nchunk, 1) * nblk * sizeof(double));
-  if (Vxc) ws.Vacc.ensure((size_t)std::max(ws.nbr, 1) * nao * nao * sizeof(double));
+  if (Vxc) ws.Vacc.ensure((size_t)std::max(ws.nbr, 1) * v_parts(nao) * nao * nao * sizeof(double));
   const void* args[4] = {P, Vxc, pts, w};
   const bool same = std::equal(args, args + 4, ws.g_args);
   if (ws.exec && same) {

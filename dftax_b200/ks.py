@@ -54,7 +54,7 @@ class KSResult:
     xc_chunk: int = 0                # grid points per XC chunk (set or autotuned)
     xc_graph: bool = False           # XC evaluations replayed a captured CUDA graph
     n_eig: int = 0                   # densities built by the eigensolver (guess, fallbacks)
-    xc_gemm_flop: float = 0.0        # float64 FLOP of one XC evaluation's two DGEMMs
+    xc_gemm_flop: float = 0.0        # float64 FLOP of one XC evaluation's two products
 
 
 DENSITY_ROUTES = {"eigh": 0, "purify": 1}
@@ -107,7 +107,7 @@ class KS:
                                                              device=self.ctx.device)
         self._diis, self._lindep = diis_space, lindep_thresh
         self._ao_thresh, self._grid_chunk = float(ao_thresh), int(grid_chunk)
-        self._xc_streams = int(xc_streams)   # 0: 8 concurrent XC streams; the batch engine uses 1
+        self._xc_streams = int(xc_streams)   # 0: 4 concurrent XC streams; the batch engine uses 1
         self._density = DENSITY_ROUTES[density]
         self.h = ctypes.c_void_p()
         self._create()
@@ -251,7 +251,7 @@ def _main(argv=None):
     ap.add_argument("--guess", default="core", choices=["core", "sad"])
     ap.add_argument("--density", default="purify", choices=sorted(DENSITY_ROUTES))
     ap.add_argument("--xc-streams", type=int, default=0,
-                    help="concurrent streams of the XC chunks (0: 8; the batch engine uses 1)")
+                    help="concurrent streams of the XC chunks (0: 4; the batch engine uses 1)")
     ap.add_argument("--streamed", action="store_true",
                     help="streamed DF (B rebuilt per J/K call, not held): df(aux, chunk=...)")
     a = ap.parse_args(argv)

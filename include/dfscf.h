@@ -42,10 +42,10 @@ typedef struct {
   int32_t max_iter;     /* 128                                                          */
   int32_t diis_space;   /* DIIS history depth (8)                                        */
   int64_t grid_chunk;   /* grid points per XC chunk, spatially sorted (0: chosen by
-                           timing 2048, 4096, 8192 and 16384 on the first molecule of each
+                           timing 512 to 16384 on the first molecule of each
                            size and XC stream count; the choice is kept for the
                            process)                                                    */
-  int32_t xc_streams;   /* concurrent streams the XC chunks run on, 1..8 (0: 8); the
+  int32_t xc_streams;   /* concurrent streams the XC chunks run on, 1..8 (0: 4); the
                            batch engine runs its solves, which already overlap one
                            another, with 1                                             */
   int32_t density;      /* how each iteration's density comes from the DIIS Fock matrix:
@@ -80,7 +80,7 @@ typedef struct {
   int32_t n_eig;        /* densities built by the eigensolver in the last dfscf_run: the
                            core guess and every iteration with density 0; the core
                            guess and the fallbacks with density 1                       */
-  double xc_gemm_flop;  /* float64 FLOP of the two DGEMMs of one XC evaluation (X = Phi P
+  double xc_gemm_flop;  /* float64 FLOP of the two products of one XC evaluation (X = Phi P
                            and Phi^T W per chunk: 4 G n_chunk^2 summed over the chunks) */
 } dfscf_result;
 

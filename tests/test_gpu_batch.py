@@ -126,8 +126,11 @@ def test_refused_request_fails_alone(grid):
 
 
 def test_poisson_stream_matches_solo(solo, grid):
-    """Requests arrive with seeded exponential gaps (mean 0.15 s) while
-    earlier ones are on the GPU; each is admitted as memory frees up."""
+    """Requests arrive with seeded exponential gaps (mean 0.03 s) while
+    earlier ones are on the GPU; each is admitted as memory frees up.  The
+    smallest of these gaps is 0.3 of the mean, and a solve takes 25 to 40 ms:
+    some solve is still running at the next arrival as long as the mean is
+    below 25 ms / 0.3 = 80 ms."""
     from dftax_b200.batch import BatchEngine
 
     rng = np.random.default_rng(8)
@@ -137,7 +140,7 @@ def test_poisson_stream_matches_solo(solo, grid):
         ids = []
         for k in order:
             ids.append((k, eng.submit(*mols[k], grid=grid)))
-            time.sleep(float(rng.exponential(0.15)))
+            time.sleep(float(rng.exponential(0.03)))
         res = [(k, eng.wait(i)) for k, i in ids]
     lat = []
     for k, r in res:
