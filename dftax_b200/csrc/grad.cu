@@ -15,10 +15,12 @@
 // G and W are contracted with the integral derivatives on the fly
 // (grad3c.cuh; grad2c_kernel below); nothing of size rows x naux beyond one
 // chunk of G is kept.
+#include "dmma.cuh"
 #include "grad3c.cuh"
 #include "internal.h"
 
 #include <algorithm>
+#include <cstring>
 
 namespace dfjk {
 
@@ -99,6 +101,104 @@ __global__ void h_add_kernel(const double* __restrict__ T, int64_t nao, const in
   const int64_t r = i / nx, x = i % nx;
   const double wr = kind[r] == 2 ? 2.0 : 1.0;
   H[r * ldb + x0 + x] += wr * a * T[x * nao * nao + (int64_t)rm[r] * nao + rn[r]];
+}
+
+// H[r][x0 + x] += w_r a sum_j U[m][x][j] C'[n][j] for every row r = (m, n) of B:
+// block (m, 64 directions, 64 entries of m's list; rows are taken under their
+// first function) on the float64 tensor cores. Rows of U and C' are staged as
+// they lie, 16 j per step (16-byte pieces, index xor 4 (row % 2): a load phase of
+// two rows x four pieces falls in distinct banks; the j order inside a step is
+// free). The sum over j is short (the density's rank), so two stages suffice.
+constexpr int kBtT = 64, kBtK = 16;
+
+__global__ void __launch_bounds__(256) back_transform_kernel(
+    const double* __restrict__ U, const double* __restrict__ Cp, int64_t ncp, int64_t nx,
+    const int* __restrict__ kptr, const int* __restrict__ krow, const int* __restrict__ kn,
+    const int* __restrict__ rm, const int8_t* __restrict__ kind, int64_t ldb, int64_t x0, double a,
+    double* __restrict__ H) {
+  __shared__ __align__(16) double sm[2][2][kBtT * kBtK];   // [stage][entries, directions]
+  __shared__ int srow[kBtT], sn[kBtT];
+  const int m = blockIdx.x;
+  const int64_t xt = (int64_t)blockIdx.y * kBtT;
+  const int e0 = kptr[m] + blockIdx.z * kBtT, e1 = kptr[m + 1];
+  if (e0 >= e1) return;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  bool any = false;
+  if (tid < kBtT) {
+    const int e = e0 + tid;
+    int r = -1, n = 0;
+    if (e < e1 && rm[krow[e]] == m) {
+      r = krow[e];
+      n = kn[e];
+    }
+    srow[tid] = r;
+    sn[tid] = n;
+    any = r >= 0;
+  }
+  if (!__syncthreads_or(any)) return;
+  const int wr = (warp & 3) * 16, wc = (warp >> 2) * 32;
+  const int fr = lane >> 2, fk = lane & 3;
+  double acc[2][4][2];
+#pragma unroll
+  for (int i = 0; i < 2; ++i)
+#pragma unroll
+    for (int b = 0; b < 4; ++b) acc[i][b][0] = acc[i][b][1] = 0.0;
+  const int nst = (int)((ncp + kBtK - 1) / kBtK);
+  const int sr = tid >> 3, sp = tid & 7;
+  auto stage = [&](int q) {
+    const int64_t k = (int64_t)q * kBtK + 2 * sp;
+#pragma unroll
+    for (int j = 0; j < 2; ++j) {
+      const int r = sr + 32 * j, o = r * kBtK + 2 * (sp ^ (4 * (r & 1)));
+      const bool oe = k < ncp && srow[r] >= 0, ox = k < ncp && xt + r < nx;
+      cp_async16(&sm[q & 1][0][o], oe ? Cp + (int64_t)sn[r] * ncp + k : Cp, oe);
+      cp_async16(&sm[q & 1][1][o], ox ? U + ((int64_t)m * nx + xt + r) * ncp + k : U, ox);
+    }
+    cp_async_commit();
+  };
+  stage(0);
+  for (int q = 0; q < nst; ++q) {
+    if (q + 1 < nst) {
+      stage(q + 1);
+      cp_async_wait<1>();
+    } else {
+      cp_async_wait<0>();
+    }
+    __syncthreads();
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      const int piece = 2 * ((4 * h + fk) ^ (4 * (fr & 1)));
+      double2 af[2], bf[4];
+#pragma unroll
+      for (int i = 0; i < 2; ++i)
+        af[i] = *reinterpret_cast<const double2*>(&sm[q & 1][0][(wr + 8 * i + fr) * kBtK + piece]);
+#pragma unroll
+      for (int b = 0; b < 4; ++b)
+        bf[b] = *reinterpret_cast<const double2*>(&sm[q & 1][1][(wc + 8 * b + fr) * kBtK + piece]);
+#pragma unroll
+      for (int i = 0; i < 2; ++i)
+#pragma unroll
+        for (int b = 0; b < 4; ++b) {
+          dmma_8x8x4(acc[i][b], af[i].x, bf[b].x);
+          dmma_8x8x4(acc[i][b], af[i].y, bf[b].y);
+        }
+    }
+    __syncthreads();
+  }
+#pragma unroll
+  for (int i = 0; i < 2; ++i) {
+    const int r = srow[wr + 8 * i + fr];
+    if (r < 0) continue;
+    const double f = (kind[r] == 2 ? 2.0 : 1.0) * a;
+    double* row = H + (int64_t)r * ldb + x0;
+#pragma unroll
+    for (int b = 0; b < 4; ++b)
+#pragma unroll
+      for (int q = 0; q < 2; ++q) {
+        const int64_t x = xt + wc + 8 * b + 2 * fk + q;
+        if (x < nx) row[x] += f * acc[i][b][q];
+      }
+  }
 }
 
 __global__ void add2_kernel(const double* __restrict__ a, const double* __restrict__ b, int64_t n,
@@ -360,11 +460,65 @@ double energy_gradient(Plan& p, const double* P, int nspin, double hf, double* g
     const double k = (nspin == 1 ? -0.25 : -0.5) * hf;
     const int64_t xc = std::max<int64_t>(1, std::min<int64_t>(p.nfit, ((int64_t)1 << 30) / (16 * nn)));
     DevBuf Bd, T1;
-    Bd.alloc((size_t)xc * nn * sizeof(double));
-    T1.alloc((size_t)xc * nn * sizeof(double));
+    // the densities' factors P_s = C C^T (lowrank.cu): with r = rank, B_x C
+    // (half transform), C^T B_x C, C (C^T B_x C) and its product with C^T at the
+    // kept pairs cost 2 n^2 r + 4 n r^2 + n^2 r per direction instead of 4 n^3
+    struct Factors {
+      unsigned long long worst[2], scale[2];
+      int rank[2], pad[2];
+    } fh{};
+    const bool low = low_rank_supported(n);
+    if (low) {
+      p.ws_lowrank.ensure((size_t)nn * nspin * sizeof(double));
+      DevBuf fd;
+      fd.alloc(sizeof(Factors));
+      DFJK_CUDA(cudaMemsetAsync(fd.p, 0, sizeof(Factors), s));
+      Factors* f = fd.as<Factors>();
+      launch_low_rank(P, n, nspin, p.ws_lowrank.as<double>(), f->rank, f->worst, f->scale, s);
+      DFJK_CUDA(cudaMemcpyAsync(&fh, f, sizeof fh, cudaMemcpyDeviceToHost, s));
+      DFJK_CUDA(cudaStreamSynchronize(s));
+    }
+    auto value = [](unsigned long long bits) {
+      double v;
+      std::memcpy(&v, &bits, sizeof v);
+      return v;
+    };
     const double one = 1.0, zero = 0.0;
     for (int sp = 0; sp < nspin; ++sp) {
       const double* Ps = P + sp * nn;
+      // (past half the functions the dense form is no dearer)
+      if (low && 2 * fh.rank[sp] <= n && value(fh.worst[sp]) <= kLowRankAccept * value(fh.scale[sp])) {
+        const int64_t ncp = fh.rank[sp] + (fh.rank[sp] & 1);
+        if (ncp == 0) continue;
+        DevBuf Cp, X, Y;
+        Cp.alloc((size_t)n * ncp * sizeof(double));
+        pack_columns(p.ws_lowrank.as<double>() + sp * nn, n, fh.rank[sp], ncp, Cp.as<double>(), s);
+        // 64 directions at a time (the half transform's tile), up to 1 GB of X
+        int64_t xl = ((int64_t)1 << 30) / (n * ncp * (int64_t)sizeof(double)) / 64 * 64;
+        xl = std::min<int64_t>(std::max<int64_t>(xl, 64), p.nfit);
+        X.alloc((size_t)n * xl * ncp * sizeof(double));
+        Y.alloc((size_t)ncp * xl * ncp * sizeof(double));
+        for (int64_t x0 = 0; x0 < p.nfit; x0 += xl) {
+          const int64_t nx = std::min(xl, p.nfit - x0);
+          half_transform(p, Cp.as<double>(), ncp, x0, nx, X.as<double>(), s);
+          const int xj = (int)(nx * ncp);
+          DFJK_CUBLAS(cublasDgemm(c.cublas, CUBLAS_OP_N, CUBLAS_OP_T, xj, (int)ncp, (int)n, &one,
+                                  X.as<double>(), xj, Cp.as<double>(), (int)ncp, &zero,
+                                  Y.as<double>(), xj));
+          DFJK_CUBLAS(cublasDgemm(c.cublas, CUBLAS_OP_N, CUBLAS_OP_N, xj, (int)n, (int)ncp, &one,
+                                  Y.as<double>(), xj, Cp.as<double>(), (int)ncp, &zero,
+                                  X.as<double>(), xj));
+          const dim3 grid((unsigned)n, (unsigned)((nx + kBtT - 1) / kBtT), (unsigned)((n + kBtT - 1) / kBtT));
+          back_transform_kernel<<<grid, 256, 0, s>>>(
+              X.as<double>(), Cp.as<double>(), ncp, nx, p.d_kptr.as<int>(), p.d_krow.as<int>(),
+              p.d_kn.as<int>(), p.d_row_m.as<int>(), p.d_row_w.as<int8_t>(), ldb, x0, 2.0 * k,
+              H.as<double>());
+          DFJK_LAUNCHED();
+        }
+        continue;
+      }
+      Bd.ensure((size_t)xc * nn * sizeof(double));
+      T1.ensure((size_t)xc * nn * sizeof(double));
       for (int64_t x0 = 0; x0 < p.nfit; x0 += xc) {
         const int64_t nx = std::min(xc, p.nfit - x0);
         DFJK_CUDA(cudaMemsetAsync(Bd.p, 0, (size_t)nx * nn * sizeof(double), s));

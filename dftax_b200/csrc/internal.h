@@ -198,6 +198,13 @@ void launch_schwarz(const Context& c, Shells& sh, const std::vector<int>& pa,
 // ---- contractions (jk.cu) ----
 void jk_compute(Plan& p, const double* C, const double* w, int64_t ncol, double* J, double* K,
                 cudaStream_t s);
+// Float64 half transform X[m][x - x0][i] = sum_n B_x[m][n] C'[n][i] of a resident
+// B for directions [x0, x0 + n); C' row-major with ncp columns, ncp even, 16-byte
+// aligned
+void half_transform(Plan& p, const double* Cp, int64_t ncp, int64_t x0, int64_t n, double* X,
+                    cudaStream_t s);
+// C'[m][j] = Ct[j][m] for j < rank, zero up to ncp columns
+void pack_columns(const double* Ct, int64_t nao, int64_t rank, int64_t ncp, double* Cp, cudaStream_t s);
 // gamma = B^T vec(Ptot) over the plan's rows (ldb doubles; the J intermediate)
 void gamma_from_density(Plan& p, const double* Ptot, double* gamma, cudaStream_t s);
 

@@ -604,6 +604,20 @@ __global__ void scale_cols_kernel(const double* __restrict__ C, const double* __
   out[i] = v;
 }
 
+void pack_columns(const double* Ct, int64_t nao, int64_t rank, int64_t ncp, double* Cp, cudaStream_t s) {
+  scale_cols_kernel<<<(unsigned)((nao * ncp + 255) / 256), 256, 0, s>>>(Ct, nullptr, nao, 1, nao, nullptr,
+                                                                       rank, ncp, Cp);
+  DFJK_LAUNCHED();
+}
+
+void half_transform(Plan& p, const double* Cp, int64_t ncp, int64_t x0, int64_t n, double* X,
+                    cudaStream_t s) {
+  launch_half_any(ncp, (const double*)p.d_B.as<double>(), p.ldb, x0, n, Cp, ncp,
+                  (const int*)p.d_kptr.as<int>(), (const int*)nullptr,
+                  (const int*)p.d_krow.as<int>(), (const int*)p.d_kn.as<int>(), (int64_t)0, 0,
+                  (int64_t)p.nao, X, s);
+}
+
 // K (+)= sign * X X^T (float64, full square) for X nao x kt row-major: lower
 // 64 x 64 tile pairs times k slices, then a fixed-order sum of the slices
 // (bit-reproducible). Three blocks run per SM; the slice count is the one whose
@@ -714,10 +728,7 @@ static void k_accumulate(Plan& p, const double* C, int64_t sm, int64_t sc, const
       if (x0 == 0) ozaki_prepare_c(p, Cc, ncp, s);
       ozaki_k1(p, ncp, x0, n, X.as<double>(), s);   // int8 tensor cores, exact accumulation
     } else {
-      launch_half_any(ncp, (const double*)p.d_B.as<double>(), p.ldb, x0, n,
-                      Cc, ncp, (const int*)p.d_kptr.as<int>(),
-                      (const int*)nullptr, (const int*)p.d_krow.as<int>(),
-                      (const int*)p.d_kn.as<int>(), (int64_t)0, 0, nao, X.as<double>(), s);
+      half_transform(p, Cc, ncp, x0, n, X.as<double>(), s);
     }
     p.timer.mark(kPhKhalf, s);
     p.timer.mark(kPhKsyrk, s);
