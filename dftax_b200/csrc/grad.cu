@@ -20,7 +20,6 @@
 #include "internal.h"
 
 #include <algorithm>
-#include <cstring>
 
 namespace dfjk {
 
@@ -463,31 +462,22 @@ double energy_gradient(Plan& p, const double* P, int nspin, double hf, double* g
     // the densities' factors P_s = C C^T (lowrank.cu): with r = rank, B_x C
     // (half transform), C^T B_x C, C (C^T B_x C) and its product with C^T at the
     // kept pairs cost 2 n^2 r + 4 n r^2 + n^2 r per direction instead of 4 n^3
-    struct Factors {
-      unsigned long long worst[2], scale[2];
-      int rank[2], pad[2];
-    } fh{};
+    LowRankInfo fh{};
     const bool low = low_rank_supported(n);
     if (low) {
       p.ws_lowrank.ensure((size_t)nn * nspin * sizeof(double));
       DevBuf fd;
-      fd.alloc(sizeof(Factors));
-      DFJK_CUDA(cudaMemsetAsync(fd.p, 0, sizeof(Factors), s));
-      Factors* f = fd.as<Factors>();
-      launch_low_rank(P, n, nspin, p.ws_lowrank.as<double>(), f->rank, f->worst, f->scale, s);
-      DFJK_CUDA(cudaMemcpyAsync(&fh, f, sizeof fh, cudaMemcpyDeviceToHost, s));
+      fd.alloc(sizeof fh);
+      DFJK_CUDA(cudaMemsetAsync(fd.p, 0, sizeof fh, s));
+      launch_low_rank(P, n, nspin, n, p.ws_lowrank.as<double>(), fd.as<LowRankInfo>(), s);
+      DFJK_CUDA(cudaMemcpyAsync(&fh, fd.p, sizeof fh, cudaMemcpyDeviceToHost, s));
       DFJK_CUDA(cudaStreamSynchronize(s));
     }
-    auto value = [](unsigned long long bits) {
-      double v;
-      std::memcpy(&v, &bits, sizeof v);
-      return v;
-    };
     const double one = 1.0, zero = 0.0;
     for (int sp = 0; sp < nspin; ++sp) {
       const double* Ps = P + sp * nn;
       // (past half the functions the dense form is no dearer)
-      if (low && 2 * fh.rank[sp] <= n && value(fh.worst[sp]) <= kLowRankAccept * value(fh.scale[sp])) {
+      if (low && 2 * fh.rank[sp] <= n && fh.within(sp, kLowRankAccept)) {
         const int64_t ncp = fh.rank[sp] + (fh.rank[sp] & 1);
         if (ncp == 0) continue;
         DevBuf Cp, X, Y;

@@ -217,10 +217,16 @@ constexpr double kLowRankTol = 1e-14;
 constexpr double kLowRankAccept = 3e-14;
 bool low_rank_supported(int64_t n);   // its workspace fits in shared memory
 // per spin channel of P (nspin x n x n, symmetric): columns Ct[k][i] (k < rank,
-// n x n per channel), the rank, max |P - C C^T| and max |P| (bits of a double;
-// the caller zeroes them). Enqueued only.
-void launch_low_rank(const double* P, int64_t n, int nspin, double* Ct, int* rank,
-                     unsigned long long* worst, unsigned long long* scale, cudaStream_t s);
+// n x n per channel), the rank (at most max_rank), max |P - C C^T| and max |P|
+// (bits of a double; the caller zeroes them). Enqueued only.
+struct LowRankInfo {
+  unsigned long long worst[2], scale[2];
+  int rank[2];
+  // max |P - C C^T| <= tol max |P| for channel sp
+  bool within(int sp, double tol) const;
+};
+void launch_low_rank(const double* P, int64_t n, int nspin, int64_t max_rank, double* Ct,
+                     LowRankInfo* info, cudaStream_t s);
 
 // ---- nuclear gradient of the DF energy (grad.cu) ----
 // E and dE/dR at a fixed density P (nspin x nao x nao, device): per orbital

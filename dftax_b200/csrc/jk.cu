@@ -18,7 +18,6 @@
 
 #include <algorithm>
 #include <cmath>
-#include <cstring>
 
 namespace dfjk {
 
@@ -847,8 +846,7 @@ __global__ void __launch_bounds__(256) dot_axpy_kernel(const double* __restrict_
 // what an energy reads back from the device (ws_scal)
 struct EnergyScalars {
   double dot[5];                      // gamma . gamma, then Tr(P_s K) per spin and operator
-  unsigned long long worst[2], scale[2];
-  int rank[2];
+  LowRankInfo low;
   int nonfinite;
   unsigned count;                     // of dot_axpy_kernel
 };
@@ -931,8 +929,7 @@ double energy(Plan& p, const double* P, int nspin, double hf, double hf_lr, doub
   // the density's factor, a chain of small steps on a few SMs, runs beside J
   SideFork side(*p.ctx, low ? 1 : 0, s);
   if (low)
-    launch_low_rank(P, n, nspin, p.ws_lowrank.as<double>(), sc->rank, sc->worst, sc->scale,
-                    side.stream(0));
+    launch_low_rank(P, n, nspin, n, p.ws_lowrank.as<double>(), &sc->low, side.stream(0));
   const double* Pt = P;
   if (nspin == 2) {
     p.ws_Ptot.ensure(nn * sizeof(double));
@@ -955,17 +952,11 @@ double energy(Plan& p, const double* P, int nspin, double hf, double hf_lr, doub
   DFJK_CUDA(cudaStreamSynchronize(s));
   if (h.nonfinite) fail(DFJK_ERR_NUMERIC, "non-finite values in the density");
   if (!exch) return 0.5 * h.dot[0];
-  auto value = [](unsigned long long bits) {
-    double v;
-    static_assert(sizeof v == sizeof bits, "bits of a double");
-    std::memcpy(&v, &bits, sizeof v);
-    return v;
-  };
   p.ws_K.ensure(nn * sizeof(double));
   double* K = p.ws_K.as<double>();
   for (int sp = 0; sp < nspin; ++sp) {
     const double* Ps = P + sp * nn;
-    const bool factored = low && value(h.worst[sp]) <= kLowRankAccept * value(h.scale[sp]);
+    const bool factored = low && h.low.within(sp, kLowRankAccept);
     DevBuf Ct, dw;
     if (!factored) density_factor(p, Ps, Ct, dw, s);   // indefinite, or too rough a factor
     const struct { Plan* plan; double coeff; } terms[2] = {{&p, hf},
@@ -975,8 +966,8 @@ double energy(Plan& p, const double* P, int nspin, double hf, double hf_lr, doub
       Plan& q = *terms[t].plan;
       if (!factored) {
         k_compute(q, Ct.as<double>(), dw.as<double>(), n, K, s);
-      } else if (h.rank[sp] > 0) {
-        k_accumulate(q, p.ws_lowrank.as<double>() + sp * nn, 1, n, nullptr, nullptr, h.rank[sp],
+      } else if (h.low.rank[sp] > 0) {
+        k_accumulate(q, p.ws_lowrank.as<double>() + sp * nn, 1, n, nullptr, nullptr, h.low.rank[sp],
                      1.0, true, K, s);
       } else {
         DFJK_CUDA(cudaMemsetAsync(K, 0, nn * sizeof(double), s));

@@ -13,6 +13,9 @@
 // eigensolver when it is not small.
 #include "internal.h"
 
+#include <algorithm>
+#include <cstring>
+
 namespace dfjk {
 namespace {
 
@@ -36,7 +39,7 @@ __device__ __forceinline__ Pivot better(Pivot a, Pivot b) {
 }
 
 // Columns Ct[k][i] (k < rank) of P[spin] for the cluster of blockIdx.x / 8;
-// rank[spin] out. Left-looking: step k forms column p of the residual from P
+// the rank out. Left-looking: step k forms column p of the residual from P
 // and the k columns so far, C[i][k] = (P[p][i] - sum_q C[i][q] C[p][q]) /
 // sqrt(d_p), and updates the residual diagonal d. Each CTA owns a run of rows
 // (its part of d in shared memory); a warp per k lane sums every eighth q
@@ -45,8 +48,8 @@ __device__ __forceinline__ Pivot better(Pivot a, Pivot b) {
 // column visible. Bound by that barrier and the L2 latency of the pivot row,
 // about 2 us a step; the arithmetic is n r^2 in all.
 __global__ void __cluster_dims__(kCta, 1, 1) __launch_bounds__(kLanes * 32)
-    pivoted_cholesky_kernel(const double* __restrict__ Pall, int64_t n, double rel_tol,
-                            double* Ctall, int* __restrict__ rank) {
+    pivoted_cholesky_kernel(const double* __restrict__ Pall, int64_t n, int64_t max_rank,
+                            double rel_tol, double* Ctall, LowRankInfo* __restrict__ info) {
   extern __shared__ double sm[];
   __shared__ double red[kLanes][kRows];
   __shared__ Pivot slot[2][kCta];
@@ -88,7 +91,7 @@ __global__ void __cluster_dims__(kCta, 1, 1) __launch_bounds__(kLanes * 32)
     for (int c = 1; c < kCta; ++c) p = better(p, slot[k & 1][c]);
     if (k == 0) first = p.v;
     // the same decision in every CTA: all read the same eight candidates
-    if (k == n || !(p.v > rel_tol * first) || !(p.v > 0.0)) break;
+    if (k == max_rank || !(p.v > rel_tol * first) || !(p.v > 0.0)) break;
     for (int64_t q = threadIdx.x; q < k; q += kLanes * 32) crow[q] = __ldcg(Ct + q * n + p.i);
     __syncthreads();
     const double inv = 1.0 / sqrt(p.v);
@@ -122,7 +125,7 @@ __global__ void __cluster_dims__(kCta, 1, 1) __launch_bounds__(kLanes * 32)
     }
   }
   // (the last barrier of the loop: no CTA still writes into another's slots)
-  if (cta == 0 && threadIdx.x == 0) rank[spin] = (int)k;
+  if (cta == 0 && threadIdx.x == 0) info->rank[spin] = (int)k;
 }
 
 // worst[spin] = max |P - C C^T| over every element, and scale[spin] = max |P|
@@ -130,14 +133,12 @@ __global__ void __cluster_dims__(kCta, 1, 1) __launch_bounds__(kLanes * 32)
 // read on the device
 __global__ void __launch_bounds__(256) residual_kernel(const double* __restrict__ Pall, int64_t n,
                                                        const double* __restrict__ Ctall,
-                                                       const int* __restrict__ rank,
-                                                       unsigned long long* __restrict__ worst,
-                                                       unsigned long long* __restrict__ scale) {
+                                                       LowRankInfo* __restrict__ info) {
   __shared__ double A[32][33], B[32][33];
   const int spin = blockIdx.z;
   const double* P = Pall + (int64_t)spin * n * n;
   const double* Ct = Ctall + (int64_t)spin * n * n;
-  const int r = rank[spin];
+  const int r = info->rank[spin];
   const int64_t i0 = blockIdx.y * 32, j0 = blockIdx.x * 32;
   const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
   double s[4] = {0.0, 0.0, 0.0, 0.0};
@@ -173,8 +174,8 @@ __global__ void __launch_bounds__(256) residual_kernel(const double* __restrict_
     m = fmax(m, __shfl_xor_sync(0xffffffffu, m, o));
   }
   if (tx == 0) {
-    atomicMax(worst + spin, (unsigned long long)__double_as_longlong(w));
-    atomicMax(scale + spin, (unsigned long long)__double_as_longlong(m));
+    atomicMax(&info->worst[spin], (unsigned long long)__double_as_longlong(w));
+    atomicMax(&info->scale[spin], (unsigned long long)__double_as_longlong(m));
   }
 }
 
@@ -184,15 +185,23 @@ size_t chol_smem(int64_t n) { return (size_t)((n + kCta - 1) / kCta + n) * sizeo
 
 bool low_rank_supported(int64_t n) { return chol_smem(n) <= (size_t)200 << 10; }
 
-void launch_low_rank(const double* P, int64_t n, int nspin, double* Ct, int* rank,
-                     unsigned long long* worst, unsigned long long* scale, cudaStream_t s) {
+bool LowRankInfo::within(int sp, double tol) const {
+  double w, m;
+  std::memcpy(&w, &worst[sp], sizeof w);
+  std::memcpy(&m, &scale[sp], sizeof m);
+  return w <= tol * m;
+}
+
+void launch_low_rank(const double* P, int64_t n, int nspin, int64_t max_rank, double* Ct,
+                     LowRankInfo* info, cudaStream_t s) {
   const size_t smem = chol_smem(n);
   DFJK_CUDA(cudaFuncSetAttribute(pivoted_cholesky_kernel,
                                  cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  pivoted_cholesky_kernel<<<kCta * nspin, kLanes * 32, smem, s>>>(P, n, kLowRankTol, Ct, rank);
+  pivoted_cholesky_kernel<<<kCta * nspin, kLanes * 32, smem, s>>>(P, n, std::min(max_rank, n), kLowRankTol,
+                                                                   Ct, info);
   DFJK_LAUNCHED();
   const unsigned t = (unsigned)((n + 31) / 32);
-  residual_kernel<<<dim3(t, t, (unsigned)nspin), 256, 0, s>>>(P, n, Ct, rank, worst, scale);
+  residual_kernel<<<dim3(t, t, (unsigned)nspin), 256, 0, s>>>(P, n, Ct, info);
   DFJK_LAUNCHED();
 }
 

@@ -14,8 +14,8 @@
 //   optional level shift b (S - S P S / 2) (scf.py:367);
 //   X^T F X diagonalized in float64 (cuSOLVER syevd), C = X C', P_{k+1} =
 //   2 C_occ C_occ^T (scf.py:319-327); or, with the purification option, the
-//   same aufbau projector of X^T F X by SP2 iterations (GEMMs), C_occ from a
-//   projected Cholesky QR, and the eigensolver once at the end for the
+//   same aufbau projector of X^T F X by SP2 iterations (GEMMs), C_occ from its
+//   pivoted Cholesky factor, and the eigensolver once at the end for the
 //   orbitals and their energies;
 //   E(P_{k+1}) and F(P_{k+1}) together; converged when |E_{k+1} - E_k| < e_tol
 //   and |err_k| < d_tol (scf.py:371).
@@ -56,8 +56,7 @@ struct dfscf {
   // captured XC graph reads and writes these, whatever buffers a call brings
   dfjk::DevBuf Pin, Vout;
   dfjk::DevBuf dots;                                 // results of a batch of dot products
-  dfjk::DevBuf sp_X, sp_X2, sp_Z, sp_Y, sp_Q, sp_st, sp_info, sp_work;   // purification
-  bool sp_have_Q = false;      // sp_Q holds the last occupied orbitals (X^T-basis)
+  dfjk::DevBuf sp_X, sp_X2, sp_Z, sp_st, sp_low;    // purification
   int sp_steps = 16;           // projection steps the last converged density took
   dfjk::XcWork xcw;
   std::vector<double> B;   // DIIS error overlaps, m x m
@@ -166,10 +165,12 @@ __global__ void sp2_init_kernel(const double* __restrict__ A, int m, const doubl
 // traces t1 = Tr X and t2 = Tr Z, reduced by every block in the same fixed
 // order so all take the same branch, then Xn = sym(Z) when Tr X^2 is nearer
 // nocc than Tr(2X - X^2), else 2X - sym(Z). Block 0 records {t1, t2, branch}.
+// force: 1 or 2 takes X^2 or 2X - X^2 whatever the traces.
 constexpr int kSp2Threads = 512;
 __global__ void __launch_bounds__(kSp2Threads) sp2_step_kernel(const double* __restrict__ X,
                                                               const double* __restrict__ Z, int m,
-                                                              int nocc, double* __restrict__ Xn,
+                                                              int nocc, int force,
+                                                              double* __restrict__ Xn,
                                                               double* __restrict__ rec) {
   __shared__ double s1[kSp2Threads], s2[kSp2Threads];
   double a = 0.0, b = 0.0;
@@ -188,7 +189,7 @@ __global__ void __launch_bounds__(kSp2Threads) sp2_step_kernel(const double* __r
     __syncthreads();
   }
   const double t1 = s1[0], t2 = s2[0], N = (double)nocc;
-  const bool sq = fabs(t2 - N) < fabs(2.0 * t1 - t2 - N);
+  const bool sq = force ? force == 1 : fabs(t2 - N) < fabs(2.0 * t1 - t2 - N);
   if (blockIdx.x == 0 && threadIdx.x == 0) {
     rec[0] = t1;
     rec[1] = t2;
@@ -201,18 +202,6 @@ __global__ void __launch_bounds__(kSp2Threads) sp2_step_kernel(const double* __r
     const double z = 0.5 * (Z[i] + Z[c + r * (int64_t)m]);
     Xn[i] = sq ? z : 2.0 * X[i] - z;
   }
-}
-
-// deterministic start vectors in [-1, 1): splitmix64 (Steele, Lea and Flood,
-// OOPSLA 2014) of the element index
-__global__ void fill_hash_kernel(double* __restrict__ R, int64_t n) {
-  const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  uint64_t z = (uint64_t)i + 0x9E3779B97F4A7C15ull;
-  z = (z ^ (z >> 30)) * 0xBF58476D1CE4E5B9ull;
-  z = (z ^ (z >> 27)) * 0x94D049BB133111EBull;
-  z ^= z >> 31;
-  R[i] = (double)(z >> 11) * 0x1.0p-52 - 1.0;
 }
 
 // adds the milliseconds of the device work enqueued on s since the last mark
@@ -429,7 +418,7 @@ int sp2_steps(dfscf& f, double* const (&Xb)[2], double* Z, double* st, bool* don
     const int g = std::min(it == 0 ? std::max(f.sp_steps, 4) : 4, kSp2Max - it);
     for (int j = 0; j < g; ++j) {
       gemm(c, CUBLAS_OP_N, CUBLAS_OP_N, m, m, m, 1.0, Xb[cur], m, Xb[cur], m, 0.0, Z, m, s);
-      sp2_step_kernel<<<grid, kSp2Threads, 0, s>>>(Xb[cur], Z, m, k, Xb[cur ^ 1],
+      sp2_step_kernel<<<grid, kSp2Threads, 0, s>>>(Xb[cur], Z, m, k, 0, Xb[cur ^ 1],
                                                    st + 2 + 3 * (it + j));
       DFJK_LAUNCHED();
       cur ^= 1;
@@ -455,6 +444,14 @@ int sp2_steps(dfscf& f, double* const (&Xb)[2], double* Z, double* st, bool* don
     if (bad) break;
     it += g;
   }
+  // the traces no longer tell the branches apart: X^2 and then 2X - X^2 square the
+  // errors of both ends of the spectrum
+  for (int j = 0; *done && j < kSp2Extra; ++j) {
+    gemm(c, CUBLAS_OP_N, CUBLAS_OP_N, m, m, m, 1.0, Xb[cur], m, Xb[cur], m, 0.0, Z, m, s);
+    sp2_step_kernel<<<grid, kSp2Threads, 0, s>>>(Xb[cur], Z, m, k, j + 1, Xb[cur ^ 1], st);
+    DFJK_LAUNCHED();
+    cur ^= 1;
+  }
   return cur;
 }
 
@@ -472,70 +469,40 @@ bool sp2_density(dfscf& f, const double* Fm, cudaStream_t s) {
   double* Xb[2] = {f.sp_X.as<double>(), f.sp_X2.as<double>()};
   double* Z = f.sp_Z.as<double>();
   double* st = f.sp_st.as<double>();   // [0..1] bounds, then 3 per step
-  double t1_last = 0.0;
-  bool done = false;
+  double rec[3] = {0.0, 0.0, 0.0};   // steps, the last Tr X, converged
   int cur = 0;
   if (m <= kSp2ClusterMax) {
-    launch_sp2_cluster(f.Fo.as<double>(), m, k, kSp2Max, Xb[0], st, s);
-    double rec[3];
+    launch_sp2_cluster(f.Fo.as<double>(), m, k, kSp2Max, Xb[1], Xb[0], st, s);
     DFJK_CUDA(cudaMemcpyAsync(rec, st, sizeof rec, cudaMemcpyDeviceToHost, s));
-    DFJK_CUDA(cudaStreamSynchronize(s));
-    t1_last = rec[1];
-    done = rec[2] == 1.0;
   } else {
-    cur = sp2_steps(f, Xb, Z, st, &done, &t1_last, s);
+    bool done = false;
+    cur = sp2_steps(f, Xb, Z, st, &done, &rec[1], s);
+    rec[2] = done ? 1.0 : 0.0;
   }
-  const double* Xs = Xb[cur];
-  if (!done || !(std::fabs(t1_last - k) < 1e-6)) {
-    tm.add(f.res.ms_diag);
-    return false;
-  }
-  // C'_occ: X applied to the last occupied orbitals (or to fixed
-  // pseudo-random vectors), orthonormalized by Cholesky QR, twice; the second
-  // pass projects out what the first left outside range(X)
-  double* Y = f.sp_Y.as<double>();
-  double* Q = f.sp_Q.as<double>();
-  double* M = f.A2.as<double>();   // k x k
-  const int64_t mk = (int64_t)m * k;
-  if (!f.sp_have_Q) {
-    fill_hash_kernel<<<blocks(mk), 256, 0, s>>>(Q, mk);
-    DFJK_LAUNCHED();
-  }
-  f.sp_have_Q = false;
-  const double one = 1.0, zero = 0.0, mone = -1.0;
-  DFJK_CUSOLVER(cusolverDnSetStream(c.cusolver, s));
-  int lwork = 0;
-  DFJK_CUSOLVER(cusolverDnDpotrf_bufferSize(c.cusolver, CUBLAS_FILL_MODE_LOWER, k, M, k, &lwork));
-  f.sp_work.ensure((size_t)std::max(lwork, 1) * sizeof(double));
-  for (int pass = 0; pass < 2; ++pass) {
-    gemm(c, CUBLAS_OP_N, CUBLAS_OP_N, m, k, m, 1.0, Xs, m, Q, m, 0.0, Y, m, s);
-    DFJK_CUBLAS(cublasSetStream(c.cublas, s));
-    DFJK_CUBLAS(cublasDsyrk(c.cublas, CUBLAS_FILL_MODE_LOWER, CUBLAS_OP_T, k, m, &one, Y, m, &zero,
-                            M, k));
-    DFJK_CUSOLVER(cusolverDnDpotrf(c.cusolver, CUBLAS_FILL_MODE_LOWER, k, M, k,
-                                   f.sp_work.as<double>(), lwork, f.sp_info.as<int>() + pass));
-    // Y <- Y L^-T, then Q = Y
-    DFJK_CUBLAS(cublasDtrsm(c.cublas, CUBLAS_SIDE_RIGHT, CUBLAS_FILL_MODE_LOWER, CUBLAS_OP_T,
-                            CUBLAS_DIAG_NON_UNIT, m, k, &one, M, k, Y, m));
-    DFJK_CUDA(cudaMemcpyAsync(Q, Y, mk * sizeof(double), cudaMemcpyDeviceToDevice, s));
-  }
-  // |X Q - Q|_F: Q must lie in range(X)
-  gemm(c, CUBLAS_OP_N, CUBLAS_OP_N, m, k, m, 1.0, Xs, m, Q, m, 0.0, Y, m, s);
-  DFJK_CUBLAS(cublasDaxpy(c.cublas, (int)mk, &mone, Q, 1, Y, 1));
-  double res = 0.0;
-  DFJK_CUBLAS(cublasDnrm2(c.cublas, (int)mk, Y, 1, &res));
-  int hinfo[2] = {0, 0};
-  DFJK_CUDA(cudaMemcpyAsync(hinfo, f.sp_info.p, 2 * sizeof(int), cudaMemcpyDeviceToHost, s));
+  // C'_occ: the projector's own factor X = C' C'^T by pivoted Cholesky
+  // (lowrank.cu), whose columns are orthonormal as far as X is idempotent
+  // (X^2 = X gives C' (C'^T C' - I) C'^T = 0); one Newton step C' (3 I - C'^T C')
+  // / 2 squares what is left. (A Cholesky QR of X applied to the last orbitals,
+  // twice, took a dozen launches and a potrf of 37 us each.)
+  LowRankInfo low{};
+  DFJK_CUDA(cudaMemsetAsync(f.sp_low.p, 0, sizeof low, s));
+  launch_low_rank(Xb[cur], m, 1, k, Z, f.sp_low.as<LowRankInfo>(), s);
+  DFJK_CUDA(cudaMemcpyAsync(&low, f.sp_low.p, sizeof low, cudaMemcpyDeviceToHost, s));
   DFJK_CUDA(cudaStreamSynchronize(s));
-  if (hinfo[0] != 0 || hinfo[1] != 0 || !(res < 1e-10 * std::sqrt((double)k))) {
+  // converged to a projector of rank nocc: X keeps the rounding of its first
+  // steps, eps times the spectrum's width over the gap (1e-12 for carbon's sets)
+  if (rec[2] != 1.0 || !(std::fabs(rec[1] - k) < 1e-6) || low.rank[0] != k || !low.within(0, 1e-10)) {
     tm.add(f.res.ms_diag);
     return false;
   }
-  f.sp_have_Q = true;
+  double* Q = Xb[cur ^ 1];
+  DFJK_CUDA(cudaMemcpyAsync(Q, Z, (size_t)m * k * sizeof(double), cudaMemcpyDeviceToDevice, s));
+  gemm(c, CUBLAS_OP_T, CUBLAS_OP_N, k, k, m, 1.0, Z, m, Z, m, 0.0, f.A2.as<double>(), k, s);
+  gemm(c, CUBLAS_OP_N, CUBLAS_OP_N, m, k, k, -0.5, Z, m, f.A2.as<double>(), k, 1.5, Q, m, s);
   // C_occ = X C'_occ (first k columns of f.C), P = 2 C_occ C_occ^T
   gemm(c, CUBLAS_OP_N, CUBLAS_OP_N, n, k, m, 1.0, f.X.as<double>(), n, Q, m, 0.0, f.C.as<double>(),
        n, s);
-  const double two = 2.0;
+  const double two = 2.0, zero = 0.0;
   DFJK_CUBLAS(cublasSetStream(c.cublas, s));
   DFJK_CUBLAS(cublasDsyrk(c.cublas, CUBLAS_FILL_MODE_LOWER, CUBLAS_OP_N, n, k, &two,
                           f.C.as<double>(), n, &zero, f.P.as<double>(), n));
@@ -548,7 +515,7 @@ bool sp2_density(dfscf& f, const double* Fm, cudaStream_t s) {
 
 // the aufbau density of F into f.P with C_occ in f.C, by the configured route
 void make_density(dfscf& f, const double* Fm, cudaStream_t s) {
-  if (f.o.density == 1 && f.nocc < f.nmo && sp2_density(f, Fm, s)) return;
+  if (f.o.density == 1 && f.nocc < f.nmo && low_rank_supported(f.nmo) && sp2_density(f, Fm, s)) return;
   make_density_eig(f, Fm, s);
 }
 
@@ -888,12 +855,10 @@ dfjk_status dfscf_create(dfjk_plan* pl, int32_t natom, const double* atom_xyz,
     f->Fx.alloc(nn * sizeof(double));
     if (f->o.density == 1) {
       f->sp_X.alloc(m * m * sizeof(double));
-      f->sp_X2.alloc(m * m * sizeof(double));
+      f->sp_X2.alloc(std::max((size_t)(m * m) * sizeof(double), sp2_cluster_bytes((int)m)));
       f->sp_Z.alloc(m * m * sizeof(double));
-      f->sp_Y.alloc(m * nocc * sizeof(double));
-      f->sp_Q.alloc(m * nocc * sizeof(double));
       f->sp_st.alloc((2 + 3 * kSp2Max) * sizeof(double));
-      f->sp_info.alloc(2 * sizeof(int));
+      f->sp_low.alloc(sizeof(LowRankInfo));
     }
     upload(f->wocc, std::vector<double>(nocc, 2.0));
     f->dF.alloc((size_t)f->o.diis_space * nn * sizeof(double));

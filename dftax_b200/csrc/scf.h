@@ -99,10 +99,13 @@ struct XcWork {
 
 // The SP2 projection of A (m x m symmetric, m <= kSp2ClusterMax) onto its nocc
 // lowest eigenvalues in one launch (sp2.cu): X, and rec = {steps, Tr X, 1 when
-// converged}. kSp2ClusterMax: a copy of X fits in a CTA's shared memory.
+// converged}; Xg: sp2_cluster_bytes(m) of scratch. kSp2ClusterMax: a copy of X
+// fits in a CTA's shared memory.
 constexpr int kSp2ClusterMax = 160;
-void launch_sp2_cluster(const double* A, int m, int nocc, int max_steps, double* X, double* rec,
-                        cudaStream_t s);
+constexpr int kSp2Extra = 2;   // steps after the stopping rule holds: X^2, then 2X - X^2
+size_t sp2_cluster_bytes(int m);
+void launch_sp2_cluster(const double* A, int m, int nocc, int max_steps, double* Xg, double* X,
+                        double* rec, cudaStream_t s);
 
 // Sorts the points (and weights) along a Morton curve over 1-Bohr cells;
 // pts [n][3] and w [n] are host arrays, reordered in place.

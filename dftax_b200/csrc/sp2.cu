@@ -7,8 +7,11 @@
 // of X in each shared memory and runs every step: 8 x 8 tiles of the lower
 // triangle of X^2 on the float64 tensor cores (X is symmetric, so rows serve
 // as columns), spread over the 64 warps; the owners write the new tile and its
-// mirror image into all eight copies. Two cluster barriers per step.
-// Bound by those barriers and the remote stores, 3-4 us a step.
+// mirror image to memory, laid out as in shared memory, and every CTA copies the
+// new X back from L2 in one sweep of 16-byte asynchronous copies (stored
+// straight into all eight shared memories, 16 scattered 8-byte remote stores per
+// value, a step of m = 150 took 20 us). Two cluster barriers per step.
+// Bound by those barriers and the L2 round trip.
 #include "dmma.cuh"
 #include "scf.h"
 
@@ -44,12 +47,15 @@ __device__ __forceinline__ double warp_sum(double v) {
 }
 
 // A: m x m symmetric (the lower triangle is read); Xout: the projector; rec:
-// {steps, Tr X before the last step, 1 when converged}. The stopping rule is
-// that of the stepwise path: the idempotency error Tr X - Tr X^2 below 1e-15 m,
-// or below 1e-9 and not below its value two steps before.
+// {steps, Tr X before the last step, 1 when converged}; Xg: scratch of mp rows of
+// mp + 4 (mp = m rounded up to 8). The stopping rule is that of the stepwise
+// path: the idempotency error Tr X - Tr X^2 below 1e-15 m, or below 1e-9 and not
+// below its value two steps before. By then the traces no longer tell the
+// branches apart, so X^2 and then 2X - X^2 follow, which square the errors of
+// both ends of the spectrum (kSp2Extra steps).
 __global__ void __cluster_dims__(kCta, 1, 1) __launch_bounds__(kWarps * 32)
     sp2_cluster_kernel(const double* __restrict__ A, int m, int nocc, int max_steps,
-                       double* __restrict__ Xout, double* __restrict__ rec) {
+                       double* Xg, double* __restrict__ Xout, double* __restrict__ rec) {
   extern __shared__ __align__(16) double X[];   // [mp][P]
   __shared__ double tz[2][kMaxTiles];           // diagonal tiles' traces of X^2
   __shared__ double rlo[kWarps], rhi[kWarps];
@@ -106,14 +112,11 @@ __global__ void __cluster_dims__(kCta, 1, 1) __launch_bounds__(kWarps * 32)
     ti[q] = t < nt ? a : -1;
     tj[q] = t - a * (a + 1) / 2;
   }
-  uint32_t xb[kCta];   // X in every CTA
-#pragma unroll
-  for (int c = 0; c < kCta; ++c) xb[c] = remote(X, c);
   double e1 = INFINITY, e2 = INFINITY, t1 = 0.0;
   const double N = (double)nocc;
-  int it = 0;
+  int it = 0, last = max_steps;
   bool done = false;
-  for (; it < max_steps && !done; ++it) {
+  for (; it < last; ++it) {
     double z[kTilesPerWarp][2];
 #pragma unroll
     for (int q = 0; q < kTilesPerWarp; ++q) {
@@ -138,9 +141,12 @@ __global__ void __cluster_dims__(kCta, 1, 1) __launch_bounds__(kWarps * 32)
     t1 = warp_sum(d);
     cluster_barrier();   // no CTA reads the old X any more; the traces have arrived
     const double t2 = warp_sum(lane < mt ? tz[it & 1][lane] : 0.0);
-    const bool sq = fabs(t2 - N) < fabs(2.0 * t1 - t2 - N);
+    const bool sq = done ? it == last - 2 : fabs(t2 - N) < fabs(2.0 * t1 - t2 - N);
     const double e = fabs(t1 - t2);
-    done = e < 1e-15 * m || (e < 1e-9 && e >= e2);
+    if (!done && (e < 1e-15 * m || (e < 1e-9 && e >= e2))) {
+      done = true;
+      last = it + 1 + kSp2Extra;
+    }
     e2 = e1;
     e1 = e;
     const bool bad = !(e < INFINITY);
@@ -152,16 +158,19 @@ __global__ void __cluster_dims__(kCta, 1, 1) __launch_bounds__(kWarps * 32)
       for (int r = 0; r < 2; ++r) {
         const int j = j0 + r;
         if (i < j) continue;   // a diagonal tile writes its lower half and the mirror image
-        const uint32_t at = (i * P + j) * 8, mir = (j * P + i) * 8;
         const double v = sq ? z[q][r] : 2.0 * X[i * P + j] - z[q][r];
-#pragma unroll
-        for (int c = 0; c < kCta; ++c) {
-          remote_store(xb[c] + at, v);
-          if (i != j) remote_store(xb[c] + mir, v);
-        }
+        Xg[i * P + j] = v;
+        Xg[j * P + i] = v;
       }
     }
-    cluster_barrier();   // the new X is complete in every copy
+    cluster_barrier();   // the new X is complete in memory (and visible: release, acquire)
+    for (int q = tid; q < mp * P / 2; q += kWarps * 32) {
+      // (the four doubles past a row's mp are never read)
+      cp_async16(X + 2 * q, Xg + 2 * q, true);
+    }
+    cp_async_commit();
+    cp_async_wait<0>();
+    __syncthreads();
     if (bad) break;      // (the same in every CTA: all see the same traces)
   }
   if (cta != 0) return;
@@ -175,13 +184,17 @@ __global__ void __cluster_dims__(kCta, 1, 1) __launch_bounds__(kWarps * 32)
 
 }  // namespace
 
-void launch_sp2_cluster(const double* A, int m, int nocc, int max_steps, double* X, double* rec,
-                        cudaStream_t s) {
+size_t sp2_cluster_bytes(int m) {
   const int mp = (m + 7) / 8 * 8;
-  const size_t smem = (size_t)mp * (mp + 4) * sizeof(double);
+  return (size_t)mp * (mp + 4) * sizeof(double);
+}
+
+void launch_sp2_cluster(const double* A, int m, int nocc, int max_steps, double* Xg, double* X,
+                        double* rec, cudaStream_t s) {
+  const size_t smem = sp2_cluster_bytes(m);
   DFJK_CUDA(cudaFuncSetAttribute(sp2_cluster_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  (int)smem));
-  sp2_cluster_kernel<<<kCta, kWarps * 32, smem, s>>>(A, m, nocc, max_steps, X, rec);
+  sp2_cluster_kernel<<<kCta, kWarps * 32, smem, s>>>(A, m, nocc, max_steps, Xg, X, rec);
   DFJK_LAUNCHED();
 }
 
