@@ -25,6 +25,13 @@ namespace dfjk {
 // J
 // ---------------------------------------------------------------------------
 
+// 32 bytes of B, read once: no L1 allocation (p 32-byte aligned)
+__device__ __forceinline__ void load4(const double* p, double (&v)[4]) {
+  asm volatile("ld.global.nc.L1::no_allocate.v4.f64 {%0, %1, %2, %3}, [%4];"
+               : "=d"(v[0]), "=d"(v[1]), "=d"(v[2]), "=d"(v[3])
+               : "l"(p));
+}
+
 // The density whose J is taken: sum_i w_i C[m][i] C[n][i] of ncol orbitals (w
 // null: ones), or the matrix D when C is null.
 struct DensitySource {
@@ -36,7 +43,9 @@ struct DensitySource {
 
 // gamma partials: CTA (bx, by) sums rows [r0, r1) for columns [by*2048, +2048).
 // The rows' weights d[r] = w_r D[m, n] are formed 32 at a time by the block
-// itself (a warp takes four), so no launch and no array come before it.
+// itself (a warp takes four), so no launch and no array come before it. Bound by
+// memory: 32-byte loads, four rows in flight per thread, four blocks per SM read
+// 7.2 TB/s of a 14.5 GB B (16-byte loads of two rows: 6.7).
 constexpr int kGtThreads = 256;
 constexpr int kGtCols = kGtThreads * 8;
 constexpr int kGtRows = 32;
@@ -48,11 +57,14 @@ __global__ void __launch_bounds__(kGtThreads) gamma_partial_kernel(
   __shared__ double sd[kGtRows];
   const int64_t r0 = blockIdx.x * rows_per_cta;
   const int64_t r1 = min(nrows, r0 + rows_per_cta);
-  const int64_t c0 = (int64_t)blockIdx.y * kGtCols + 2 * threadIdx.x;
+  // columns c0 .. + 3 and c0 + 1024 .. + 3 (ldb is a multiple of 8)
+  const int64_t c0 = (int64_t)blockIdx.y * kGtCols + 4 * threadIdx.x;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  double2 acc[4];
+  double acc[2][4];
 #pragma unroll
-  for (int j = 0; j < 4; ++j) acc[j] = make_double2(0.0, 0.0);
+  for (int j = 0; j < 2; ++j)
+#pragma unroll
+    for (int u = 0; u < 4; ++u) acc[j][u] = 0.0;
   for (int64_t t0 = r0; t0 < r1; t0 += kGtRows) {
     if (src.C) {
 #pragma unroll
@@ -77,26 +89,29 @@ __global__ void __launch_bounds__(kGtThreads) gamma_partial_kernel(
     }
     __syncthreads();
     const int nr = (int)min(r1 - t0, (int64_t)kGtRows);
-#pragma unroll 2
+#pragma unroll 4
     for (int q = 0; q < nr; ++q) {
       const double d = sd[q];
       const double* row = B + (t0 + q) * ldb;
 #pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        const int64_t c = c0 + j * 2 * kGtThreads;
+      for (int j = 0; j < 2; ++j) {
+        const int64_t c = c0 + j * 4 * kGtThreads;
         if (c < ldb) {
-          const double2 b = __ldcs(reinterpret_cast<const double2*>(row + c));
-          acc[j].x += d * b.x;
-          acc[j].y += d * b.y;
+          double v[4];
+          load4(row + c, v);
+#pragma unroll
+          for (int u = 0; u < 4; ++u) acc[j][u] += d * v[u];
         }
       }
     }
     __syncthreads();
   }
 #pragma unroll
-  for (int j = 0; j < 4; ++j) {
-    const int64_t c = c0 + j * 2 * kGtThreads;
-    if (c < ldb) *reinterpret_cast<double2*>(part + blockIdx.x * ldb + c) = acc[j];
+  for (int j = 0; j < 2; ++j) {
+    const int64_t c = c0 + j * 4 * kGtThreads;
+    if (c < ldb)
+#pragma unroll
+      for (int u = 0; u < 4; ++u) part[blockIdx.x * ldb + c + u] = acc[j][u];
   }
 }
 
@@ -133,35 +148,38 @@ static void launch_reduce_rows(const double* part, int64_t nparts, int64_t ldb, 
   DFJK_LAUNCHED();
 }
 
-// J rows: one warp per row, J[m, n] and J[n, m]
-__global__ void j_rows_kernel(const double* __restrict__ B, int64_t ldb, int64_t nrows,
-                              const double* __restrict__ gamma, const int* __restrict__ rm,
-                              const int* __restrict__ rn, const int8_t* __restrict__ kind,
-                              int64_t nao, double* __restrict__ J) {
+// J rows: one warp per row, J[m, n] and J[n, m]. Bound by memory: two 32-byte
+// loads per lane in flight, 64 warps per SM (6.8 TB/s of a 14.5 GB B; four
+// 16-byte loads: 5.7).
+__global__ void __launch_bounds__(256) j_rows_kernel(
+    const double* __restrict__ B, int64_t ldb, int64_t nrows, const double* __restrict__ gamma,
+    const int* __restrict__ rm, const int* __restrict__ rn, const int8_t* __restrict__ kind,
+    int64_t nao, double* __restrict__ J) {
   const int lane = threadIdx.x & 31;
   const int64_t nwarps = (gridDim.x * (int64_t)blockDim.x) >> 5;
   for (int64_t r = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5; r < nrows; r += nwarps) {
     const double* row = B + r * ldb;
-    // four 16-byte loads in flight per lane (ldb is a multiple of 8 and c is
-    // even, so c + 192 < ldb keeps all four pairs inside the row)
-    double s4[4] = {0.0, 0.0, 0.0, 0.0};
-    int64_t c = 2 * lane;
-    for (; c + 192 < ldb; c += 256) {
-      double2 b[4], g[4];
-#pragma unroll
-      for (int u = 0; u < 4; ++u) {
-        b[u] = __ldcs(reinterpret_cast<const double2*>(row + c + 64 * u));
-        g[u] = __ldg(reinterpret_cast<const double2*>(gamma + c + 64 * u));
-      }
-#pragma unroll
-      for (int u = 0; u < 4; ++u) s4[u] += b[u].x * g[u].x + b[u].y * g[u].y;
+    // ldb is a multiple of 8 and c of 4: a load that starts inside the row ends there
+    double s2[2] = {0.0, 0.0};
+    auto add = [&](const double (&b)[4], int64_t c, double& s) {
+      const double2 g0 = __ldg(reinterpret_cast<const double2*>(gamma + c));
+      const double2 g1 = __ldg(reinterpret_cast<const double2*>(gamma + c + 2));
+      s += b[0] * g0.x + b[1] * g0.y + b[2] * g1.x + b[3] * g1.y;
+    };
+    int64_t c = 4 * lane;
+    for (; c + 128 < ldb; c += 256) {
+      double b0[4], b1[4];
+      load4(row + c, b0);
+      load4(row + c + 128, b1);
+      add(b0, c, s2[0]);
+      add(b1, c + 128, s2[1]);
     }
-    for (; c < ldb; c += 64) {
-      const double2 b = __ldcs(reinterpret_cast<const double2*>(row + c));
-      const double2 g = __ldg(reinterpret_cast<const double2*>(gamma + c));
-      s4[0] += b.x * g.x + b.y * g.y;
+    if (c < ldb) {
+      double b0[4];
+      load4(row + c, b0);
+      add(b0, c, s2[0]);
     }
-    double s = (s4[0] + s4[1]) + (s4[2] + s4[3]);
+    double s = s2[0] + s2[1];
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
     if (lane == 0) {
@@ -633,7 +651,7 @@ static void syrk_fp64(Plan& p, const double* X, int64_t kt, double sign, bool be
   int64_t best = INT64_MAX;
   for (int64_t q = 1; q <= most; ++q) {
     const int64_t t = (tiles * q + slots - 1) / slots * ((kt + q - 1) / q + 128);
-    if (t < best) {
+    if (best == INT64_MAX || 100 * t < 98 * best) {   // (a slice costs a partial of K)
       best = t;
       nsplit = q;
     }

@@ -520,7 +520,7 @@ static int64_t syrk_slice(int64_t kt, int64_t nao, int dev) {
   for (int64_t q = least; q <= most; ++q) {
     const int64_t per = (ktiles + q - 1) / q;
     const int64_t t = (tiles * q + sm - 1) / sm * (per + 14);
-    if (t < best) {
+    if (best == INT64_MAX || 100 * t < 98 * best) {   // (a slice costs a partial of K)
       best = t;
       slice = per * sh.box_k;
     }
