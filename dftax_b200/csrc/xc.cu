@@ -470,6 +470,12 @@ __global__ void __launch_bounds__(256, 3) rho_kernel(
     if (q < steps) stage(q);
     cp_async_commit();
   }
+  // a column block's dPhi, 512 bytes of 3 x 64 rows, on its way to L2 while the
+  // block's products run: its epilogue reads it
+  auto ahead = [&](int cb) {
+    const int d = tid >> 6, c = cb * kRpCols + (tid & 63);
+    if (d < 3 && c < nsig) prefetch_l2(dphi + d * plane + c * G + g0, kRpPts * sizeof(double));
+  };
   double acc[2][4][2], sum[4][2];   // sum: rho, grad of the lane's two points
 #pragma unroll
   for (int a = 0; a < 2; ++a)
@@ -484,6 +490,7 @@ __global__ void __launch_bounds__(256, 3) rho_kernel(
     cp_async_commit();
     const double* As = rsm + (q % kRpStages) * kRpStage;
     const double* Bs = As + kRpK * kRpPitch;
+    if (q % nk == 0) ahead(q / nk);
     if (q / nk * kRpCols + wi < nsig) {   // else the warp's columns lie past the functions
 #pragma unroll
       for (int kk = 0; kk < kRpK; kk += 4) {
@@ -845,19 +852,21 @@ void xc_chunk(const Shells& sh, const int (&nout)[8], const std::vector<double>&
     grp = XcGroup{};
     phi = pc = part = 0;
   };
+  // each chunk's shells
+  struct Chunk {
+    int64_t g0, ng;
+    int nsig;
+    std::vector<int> shells;
+  };
+  std::vector<Chunk> chunks;
   for (int64_t g0 = 0; g0 < n; g0 += G) {
-    const int64_t ng = std::min(G, n - g0);
+    Chunk ch{g0, std::min(G, n - g0), 0, {}};
     double bl[3] = {INFINITY, INFINITY, INFINITY}, bh[3] = {-INFINITY, -INFINITY, -INFINITY};
-    for (int64_t i = g0; i < g0 + ng; ++i)
+    for (int64_t i = g0; i < g0 + ch.ng; ++i)
       for (int d = 0; d < 3; ++d) {
         bl[d] = std::min(bl[d], pts[3 * i + d]);
         bh[d] = std::max(bh[d], pts[3 * i + d]);
       }
-    std::vector<Entry> mine;
-    int nsig = 0;
-    const int64_t ao = (int64_t)aomap.size();
-    pos.resize(pos.size() + nao, -1);
-    int* ps = pos.data() + pos.size() - nao;
     for (int s = 0; s < sh.n; ++s) {
       double d2 = 0.0;
       for (int d = 0; d < 3; ++d) {
@@ -866,17 +875,34 @@ void xc_chunk(const Shells& sh, const int (&nout)[8], const std::vector<double>&
         d2 += e * e;
       }
       if (bound(s, std::sqrt(d2)) <= thresh) continue;
-      mine.push_back({s, nsig, 0});
+      ch.shells.push_back(s);
+      ch.nsig += nout[sh.l[s]];
+    }
+    chunks.push_back(std::move(ch));
+  }
+  // the chunks with the most functions first: a group's chunks are then alike,
+  // and a launch ends on its shortest blocks
+  std::stable_sort(chunks.begin(), chunks.end(),
+                   [](const Chunk& a, const Chunk& b) { return a.nsig > b.nsig; });
+  for (const Chunk& ch : chunks) {
+    const int nsig = ch.nsig;
+    const int64_t ao = (int64_t)aomap.size();
+    pos.resize(pos.size() + nao, -1);
+    int* ps = pos.data() + pos.size() - nao;
+    int c = 0;
+    std::vector<Entry> mine;
+    for (int s : ch.shells) {
+      mine.push_back({s, c, 0});
       const int no = nout[sh.l[s]];
       for (int m = 0; m < no; ++m) {
         aomap.push_back(sh.out0[s] + m);
-        ps[sh.out0[s] + m] = nsig + m;
+        ps[sh.out0[s] + m] = c + m;
       }
-      nsig += no;
+      c += no;
     }
     // AO values, three gradients and the weighted AOs: 40 bytes per function and point
     if (grp.count > 0 && (phi + (int64_t)nsig * G) * 40 > kXcGroupBytes) close();
-    XcChunkInfo ci{nsig, nsig + (nsig & 1), g0, ng, phi, pc, part, ao};
+    XcChunkInfo ci{nsig, nsig + (nsig & 1), ch.g0, ch.ng, phi, pc, part, ao};
     if (grp.count == 0) grp.first = (int)out.info.size();
     for (Entry e : mine) {
       e.chunk = grp.count;
