@@ -519,7 +519,11 @@ __global__ void __launch_bounds__(256, 3) syrk_part_kernel(const double* __restr
   const int64_t k0 = (int64_t)blockIdx.y * kslice;
   const int64_t k1 = k0 + kslice < kt ? k0 + kslice : kt;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int wr = (warp & 3) * 16, wc = (warp >> 2) * 32;
+  // 16 rows x 32 columns a warp. Warps with nothing to do (above the diagonal, past
+  // nao) leave the tensor pipe of their quarter of the SM idle, so the rows go to
+  // the warps turned by block and column half.
+  const int wr = ((warp + (warp >> 1 & 2) + (int)(blockIdx.x + blockIdx.y)) & 3) * 16;
+  const int wc = (warp >> 2) * 32;
   const int fr = lane >> 2, fk = lane & 3;
   const bool work = r0 + wr < nao && c0 + wc < nao && !(diag && wc > wr + 15);
   double acc[2][4][2];

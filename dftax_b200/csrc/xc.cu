@@ -579,7 +579,10 @@ __global__ void __launch_bounds__(256, 3) v_kernel(const double* __restrict__ ph
   const int64_t k0 = blockIdx.y * (int64_t)kVSlice;
   const int64_t k1 = k0 + kVSlice < G ? k0 + kVSlice : G;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int wr = (warp & 3) * 16, wc = (warp >> 2) * 32;
+  // rows turned by block and column half: the warps past nsig then leave different
+  // quarters of the SM, with their tensor pipes, idle
+  const int wr = ((warp + (warp >> 1 & 2) + (int)(blockIdx.x + blockIdx.y + blockIdx.z)) & 3) * 16;
+  const int wc = (warp >> 2) * 32;
   const int fr = lane >> 2, fk = lane & 3;
   const bool work = r0 + wr < nsig && c0 + wc < nsig;
   double acc[2][4][2];
