@@ -116,10 +116,10 @@ int64_t estimate(const dfbatch_request* r) {
   b += (22 + 2 * diis) * nao * nao * 8;                          // SCF matrices (purification, density factor too), DIIS
   const int64_t G = r->scf_opts.grid_chunk > 0 ? r->scf_opts.grid_chunk : 16384;
   // XC chunk buffers and a V accumulator on each of the solve's XC streams
-  // (one unless the request asks for more: xc.cu), the grid
+  // (one unless the request asks for more: xc.cu), the grid and its sort
   const int64_t nbr = r->scf_opts.xc_streams > 0 ? r->scf_opts.xc_streams : 1;
   const int64_t grp = std::max<int64_t>(dfjk::kXcGroupBytes, 5 * nao * G * 8);
-  b += nbr * (grp + (G / 512 + 3) * nao * nao * 8) + r->npoint * 4 * 8;
+  b += nbr * (grp + (G / 512 + 3) * nao * nao * 8) + r->npoint * 11 * 8;
   return b + b / 10 + ((int64_t)256 << 20);
 }
 

@@ -677,7 +677,7 @@ std::map<std::tuple<int, int, int>, int64_t>& tuned() {
   return *m;
 }
 
-void autotune_chunk(dfscf& f, const int (&nout)[8], const std::vector<double>& pv,
+void autotune_chunk(dfscf& f, const int (&nout)[8], const std::vector<double>& boxes,
                     cudaStream_t s) {
   int lg = 0;
   while ((int64_t(1) << (lg + 1)) <= f.npts) ++lg;
@@ -696,7 +696,7 @@ void autotune_chunk(dfscf& f, const int (&nout)[8], const std::vector<double>& p
       if (G < 4096 && f.npts < ((int64_t)1 << 16)) continue;
       // as the SCF runs it: the first call launches directly, the second
       // captures the CUDA graph, the timed ones replay it
-      xc_chunk(f.p->orb, nout, pv, G, f.o.ao_thresh, f.xcw);
+      xc_chunk(f.p->orb, nout, f.npts, boxes, G, f.o.ao_thresh, f.xcw);
       for (int rep = 0; rep < 2; ++rep)
         xc_energy_fock(*f.c, f.ov, f.pts.as<double>(), f.wts.as<double>(), f.P.as<double>(),
                        f.Vxc.as<double>(), xc_params(f), f.xcw, s);
@@ -714,7 +714,7 @@ void autotune_chunk(dfscf& f, const int (&nout)[8], const std::vector<double>& p
     tuned().emplace(key, best);
   }
   f.tuned_chunk = best;
-  xc_chunk(f.p->orb, nout, pv, best, f.o.ao_thresh, f.xcw);   // also a fresh graph state
+  xc_chunk(f.p->orb, nout, f.npts, boxes, best, f.o.ao_thresh, f.xcw);   // also a fresh graph state
 }
 
 }  // namespace
@@ -785,18 +785,15 @@ dfjk_status dfscf_create(dfjk_plan* pl, int32_t natom, const double* atom_xyz,
     upload(f->atom_xyz, std::vector<double>(atom_xyz, atom_xyz + 3 * natom));
     upload(f->atom_z, std::vector<double>(atom_charge, atom_charge + natom));
     if (!(f->o.ao_thresh >= 0.0)) fail(DFJK_ERR_INVALID, "ao_thresh must be >= 0");
-    std::vector<double> pv, wv;
+    cudaStream_t s = static_cast<cudaStream_t>(stream);
+    std::vector<double> boxes;
     int nout[8];
     for (int l = 0; l < 8; ++l) nout[l] = p.orb.spherical ? 2 * l + 1 : ncart(l);
     if (npoint > 0) {
       // spatially sorted chunks with their non-negligible shells
-      pv.assign(grid_xyz, grid_xyz + 3 * npoint);
-      wv.assign(grid_w, grid_w + npoint);
-      xc_sort(pv, wv);
+      sort_points(grid_xyz, grid_w, npoint, f->pts, f->wts, boxes, s);
       const int64_t G = f->o.grid_chunk > 0 ? (f->o.grid_chunk + 255) / 256 * 256 : 8192;
-      if (!tunes(*f)) xc_chunk(p.orb, nout, pv, G, f->o.ao_thresh, f->xcw);
-      upload(f->pts, pv);
-      upload(f->wts, wv);
+      if (!tunes(*f)) xc_chunk(p.orb, nout, npoint, boxes, G, f->o.ao_thresh, f->xcw);
     }
     double enn = 0.0;
     for (int a = 0; a < natom; ++a)
@@ -821,7 +818,6 @@ dfjk_status dfscf_create(dfjk_plan* pl, int32_t natom, const double* atom_xyz,
     const int64_t n = p.nao, nn = n * n;
     for (DevBuf* b : {&f->S, &f->T, &f->V, &f->H, &f->P, &f->F, &f->J, &f->K, &f->Vxc, &f->A1, &f->A2})
       b->alloc(nn * sizeof(double));
-    cudaStream_t s = static_cast<cudaStream_t>(stream);
     launch_one_electron(*c, ov, f->nshell, p.orb.l, natom, f->atom_xyz.as<double>(),
                         f->atom_z.as<double>(), f->S.as<double>(), f->T.as<double>(),
                         f->V.as<double>(), s);
@@ -865,7 +861,7 @@ dfjk_status dfscf_create(dfjk_plan* pl, int32_t natom, const double* atom_xyz,
     f->dE.alloc((size_t)f->o.diis_space * m * m * sizeof(double));
     DFJK_CUDA(cudaMemsetAsync(f->dE.p, 0, (size_t)f->o.diis_space * m * m * sizeof(double), s));
     DFJK_CUDA(cudaMemsetAsync(f->dF.p, 0, (size_t)f->o.diis_space * nn * sizeof(double), s));
-    if (tunes(*f)) autotune_chunk(*f, nout, pv, s);
+    if (tunes(*f)) autotune_chunk(*f, nout, boxes, s);
     DFJK_CUDA(cudaStreamSynchronize(s));
   });
   if (st != DFJK_OK) {

@@ -107,14 +107,18 @@ size_t sp2_cluster_bytes(int m);
 void launch_sp2_cluster(const double* A, int m, int nocc, int max_steps, double* Xg, double* X,
                         double* rec, cudaStream_t s);
 
-// Sorts the points (and weights) along a Morton curve over 1-Bohr cells;
-// pts [n][3] and w [n] are host arrays, reordered in place.
-void xc_sort(std::vector<double>& pts, std::vector<double>& w);
-// Cuts sorted points into chunks of G points and keeps for each chunk the
+// Uploads the grid sorted along a Morton curve over 1-Bohr cells, points of a cell
+// in their own order (points.cu): pts [n][3] and w [n] on the device, and the
+// bounding box {low x, y, z, high x, y, z} of every kXcBox sorted points. pts_host
+// and w_host are host arrays. Host synchronizing.
+constexpr int kXcBox = 256;
+void sort_points(const double* pts_host, const double* w_host, int64_t n, DevBuf& pts, DevBuf& w,
+                 std::vector<double>& boxes, cudaStream_t s);
+// Cuts n sorted points into chunks of G points, a multiple of kXcBox, and keeps for each chunk the
 // shells whose value-and-gradient bound over the chunk's bounding box exceeds
 // thresh (uploads the shell lists); forgets any captured graph of ws.
-void xc_chunk(const Shells& sh, const int (&nout)[8], const std::vector<double>& pts, int64_t G,
-              double thresh, XcWork& ws);
+void xc_chunk(const Shells& sh, const int (&nout)[8], int64_t n, const std::vector<double>& boxes,
+              int64_t G, double thresh, XcWork& ws);
 
 struct XcParams {
   double x_scale = 0.75;        // PBE exchange share (PBE0)

@@ -30,7 +30,6 @@
 
 #include <algorithm>
 #include <cmath>
-#include <thread>
 #include <utility>
 
 namespace dfjk {
@@ -698,95 +697,6 @@ void launch_becke_partition(const double* pts, const int* owner, const double* r
   DFJK_CUDA(cudaStreamSynchronize(s));   // the pair tables are freed on return
 }
 
-// interleaves the low 21 bits of x, y, z (Morton order)
-static uint64_t morton3(uint64_t x, uint64_t y, uint64_t z) {
-  auto spread = [](uint64_t v) {
-    v &= 0x1fffffULL;
-    v = (v | v << 32) & 0x1f00000000ffffULL;
-    v = (v | v << 16) & 0x1f0000ff0000ffULL;
-    v = (v | v << 8) & 0x100f00f00f00f00fULL;
-    v = (v | v << 4) & 0x10c30c30c30c30c3ULL;
-    v = (v | v << 2) & 0x1249249249249249ULL;
-    return v;
-  };
-  return spread(x) | spread(y) << 1 | spread(z) << 2;
-}
-
-void xc_sort(std::vector<double>& pts, std::vector<double>& w) {
-  const int64_t n = (int64_t)w.size();
-  if (n == 0) return;
-  // contiguous index ranges of at least 32 k points, one per host thread (starting
-  // 15 threads for each of the seven passes cost more than sorting 100 k points)
-  const int T = (int)std::max<int64_t>(
-      1, std::min<int64_t>(n >> 15, std::min<unsigned>(16, std::max(1u, std::thread::hardware_concurrency()))));
-  auto lo_of = [&](int t) { return n * t / T; };
-  // Morton order of 1-Bohr cells
-  std::vector<double> los((size_t)3 * T, INFINITY);
-  run_on_threads(T, [&](int t) {
-    for (int64_t i = lo_of(t); i < lo_of(t + 1); ++i)
-      for (int d = 0; d < 3; ++d) los[3 * t + d] = std::min(los[3 * t + d], pts[3 * i + d]);
-  });
-  double lo[3] = {INFINITY, INFINITY, INFINITY};
-  for (int t = 0; t < T; ++t)
-    for (int d = 0; d < 3; ++d) lo[d] = std::min(lo[d], los[3 * t + d]);
-  std::vector<uint64_t> code(n), ktmp(n), cmaxs(T, 0);
-  std::vector<int64_t> order(n), otmp(n);
-  run_on_threads(T, [&](int t) {
-    for (int64_t i = lo_of(t); i < lo_of(t + 1); ++i) {
-      uint64_t c[3];
-      for (int d = 0; d < 3; ++d) c[d] = (uint64_t)std::floor(pts[3 * i + d] - lo[d]);
-      code[i] = morton3(c[0], c[1], c[2]);
-      cmaxs[t] = std::max(cmaxs[t], code[i]);
-      order[i] = i;
-    }
-  });
-  const uint64_t cmax = *std::max_element(cmaxs.begin(), cmaxs.end());
-  // order by (code, index): a stable LSD radix sort of the codes, 11 bits a
-  // pass over the bits cmax needs. Per pass each thread counts its range;
-  // the offsets run bucket by bucket and, within a bucket, thread by thread,
-  // so every thread's elements land after those of lower indices (stable)
-  int bits = 0;
-  while (bits < 64 && (cmax >> bits) != 0) ++bits;
-  constexpr int kRadixBits = 11;
-  constexpr uint64_t kBuckets = (uint64_t)1 << kRadixBits, kMask = kBuckets - 1;
-  std::vector<int64_t> hist((size_t)T * kBuckets);
-  for (int shift = 0; shift < bits; shift += kRadixBits) {
-    run_on_threads(T, [&](int t) {
-      int64_t* h = hist.data() + (size_t)t * kBuckets;
-      std::fill(h, h + kBuckets, 0);
-      for (int64_t i = lo_of(t); i < lo_of(t + 1); ++i) h[(code[i] >> shift) & kMask]++;
-    });
-    int64_t run = 0;
-    for (uint64_t b = 0; b < kBuckets; ++b)
-      for (int t = 0; t < T; ++t) {
-        int64_t& h = hist[(size_t)t * kBuckets + b];
-        const int64_t c = h;
-        h = run;
-        run += c;
-      }
-    run_on_threads(T, [&](int t) {
-      int64_t* h = hist.data() + (size_t)t * kBuckets;
-      for (int64_t i = lo_of(t); i < lo_of(t + 1); ++i) {
-        const int64_t dst = h[(code[i] >> shift) & kMask]++;
-        ktmp[dst] = code[i];
-        otmp[dst] = order[i];
-      }
-    });
-    code.swap(ktmp);
-    order.swap(otmp);
-  }
-  std::vector<double> p2(3 * n), w2(n);
-  run_on_threads(T, [&](int t) {
-    for (int64_t i = lo_of(t); i < lo_of(t + 1); ++i) {
-      const int64_t j = order[i];
-      for (int d = 0; d < 3; ++d) p2[3 * i + d] = pts[3 * j + d];
-      w2[i] = w[j];
-    }
-  });
-  pts.swap(p2);
-  w.swap(w2);
-}
-
 // slices of a chunk's V product
 static int64_t xc_slices(int64_t G) { return (G + kVSlice - 1) / kVSlice; }
 
@@ -796,10 +706,9 @@ static int64_t v_parts(int64_t nao) {
   return std::min<int64_t>(8, std::max<int64_t>(1, ((int64_t)1 << 18) / (nao * nao)));
 }
 
-void xc_chunk(const Shells& sh, const int (&nout)[8], const std::vector<double>& pts, int64_t G,
-              double thresh, XcWork& ws) {
+void xc_chunk(const Shells& sh, const int (&nout)[8], int64_t n, const std::vector<double>& boxes,
+              int64_t G, double thresh, XcWork& ws) {
   XcChunks& out = ws.ch;
-  const int64_t n = (int64_t)pts.size() / 3;
   out.info.clear();
   out.groups.clear();
   out.max_phi = out.max_pc = out.max_part = out.max_points = 0;
@@ -865,10 +774,10 @@ void xc_chunk(const Shells& sh, const int (&nout)[8], const std::vector<double>&
   for (int64_t g0 = 0; g0 < n; g0 += G) {
     Chunk ch{g0, std::min(G, n - g0), 0, {}};
     double bl[3] = {INFINITY, INFINITY, INFINITY}, bh[3] = {-INFINITY, -INFINITY, -INFINITY};
-    for (int64_t i = g0; i < g0 + ch.ng; ++i)
+    for (int64_t b = g0 / kXcBox; b < (g0 + ch.ng + kXcBox - 1) / kXcBox; ++b)
       for (int d = 0; d < 3; ++d) {
-        bl[d] = std::min(bl[d], pts[3 * i + d]);
-        bh[d] = std::max(bh[d], pts[3 * i + d]);
+        bl[d] = std::min(bl[d], boxes[6 * b + d]);
+        bh[d] = std::max(bh[d], boxes[6 * b + 3 + d]);
       }
     for (int s = 0; s < sh.n; ++s) {
       double d2 = 0.0;

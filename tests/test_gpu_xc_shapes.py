@@ -39,3 +39,33 @@ def test_xc_shapes(name, npts, chunk):
         assert np.linalg.norm(V.cpu().numpy() - V0) <= REL * np.linalg.norm(V0)
     e1, none = ks.xc_energy(P, want_fock=False)
     assert none is None and abs(e1 - e0) <= REL * abs(e0)
+
+
+@pytest.mark.parametrize("npts,far", [(2047, 30.0), (2049, 300.0), (6000, 1e5), (5000, 1e7)])
+def test_scattered_points(npts, far):
+    """The device sort of the grid at tile edges (2048 points), with many points in
+    one cell (equal keys) and with one to eight digits of key: half of the points
+    lie up to `far` Bohr out, where the density vanishes."""
+    import torch
+
+    from dftax_b200 import df, systems
+    from dftax_b200.ks import KS
+    from oracle import ks as oks
+
+    sym, xyz, orb, aux, nocc = systems.workload("water", seed=1)
+    rng = np.random.default_rng(npts)
+    pts = xyz[rng.integers(0, len(xyz), npts)] + rng.standard_normal((npts, 3))
+    pts[::2] += rng.uniform(-far, far, pts[::2].shape)
+    w = rng.uniform(0.01, 0.1, npts)
+    C = systems.random_occupied(orb.nao, nocc, seed=3)
+    P = 2.0 * C @ C.T
+    e0, V0 = oks.exc_and_vxc(orb, pts, w, P)
+    e = []
+    for _ in range(2):
+        ks = KS(sym, xyz, orb, coulomb=df(aux), grid=(pts, w), grid_chunk=512)
+        e1, V = ks.xc_energy(torch.as_tensor(P, device="cuda"))
+        assert abs(e1 - e0) <= REL * abs(e0)
+        assert np.linalg.norm(V.cpu().numpy() - V0) <= REL * np.linalg.norm(V0)
+        e.append(e1)
+        ks.close()
+    assert e[0] == e[1]
