@@ -72,6 +72,18 @@ struct Error {
     ::dfjk::count_launch();             \
   } while (0)
 
+// Lets a kernel whose dynamic shared memory depends on the call take up to the 227 KB
+// of a block. The limit belongs to the function, for all threads of the process: were
+// it set to each call's own size, a smaller call of another thread could lower it
+// before this one's launch, which would then be refused.
+template <class Kernel>
+void allow_shared(Kernel* kernel) {
+  cudaFuncAttributes at{};
+  DFJK_CUDA(cudaFuncGetAttributes(&at, kernel));
+  DFJK_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 232448 - (int)at.sharedSizeBytes));
+}
+
 // Device memory cache (api.cu): freed DevBufs are kept for reuse per device.
 // Synchronizes device dev and records that every buffer freed before the
 // synchronization began is idle (may be handed out again without waiting).

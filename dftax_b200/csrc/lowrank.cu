@@ -195,8 +195,7 @@ bool LowRankInfo::within(int sp, double tol) const {
 void launch_low_rank(const double* P, int64_t n, int nspin, int64_t max_rank, double* Ct,
                      LowRankInfo* info, cudaStream_t s) {
   const size_t smem = chol_smem(n);
-  DFJK_CUDA(cudaFuncSetAttribute(pivoted_cholesky_kernel,
-                                 cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  allow_shared(pivoted_cholesky_kernel);
   pivoted_cholesky_kernel<<<kCta * nspin, kLanes * 32, smem, s>>>(P, n, std::min(max_rank, n), kLowRankTol,
                                                                    Ct, info);
   DFJK_LAUNCHED();

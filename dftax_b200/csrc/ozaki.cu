@@ -305,8 +305,7 @@ void check_oz_err(Plan& p, cudaStream_t s) {
 template <int XB>
 static void launch_kplanes(Plan& p, int64_t plane, cudaStream_t s) {
   const size_t smem = (size_t)4 * XB * (p.nao_p16 + 4);
-  DFJK_CUDA(cudaFuncSetAttribute(kplanes_kernel<XB>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)smem));
+  allow_shared(kplanes_kernel<XB>);
   const int64_t nxb = (p.nfit + XB - 1) / XB;
   for (int64_t b0 = 0; b0 < nxb; b0 += 65535) {
     const int64_t nb = std::min<int64_t>(65535, nxb - b0);

@@ -192,8 +192,7 @@ size_t sp2_cluster_bytes(int m) {
 void launch_sp2_cluster(const double* A, int m, int nocc, int max_steps, double* Xg, double* X,
                         double* rec, cudaStream_t s) {
   const size_t smem = sp2_cluster_bytes(m);
-  DFJK_CUDA(cudaFuncSetAttribute(sp2_cluster_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)smem));
+  allow_shared(sp2_cluster_kernel);
   sp2_cluster_kernel<<<kCta, kWarps * 32, smem, s>>>(A, m, nocc, max_steps, Xg, X, rec);
   DFJK_LAUNCHED();
 }

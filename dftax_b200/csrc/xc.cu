@@ -689,8 +689,7 @@ void launch_becke_partition(const double* pts, const int* owner, const double* r
   int threads = 64;
   const size_t smem = (size_t)natom * threads * sizeof(double);
   if (smem > 200 * 1024) fail(DFJK_ERR_UNSUPPORTED, "Becke partition supports at most 400 atoms");
-  DFJK_CUDA(cudaFuncSetAttribute(becke_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)std::max<size_t>(smem, 1)));
+  allow_shared(becke_kernel);
   becke_kernel<<<(unsigned)((n + threads - 1) / threads), threads, smem, s>>>(
       pts, owner, raw, n, dxyz.as<double>(), dinv.as<double>(), daab.as<double>(), natom, w);
   DFJK_LAUNCHED();

@@ -67,3 +67,38 @@ def test_energy_of_any_density(name, precision, hf_lr):
         assert abs(e - ref) <= rel * size * max(float(Pt.norm()), 1e-300), (what, e, ref)
         e2, F2 = plan.energy(Pt, 0.25, hf_coeff_lr=hf_lr)
         assert e2 == e and torch.equal(F, F2), what
+
+
+def test_sizes_on_two_threads():
+    """Threads that factor densities of different sizes at once, each on its own
+    context and stream: every energy is the one of a lone call."""
+    import threading
+
+    import torch
+
+    from dftax_b200 import Plan, systems
+    from dftax_b200.coulomb import Context
+
+    plans, dens, alone = [], [], []
+    for name in ("water", "water6"):
+        _, _, orb, aux, nocc = systems.workload(name, seed=2)
+        plans.append(Plan(orb, aux, ctx=Context(0)).build())
+        C = systems.random_occupied(orb.nao, nocc, seed=5)
+        dens.append(torch.as_tensor(2.0 * C @ C.T, device="cuda"))
+        alone.append(plans[-1].energy(dens[-1], 0.25)[0])
+    errors = []
+
+    def work(q):
+        try:
+            with torch.cuda.stream(torch.cuda.Stream()):
+                for _ in range(300):
+                    assert abs(plans[q].energy(dens[q], 0.25)[0] - alone[q]) <= 1e-10 * abs(alone[q])
+        except Exception as e:  # noqa: BLE001
+            errors.append(repr(e))
+
+    threads = [threading.Thread(target=work, args=(q,)) for q in (0, 1)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not errors, errors[0]
