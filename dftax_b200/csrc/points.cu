@@ -189,25 +189,29 @@ void sort_points(const double* pts_host, const double* w_host, int64_t n, DevBuf
   if (n >= (int64_t)1 << 31) fail(DFJK_ERR_UNSUPPORTED, "%lld grid points", (long long)n);
   const int64_t nbox = (n + kXcBox - 1) / kXcBox, tiles = (n + kTile - 1) / kTile;
   static_assert(kXcBox == kThreads, "a box is a block's points");
-  DevBuf raw, raw_w, key[2], idx[2], hist, box;
   pts.alloc(3 * n * sizeof(double));
   w.alloc(n * sizeof(double));
-  raw.alloc(3 * n * sizeof(double));
-  raw_w.alloc(n * sizeof(double));
-  box.alloc(6 * nbox * sizeof(double));
-  for (int q = 0; q < 2; ++q) {
-    key[q].alloc(n * sizeof(uint64_t));
-    idx[q].alloc(n * sizeof(uint32_t));
-  }
-  hist.alloc(kDigits * tiles * sizeof(int));
+  // one buffer for all scratch: each one taken from the cache may wait for the device
+  DevBuf scratch;
+  scratch.alloc((4 * n + 6 * nbox) * sizeof(double) + 2 * n * sizeof(uint64_t) +
+                (2 * n + kDigits * tiles) * sizeof(uint32_t));
+  double* raw = scratch.as<double>();
+  double *raw_w = raw + 3 * n, *box = raw_w + n;
+  uint64_t* key[2];
+  key[0] = reinterpret_cast<uint64_t*>(box + 6 * nbox);
+  key[1] = key[0] + n;
+  uint32_t* idx[2];
+  idx[0] = reinterpret_cast<uint32_t*>(key[1] + n);
+  idx[1] = idx[0] + n;
+  int* hist = reinterpret_cast<int*>(idx[1] + n);
   boxes.resize(6 * nbox);
-  DFJK_CUDA(cudaMemcpyAsync(raw.p, pts_host, 3 * n * sizeof(double), cudaMemcpyHostToDevice, s));
-  DFJK_CUDA(cudaMemcpyAsync(raw_w.p, w_host, n * sizeof(double), cudaMemcpyHostToDevice, s));
+  DFJK_CUDA(cudaMemcpyAsync(raw, pts_host, 3 * n * sizeof(double), cudaMemcpyHostToDevice, s));
+  DFJK_CUDA(cudaMemcpyAsync(raw_w, w_host, n * sizeof(double), cudaMemcpyHostToDevice, s));
   auto gather = [&](const uint32_t* order) {
-    gather_kernel<<<(unsigned)nbox, kThreads, 0, s>>>(raw.as<double>(), raw_w.as<double>(), n, order,
-                                                      pts.as<double>(), w.as<double>(), box.as<double>());
+    gather_kernel<<<(unsigned)nbox, kThreads, 0, s>>>(raw, raw_w, n, order, pts.as<double>(),
+                                                      w.as<double>(), box);
     DFJK_LAUNCHED();
-    DFJK_CUDA(cudaMemcpyAsync(boxes.data(), box.p, 6 * nbox * sizeof(double), cudaMemcpyDeviceToHost, s));
+    DFJK_CUDA(cudaMemcpyAsync(boxes.data(), box, 6 * nbox * sizeof(double), cudaMemcpyDeviceToHost, s));
     DFJK_CUDA(cudaStreamSynchronize(s));
   };
   gather(nullptr);
@@ -219,21 +223,19 @@ void sort_points(const double* pts_host, const double* w_host, int64_t n, DevBuf
   // cells 0 .. floor(ext) a side: three bits of the key for each of theirs
   int bits = 0;
   while (bits < 21 && std::floor(ext) >= (double)((int64_t)1 << bits)) ++bits;
-  keys_kernel<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(raw.as<double>(), n, lo[0], lo[1], lo[2],
-                                                          key[0].as<uint64_t>(), idx[0].as<uint32_t>());
+  keys_kernel<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(raw, n, lo[0], lo[1], lo[2], key[0], idx[0]);
   DFJK_LAUNCHED();
   int q = 0;
   for (int shift = 0; shift < 3 * bits; shift += 8, q ^= 1) {
-    hist_kernel<<<(unsigned)tiles, kThreads, 0, s>>>(key[q].as<uint64_t>(), n, shift, hist.as<int>());
+    hist_kernel<<<(unsigned)tiles, kThreads, 0, s>>>(key[q], n, shift, hist);
     DFJK_LAUNCHED();
-    scan_kernel<<<1, kScanThreads, 0, s>>>(hist.as<int>(), kDigits * tiles);
+    scan_kernel<<<1, kScanThreads, 0, s>>>(hist, kDigits * tiles);
     DFJK_LAUNCHED();
-    scatter_kernel<<<(unsigned)tiles, kThreads, 0, s>>>(key[q].as<uint64_t>(), idx[q].as<uint32_t>(), n,
-                                                        shift, hist.as<int>(), key[q ^ 1].as<uint64_t>(),
-                                                        idx[q ^ 1].as<uint32_t>());
+    scatter_kernel<<<(unsigned)tiles, kThreads, 0, s>>>(key[q], idx[q], n, shift, hist, key[q ^ 1],
+                                                        idx[q ^ 1]);
     DFJK_LAUNCHED();
   }
-  gather(idx[q].as<uint32_t>());
+  gather(idx[q]);
 }
 
 }  // namespace dfjk
