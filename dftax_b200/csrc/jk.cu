@@ -521,7 +521,7 @@ __global__ void __launch_bounds__(256, 3) syrk_part_kernel(const double* __restr
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   // 16 rows x 32 columns a warp. Warps with nothing to do (above the diagonal, past
   // nao) leave the tensor pipe of their quarter of the SM idle, so the rows go to
-  // the warps turned by block and column half.
+  // the warps turned by block and column half ((H2O)_12: 572 -> 562 us).
   const int wr = ((warp + (warp >> 1 & 2) + (int)(blockIdx.x + blockIdx.y)) & 3) * 16;
   const int wc = (warp >> 2) * 32;
   const int fr = lane >> 2, fk = lane & 3;
