@@ -61,6 +61,7 @@ __global__ void __cluster_dims__(kCta, 1, 1) __launch_bounds__(kLanes * 32)
   double* d = sm;            // residual diagonal of rows lo .. hi - 1 (-1: pivoted)
   double* crow = sm + per;   // C[p][0 .. k - 1]
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  cluster_barrier();   // every CTA runs before anything is written into it
   Pivot best{-1.0, 0};
   if (warp == 0)
     for (int64_t i = lo + lane; i < hi; i += 32) {
