@@ -126,21 +126,25 @@ def test_refused_request_fails_alone(grid):
 
 
 def test_poisson_stream_matches_solo(solo, grid):
-    """Requests arrive with seeded exponential gaps (mean 0.03 s) while
-    earlier ones are on the GPU; each is admitted as memory frees up.  The
-    smallest of these gaps is 0.3 of the mean, and a solve takes 25 to 40 ms:
-    some solve is still running at the next arrival as long as the mean is
-    below 25 ms / 0.3 = 80 ms."""
+    """Requests arrive with seeded exponential gaps while earlier ones are on
+    the GPU; each is admitted as memory frees up.  The mean gap is the engine's
+    own shortest solve, run before the stream: the sixth gap, 0.3 of the mean,
+    then ends while the request before it is being solved, however fast a solve
+    is.  (The requests are prepared beforehand, so a gap holds nothing else.)"""
     from dftax_b200.batch import BatchEngine
 
     rng = np.random.default_rng(8)
     mols = molecules()
     order = [0, 3, 1, 4, 2, 3, 0]
     with BatchEngine(workers=3) as eng:
+        first = [eng.wait(eng.submit(*m, grid=grid)) for m in mols]
+        assert all(r.status == 0 for r in first)
+        unit = min(r.t_end - r.t_start for r in first)
+        reqs = [eng.request(*mols[k], grid=grid) for k in order]
         ids = []
-        for k in order:
-            ids.append((k, eng.submit(*mols[k], grid=grid)))
-            time.sleep(float(rng.exponential(0.03)))
+        for k, req in zip(order, reqs):
+            ids.append((k, eng.submit_request(req)))
+            time.sleep(float(rng.exponential(unit)))
         res = [(k, eng.wait(i)) for k, i in ids]
     lat = []
     for k, r in res:
