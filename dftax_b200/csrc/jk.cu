@@ -981,6 +981,18 @@ double energy(Plan& p, const double* P, int nspin, double hf, double hf_lr, doub
     const bool factored = low && h.low.within(sp, kLowRankAccept);
     DevBuf Ct, dw;
     if (!factored) density_factor(p, Ps, Ct, dw, s);   // indefinite, or too rough a factor
+    // the factor's columns C[m][k] at Cf[m * sm + k * sk]; mixed products take them
+    // spread out and laid out as they are read
+    const double* Cf = p.ws_lowrank.as<double>() + sp * nn;
+    int64_t sm = 1, sk = n;
+    const int64_t rank = factored ? h.low.rank[sp] : 0;
+    if (rank > 0 && p.opts.precision == DFJK_MIXED && !p.opts.streamed) {
+      sm = rank + (rank & 1);
+      sk = 1;
+      p.ws_Cp.ensure((size_t)n * sm * sizeof(double));
+      spread_columns(Cf, n, rank, sm, sm, 1, p.ws_Cp.as<double>(), s);
+      Cf = p.ws_Cp.as<double>();
+    }
     const struct { Plan* plan; double coeff; } terms[2] = {{&p, hf},
                                                            {p.lr ? &p.lr->p : nullptr, hf_lr}};
     for (int t = 0; t < 2; ++t) {
@@ -988,9 +1000,8 @@ double energy(Plan& p, const double* P, int nspin, double hf, double hf_lr, doub
       Plan& q = *terms[t].plan;
       if (!factored) {
         k_compute(q, Ct.as<double>(), dw.as<double>(), n, K, s);
-      } else if (h.low.rank[sp] > 0) {
-        k_accumulate(q, p.ws_lowrank.as<double>() + sp * nn, 1, n, nullptr, nullptr, h.low.rank[sp],
-                     1.0, true, K, s);
+      } else if (rank > 0) {
+        k_accumulate(q, Cf, sm, sk, nullptr, nullptr, rank, 1.0, true, K, s);
       } else {
         DFJK_CUDA(cudaMemsetAsync(K, 0, nn * sizeof(double), s));
       }

@@ -180,6 +180,39 @@ __global__ void __launch_bounds__(256) residual_kernel(const double* __restrict_
   }
 }
 
+// out(i, j) = sum_q Ct[q][i] H[q][j], H[q][j] = (cos + sin)(2 pi q j / r) / sqrt r
+// (Hartley's matrix, orthogonal and symmetric for every r), at out[i * si + j * sj];
+// j in [r, ncp): zero. The r values that H consists of, by q j mod r, in shared
+// memory. A block has 32 rows and eight columns, so that a few dozen orbitals
+// already give some forty blocks; bound by the latency of the loads of Ct.
+constexpr int kSpRows = 32, kSpCols = 8;
+__global__ void __launch_bounds__(kSpRows * kSpCols) spread_kernel(const double* __restrict__ Ct,
+                                                                   int64_t n, int r, int64_t ncp,
+                                                                   int64_t si, int64_t sj,
+                                                                   double* __restrict__ out) {
+  extern __shared__ double cas[];
+  for (int t = threadIdx.x; t < r; t += kSpRows * kSpCols) {
+    double sn, cs;
+    sincospi(2.0 * t / r, &sn, &cs);
+    cas[t] = (cs + sn) / sqrt((double)r);
+  }
+  __syncthreads();
+  const int64_t i = blockIdx.x * (int64_t)kSpRows + threadIdx.x % kSpRows;
+  const int64_t j = blockIdx.y * (int64_t)kSpCols + threadIdx.x / kSpRows;
+  if (i >= n || j >= ncp) return;
+  double acc = 0.0;
+  if (j < r) {
+    int t = 0;
+#pragma unroll 8
+    for (int q = 0; q < r; ++q) {
+      acc += Ct[q * n + i] * cas[t];
+      t += (int)j;
+      if (t >= r) t -= r;
+    }
+  }
+  out[i * si + j * sj] = acc;
+}
+
 size_t chol_smem(int64_t n) { return (size_t)((n + kCta - 1) / kCta + n) * sizeof(double); }
 
 }  // namespace
@@ -202,6 +235,14 @@ void launch_low_rank(const double* P, int64_t n, int nspin, int64_t max_rank, do
   DFJK_LAUNCHED();
   const unsigned t = (unsigned)((n + 31) / 32);
   residual_kernel<<<dim3(t, t, (unsigned)nspin), 256, 0, s>>>(P, n, Ct, info);
+  DFJK_LAUNCHED();
+}
+
+void spread_columns(const double* Ct, int64_t n, int64_t rank, int64_t ncp, int64_t si, int64_t sj,
+                    double* out, cudaStream_t s) {
+  allow_shared(spread_kernel);
+  const dim3 grid((unsigned)((n + kSpRows - 1) / kSpRows), (unsigned)((ncp + kSpCols - 1) / kSpCols));
+  spread_kernel<<<grid, kSpRows * kSpCols, (size_t)rank * sizeof(double), s>>>(Ct, n, (int)rank, ncp, si, sj, out);
   DFJK_LAUNCHED();
 }
 
