@@ -461,7 +461,8 @@ double energy_gradient(Plan& p, const double* P, int nspin, double hf, double* g
     DevBuf Bd, T1;
     // the densities' factors P_s = C C^T (lowrank.cu): with r = rank, B_x C
     // (half transform), C^T B_x C, C (C^T B_x C) and its product with C^T at the
-    // kept pairs cost 2 n^2 r + 4 n r^2 + n^2 r per direction instead of 4 n^3
+    // kept pairs cost 2 n^2 r + 4 n r^2 + n^2 r per direction instead of 4 n^3; past
+    // half the functions the dense form is no dearer, and the factor stops there
     LowRankInfo fh{};
     const bool low = low_rank_supported(n);
     if (low) {
@@ -469,15 +470,15 @@ double energy_gradient(Plan& p, const double* P, int nspin, double hf, double* g
       DevBuf fd;
       fd.alloc(sizeof fh);
       DFJK_CUDA(cudaMemsetAsync(fd.p, 0, sizeof fh, s));
-      launch_low_rank(P, n, nspin, n, p.ws_lowrank.as<double>(), fd.as<LowRankInfo>(), s);
+      launch_low_rank(P, n, nspin, n / 2, p.ws_lowrank.as<double>(), kLowRankAccept,
+                      fd.as<LowRankInfo>(), s);
       DFJK_CUDA(cudaMemcpyAsync(&fh, fd.p, sizeof fh, cudaMemcpyDeviceToHost, s));
       DFJK_CUDA(cudaStreamSynchronize(s));
     }
     const double one = 1.0, zero = 0.0;
     for (int sp = 0; sp < nspin; ++sp) {
       const double* Ps = P + sp * nn;
-      // (past half the functions the dense form is no dearer)
-      if (low && 2 * fh.rank[sp] <= n && fh.within(sp, kLowRankAccept)) {
+      if (low && fh.within(sp, kLowRankAccept)) {
         const int64_t ncp = fh.rank[sp] + (fh.rank[sp] & 1);
         if (ncp == 0) continue;
         DevBuf Cp, X, Y;

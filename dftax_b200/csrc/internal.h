@@ -215,10 +215,19 @@ constexpr double kLowRankTol = 1e-14;
 // the factor stands for P when no element of P - C C^T exceeds this share of
 // max |P|: the pivots left out plus the rounding of r-term sums
 constexpr double kLowRankAccept = 3e-14;
+// Columns after which a density of n functions goes to the eigensolver: all of them
+// up to 1024 functions (for 480 functions the chain of every column takes 1.9 ms
+// and the eigensolver 4.8, for 960 7.8 and 11), half of them beyond (1920: 44 ms
+// for all, 18 for half, against 29). A density that is refused after the last
+// column, as one with an eigenvalue just below zero under a full spectrum, costs
+// the chain on top: 1% of a Fock build of 180 functions, 8% of 318, 3% of 960.
+inline int64_t low_rank_cap(int64_t n) { return n <= 1024 ? n : n / 2; }
 bool low_rank_supported(int64_t n);   // its workspace fits in shared memory
 // per spin channel of P (nspin x n x n, symmetric): columns Ct[k][i] (k < rank,
-// n x n per channel), the rank (at most max_rank), max |P - C C^T| and max |P|
-// (bits of a double; the caller zeroes them). Enqueued only.
+// n x n per channel), the rank (at most max_rank; -1 when a residual diagonal fell
+// below -accept times the largest one, P then being further than accept from any
+// factor), max |P - C C^T| and max |P| (bits of a double; the caller zeroes them).
+// Enqueued only.
 struct LowRankInfo {
   unsigned long long worst[2], scale[2];
   int rank[2];
@@ -226,7 +235,7 @@ struct LowRankInfo {
   bool within(int sp, double tol) const;
 };
 void launch_low_rank(const double* P, int64_t n, int nspin, int64_t max_rank, double* Ct,
-                     LowRankInfo* info, cudaStream_t s);
+                     double accept, LowRankInfo* info, cudaStream_t s);
 // The columns of a pivoted Cholesky factor (Ct[k][i], n each, rank of them) rotated
 // by an orthogonal matrix that spreads every one over all: out[i * si + j * sj], zero
 // in the columns from rank up to ncp. C C^T stays what it is. For the mixed half

@@ -951,7 +951,8 @@ double energy(Plan& p, const double* P, int nspin, double hf, double hf_lr, doub
   // the density's factor, a chain of small steps on a few SMs, runs beside J
   SideFork side(*p.ctx, low ? 1 : 0, s);
   if (low)
-    launch_low_rank(P, n, nspin, n, p.ws_lowrank.as<double>(), &sc->low, side.stream(0));
+    launch_low_rank(P, n, nspin, low_rank_cap(n), p.ws_lowrank.as<double>(), kLowRankAccept, &sc->low,
+                    side.stream(0));
   const double* Pt = P;
   if (nspin == 2) {
     p.ws_Ptot.ensure(nn * sizeof(double));

@@ -21,7 +21,8 @@ namespace {
 
 constexpr int kCta = 8;         // CTAs per cluster, one cluster per spin channel
 constexpr int kLanes = 8;       // k lanes (warps) per block
-constexpr int kRows = 32;       // rows per pass
+constexpr int kPer = 4;         // rows per lane and pass
+constexpr int kRows = 32 * kPer;
 
 __device__ __forceinline__ void cluster_barrier() {
   asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
@@ -43,13 +44,19 @@ __device__ __forceinline__ Pivot better(Pivot a, Pivot b) {
 // and the k columns so far, C[i][k] = (P[p][i] - sum_q C[i][q] C[p][q]) /
 // sqrt(d_p), and updates the residual diagonal d. Each CTA owns a run of rows
 // (its part of d in shared memory); a warp per k lane sums every eighth q
-// over 32 rows at a time. One cluster barrier per step carries the CTAs' pivot
+// over up to 128 rows at a time. One cluster barrier per step carries the CTAs' pivot
 // candidates (distributed shared memory, two sets of slots) and makes the new
 // column visible. Bound by that barrier and the L2 latency of the pivot row,
-// about 2 us a step; the arithmetic is n r^2 in all.
+// about 2 us a step, and past some hundred columns by the reads of the former
+// ones, n r^2 / 2 values in all on eight SMs.
+// A residual diagonal only falls, so one below -accept times the largest diagonal
+// shows that the factor would be refused: its CTA sends an infinite candidate, and
+// every CTA stops with rank -1 (a difference of densities after the columns of its
+// positive part).
 __global__ void __cluster_dims__(kCta, 1, 1) __launch_bounds__(kLanes * 32)
     pivoted_cholesky_kernel(const double* __restrict__ Pall, int64_t n, int64_t max_rank,
-                            double rel_tol, double* Ctall, LowRankInfo* __restrict__ info) {
+                            double rel_tol, double accept, double* Ctall,
+                            LowRankInfo* __restrict__ info) {
   extern __shared__ double sm[];
   __shared__ double red[kLanes][kRows];
   __shared__ Pivot slot[2][kCta];
@@ -91,6 +98,10 @@ __global__ void __cluster_dims__(kCta, 1, 1) __launch_bounds__(kLanes * 32)
 #pragma unroll
     for (int c = 1; c < kCta; ++c) p = better(p, slot[k & 1][c]);
     if (k == 0) first = p.v;
+    if (p.v == INFINITY) {
+      k = -1;
+      break;
+    }
     // the same decision in every CTA: all read the same eight candidates
     if (k == max_rank || !(p.v > rel_tol * first) || !(p.v > 0.0)) break;
     for (int64_t q = threadIdx.x; q < k; q += kLanes * 32) crow[q] = __ldcg(Ct + q * n + p.i);
@@ -98,29 +109,43 @@ __global__ void __cluster_dims__(kCta, 1, 1) __launch_bounds__(kLanes * 32)
     const double inv = 1.0 / sqrt(p.v);
     best = Pivot{-1.0, 0};
     for (int64_t r0 = lo; r0 < hi; r0 += kRows) {
-      const int64_t i = r0 + lane;
-      double s = 0.0;
-      if (i < hi)
-        for (int64_t q = warp; q < k; q += kLanes) s += Ct[q * n + i] * crow[q];
-      red[warp][lane] = s;
-      __syncthreads();
-      if (warp == 0 && i < hi) {
-        double t = 0.0;
+      double sum[kPer] = {};
+#pragma unroll 4
+      for (int64_t q = warp; q < k; q += kLanes) {
+        const double c = crow[q];
+        const double* col = Ct + q * n + r0 + lane;
 #pragma unroll
-        for (int w = 0; w < kLanes; ++w) t += red[w][lane];
-        double di = d[i - lo], c = 0.0;
-        if (i == p.i) {
-          c = sqrt(p.v);
-          di = -1.0;
-        } else if (di >= 0.0) {
-          // (rounding can leave a residual diagonal just below zero: its row
-          // is finished then, as a pivoted one is)
-          c = (P[p.i * n + i] - t) * inv;
-          di -= c * c;
+        for (int u = 0; u < kPer; ++u)
+          if (r0 + lane + 32 * u < hi) sum[u] += col[32 * u] * c;
+      }
+#pragma unroll
+      for (int u = 0; u < kPer; ++u) red[warp][lane + 32 * u] = sum[u];
+      __syncthreads();
+      if (warp == 0) {
+#pragma unroll
+        for (int u = 0; u < kPer; ++u) {
+          const int64_t i = r0 + lane + 32 * u;
+          if (i >= hi) break;
+          double t = 0.0;
+#pragma unroll
+          for (int w = 0; w < kLanes; ++w) t += red[w][lane + 32 * u];
+          double di = d[i - lo], c = 0.0;
+          bool below = k == 0 && di < -accept * first;
+          if (i == p.i) {
+            c = sqrt(p.v);
+            di = -1.0;
+          } else if (di >= 0.0) {
+            // (rounding can leave a residual diagonal just below zero: its row
+            // is finished then, as a pivoted one is)
+            c = (P[p.i * n + i] - t) * inv;
+            di -= c * c;
+            below = di < -accept * first;
+          }
+          d[i - lo] = di;
+          Ct[k * n + i] = c;
+          if (below) best = Pivot{INFINITY, i};
+          else if (di >= 0.0) best = better(best, Pivot{di, i});
         }
-        d[i - lo] = di;
-        Ct[k * n + i] = c;
-        if (di >= 0.0) best = better(best, Pivot{di, i});
       }
       __syncthreads();
     }
@@ -227,11 +252,11 @@ bool LowRankInfo::within(int sp, double tol) const {
 }
 
 void launch_low_rank(const double* P, int64_t n, int nspin, int64_t max_rank, double* Ct,
-                     LowRankInfo* info, cudaStream_t s) {
+                     double accept, LowRankInfo* info, cudaStream_t s) {
   const size_t smem = chol_smem(n);
   allow_shared(pivoted_cholesky_kernel);
   pivoted_cholesky_kernel<<<kCta * nspin, kLanes * 32, smem, s>>>(P, n, std::min(max_rank, n), kLowRankTol,
-                                                                   Ct, info);
+                                                                   accept, Ct, info);
   DFJK_LAUNCHED();
   const unsigned t = (unsigned)((n + 31) / 32);
   residual_kernel<<<dim3(t, t, (unsigned)nspin), 256, 0, s>>>(P, n, Ct, info);

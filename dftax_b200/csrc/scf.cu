@@ -484,14 +484,16 @@ bool sp2_density(dfscf& f, const double* Fm, cudaStream_t s) {
   // (X^2 = X gives C' (C'^T C' - I) C'^T = 0); one Newton step C' (3 I - C'^T C')
   // / 2 squares what is left. (A Cholesky QR of X applied to the last orbitals,
   // twice, took a dozen launches and a potrf of 37 us each.)
+  // X keeps the rounding of its first steps, eps times the spectrum's width over
+  // the gap (1e-12 for carbon's sets)
+  constexpr double kAccept = 1e-10;
   LowRankInfo low{};
   DFJK_CUDA(cudaMemsetAsync(f.sp_low.p, 0, sizeof low, s));
-  launch_low_rank(Xb[cur], m, 1, k, Z, f.sp_low.as<LowRankInfo>(), s);
+  launch_low_rank(Xb[cur], m, 1, k, Z, kAccept, f.sp_low.as<LowRankInfo>(), s);
   DFJK_CUDA(cudaMemcpyAsync(&low, f.sp_low.p, sizeof low, cudaMemcpyDeviceToHost, s));
   DFJK_CUDA(cudaStreamSynchronize(s));
-  // converged to a projector of rank nocc: X keeps the rounding of its first
-  // steps, eps times the spectrum's width over the gap (1e-12 for carbon's sets)
-  if (rec[2] != 1.0 || !(std::fabs(rec[1] - k) < 1e-6) || low.rank[0] != k || !low.within(0, 1e-10)) {
+  // converged to a projector of rank nocc
+  if (rec[2] != 1.0 || !(std::fabs(rec[1] - k) < 1e-6) || low.rank[0] != k || !low.within(0, kAccept)) {
     tm.add(f.res.ms_diag);
     return false;
   }

@@ -131,3 +131,47 @@ def test_mixed_factor_is_as_precise_as_eigenvectors():
         eig += float(((K - K0).norm() / K0.norm()) ** 2)
     print("factor / eigenvectors:", (factor / eig) ** 0.5)
     assert factor <= 1.1 ** 2 * eig, (factor / eig) ** 0.5
+
+
+@pytest.mark.parametrize("n", [6, 35])
+def test_rank_cap(n):
+    """Ranks at the columns where the factor gives way: the gradient's half of the
+    functions, Fock's half past 1024 functions (35 waters: 1050), full rank, and
+    densities whose residual turns negative at once, after some columns and after
+    nearly all. One s shell on each oxygen as the auxiliary set keeps the
+    contractions small."""
+    import torch
+
+    from dftax_b200 import Plan, build_basis_data, systems
+
+    sym, xyz = systems.water_cluster(n, seed=1)
+    orb, _ = systems.basis_for(sym, xyz)
+    ox = [i for i, s in enumerate(sym) if s == "O"]
+    aux = build_basis_data(["O"] * n, xyz[ox], {"O": [(0, [0.8], [1.0])]})
+    plan = Plan(orb, aux).build()
+    T, V = plan.eri3c_dense(), plan.metric_pinv()
+    m = orb.nao
+    g = torch.Generator().manual_seed(n)
+    q = torch.linalg.qr(torch.randn(m, m, generator=g, dtype=torch.float64).cuda())[0]
+    w = torch.rand(m, generator=g, dtype=torch.float64).cuda() + 0.1
+
+    def form(q, w):
+        P = (q * w) @ q.T
+        return 0.5 * (P + P.T)
+
+    half = m // 2
+    cases = [form(q[:, :r], w[:r]) for r in (half - 1, half, half + 1, m)]
+    cases += [form(q, w - 0.12), form(q[:, :20], torch.sign(w[:20] - 0.6)),
+              form(q[:, :half], torch.where(torch.arange(half, device="cuda") < half - 2, 1.0, -1e-3))]
+    for P in cases:
+        J = T @ (V @ torch.einsum("mnP,mn->P", T, P))
+        X = torch.einsum("mnP,PQ->mnQ", T, torch.linalg.cholesky(V))
+        K = torch.einsum("mlQ,ls,nsQ->mn", X, P, X)
+        F0 = J - 0.125 * K
+        e0 = 0.5 * float((J * P).sum()) - 0.0625 * float((K * P).sum())
+        e, F = plan.energy(P[None], 0.25)
+        assert float((F.reshape(F0.shape) - F0).norm()) < REL * float(J.norm() + K.norm())
+        assert abs(e - e0) < REL * float((J * P).abs().sum() + (K * P).abs().sum())
+        if n == 6:   # both forms of the gradient's K part: the energy goes through it
+            eg, _ = plan.energy_grad(P[None], 0.25, xyz)
+            assert abs(eg - e0) < REL * float((J * P).abs().sum() + (K * P).abs().sum())
