@@ -145,7 +145,7 @@ struct Plan {
   // float64 K = X X^T: per-slice partials
   DevBuf ws_syrk;
   // density path: total density, low-rank columns, scalars read back, block partials of the dots, K
-  DevBuf ws_Ptot, ws_lowrank, ws_scal, ws_dots, ws_K;
+  DevBuf ws_Ptot, ws_lowrank, ws_spread, ws_scal, ws_dots, ws_K;
 };
 
 // ---- mixed precision on the int8 tensor cores (ozaki.cu) ----
@@ -236,15 +236,15 @@ struct LowRankInfo {
 };
 void launch_low_rank(const double* P, int64_t n, int nspin, int64_t max_rank, double* Ct,
                      double accept, LowRankInfo* info, cudaStream_t s);
-// The columns of a pivoted Cholesky factor (Ct[k][i], n each, rank of them) rotated
-// by an orthogonal matrix that spreads every one over all: out[i * si + j * sj], zero
-// in the columns from rank up to ncp. C C^T stays what it is. For the mixed half
-// transform, whose digits of a column are relative to its largest element: that of a
-// Cholesky column is its pivot, up to sqrt(rank) times the rest, so that the digits'
-// error grew with the rank (sum of the squared column maxima, random occupied
-// orbitals: 2.9 times that of eigenvectors at n = 318, 25 columns, 8.2 times at 960,
-// 160; rotated 0.97 and 0.73 times).
-void spread_columns(const double* Ct, int64_t n, int64_t rank, int64_t ncp, int64_t si, int64_t sj,
+// The columns Ct of launch_low_rank (of one channel, their number *rank read on the
+// device) rotated by an orthogonal matrix that spreads every one over all; C C^T
+// stays what it is. rows: out[i][j], rows of rank rounded up to even, the padding
+// zero; else out[j][i]. For the mixed half transform, whose digits of a column are
+// relative to its largest element: that of a Cholesky column is its pivot, up to
+// sqrt(rank) times the rest, so that the digits' error grew with the rank (sum of
+// the squared column maxima, random occupied orbitals: 2.9 times that of eigenvectors
+// at n = 318, 25 columns, 8.2 times at 960, 160; rotated 0.97 and 0.73 times).
+void spread_columns(const double* Ct, int64_t n, int64_t max_rank, const int* rank, bool rows,
                     double* out, cudaStream_t s);
 
 // ---- nuclear gradient of the DF energy (grad.cu) ----

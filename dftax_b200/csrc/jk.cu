@@ -947,12 +947,19 @@ double energy(Plan& p, const double* P, int nspin, double hf, double hf_lr, doub
   nonfinite_kernel<<<(unsigned)((nn * nspin + 255) / 256), 256, 0, s>>>(P, nn * nspin, &sc->nonfinite);
   DFJK_LAUNCHED();
   const bool low = exch && low_rank_supported(n);
+  // mixed products take the factor's columns spread out and laid out as they are read
+  const bool spread = low && p.opts.precision == DFJK_MIXED && !p.opts.streamed;
+  const int64_t cap = low_rank_cap(n), ns = n * (cap + (cap & 1));
   if (low) p.ws_lowrank.ensure((size_t)nn * nspin * sizeof(double));
+  if (spread) p.ws_spread.ensure((size_t)ns * nspin * sizeof(double));
   // the density's factor, a chain of small steps on a few SMs, runs beside J
   SideFork side(*p.ctx, low ? 1 : 0, s);
-  if (low)
-    launch_low_rank(P, n, nspin, low_rank_cap(n), p.ws_lowrank.as<double>(), kLowRankAccept, &sc->low,
-                    side.stream(0));
+  if (low) {
+    launch_low_rank(P, n, nspin, cap, p.ws_lowrank.as<double>(), kLowRankAccept, &sc->low, side.stream(0));
+    for (int sp = 0; spread && sp < nspin; ++sp)
+      spread_columns(p.ws_lowrank.as<double>() + sp * nn, n, cap, &sc->low.rank[sp], true,
+                     p.ws_spread.as<double>() + sp * ns, side.stream(0));
+  }
   const double* Pt = P;
   if (nspin == 2) {
     p.ws_Ptot.ensure(nn * sizeof(double));
@@ -982,18 +989,10 @@ double energy(Plan& p, const double* P, int nspin, double hf, double hf_lr, doub
     const bool factored = low && h.low.within(sp, kLowRankAccept);
     DevBuf Ct, dw;
     if (!factored) density_factor(p, Ps, Ct, dw, s);   // indefinite, or too rough a factor
-    // the factor's columns C[m][k] at Cf[m * sm + k * sk]; mixed products take them
-    // spread out and laid out as they are read
-    const double* Cf = p.ws_lowrank.as<double>() + sp * nn;
-    int64_t sm = 1, sk = n;
+    // the factor's columns: C[m][k] at Cf[m * sm + k * sk]
     const int64_t rank = factored ? h.low.rank[sp] : 0;
-    if (rank > 0 && p.opts.precision == DFJK_MIXED && !p.opts.streamed) {
-      sm = rank + (rank & 1);
-      sk = 1;
-      p.ws_Cp.ensure((size_t)n * sm * sizeof(double));
-      spread_columns(Cf, n, rank, sm, sm, 1, p.ws_Cp.as<double>(), s);
-      Cf = p.ws_Cp.as<double>();
-    }
+    const double* Cf = (spread ? p.ws_spread : p.ws_lowrank).as<double>() + sp * (spread ? ns : nn);
+    const int64_t sm = spread ? rank + (rank & 1) : 1, sk = spread ? 1 : n;
     const struct { Plan* plan; double coeff; } terms[2] = {{&p, hf},
                                                            {p.lr ? &p.lr->p : nullptr, hf_lr}};
     for (int t = 0; t < 2; ++t) {

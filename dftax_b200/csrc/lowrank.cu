@@ -205,17 +205,19 @@ __global__ void __launch_bounds__(256) residual_kernel(const double* __restrict_
   }
 }
 
-// out(i, j) = sum_q Ct[q][i] H[q][j], H[q][j] = (cos + sin)(2 pi q j / r) / sqrt r
-// (Hartley's matrix, orthogonal and symmetric for every r), at out[i * si + j * sj];
-// j in [r, ncp): zero. The r values that H consists of, by q j mod r, in shared
-// memory. A block has 32 rows and eight columns, so that a few dozen orbitals
-// already give some forty blocks; bound by the latency of the loads of Ct.
+// sum_q Ct[q][i] H[q][j], H[q][j] = (cos + sin)(2 pi q j / r) / sqrt r (Hartley's
+// matrix, orthogonal and symmetric for every r), at out[i][j] (rows of r rounded up
+// to even, zero there) or out[j][i]. The r values that H consists of, by q j mod r,
+// in shared memory. A block has 32 rows and eight columns, so that a few dozen
+// orbitals already give some forty blocks (those past r leave at once); bound by
+// the latency of the loads of Ct.
 constexpr int kSpRows = 32, kSpCols = 8;
 __global__ void __launch_bounds__(kSpRows * kSpCols) spread_kernel(const double* __restrict__ Ct,
-                                                                   int64_t n, int r, int64_t ncp,
-                                                                   int64_t si, int64_t sj,
-                                                                   double* __restrict__ out) {
+                                                                   int64_t n, const int* __restrict__ rank,
+                                                                   bool rows, double* __restrict__ out) {
   extern __shared__ double cas[];
+  const int r = *rank, ncp = rows ? r + (r & 1) : r;
+  if ((int)blockIdx.y * kSpCols >= ncp) return;   // (r may be -1)
   for (int t = threadIdx.x; t < r; t += kSpRows * kSpCols) {
     double sn, cs;
     sincospi(2.0 * t / r, &sn, &cs);
@@ -223,7 +225,7 @@ __global__ void __launch_bounds__(kSpRows * kSpCols) spread_kernel(const double*
   }
   __syncthreads();
   const int64_t i = blockIdx.x * (int64_t)kSpRows + threadIdx.x % kSpRows;
-  const int64_t j = blockIdx.y * (int64_t)kSpCols + threadIdx.x / kSpRows;
+  const int j = blockIdx.y * kSpCols + threadIdx.x / kSpRows;
   if (i >= n || j >= ncp) return;
   double acc = 0.0;
   if (j < r) {
@@ -231,11 +233,11 @@ __global__ void __launch_bounds__(kSpRows * kSpCols) spread_kernel(const double*
 #pragma unroll 8
     for (int q = 0; q < r; ++q) {
       acc += Ct[q * n + i] * cas[t];
-      t += (int)j;
+      t += j;
       if (t >= r) t -= r;
     }
   }
-  out[i * si + j * sj] = acc;
+  out[rows ? i * ncp + j : j * n + i] = acc;
 }
 
 size_t chol_smem(int64_t n) { return (size_t)((n + kCta - 1) / kCta + n) * sizeof(double); }
@@ -263,11 +265,12 @@ void launch_low_rank(const double* P, int64_t n, int nspin, int64_t max_rank, do
   DFJK_LAUNCHED();
 }
 
-void spread_columns(const double* Ct, int64_t n, int64_t rank, int64_t ncp, int64_t si, int64_t sj,
+void spread_columns(const double* Ct, int64_t n, int64_t max_rank, const int* rank, bool rows,
                     double* out, cudaStream_t s) {
+  max_rank = std::max<int64_t>(1, std::min(max_rank, n));
   allow_shared(spread_kernel);
-  const dim3 grid((unsigned)((n + kSpRows - 1) / kSpRows), (unsigned)((ncp + kSpCols - 1) / kSpCols));
-  spread_kernel<<<grid, kSpRows * kSpCols, (size_t)rank * sizeof(double), s>>>(Ct, n, (int)rank, ncp, si, sj, out);
+  const dim3 grid((unsigned)((n + kSpRows - 1) / kSpRows), (unsigned)((max_rank + kSpCols) / kSpCols));
+  spread_kernel<<<grid, kSpRows * kSpCols, (size_t)max_rank * sizeof(double), s>>>(Ct, n, rank, rows, out);
   DFJK_LAUNCHED();
 }
 

@@ -490,6 +490,11 @@ bool sp2_density(dfscf& f, const double* Fm, cudaStream_t s) {
   LowRankInfo low{};
   DFJK_CUDA(cudaMemsetAsync(f.sp_low.p, 0, sizeof low, s));
   launch_low_rank(Xb[cur], m, 1, k, Z, kAccept, f.sp_low.as<LowRankInfo>(), s);
+  if (f.p->opts.precision == DFJK_MIXED && !f.p->opts.streamed) {
+    // the orbitals go to the mixed K (Xb[cur] is read no more)
+    spread_columns(Z, m, k, f.sp_low.as<LowRankInfo>()->rank, false, Xb[cur], s);
+    Z = Xb[cur];
+  }
   DFJK_CUDA(cudaMemcpyAsync(&low, f.sp_low.p, sizeof low, cudaMemcpyDeviceToHost, s));
   DFJK_CUDA(cudaStreamSynchronize(s));
   // converged to a projector of rank nocc
@@ -498,11 +503,6 @@ bool sp2_density(dfscf& f, const double* Fm, cudaStream_t s) {
     return false;
   }
   double* Q = Xb[cur ^ 1];
-  if (f.p->opts.precision == DFJK_MIXED && !f.p->opts.streamed) {
-    // the orbitals go to the mixed K (Xb[cur] is read no more)
-    spread_columns(Z, m, k, k, 1, m, Xb[cur], s);
-    Z = Xb[cur];
-  }
   DFJK_CUDA(cudaMemcpyAsync(Q, Z, (size_t)m * k * sizeof(double), cudaMemcpyDeviceToDevice, s));
   gemm(c, CUBLAS_OP_T, CUBLAS_OP_N, k, k, m, 1.0, Z, m, Z, m, 0.0, f.A2.as<double>(), k, s);
   gemm(c, CUBLAS_OP_N, CUBLAS_OP_N, m, k, k, -0.5, Z, m, f.A2.as<double>(), k, 1.5, Q, m, s);
