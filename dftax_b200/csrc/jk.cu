@@ -790,9 +790,13 @@ static void k_compute(Plan& p, const double* C, const double* w, int64_t ncol, d
   k_accumulate(p, C, ncol, 1, w, &neg, (int64_t)neg.size(), -1.0, pos.empty(), K, s, fuse);
 }
 
+static void reset_jk_phases(Plan& p) {
+  for (int ph = kPhJ; ph <= kPhKsyrk; ++ph) p.timer.reset(ph);
+}
+
 void jk_compute(Plan& p, const double* C, const double* w, int64_t ncol, double* J, double* K,
                 cudaStream_t s) {
-  for (int ph = kPhJ; ph <= kPhKsyrk; ++ph) p.timer.reset(ph);
+  reset_jk_phases(p);
   if (J) {
     p.timer.mark(kPhJ, s);
     DevBuf& gamma = p.ws_gamma;
@@ -941,6 +945,8 @@ double energy(Plan& p, const double* P, int nspin, double hf, double hf_lr, doub
               cudaStream_t s) {
   const int64_t n = p.nao, nn = n * n;
   const bool exch = hf != 0.0 || hf_lr != 0.0;
+  reset_jk_phases(p);
+  if (hf_lr != 0.0) reset_jk_phases(p.lr->p);
   p.ws_scal.ensure(sizeof(EnergyScalars));
   EnergyScalars* sc = p.ws_scal.as<EnergyScalars>();
   DFJK_CUDA(cudaMemsetAsync(sc, 0, sizeof(EnergyScalars), s));

@@ -199,7 +199,8 @@ dfjk_status dfjk_j_noalloc(dfjk_plan* plan, const double* C, const double* w, in
 /* ---- tracing ------------------------------------------------------------ */
 
 /* Phases timed with CUDA events on the stream of the last dfjk_build / dfjk_jk
- * (dfjk_energy's J and K count as dfjk_jk). */
+ * (dfjk_energy counts as dfjk_jk; of its parts only those of K are timed, J
+ * reads 0). */
 enum {
   DFJK_PHASE_METRIC = 0, /* (P|Q), eigensolver, factor L                      */
   DFJK_PHASE_PAIRS = 1,  /* primitive-pair setup (E tables in spherical form) */

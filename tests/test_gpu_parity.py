@@ -335,3 +335,32 @@ def test_oversized_plan_reports_memory(water_golden):
     small = Plan(golden_basis(g, "orb"), golden_basis(g, "aux")).build()
     J, K = small.jk(g["C"])
     assert rel(K.cpu().numpy(), g["K"]) < NOISE_REL
+
+
+def test_phase_times_are_of_the_last_energy():
+    """dfjk_energy counts as the last J-K call: the phases of its K are measured and
+    do not add up over repeated calls (20 calls of the same density, so at most a few
+    times one call's time), for the plan and its long-range partner; J reads zero."""
+    import torch
+
+    from dftax_b200 import Plan, systems
+
+    _, _, orb, aux, nocc = systems.workload("water2", seed=0)
+    C = torch.as_tensor(systems.random_occupied(orb.nao, nocc, seed=0), device="cuda")
+    P = (2.0 * C @ C.T)[None]
+    plan = Plan(orb, aux, omega=0.3).build()
+
+    def one():
+        plan.energy(P, 0.25, hf_coeff_lr=0.4)
+        return [p.phase_times() for p in (plan, plan.long_range)]
+
+    one()
+    runs = [one() for _ in range(20)]
+    assert plan.phase_times()["j"] == 0.0
+    for k in (0, 1):
+        for ph in ("khalf", "ksyrk"):
+            first = [r[k][ph] for r in runs[:3]]
+            assert min(first) > 0.0, ph
+            assert runs[-1][k][ph] < 3.0 * max(first), (ph, first, runs[-1][k][ph])
+    plan.energy(P, 0.0, want_grad=False)
+    assert plan.phase_times()["khalf"] == 0.0
