@@ -38,8 +38,10 @@ struct XcChunkInfo {
 };
 
 // A run of chunks whose kernels share their launches: the chunks' AO values,
-// gradients and weighted AOs take at most kXcGroupBytes (or one chunk).
+// gradients and weighted AOs take at most kXcGroupBytes (or one chunk). Chunks
+// have a function and 256 points at least, so a group's count stays below 2^16.
 constexpr int64_t kXcGroupBytes = (int64_t)256 << 20;
+static_assert(kXcGroupBytes / (40 * 256) < 65536, "chunks of a group: a grid dimension");
 struct XcGroup {
   int first = 0, count = 0;            // chunks
   int max_nsig = 0;

@@ -790,7 +790,9 @@ void xc_chunk(const Shells& sh, const int (&nout)[8], int64_t n, const std::vect
       ch.shells.push_back(s);
       ch.nsig += nout[sh.l[s]];
     }
-    chunks.push_back(std::move(ch));
+    // (without functions a chunk adds nothing: it stays out of the launches, which
+    // take a group's chunks in a grid dimension of at most 65535)
+    if (ch.nsig > 0) chunks.push_back(std::move(ch));
   }
   // the chunks with the most functions first: a group's chunks are then alike,
   // and a launch ends on its shortest blocks ((H2O)_6: 1052 -> 1040 us, (H2O)_8:

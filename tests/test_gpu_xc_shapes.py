@@ -69,3 +69,51 @@ def test_scattered_points(npts, far):
         e.append(e1)
         ks.close()
     assert e[0] == e[1]
+
+
+def test_many_chunks_without_functions():
+    """More chunks that no function reaches than a launch dimension holds (65535):
+    16.8 million far points beside 4096 near ones, 256 points a chunk. They add
+    nothing: the result is that of the near points alone."""
+    import torch
+
+    from dftax_b200 import df, systems
+    from dftax_b200.ks import KS
+
+    sym, xyz, orb, aux, nocc = systems.workload("water", seed=1)
+    rng = np.random.default_rng(0)
+    near = xyz[rng.integers(0, len(xyz), 4096)] + rng.standard_normal((4096, 3))
+    w = rng.uniform(0.01, 0.1, 4096)
+    far = 65540 * 256
+    pts = np.full((far + 4096, 3), 300.0)
+    pts[far // 2:far // 2 + 4096] = near
+    ws = np.full(far + 4096, 0.5)
+    ws[far // 2:far // 2 + 4096] = w
+    C = systems.random_occupied(orb.nao, nocc, seed=3)
+    P = torch.as_tensor(2.0 * C @ C.T, device="cuda")
+    out = []
+    for grid in ((near, w), (pts, ws)):
+        ks = KS(sym, xyz, orb, coulomb=df(aux), grid=grid, grid_chunk=256)
+        for _ in range(3):   # direct, captured, replayed
+            e, V = ks.xc_energy(P)
+        out.append((e, V))
+        ks.close()
+    (e0, V0), (e1, V1) = out
+    assert abs(e1 - e0) <= REL * abs(e0)
+    assert float((V1 - V0).norm()) <= REL * float(V0.norm())
+
+
+def test_no_chunk_has_functions():
+    """A grid that no function reaches: zero energy and matrix."""
+    import torch
+
+    from dftax_b200 import df, systems
+    from dftax_b200.ks import KS
+
+    sym, xyz, orb, aux, nocc = systems.workload("water", seed=1)
+    ks = KS(sym, xyz, orb, coulomb=df(aux), grid=(np.full((700, 3), 300.0), np.ones(700)),
+            grid_chunk=256)
+    C = systems.random_occupied(orb.nao, nocc, seed=3)
+    for _ in range(3):
+        e, V = ks.xc_energy(torch.as_tensor(2.0 * C @ C.T, device="cuda"))
+        assert e == 0.0 and not V.any()
