@@ -114,7 +114,7 @@ int64_t estimate(const dfbatch_request* r) {
   b += x + x * 5 / 8 + (2 * (ldb * nocc / 8192) + 66) * nao * nao * 8;
   const int64_t diis = r->scf_opts.diis_space > 0 ? r->scf_opts.diis_space : 8;
   b += (23 + 2 * diis) * nao * nao * 8;                          // SCF matrices (purification, density factor too), DIIS
-  const int64_t G = r->scf_opts.grid_chunk > 0 ? r->scf_opts.grid_chunk : 16384;
+  const int64_t G = r->scf_opts.grid_chunk > 0 ? std::min(r->scf_opts.grid_chunk, dfjk::kXcMaxChunk) : 16384;
   // XC chunk buffers and a V accumulator on each of the solve's XC streams
   // (one unless the request asks for more: xc.cu), the grid and its sort
   const int64_t nbr = r->scf_opts.xc_streams > 0 ? r->scf_opts.xc_streams : 1;

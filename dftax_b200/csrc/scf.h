@@ -42,6 +42,8 @@ struct XcChunkInfo {
 // have a function and 256 points at least, so a group's count stays below 2^16.
 constexpr int64_t kXcGroupBytes = (int64_t)256 << 20;
 static_assert(kXcGroupBytes / (40 * 256) < 65536, "chunks of a group: a grid dimension");
+// Points of a chunk, at most: its 512-point slices are a grid dimension too.
+constexpr int64_t kXcMaxChunk = (int64_t)1 << 24;
 struct XcGroup {
   int first = 0, count = 0;            // chunks
   int max_nsig = 0;

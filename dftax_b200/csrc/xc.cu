@@ -698,6 +698,7 @@ void launch_becke_partition(const double* pts, const int* owner, const double* r
 }
 
 // slices of a chunk's V product
+static_assert(kXcMaxChunk / kVSlice < 65536, "slices: a grid dimension");
 static int64_t xc_slices(int64_t G) { return (G + kVSlice - 1) / kVSlice; }
 
 // V accumulators per branch: enough that their nao^2 threads each come to about

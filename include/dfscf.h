@@ -41,7 +41,8 @@ typedef struct {
                            every shell, the dense quadrature)                          */
   int32_t max_iter;     /* 128                                                          */
   int32_t diis_space;   /* DIIS history depth (8)                                        */
-  int64_t grid_chunk;   /* grid points per XC chunk, spatially sorted (0: chosen by
+  int64_t grid_chunk;   /* grid points per XC chunk, spatially sorted, rounded up to
+                           256 and cut at 2^24 (0: chosen by
                            timing 512 to 16384 on the first molecule of each
                            size and XC stream count; the choice is kept for the
                            process)                                                    */

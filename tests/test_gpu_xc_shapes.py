@@ -117,3 +117,27 @@ def test_no_chunk_has_functions():
     for _ in range(3):
         e, V = ks.xc_energy(torch.as_tensor(2.0 * C @ C.T, device="cuda"))
         assert e == 0.0 and not V.any()
+
+
+def test_chunk_larger_than_a_launch():
+    """A chunk size whose 512-point slices exceed a launch dimension is cut: H2 with
+    an s shell on each atom, as with ordinary chunks."""
+    import torch
+
+    from dftax_b200 import build_basis_data, df
+    from dftax_b200.ks import KS
+
+    xyz = np.array([[0.0, 0.0, 0.0], [0.0, 0.0, 1.4]])
+    orb = build_basis_data(["H", "H"], xyz, {"H": [(0, [0.8], [1.0])]})
+    aux = build_basis_data(["H", "H"], xyz, {"H": [(0, [1.1], [1.0])]})
+    rng = np.random.default_rng(4)
+    grid = (xyz[rng.integers(0, 2, 3000)] + rng.standard_normal((3000, 3)), rng.uniform(0.01, 0.1, 3000))
+    P = torch.tensor([[0.6, 0.5], [0.5, 0.6]], dtype=torch.float64, device="cuda")
+    out = []
+    for chunk in (256, 1 << 26):
+        ks = KS(["H", "H"], xyz, orb, coulomb=df(aux), grid=grid, grid_chunk=chunk)
+        out.append(ks.xc_energy(P))
+        ks.close()
+    (e0, V0), (e1, V1) = out
+    assert abs(e1 - e0) <= REL * abs(e0)
+    assert float((V1 - V0).norm()) <= REL * float(V0.norm())
