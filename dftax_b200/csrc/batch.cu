@@ -114,12 +114,17 @@ int64_t estimate(const dfbatch_request* r) {
   b += x + x * 5 / 8 + (2 * (ldb * nocc / 8192) + 66) * nao * nao * 8;
   const int64_t diis = r->scf_opts.diis_space > 0 ? r->scf_opts.diis_space : 8;
   b += (23 + 2 * diis) * nao * nao * 8;                          // SCF matrices (purification, density factor too), DIIS
-  const int64_t G = r->scf_opts.grid_chunk > 0 ? std::min(r->scf_opts.grid_chunk, dfjk::kXcMaxChunk) : 16384;
-  // XC chunk buffers and a V accumulator on each of the solve's XC streams
-  // (one unless the request asks for more: xc.cu), the grid and its sort
+  // XC buffers of each of the solve's XC streams (one unless the request asks for
+  // more: xc.cu), the largest over the chunk sizes that are tried; the grid and its
+  // sort; the chunks' maps between their functions and all
   const int64_t nbr = r->scf_opts.xc_streams > 0 ? r->scf_opts.xc_streams : 1;
-  const int64_t grp = std::max<int64_t>(dfjk::kXcGroupBytes, 5 * nao * G * 8);
-  b += nbr * (grp + (G / 512 + 3) * nao * nao * 8) + r->npoint * 11 * 8;
+  int64_t branch = 0, maps = 0;
+  for (int64_t G : r->scf_opts.grid_chunk > 0 ? std::vector<int64_t>{dfjk::xc_points(r->scf_opts.grid_chunk)}
+                                              : std::vector<int64_t>{512, 1024, 2048, 4096, 8192, 16384}) {
+    branch = std::max(branch, dfjk::xc_branch_bytes(nao, G, r->npoint));
+    maps = std::max(maps, (r->npoint / G + 1) * nao * 8);
+  }
+  if (r->npoint > 0) b += nbr * branch + maps + r->npoint * 11 * 8;
   return b + b / 10 + ((int64_t)256 << 20);
 }
 

@@ -799,7 +799,7 @@ dfjk_status dfscf_create(dfjk_plan* pl, int32_t natom, const double* atom_xyz,
     if (npoint > 0) {
       // spatially sorted chunks with their non-negligible shells
       sort_points(grid_xyz, grid_w, npoint, f->pts, f->wts, boxes, s);
-      const int64_t G = f->o.grid_chunk > 0 ? std::min(kXcMaxChunk, (f->o.grid_chunk + 255) / 256 * 256) : 8192;
+      const int64_t G = f->o.grid_chunk > 0 ? xc_points(f->o.grid_chunk) : 8192;
       if (!tunes(*f)) xc_chunk(p.orb, nout, npoint, boxes, G, f->o.ao_thresh, f->xcw);
     }
     double enn = 0.0;

@@ -44,6 +44,9 @@ constexpr int64_t kXcGroupBytes = (int64_t)256 << 20;
 static_assert(kXcGroupBytes / (40 * 256) < 65536, "chunks of a group: a grid dimension");
 // Points of a chunk, at most: its 512-point slices are a grid dimension too.
 constexpr int64_t kXcMaxChunk = (int64_t)1 << 24;
+inline int64_t xc_points(int64_t grid_chunk) {   // of a chunk for a requested size
+  return grid_chunk < kXcMaxChunk ? (grid_chunk + 255) / 256 * 256 : kXcMaxChunk;
+}
 struct XcGroup {
   int first = 0, count = 0;            // chunks
   int max_nsig = 0;
@@ -73,6 +76,10 @@ struct XcBranch {
   DevBuf Pc, Vc;                // P on each chunk's AOs, the slices of its V block
   DevBuf vals;                  // per chunk [4][G]: rho, grad rho, then v_rho / 2, v_grad
 };
+
+// Upper bound of a branch's buffers (its V accumulators too) for chunks of G of
+// npoint points and nao functions
+int64_t xc_branch_bytes(int64_t nao, int64_t G, int64_t npoint);
 
 // branches of an evaluation unless the caller asks for another number. (H2O)_6 by
 // group size and branches, 1024-point chunks: 48 MB x 2 (both groups in L2)
