@@ -200,7 +200,9 @@ dfjk_status dfjk_j_noalloc(dfjk_plan* plan, const double* C, const double* w, in
 
 /* Phases timed with CUDA events on the stream of the last dfjk_build / dfjk_jk
  * (dfjk_energy counts as dfjk_jk; of its parts only those of K are timed, J
- * reads 0). */
+ * reads 0). The phases of a build may overlap: where its rows fit in one chunk and
+ * the metric is computed anew, pairs and 3-center rows run beside the metric, and
+ * their sum exceeds the build's time. */
 enum {
   DFJK_PHASE_METRIC = 0, /* (P|Q), eigensolver, factor L                      */
   DFJK_PHASE_PAIRS = 1,  /* primitive-pair setup (E tables in spherical form) */
