@@ -418,6 +418,7 @@ void launch_grad3c_pairs(Plan& p, const ClassRange& cr, int64_t b, int64_t e, do
     a.row_base = row_base;
     a.ld = p.naux;
     a.G = G;
+    a.sms = num_sms(c.device);
     a.omega = p.atten;
     a.grad_orb = grad_orb;
     a.grad_aux = grad_aux;

@@ -121,6 +121,7 @@ struct Grad3cArgs {
   int64_t row_base;          // global row of G[0]
   int64_t ld;
   const double* G;
+  int sms;                   // of the device (the launch reads it)
   double omega;
   double* grad_orb;          // [orbital shell][3]
   double* grad_aux;          // [aux shell][3]
@@ -323,7 +324,7 @@ inline void launch_grad3c_one(unsigned npair, cudaStream_t s, const Grad3cArgs& 
     cudaFuncSetAttribute(grad3c_kernel<LA, LB, LC>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                          (int)S::smem);
   const unsigned full = (unsigned)((a.aux_count + S::GPB - 1) / S::GPB);
-  const unsigned gy = (uint64_t)npair * full > 8 * 148 ? (full + 3) / 4 : full;
+  const unsigned gy = (uint64_t)npair * full > 8 * (uint64_t)a.sms ? (full + 3) / 4 : full;
   grad3c_kernel<LA, LB, LC><<<dim3(npair, gy), 128, S::smem, s>>>(a);
 }
 

@@ -196,6 +196,7 @@ void launch_schwarz(const Context& c, Shells& sh, const std::vector<int>& pa,
                     const std::vector<int>& pb, std::vector<double>& qmax);
 
 // ---- contractions (jk.cu) ----
+int num_sms(int dev);
 void jk_compute(Plan& p, const double* C, const double* w, int64_t ncol, double* J, double* K,
                 cudaStream_t s);
 // Float64 half transform X[m][x - x0][i] = sum_n B_x[m][n] C'[n][i] of a resident

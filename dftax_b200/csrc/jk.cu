@@ -10,8 +10,8 @@
 //      K = X X^T over the (x, i) index, C' = C sqrt|w|
 // Float64 plans run both K products on the float64 tensor cores (mma.sync
 // m8n8k4 f64: the gathered half transform, then a split-k X X^T); mixed plans
-// run them on the int8 tensor cores (ozaki.cu). J is float64 in both.
-// which are the P-gradients of dftax's DFCoulomb.energy (terms.py:592-613):
+// run them on the int8 tensor cores (ozaki.cu). J is float64 in both. J and K
+// are the P-gradients of dftax's DFCoulomb.energy (terms.py:592-613):
 // J = int3c (V+ gamma), K = einsum("mlP,PQ,nsQ,ls->mn") (hybrid.py:23-41).
 #include "dmma.cuh"
 #include "internal.h"
@@ -192,7 +192,7 @@ __global__ void __launch_bounds__(256) j_rows_kernel(
   }
 }
 
-static int num_sms(int dev) {
+int num_sms(int dev) {
   int n = 0;
   cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev);
   return n > 0 ? n : 148;
@@ -673,17 +673,17 @@ static void syrk_fp64(Plan& p, const double* X, int64_t kt, double sign, bool be
   DFJK_LAUNCHED();
 }
 
-// K (+)= sign * X X^T for the selected columns of C (scaled by sqrt|w|)
-// fuse (streamed plans only, may be null): gamma = B^T d is also summed in the
-// first pass over B's chunks (one rebuild of B fewer per J/K call).
+// Streamed plans: gamma = B^T d summed in the K half transform's first pass over
+// B's chunks (one rebuild of B fewer per J/K call).
 struct GammaFuse {
   DensitySource src;
   double* gamma = nullptr;
   bool done = false;
 };
 
-// nsel columns of C: those of `sel` (host indices), or the first nsel when
-// null; C[m][j] lies at C[m * sm + j * sc]
+// K (+)= sign * X X^T for nsel columns of C (scaled by sqrt|w|): those of `sel`
+// (host indices), or the first nsel when null; C[m][j] lies at C[m * sm + j * sc].
+// fuse (streamed plans only) may be null
 static void k_accumulate(Plan& p, const double* C, int64_t sm, int64_t sc, const double* w,
                          const std::vector<int>* sel, int64_t nsel, double sign, bool first,
                          double* K, cudaStream_t s, GammaFuse* fuse = nullptr) {
@@ -891,8 +891,6 @@ static void dot_axpy(Plan& p, const double* a, const double* b, double c, int64_
   DFJK_LAUNCHED();
 }
 
-// K of a symmetric density Q (device, nao x nao): Q = V diag(l) V^T on the
-// device, K(Q) = sum_k l_k K(v_k v_k^T) over |l_k| > 1e-14 max|l|.
 // Eigen-factor of a symmetric Q (nao x nao): Ct row-major with Q = Ct diag(dw) Ct^T,
 // eigenvalues below 1e-14 of the largest set to zero, so K(Q) = k_compute(Ct, dw).
 static void density_factor(Plan& p, const double* Q, DevBuf& Ct, DevBuf& dw, cudaStream_t s) {
@@ -933,14 +931,13 @@ static void density_factor(Plan& p, const double* Q, DevBuf& Ct, DevBuf& dw, cud
   upload(dw, wsel);
 }
 
-// hf_lr: the long-range exchange of range-separated hybrids through the plan's
-// long-range fit (terms.py:604-612)
 void gamma_from_density(Plan& p, const double* Ptot, double* gamma, cudaStream_t s) {
   gamma_of(p, DensitySource{nullptr, nullptr, 0, Ptot}, gamma, s);
 }
 
-// Two host synchronizations: the ranks (with the density check), and the
-// scalars at the end.
+// hf_lr: the long-range exchange of range-separated hybrids through the plan's
+// long-range fit (terms.py:604-612). Two host synchronizations: the ranks (with
+// the density check), and the scalars at the end.
 double energy(Plan& p, const double* P, int nspin, double hf, double hf_lr, double* F,
               cudaStream_t s) {
   const int64_t n = p.nao, nn = n * n;

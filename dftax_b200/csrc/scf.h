@@ -25,7 +25,7 @@ void launch_one_electron(const Context& c, const OrbView& ov, int nshell, const 
                          double* T, double* V, cudaStream_t s);
 
 // Chunks of spatially sorted grid points, each with the orbital shells that
-// are not negligible anywhere in its bounding box (xc_prepare)
+// are not negligible anywhere in its bounding box (xc_chunk)
 constexpr int kXcMaxL = 3;   // orbital l the AO kernel evaluates (f)
 
 // What the kernels read about a chunk; the offsets (in doubles) lie within the
@@ -81,10 +81,12 @@ struct XcBranch {
 // npoint points and nao functions
 int64_t xc_branch_bytes(int64_t nao, int64_t G, int64_t npoint);
 
-// branches of an evaluation unless the caller asks for another number. (H2O)_6 by
-// group size and branches, 1024-point chunks: 48 MB x 2 (both groups in L2)
-// 1900 us, 96 x 4 1250, 256 x 2 1205, 256 x 4 1108, 1024 x 1 1374: launches that
-// fill the device count for more than L2 residency.
+// branches of an evaluation unless the caller asks for another number. us by group
+// size and branches, 512-point chunks, (H2O)_6 / (H2O)_16 / C8H18: 96 MB x 4 860 /
+// 4940 / 5070, 256 x 1 986 / 6130 / 6330, 256 x 2 893 / 5070 / 5130, 256 x 4 821 /
+// 4820 / 4800, 256 x 8 836 / 4770 / 4810, 1024 x 4 879 / 4840 / 4850 (2048-point
+// chunks order alike): launches that fill the device count for more than groups
+// that stay in L2, and past four branches or 256 MB there is nothing left to fill.
 constexpr int kXcDefaultBranches = 4;
 
 struct XcWork {
@@ -139,7 +141,7 @@ struct XcParams {
 
 // E_xc of the closed-shell density P (nao x nao, symmetric, device) and, when
 // Vxc != nullptr, its P-gradient symmetrized (device, nao x nao), over the grid
-// points pts [n][3] with weights w [n] (device, in xc_prepare's order), chunk
+// points pts [n][3] with weights w [n] (device, in sort_points' order), chunk
 // by chunk as ws.ch lays them out, on the context's branch streams forked from
 // and joined to s. Returns E_xc (host synchronizing); Vcopy, when given,
 // receives a copy of Vxc before that.
