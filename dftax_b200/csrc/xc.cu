@@ -710,8 +710,10 @@ static int64_t v_parts(int64_t nao) {
 // A chunk of nsig functions takes 40 nsig G bytes of its group's, and beside them
 // 8 nsig (nsig + 1) for its P block and 8 nsig^2 per slice of V: most, as a share of
 // the group, with all nao functions. Four values a point, a function a point at least.
+// A small grid does not fill a group.
 int64_t xc_branch_bytes(int64_t nao, int64_t G, int64_t npoint) {
-  const int64_t group = std::max(kXcGroupBytes, 40 * nao * G);
+  const int64_t all = 40 * nao * ((npoint + G - 1) / G * G);
+  const int64_t group = std::max(std::min(kXcGroupBytes, all), 40 * nao * G);
   const double share = (double)(nao + 1 + xc_slices(G) * nao) / (5.0 * (double)G);
   return group + (int64_t)(share * (double)group) + 32 * std::min(npoint + G, group / 40) +
          v_parts(nao) * nao * nao * 8;

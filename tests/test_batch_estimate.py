@@ -36,3 +36,11 @@ def test_a_stream_covers_its_group(name, chunk):
             blocks = 8 * count * (nsig * (nsig + 1) + -(-G // 512) * nsig * nsig)
             need = count * (40 * nsig + 32) * G + blocks + 8 * nao * nao
             assert per_stream >= need, (G, nsig)
+
+
+def test_a_small_grid_fills_no_group():
+    """One water with 28000 points holds 34 MB of AO planes: its request fits a budget
+    of 400 MB, 256 of which the estimate always keeps."""
+    from dftax_b200 import systems
+
+    assert _estimate(systems.workload("water", seed=0), 1, 0, 28000) < 400 << 20
